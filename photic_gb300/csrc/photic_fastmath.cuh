@@ -162,6 +162,28 @@ PHOTIC_FM_HD double div_by(double a, double b, double inv) {
   return fma(r, inv, q);
 }
 
+// a / b for a small divisor or pi, fixed in advance, in two FP64 operations:
+// the reciprocal held as hi = RN(1/b) and lo = RN(1/b - hi), the quotient
+// RN(a hi + RN(a lo)) (the product by an unevaluated constant of
+// N. Brisebarre and J.-M. Muller, "Correctly rounded multiplication by
+// arbitrary precision constants", IEEE Trans. Comput. 57(2), 2008).  The sum
+// before the last rounding is within 2^-54 ulp of the quotient, and a
+// quotient by b = 2^k c, c odd and below 2^50, stays 1/(2c) ulp from the
+// middle of two doubles: the result is the IEEE quotient (pi's significand
+// ends in three zeros, c = 2^49.7).  Subnormal and special operands are
+// divided.
+PHOTIC_FM_HD double div_const(double a, double b, double hi, double lo) {
+  const int64_t e = (bits(a) >> 52) & 0x7ff;
+  if (e < 256 || e > 1790) return a / b;
+  return fma(a, hi, a * lo);
+}
+constexpr double kPiHi = 0x1.45f306dc9c883p-2, kPiLo = -0x1.0c3b15964a2c2p-57;
+constexpr double k120Hi = 0x1.1111111111111p-7, k120Lo = 0x1.1111111111111p-63;
+constexpr double k6Hi = 0x1.5555555555555p-3, k6Lo = 0x1.5555555555555p-57;
+PHOTIC_FM_HD double div_pi(double a) { return div_const(a, 3.141592653589793, kPiHi, kPiLo); }
+PHOTIC_FM_HD double div_120(double a) { return div_const(a, 120.0, k120Hi, k120Lo); }
+PHOTIC_FM_HD double div_6(double a) { return div_const(a, 6.0, k6Hi, k6Lo); }
+
 // q / q: 1 for finite non-zero q, NaN for zero, infinite or NaN q.
 PHOTIC_FM_HD double self_ratio(double q) {
   const int64_t a = bits(q) & 0x7fffffffffffffffLL;

@@ -19,10 +19,24 @@
 
 #include "photic_fastmath.cuh"
 #include "photic_params.h"
+#include "photic_softfp.cuh"
+
+#if defined(__CUDACC__)
+#define PHOTIC_NOINLINE __noinline__
+#else
+#define PHOTIC_NOINLINE inline
+#endif
 
 namespace photic {
 
 constexpr double kPi = 3.141592653589793;  // model/common.h:19
+
+// Library functions that run once a pixel or a start, out of line: the
+// kernels' loops stay within the instruction cache (32 KB streams at full
+// rate, beyond it a warp instruction was measured at two to eight times the
+// clocks).
+static __device__ PHOTIC_NOINLINE double pow_call(double a, double b) { return pow(a, b); }
+static __device__ PHOTIC_NOINLINE double div_call(double a, double b) { return sf::div(a, b); }
 
 // Measured-spectrum constants of one pixel and scene that do not change
 // during the fit: the Y exponent depends only on the measured
@@ -73,27 +87,127 @@ __device__ __forceinline__ void pixel_setup_f64(const FitParams &fp, const Scene
   double Y = 3.44 * (1.0 - 3.17 * fm::exp_t(-2.01 * chi));
   if (Y < 0.0) Y = 0.0;
   if (Y > 2.5) Y = 2.5;
-#pragma unroll
-  for (int b = 0; b < NB; b++)
-    if (b < nb) px.pw[b] = pow(sc.ratio440[b], Y);
+#pragma unroll 1
+  for (int b = 0; b < nb; b++) px.pw[b] = pow_call(sc.ratio440[b], Y);
   px.mean = tot / (double)nb;
+}
+
+// Whether a K takes part in the minimum: the reference compares it, cast to
+// float, with zero (model/samodel.c:2698), and a double rounds to float zero
+// up to 2^-150.
+__device__ __forceinline__ bool k_counts(double K) {
+  return (fm::bits(K) & 0x7fffffffffffffffLL) > 0x3690000000000000LL;
 }
 
 // Depth-dependent K penalty and very-high-K penalty
 // (model/samodel.c:2696-2732) for one scene whose min K is K_min.
 __device__ __forceinline__ double k_penalty_f64(const KPenalty &kp, double H, double K_min) {
   double e = 0.0;
-  int c = -1;
-  if (H < 1.0 && K_min < kp.k_thr[0]) c = 0;
-  else if (H < 2.0 && K_min < kp.k_thr[1]) c = 1;
-  else if (H < 3.0 && K_min < kp.k_thr[2]) c = 2;
-  else if (H < 4.0 && K_min < kp.k_thr[3]) c = 3;
-  else if (H < 5.0 && K_min < kp.k_thr[4]) c = 4;
-  if (c >= 0) {
-    double d = 1.0 / (0.01 + K_min) - kp.inv_t[c];
-    e = e + 100.0 * (d * d);
+  if (sf::lt(H, 5.0)) {  // every band of depth below needs it
+    int c = -1;
+    if (sf::lt(H, 1.0) && sf::lt(K_min, kp.k_thr[0])) c = 0;
+    else if (sf::lt(H, 2.0) && sf::lt(K_min, kp.k_thr[1])) c = 1;
+    else if (sf::lt(H, 3.0) && sf::lt(K_min, kp.k_thr[2])) c = 2;
+    else if (sf::lt(H, 4.0) && sf::lt(K_min, kp.k_thr[3])) c = 3;
+    else if (sf::lt(K_min, kp.k_thr[4])) c = 4;
+    if (c >= 0) {
+      double d = sf::div(1.0, 0.01 + K_min) - kp.inv_t[c];
+      e = e + 100.0 * (d * d);
+    }
   }
   return e;
+}
+
+// One band term of the cost: samodel_Rrs (model/samodel.c:2846-2949) for one
+// band, region and scene, and its squared residual (:2571).
+struct BandTerm {
+  double K;      // diffuse attenuation, clamped to [0, 2.5]
+  double rrs_B;  // bottom part of the subsurface reflectance
+  double rrs;    // subsurface reflectance
+  double Rm;     // modelled Rrs
+  double dd;     // (Rm - measured)^2
+};
+
+// With every operation compiled (any operands).
+static __device__ PHOTIC_NOINLINE void band_term_general(const SceneConsts &sc, int b, double sec_sun,
+                                                      double H, double rho, double P, double lnP,
+                                                      double G, double X, double pw, double r,
+                                                      BandTerm *t) {
+  const double a_phi = (sc.a0[b] + sc.a1[b] * lnP) * P;
+  const double a_g = G * sc.eS[b];
+  const double a = sc.aw[b] + a_phi + a_g;
+  const double bb = sc.bbw[b] + X * pw;
+  const double u = bb / (a + bb);
+  double K = a + bb;
+  if (K < 0.0) K = 0.0;
+  if (K > 2.5) K = 2.5;
+  const double rrs_dp = (0.084 + 0.170 * u) * u;
+  const double DuC = 1.03 * sqrt(1.0 + 2.4 * u);
+  const double DuB = 1.04 * sqrt(1.0 + 5.4 * u);
+  double M = sec_sun + DuC * sc.sec_view;
+  const double rrs_C = rrs_dp * (1.0 - fm::exp_t(-M * K * H));
+  M = sec_sun + DuB * sc.sec_view;
+  const double rrs_B = fm::div_by(rho, kPi, fm::kInvPi) * fm::exp_t(-M * K * H);
+  const double rrs = rrs_C + rrs_B;
+  const double Rm = 0.5 * rrs / (1.0 - 1.5 * rrs);
+  const double d = Rm - r;
+  t->K = K;
+  t->rrs_B = rrs_B;
+  t->rrs = rrs;
+  t->Rm = Rm;
+  t->dd = d * d;
+}
+
+// The same bits with the divisions, square roots, products and comparisons on
+// the integer and FP32 pipes (photic_softfp.cuh), the additions and the
+// exponentials' polynomials on the FP64 pipe, so that the pipes share the
+// work.  A product by the unit secant of a nadir view is skipped (exact).
+// The soft operations need normal operands: `near_x` says that H, rho, P, G,
+// X, pw and ln P are, the band's constants' bit in sc.near_mask that those
+// are, and the tests below cover the intermediates; a term that fails one
+// (an exact zero, an absurd exponent, NaN) is evaluated again above.
+__device__ __forceinline__ void band_term(const SceneConsts &sc, int b, double sec_sun, bool near_x,
+                                          double H, double rho, double P, double lnP, double G,
+                                          double X, double pw, double r, BandTerm &t) {
+  const double c = sc.a0[b] + sf::mul_mid(sc.a1[b], lnP);
+  const double a_phi = sf::mul_mid(c, P);
+  const double a_g = sf::mul_mid(G, sc.eS[b]);
+  const double a = sc.aw[b] + a_phi + a_g;
+  const double bb = sc.bbw[b] + sf::mul_mid(X, pw);
+  const double ab = a + bb;
+  const double u = sf::div_mid(bb, ab);
+  const double K = fm::bits(ab) > 0x4004000000000000LL ? 2.5 : ab;  // > 2.5 (positive here)
+  const double rrs_dp = sf::mul_mid(0.084 + sf::mul_mid(0.170, u), u);
+  double DuC = sf::mul_mid(1.03, sf::sqrt_mid(1.0 + sf::mul_mid(2.4, u)));
+  double DuB = sf::mul_mid(1.04, sf::sqrt_mid(1.0 + sf::mul_mid(5.4, u)));
+  if (sc.sec_view != 1.0) {
+    DuC = sf::mul_mid(DuC, sc.sec_view);
+    DuB = sf::mul_mid(DuB, sc.sec_view);
+  }
+  const double MC = sec_sun + DuC, MB = sec_sun + DuB;
+  const double xC = -sf::mul_mid(sf::mul_mid(MC, K), H);
+  const double xB = -sf::mul_mid(sf::mul_mid(MB, K), H);
+  const double eC = fm::exp_t(xC), eB = fm::exp_t(xB);
+  const double oC = 1.0 - eC;
+  const double rrs_C = sf::mul_mid(rrs_dp, oC);
+  const double rrs_B = sf::mul_mid(fma(rho, fm::kPiHi, rho * fm::kPiLo), eB);
+  const double rrs = rrs_C + rrs_B;
+  const double den = 1.0 - sf::mul_mid(1.5, rrs);
+  const double Rm = sf::div_mid(sf::half_mid(rrs), den);
+  const double d = Rm - r;
+  t.K = K;
+  t.rrs_B = rrs_B;
+  t.rrs = rrs;
+  t.Rm = Rm;
+  t.dd = sf::mul_mid(d, d);
+  const bool ok = near_x && ((sc.near_mask >> b) & 1) && sf::near(c) && sf::near_positive(ab) &&
+                  sf::near_positive(u) && sf::near_positive(MC) && sf::near_positive(MB) &&
+                  sf::near_positive(oC) && sf::mid_positive(eB) && sf::near_positive(rrs) && sf::near(den) && sf::near(d);
+  if (!ok) {
+    BandTerm g;
+    band_term_general(sc, b, sec_sun, H, rho, P, lnP, G, X, pw, r, &g);
+    t = g;
+  }
 }
 
 struct CostDetailsF64 {
@@ -103,12 +217,14 @@ struct CostDetailsF64 {
 
 // What a plain evaluation can keep, besides its cost, so that the products
 // at the kept optimum (model/samodel.c:2413, 1994-2079) follow from the same
-// evaluation: the bands' bottom and total subsurface reflectances and the
-// modelled Rrs, the Rrs error, K minimum and albedo.  NoKeep keeps nothing.
+// evaluation: the Rrs error, K minimum and albedo and, on the lanes that ask
+// (want), the index of optical depth's sum and the modelled Rrs.  NoKeep
+// keeps nothing.
 struct NoKeep {};
 template <int NB>
 struct BandKeep {
-  double rrs_B[NB], rrs[NB], Rm[NB];
+  bool want;
+  double iod, Rm[NB];
   double E, K_min, qB;
 };
 
@@ -131,54 +247,40 @@ __device__ __forceinline__ double cost_f64(const FitParams &fp, const SceneConst
   const double X = 0.01 * fabs(x[5]);
   const double lnP = log(P);
   const double qB = q * B;
+  const bool near_x = sf::near_positive(H) && sf::near_positive(qB) && sf::near_positive(P) &&
+                      sf::near_positive(G) && sf::near_positive(X) && sf::near(lnP);
   double err = 0.0, K_min = 1.0e4, iod = 0.0;
-#pragma unroll
-  for (int b = 0; b < NB; b++) {
-    if (b < nb) {
-      double rho = qB * sc.refl[b];
-      double a_phi = (sc.a0[b] + sc.a1[b] * lnP) * P;
-      double a_g = G * sc.eS[b];
-      double a = sc.aw[b] + a_phi + a_g;
-      double bb = sc.bbw[b] + X * px.pw[b];
-      double u = bb / (a + bb);
-      double K = a + bb;
-      if (K < 0.0) K = 0.0;
-      if (K > 2.5) K = 2.5;
-      double rrs_dp = (0.084 + 0.170 * u) * u;
-      double DuC = 1.03 * sqrt(1.0 + 2.4 * u);
-      double DuB = 1.04 * sqrt(1.0 + 5.4 * u);
-      double M = sc.sec_sun + DuC * sc.sec_view;
-      double rrs_C = rrs_dp * (1.0 - fm::exp_t(-M * K * H));
-      M = sc.sec_sun + DuB * sc.sec_view;
-      double rrs_B = fm::div_by(rho, kPi, fm::kInvPi) * fm::exp_t(-M * K * H);
-      double rrs = rrs_C + rrs_B;
-      double Rm = 0.5 * rrs / (1.0 - 1.5 * rrs);
-      double d = Rm - px.rrs[b];
-      err = err + d * d;
-      if (__double2float_rn(K) != 0.0f && K < K_min) K_min = K;
-      if (kDetails) {
-        iod = iod + rrs_B / rrs;
-        det->Rm[b] = Rm;
-      }
-      if constexpr (kKeep) {
-        keep->rrs_B[b] = rrs_B;
-        keep->rrs[b] = rrs;
-        keep->Rm[b] = Rm;
+#pragma unroll 1
+  for (int b = 0; b < nb; b++) {
+    BandTerm t;
+    band_term(sc, b, sc.sec_sun, near_x && sf::near_positive(px.pw[b]), H, qB * sc.refl[b], P, lnP,
+              G, X, px.pw[b], px.rrs[b], t);
+    err = err + t.dd;
+    if (k_counts(t.K) && sf::lt(t.K, K_min)) K_min = t.K;
+    if (kDetails) {
+      iod = iod + sf::div(t.rrs_B, t.rrs);
+      det->Rm[b] = t.Rm;
+    }
+    if constexpr (kKeep) {
+      if (keep->want) {
+        iod = iod + sf::div(t.rrs_B, t.rrs);
+        keep->Rm[b] = t.Rm;
       }
     }
   }
-  const double E = 100.0 * sqrt(fm::div_count(err, nb)) / px.mean;
+  const double E = sf::div(100.0 * sf::sqrt(fm::div_count(err, nb)), px.mean);
   double Ke = k_penalty_f64(fp.kp, H, K_min);
-  if (K_min > 0.7) {
+  if (sf::lt(0.7, K_min)) {
     double d = 4.0 * (K_min - 0.7);
     Ke = Ke + 100.0 * (d * d);
   }
   double model = 80.0 * E + 15.0 * Ke;
-  model = fm::div_by(model, 120.0, fm::kInv120);
+  model = fm::div_120(model);
   if constexpr (kKeep) {
     keep->E = E;
     keep->K_min = K_min;
     keep->qB = qB;
+    keep->iod = iod;
   }
   if (kDetails) {
     det->rrs_error = E;
@@ -193,6 +295,10 @@ __device__ __forceinline__ double cost_f64(const FitParams &fp, const SceneConst
 // The cold start of samodel_optimise_one_bottom_combination
 // (model/samodel.c:2249-2353) for one region, one scene, one bottom type;
 // the depth slot is filled per start.
+__device__ __forceinline__ double cold_P(double r490, double r550) {
+  return 100.0 * 0.072 * pow_call(r490 / r550, -1.7);
+}
+
 template <int NB>
 __device__ __forceinline__ void cold_start_f64(const FitParams &fp, const PixelF64<NB> &px,
                                                double *start, double *step) {
@@ -200,7 +306,7 @@ __device__ __forceinline__ void cold_start_f64(const FitParams &fp, const PixelF
   step[1] = 1.5 * start[1];
   start[2] = 1.0;
   step[2] = 0.5 * start[2];
-  start[3] = 100.0 * 0.072 * pow(px.r490 / px.r550, -1.7);
+  start[3] = cold_P(px.r490, px.r550);
   start[4] = 1.5 * start[3];
   start[5] = 100.0 * 30.0 * fp.aw640 * px.r640;
   step[3] = 2.0 * start[3];

@@ -335,6 +335,7 @@ __global__ void __launch_bounds__(BS) invert_kernel(const __grid_constant__ Inve
       if constexpr (P::kFused) {
         // the kept optimum is evaluated together with the other lanes' points
         typename P::template Keep<NB> keep;
+        keep.want = fin;
         y = P::template cost_keep<NB>(args, px, m.x, keep);
         if (fin) P::template details_from_keep<NB>(args, keep, y, det);
       } else {

@@ -37,8 +37,8 @@ struct PrecJ {
   static __device__ __forceinline__ T half(T a) { return a * 0.5; }
   static __device__ __forceinline__ T scale2(T a, float c) { return a * (double)c; }
   static __device__ __forceinline__ T div_n(T a, int n) { return fm::div_by(a, (double)n, 1.0 / (double)n); }
-  static __device__ __forceinline__ bool lt(T a, T b) { return a < b; }
-  static __device__ __forceinline__ bool le(T a, T b) { return a <= b; }
+  static __device__ __forceinline__ bool lt(T a, T b) { return sf::lt(a, b); }
+  static __device__ __forceinline__ bool le(T a, T b) { return sf::le(a, b); }
   static __device__ __forceinline__ T eps_step(T s) { return s * 1.0e-6; }
   static __device__ __forceinline__ T eps_scale() { return 1.0e-6; }
   static __device__ __forceinline__ long long trunc10(T y) { return photic::trunc10(y); }
@@ -124,43 +124,30 @@ __device__ __forceinline__ double jcost(const JointArgs &a, const JPixel<K, NB> 
       X = 0.01 * fabs(x[4 + 4 * s]);
     }
     const double lnP = log(P);
+    const bool near_x = sf::near_positive(H) && sf::near_positive(qB) && sf::near_positive(P) &&
+                        sf::near_positive(G) && sf::near_positive(X) && sf::near(lnP);
     double km = 1.0e4;
-#pragma unroll
+#pragma unroll 1  // the pixel is in local memory; one copy of the band term
     for (int b = 0; b < NB; b++) {
       if (b < nb) {
-        const double rho = qB * sc.refl[b];
-        const double a_phi = (sc.a0[b] + sc.a1[b] * lnP) * P;
-        const double a_g = G * sc.eS[b];
-        const double aa = sc.aw[b] + a_phi + a_g;
-        const double bb = sc.bbw[b] + X * px.pw[s][b];
-        const double u = bb / (aa + bb);
-        double Kb = aa + bb;
-        if (Kb < 0.0) Kb = 0.0;
-        if (Kb > 2.5) Kb = 2.5;
-        const double rrs_dp = (0.084 + 0.170 * u) * u;
-        const double DuC = 1.03 * sqrt(1.0 + 2.4 * u);
-        const double DuB = 1.04 * sqrt(1.0 + 5.4 * u);
-        double M = px.sec_sun[s] + DuC * sc.sec_view;
-        const double rrs_C = rrs_dp * (1.0 - fm::exp_t(-M * Kb * H));
-        M = px.sec_sun[s] + DuB * sc.sec_view;
-        const double rrs_B = fm::div_by(rho, kPi, fm::kInvPi) * fm::exp_t(-M * Kb * H);
-        const double rrs = rrs_C + rrs_B;
-        const double Rm = 0.5 * rrs / (1.0 - 1.5 * rrs);
-        const double d = Rm - px.rrs[s][b];
-        err = err + d * d;
-        if (__double2float_rn(Kb) != 0.0f && Kb < km) km = Kb;
+        BandTerm t;
+        band_term(sc, b, px.sec_sun[s], near_x && sf::near_positive(px.pw[s][b]), H,
+                  qB * sc.refl[b], P, lnP, G, X, px.pw[s][b], px.rrs[s][b], t);
+        err = err + t.dd;
+        const double Kb = t.K;
+        if (k_counts(Kb) && sf::lt(Kb, km)) km = Kb;
         if (kDetails) {
-          iod = iod + rrs_B / rrs;
-          if (__double2float_rn(Kb) != 0.0f && Kb < Kall) Kall = Kb;
+          iod = iod + t.rrs_B / t.rrs;
+          if (k_counts(Kb) && sf::lt(Kb, Kall)) Kall = Kb;
         }
       }
     }
     kmin[s] = km;
   }
-  const double E = 100.0 * sqrt(fm::div_count(err, K * nb)) / px.mean;
+  const double E = sf::div(100.0 * sf::sqrt(fm::div_count(err, K * nb)), px.mean);
   double Ke = 0.0;
   for (int s = 0; s < K; s++) Ke = Ke + k_penalty_f64(fp.kp, H, kmin[s]);
-  if (kmin[K - 1] > 0.7) {
+  if (sf::lt(0.7, kmin[K - 1])) {
     const double d = 4.0 * (kmin[K - 1] - 0.7);
     Ke = Ke + 100.0 * (d * d);
   }
@@ -380,12 +367,6 @@ cudaError_t launch_k(const JointArgs &a, int grid, cudaStream_t s) {
 template <int LAYOUT, int NB>
 cudaError_t launch_all_k(const JointArgs &a, int sms, int per_sm, cudaStream_t s,
                          const JointFork *f) {
-  const int grid = sms * (per_sm > 0 ? per_sm : 4);
-  typedef cudaError_t (*Launch)(const JointArgs &, int, cudaStream_t);
-  const Launch fn[kMaxScenes] = {launch_k<LAYOUT, 1, NB>, launch_k<LAYOUT, 2, NB>,
-                                 launch_k<LAYOUT, 3, NB>, launch_k<LAYOUT, 4, NB>,
-                                 launch_k<LAYOUT, 5, NB>, launch_k<LAYOUT, 6, NB>,
-                                 launch_k<LAYOUT, 7, NB>, launch_k<LAYOUT, 8, NB>};
   cudaError_t e;
   if (f && (e = cudaEventRecord(f->fork, s)) != cudaSuccess) return e;
   for (int k = kMaxScenes; k >= 1; k--) {
@@ -393,7 +374,16 @@ cudaError_t launch_all_k(const JointArgs &a, int sms, int per_sm, cudaStream_t s
     if (f && (e = cudaStreamWaitEvent(t, f->fork, 0)) != cudaSuccess) return e;
     // up to four bands: a group of lanes per pixel (photic_joint_group.cu);
     // more bands: one thread per pixel
-    e = NB <= 4 ? launch_joint_group(a, k, per_sm, sms, t) : fn[k - 1](a, grid, t);
+    if constexpr (NB <= 4) {
+      e = launch_joint_group(a, k, per_sm, sms, t);
+    } else {
+      typedef cudaError_t (*Launch)(const JointArgs &, int, cudaStream_t);
+      const Launch fn[kMaxScenes] = {launch_k<LAYOUT, 1, NB>, launch_k<LAYOUT, 2, NB>,
+                                     launch_k<LAYOUT, 3, NB>, launch_k<LAYOUT, 4, NB>,
+                                     launch_k<LAYOUT, 5, NB>, launch_k<LAYOUT, 6, NB>,
+                                     launch_k<LAYOUT, 7, NB>, launch_k<LAYOUT, 8, NB>};
+      e = fn[k - 1](a, sms * (per_sm > 0 ? per_sm : 4), t);
+    }
     if (e != cudaSuccess) return e;
     if (f) {
       if ((e = cudaEventRecord(f->join[k - 1], t)) != cudaSuccess) return e;

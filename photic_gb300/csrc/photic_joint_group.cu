@@ -290,28 +290,14 @@ __global__ void __launch_bounds__(kBlock) joint_group_kernel(const __grid_consta
       const double Gg = 0.01 * fabs(x[cP + 1]);
       const double Xx = 0.01 * fabs(x[cP + 2]);
       const double lnP = log(P);
-      const double rho = qB * sc.refl[bb];
-      const double a_phi = (sc.a0[bb] + sc.a1[bb] * lnP) * P;
-      const double a_g = Gg * sc.eS[bb];
-      const double aa = sc.aw[bb] + a_phi + a_g;
-      const double bbk = sc.bbw[bb] + Xx * my_pw;
-      const double u = bbk / (aa + bbk);
-      double Kb = aa + bbk;
-      if (Kb < 0.0) Kb = 0.0;
-      if (Kb > 2.5) Kb = 2.5;
-      const double rrs_dp = (0.084 + 0.170 * u) * u;
-      const double DuC = 1.03 * sqrt(1.0 + 2.4 * u);
-      const double DuB = 1.04 * sqrt(1.0 + 5.4 * u);
-      double M = my_sec + DuC * sc.sec_view;
-      const double rrs_C = rrs_dp * (1.0 - fm::exp_t(-M * Kb * H));
-      M = my_sec + DuB * sc.sec_view;
-      const double rrs_B = fm::div_by(rho, kPi, fm::kInvPi) * fm::exp_t(-M * Kb * H);
-      const double rrs = rrs_C + rrs_B;
-      const double Rm = 0.5 * rrs / (1.0 - 1.5 * rrs);
-      const double d = Rm - my_rrs;
-      g.dd[gl] = d * d;
-      g.kk[gl] = Kb;
-      if (final_eval) g.io[gl] = rrs_B / rrs;
+      const bool near_x = sf::near_positive(H) && sf::near_positive(qB) && sf::near_positive(P) &&
+                          sf::near_positive(Gg) && sf::near_positive(Xx) && sf::near(lnP) &&
+                          sf::near_positive(my_pw);
+      BandTerm t;
+      band_term(sc, bb, my_sec, near_x, H, qB * sc.refl[bb], P, lnP, Gg, Xx, my_pw, my_rrs, t);
+      g.dd[gl] = t.dd;
+      g.kk[gl] = t.K;
+      if (final_eval) g.io[gl] = t.rrs_B / t.rrs;
     }
     __syncwarp();
     // each scene's K_min and K penalty on lane s (model/samodel.c:2696-2725);
@@ -321,7 +307,7 @@ __global__ void __launch_bounds__(kBlock) joint_group_kernel(const __grid_consta
       double km = 1.0e4;
       for (int b = 0; b < nb; b++) {
         const double Kb = g.kk[gl * 4 + b];
-        if (__double2float_rn(Kb) != 0.0f && Kb < km) km = Kb;
+        if (k_counts(Kb) && sf::lt(Kb, km)) km = Kb;
       }
       g.kmin[gl] = km;
       g.kpen[gl] = k_penalty_f64(fp.kp, H, km);
@@ -338,12 +324,12 @@ __global__ void __launch_bounds__(kBlock) joint_group_kernel(const __grid_consta
           for (int b = 0; b < nb; b++) {
             const double Kb = g.kk[s * 4 + b];
             iod = iod + g.io[s * 4 + b];
-            if (__double2float_rn(Kb) != 0.0f && Kb < Kall) Kall = Kb;
+            if (k_counts(Kb) && sf::lt(Kb, Kall)) Kall = Kb;
           }
       }
       const double km = g.kmin[K - 1];
-      const double E = 100.0 * sqrt(fm::div_count(err, K * nb)) / mean;
-      if (km > 0.7) {  // the last scene's K_min (model/samodel.c:2726-2732)
+      const double E = sf::div(100.0 * sf::sqrt(fm::div_count(err, K * nb)), mean);
+      if (sf::lt(0.7, km)) {  // the last scene's K_min (model/samodel.c:2726-2732)
         const double dk = 4.0 * (km - 0.7);
         Ke = Ke + 100.0 * (dk * dk);
       }

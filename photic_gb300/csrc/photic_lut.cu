@@ -522,6 +522,7 @@ __global__ void __launch_bounds__(kLutBlock) lut_kernel(const __grid_constant__ 
       // values give the products (the final point is evaluated together
       // with the other lanes' trial points)
       BandKeep<NB> keep;
+      keep.want = m.phase == PH_FINAL;
       const double y = P::template cost_keep<NB>(ia, px, m.x, keep);
       if (m.phase == PH_FINAL) {
         typename P::Details det;

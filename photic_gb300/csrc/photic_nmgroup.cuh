@@ -30,10 +30,23 @@ struct NmGroup {
   double inv_n, inv_n1;  // RN(1 / n), RN(1 / (n + 1)) for the centroid and the variance test
   long long floor_lo;
   int32_t phase, jj, hi, lo, icount, numres, ifault, countdown, kcount, konvge;
+  // The centroid sums every coordinate over the vertices in order, and an
+  // iteration changes one vertex: ck holds the sums before vertices kCkStep,
+  // 2 kCkStep, ..., the first ck_valid of them up to date, so that the sum
+  // resumes at the changed vertex's block instead of at vertex 0 (the same
+  // additions in the same order; half of them on average).
+  static constexpr int kCkStep = 8;
+  static constexpr int kCk = ((NT > 0 ? NT : C * G) + kCkStep) / kCkStep;
+  double ck[C][kCk];
+  int32_t ck_valid;
 
   __device__ __forceinline__ int dim() const { return NT > 0 ? NT : nrt; }
   __device__ __forceinline__ int coord(int t) const { return gl + t * G; }
   __device__ __forceinline__ bool own(int t) const { return coord(t) < dim(); }
+  // Whether slot t holds a coordinate on any lane, and the coordinate that a
+  // lane reads for it (a lane without one reads its group's first).
+  __device__ __forceinline__ bool slot_used(int t) const { return t == 0 || t * G < dim(); }
+  __device__ __forceinline__ int column(int t) const { return own(t) ? coord(t) : t * G; }
   // The slot holding coordinate i on this lane, -1 if another lane owns it.
   // (Matching i against coord(t) slot by slot instead lost the match on
   // the second slot in the compiled kernel: the stepped vertex of the last
@@ -74,7 +87,7 @@ struct NmGroup {
     inv_n = inv_n1 = 1.0;
     scale = 1.0;
     floor_lo = 0;
-    phase = jj = hi = lo = icount = numres = ifault = countdown = 0;
+    phase = jj = hi = lo = icount = numres = ifault = countdown = ck_valid = 0;
   }
 
   __device__ __forceinline__ void begin(double var_limit_, int32_t konvge_, int32_t kcount_) {
@@ -98,6 +111,7 @@ struct NmGroup {
         X[coord(t)] = start[t];
         Vv(dim(), coord(t)) = start[t];
       }
+    ck_valid = 0;
     phase = PH_INIT_BASE;
   }
 
@@ -119,9 +133,10 @@ struct NmGroup {
   __device__ __forceinline__ void find_lo() {
     ylo = F(0);
     lo = 0;
+#pragma unroll 1
     for (int j = 1; j <= dim(); j++) {
       const double fj = F(j);
-      if (fj < ylo) {
+      if (sf::lt(fj, ylo)) {
         ylo = fj;
         lo = j;
       }
@@ -140,9 +155,10 @@ struct NmGroup {
       if (f0 != f0) return 0;
       double v = 0.0;
       int idx = 0x7fffffff;
+#pragma unroll 1
       for (int j = gl; j <= dim(); j += G) {
         const double f = F(j);
-        if (f == f && (idx == 0x7fffffff || v < f)) {
+        if (f == f && (idx == 0x7fffffff || sf::lt(v, f))) {
           v = f;
           idx = j;
         }
@@ -152,7 +168,7 @@ struct NmGroup {
         const double ov = __shfl_xor_sync(gmask, v, o);
         const int oi = __shfl_xor_sync(gmask, idx, o);
         if (oi != 0x7fffffff &&
-            (idx == 0x7fffffff || v < ov || (!(ov < v) && oi < idx))) {
+            (idx == 0x7fffffff || sf::lt(v, ov) || (!sf::lt(ov, v) && oi < idx))) {
           v = ov;
           idx = oi;
         }
@@ -162,9 +178,10 @@ struct NmGroup {
     }
     double yhi = F(0);
     int h = 0;
+#pragma unroll 1
     for (int j = 1; j <= dim(); j++) {
       const double fj = F(j);
-      if (yhi < fj) {
+      if (sf::lt(yhi, fj)) {
         yhi = fj;
         h = j;
       }
@@ -178,30 +195,49 @@ struct NmGroup {
     if constexpr (kSharedF) {
 #if defined(__CUDA_ARCH__)
       int c = 0;
+#pragma unroll 1
       for (int j = gl; j <= dim(); j += G)
-        if (fr_ < F(j)) c++;
+        if (sf::lt(fr_, F(j))) c++;
       return (int)__reduce_add_sync(gmask, (unsigned)c);
 #endif
     }
     int worse = 0;
+#pragma unroll 1
     for (int j = 0; j <= dim(); j++)
-      if (fr_ < F(j)) worse++;
+      if (sf::lt(fr_, F(j))) worse++;
     return worse;
   }
 
   __device__ __forceinline__ bool inner_top() {
     if (kcount <= icount) return false;
     hi = worst_vertex();
+    double z[C];
+    int m = ck_valid;
+#pragma unroll
+    for (int t = 0; t < C; t++) z[t] = m > 0 ? ck[t][m - 1] : 0.0;
+    int j = m * kCkStep;
+#pragma unroll 1
+    for (; j + kCkStep <= dim() + 1; j += kCkStep, m++) {
+#pragma unroll
+      for (int t = 0; t < C; t++)
+        if (slot_used(t)) {
+#pragma unroll
+          for (int i = 0; i < kCkStep; i++) z[t] = z[t] + Vv(j + i, column(t));
+          ck[t][m] = z[t];
+        }
+    }
+    ck_valid = m;
+#pragma unroll 1
+    for (; j <= dim(); j++) {
+#pragma unroll
+      for (int t = 0; t < C; t++)
+        if (slot_used(t)) z[t] = z[t] + Vv(j, column(t));
+    }
 #pragma unroll
     for (int t = 0; t < C; t++)
-      if (own(t)) {
-        const int i = coord(t);
-        double z = 0.0;
-        for (int j = 0; j <= dim(); j++) z = z + Vv(j, i);
-        z = z - Vv(hi, i);
-        cen[t] = fm::div_by(z, (double)dim(), inv_n);
-        refl[t] = cen[t] + (cen[t] - Vv(hi, i));
-        X[i] = refl[t];
+      if (slot_used(t)) {
+        z[t] = z[t] - Vv(hi, column(t));
+        cen[t] = fm::div_by(z[t], (double)dim(), inv_n);
       }
     phase = PH_REFLECT;
     return true;
@@ -211,16 +247,34 @@ struct NmGroup {
   // every lane of the group), so no lane ever reads a cost another lane is
   // writing, whatever the lanes' relative progress; or one shared copy
   // written between barriers (setF).
-  __device__ __forceinline__ void replace_hi(const double (&p)[C], double y) {
+  __device__ __forceinline__ void replace_hi(bool reflection, double y) {
 #pragma unroll
     for (int t = 0; t < C; t++)
-      if (own(t)) Vv(hi, coord(t)) = p[t];
+      if (own(t)) Vv(hi, coord(t)) = reflection ? refl[t] : trial[t];
+    if (hi / kCkStep < ck_valid) ck_valid = hi / kCkStep;
     setF(hi, y);
+  }
+
+  // The pending point of the iteration, cen + c (a - b) (photic_nm.cuh): the
+  // reflection, the expansion or a contraction, written once.
+  __device__ __forceinline__ void make_point(int pk) {
+    const double c = pk == PK_EXPAND ? 2.0 : (pk == PK_REFL ? 1.0 : 0.5);
+#pragma unroll
+    for (int t = 0; t < C; t++)
+      if (slot_used(t)) {
+        const double w = Vv(hi, column(t));
+        const double a = pk == PK_REFL ? cen[t] : (pk == PK_CONTRACT_IN ? w : refl[t]);
+        const double b = pk == PK_REFL ? w : cen[t];
+        const double p = cen[t] + c * (a - b);
+        if (pk == PK_REFL) refl[t] = p;
+        else trial[t] = p;
+        if (own(t)) X[coord(t)] = p;
+      }
   }
 
   __device__ __forceinline__ bool iteration_end() {
     const double fh = F(hi);
-    if (fh < ylo) {
+    if (sf::lt(fh, ylo)) {
       ylo = fh;
       lo = hi;
     }
@@ -229,14 +283,16 @@ struct NmGroup {
     if (icount <= kcount) {
       countdown = konvge;
       double z = 0.0;
+#pragma unroll 1
       for (int j = 0; j <= dim(); j++) z = z + F(j);
       const double mean = fm::div_by(z, (double)(dim() + 1), inv_n1);
       z = 0.0;
+#pragma unroll 1
       for (int j = 0; j <= dim(); j++) {
         const double d = F(j) - mean;
         z = z + d * d;
       }
-      if (z <= var_limit) return true;
+      if (sf::le(z, var_limit)) return true;
     }
     return false;
   }
@@ -260,115 +316,69 @@ struct NmGroup {
       }
   }
 
+  // Consume the cost y of the point at X and stage the next one.  Returns
+  // true when the nelmin call has returned.  As in photic_nm.cuh the switch
+  // only decides; what it decides on (a vertex replaced, a vertex shrunk, the
+  // next point) is written once below it, and the transitions between the
+  // stages only go forward.
   __device__ __forceinline__ bool step_machine(double y) {
     enum { CS_NONE = -1, CS_READY, CS_TOP, CS_ITER_END, CS_END_INNER, CS_PROBE_PLUS,
            CS_PROBE_END, CS_NM_DONE };
-    int cs = CS_NONE;
+    int cs = CS_NONE, pk = PK_NONE, rep = 0, vert = -1, shr = -1;
+    icount++;
     switch (phase) {
       case PH_INIT_BASE:
         setF(dim(), y);
-        icount++;
-        make_vertex(0);
+        vert = 0;
         break;
       case PH_INIT_VERT:
         setF(jj, y);
-        icount++;
-        if (jj + 1 < dim()) make_vertex(jj + 1);
+        if (jj + 1 < dim()) vert = jj + 1;
         else cs = CS_READY;
         break;
       case PH_REFLECT:
         fr = y;
-        icount++;
-        if (fr < ylo) {
-#pragma unroll
-          for (int t = 0; t < C; t++) trial[t] = cen[t] + 2.0 * (refl[t] - cen[t]);
-          set_x_from(trial);
+        if (sf::lt(fr, ylo)) {
+          pk = PK_EXPAND;
           phase = PH_EXPAND;
         } else {
           const int worse = count_worse(fr);
           if (worse > 1) {
-            replace_hi(refl, fr);
-            cs = CS_ITER_END;
+            rep = 1;
           } else if (worse == 0) {
-#pragma unroll
-            for (int t = 0; t < C; t++)
-              if (own(t)) trial[t] = cen[t] + (Vv(hi, coord(t)) - cen[t]) * 0.5;
-            set_x_from(trial);
+            pk = PK_CONTRACT_IN;
             phase = PH_CONTRACT_IN;
           } else {
-#pragma unroll
-            for (int t = 0; t < C; t++) trial[t] = cen[t] + (refl[t] - cen[t]) * 0.5;
-            set_x_from(trial);
+            pk = PK_CONTRACT_OUT;
             phase = PH_CONTRACT_OUT;
           }
         }
         break;
       case PH_EXPAND:
-        icount++;
-        if (fr < y) replace_hi(refl, fr);
-        else replace_hi(trial, y);
-        cs = CS_ITER_END;
+        rep = sf::lt(fr, y) ? 1 : 2;
         break;
-      case PH_CONTRACT_IN: {
-        icount++;
-        const bool shrink = F(hi) < y;
-        if (shrink) {
-#pragma unroll
-          for (int t = 0; t < C; t++)
-            if (own(t)) {
-              const int i = coord(t);
-              const double s = (Vv(0, i) + Vv(lo, i)) * 0.5;
-              Vv(0, i) = s;
-              X[i] = s;
-            }
-          jj = 0;
-          phase = PH_SHRINK;
-        } else {
-          replace_hi(trial, y);
-          cs = CS_ITER_END;
-        }
+      case PH_CONTRACT_IN:
+        // shrink every vertex towards the best (model/asa047.c:331-351)
+        if (sf::lt(F(hi), y)) shr = 0;
+        else rep = 2;
         break;
-      }
       case PH_SHRINK:
         setF(jj, y);
-        icount++;
-        if (jj < dim()) {
-          const int j = jj + 1;
-#pragma unroll
-          for (int t = 0; t < C; t++)
-            if (own(t)) {
-              const int i = coord(t);
-              const double s = (Vv(j, i) + Vv(lo, i)) * 0.5;
-              Vv(j, i) = s;
-              X[i] = s;
-            }
-          jj = j;
-        } else {
-          cs = CS_READY;
-        }
+        if (jj < dim()) shr = jj + 1;
+        else cs = CS_READY;
         break;
       case PH_CONTRACT_OUT:
-        icount++;
-        if (y <= fr) replace_hi(trial, y);
-        else replace_hi(refl, fr);
-        cs = CS_ITER_END;
+        rep = sf::le(y, fr) ? 2 : 1;
         break;
       case PH_PROBE_PLUS:
-        icount++;
+      case PH_PROBE_MINUS:
         if (trunc10(y) < floor_lo) {
           ifault = 2;
           cs = CS_PROBE_END;
-        } else {
+        } else if (phase == PH_PROBE_PLUS) {
           probe_move(-1);
           set_x_from(xmin);
           phase = PH_PROBE_MINUS;
-        }
-        break;
-      case PH_PROBE_MINUS:
-        icount++;
-        if (trunc10(y) < floor_lo) {
-          ifault = 2;
-          cs = CS_PROBE_END;
         } else {
           probe_move(0);
           jj++;
@@ -376,60 +386,72 @@ struct NmGroup {
         }
         break;
       default:
+        icount--;
         break;
     }
-    while (cs != CS_NONE) {
-      switch (cs) {
-        case CS_READY:
-          find_lo();
-          cs = CS_TOP;
-          break;
-        case CS_TOP:
-          cs = inner_top() ? CS_NONE : CS_END_INNER;
-          break;
-        case CS_ITER_END:
-          cs = iteration_end() ? CS_END_INNER : CS_TOP;
-          break;
-        case CS_END_INNER:
+    if (vert >= 0) make_vertex(vert);
+    if (shr >= 0) {
 #pragma unroll
-          for (int t = 0; t < C; t++)
-            if (own(t)) xmin[t] = Vv(lo, coord(t));
-          floor_lo = trunc10(F(lo));
-          if (kcount < icount) {
-            ifault = 2;
-            cs = CS_NM_DONE;
-          } else {
-            ifault = 0;
-            jj = 0;
-            cs = CS_PROBE_PLUS;
-          }
-          break;
-        case CS_PROBE_PLUS:
-          probe_move(+1);
-          set_x_from(xmin);
-          phase = PH_PROBE_PLUS;
-          cs = CS_NONE;
-          break;
-        case CS_PROBE_END:
-          if (ifault == 0) {
-            cs = CS_NM_DONE;
-          } else {
-#pragma unroll
-            for (int t = 0; t < C; t++) start[t] = xmin[t];
-            scale = 1.0e-6;
-            numres++;
-            restart_simplex();
-            cs = CS_NONE;
-          }
-          break;
-        case CS_NM_DONE:
-          return true;
-        default:
-          cs = CS_NONE;
-          break;
+      for (int t = 0; t < C; t++)
+        if (own(t)) {
+          const int i = coord(t);
+          const double s = (Vv(shr, i) + Vv(lo, i)) * 0.5;
+          Vv(shr, i) = s;
+          X[i] = s;
+        }
+      ck_valid = 0;
+      jj = shr;
+      phase = PH_SHRINK;
+    }
+    if (rep) {
+      replace_hi(rep == 1, rep == 1 ? fr : y);
+      cs = CS_ITER_END;
+    }
+    if (cs == CS_READY) {
+      find_lo();
+      cs = CS_TOP;
+    }
+    if (cs == CS_ITER_END) cs = iteration_end() ? CS_END_INNER : CS_TOP;
+    if (cs == CS_TOP) {
+      if (inner_top()) {
+        pk = PK_REFL;
+        cs = CS_NONE;
+      } else {
+        cs = CS_END_INNER;
       }
     }
-    return false;
+    if (pk != PK_NONE) make_point(pk);
+    if (cs == CS_END_INNER) {
+#pragma unroll
+      for (int t = 0; t < C; t++)
+        if (own(t)) xmin[t] = Vv(lo, coord(t));
+      floor_lo = trunc10(F(lo));
+      if (kcount < icount) {
+        ifault = 2;
+        cs = CS_NM_DONE;
+      } else {
+        ifault = 0;
+        jj = 0;
+        cs = CS_PROBE_PLUS;
+      }
+    }
+    if (cs == CS_PROBE_PLUS) {
+      probe_move(+1);
+      set_x_from(xmin);
+      phase = PH_PROBE_PLUS;
+    }
+    if (cs == CS_PROBE_END) {
+      if (ifault == 0) {
+        cs = CS_NM_DONE;
+      } else {
+#pragma unroll
+        for (int t = 0; t < C; t++) start[t] = xmin[t];
+        scale = 1.0e-6;
+        numres++;
+        restart_simplex();
+      }
+    }
+    return cs == CS_NM_DONE;
   }
 };
 

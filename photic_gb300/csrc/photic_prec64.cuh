@@ -32,8 +32,8 @@ struct PrecF64 {
   static __device__ __forceinline__ T scale2(T a, float c) { return a * (double)c; }
   // z / n for the simplex size n, a compile-time constant here
   static __device__ __forceinline__ T div_n(T a, int n) { return fm::div_by(a, (double)n, 1.0 / (double)n); }
-  static __device__ __forceinline__ bool lt(T a, T b) { return a < b; }
-  static __device__ __forceinline__ bool le(T a, T b) { return a <= b; }
+  static __device__ __forceinline__ bool lt(T a, T b) { return sf::lt(a, b); }
+  static __device__ __forceinline__ bool le(T a, T b) { return sf::le(a, b); }
   static __device__ __forceinline__ T eps_step(T s) { return s * 1.0e-6; }
   static __device__ __forceinline__ T eps_scale() { return 1.0e-6; }
   static __device__ __forceinline__ long long trunc10(T y) { return photic::trunc10(y); }
@@ -41,10 +41,7 @@ struct PrecF64 {
   static __device__ __forceinline__ double to_double(T a) { return a; }
   static __device__ __forceinline__ T var_limit(const InvertArgs &a) { return a.fp.reqmin * (double)kPrecN; }
   static __device__ __forceinline__ T hstart(const InvertArgs &a, int k) {
-    double h = a.fp.hstarts[0];
-    for (int i = 1; i < kMaxHStarts; i++)
-      if (i == k) h = a.fp.hstarts[i];
-    return h;
+    return a.fp.hstarts[k];
   }
   static __device__ __forceinline__ T h_step(T h) { return 1.25 * h; }
   template <int NB>
@@ -74,21 +71,17 @@ struct PrecF64 {
                                                 const T *x, Keep<NB> &k) {
     return cost_f64<false, NB, Keep<NB>>(a.fp, a.sc, px, x, nullptr, &k);
   }
-  // The products of cost_f64<true> (photic_fp64.cuh) from a kept evaluation,
-  // the index of optical depth summed in band order.
+  // The products of cost_f64<true> (photic_fp64.cuh) from a kept evaluation
+  // with keep.want set.
   template <int NB>
   static __device__ __forceinline__ void details_from_keep(const InvertArgs &a,
                                                            const Keep<NB> &k, T model,
                                                            Details &d) {
-    double iod = 0.0;
-#pragma unroll
-    for (int b = 0; b < NB; b++)
-      if (b < a.fp.n_bands) iod = iod + k.rrs_B[b] / k.rrs[b];
     d.rrs_error = k.E;
     d.model_error = model;
     d.bottom_albedo = k.qB;
     d.K_min = k.K_min == 1.0e4 ? 0.0 : k.K_min;
-    d.iod = 100.0 * iod / (double)a.fp.n_bands;
+    d.iod = 100.0 * k.iod / (double)a.fp.n_bands;
   }
   template <int NB>
   static __device__ __forceinline__ void details(const InvertArgs &a, const Pixel<NB> &px,

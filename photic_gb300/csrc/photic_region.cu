@@ -46,8 +46,8 @@ constexpr int kMaxR = kRegionMaxR, kTerms = 128, kHT = kTerms / 32, kShares = 32
 constexpr int kChainD = 3 * kRS + kTerms + 3 * kMaxScenes + 24;
 // the cost's staging, per warp: |H| and depth deviations per region, bottom
 // deviations per (type, region), K penalty and smallest K per scene, mean
-// share per type
-constexpr int kStage = 64;
+// share per type, ln P per scene
+constexpr int kStage = 72;
 
 // Launch shapes: C coordinates per lane, vertex row stride CG.
 template <int C, int CG>
@@ -60,7 +60,7 @@ struct Shape {
   // per-(region, bottom) shares of the bottom-continuity term, and the
   // chain mode's arrays
   static constexpr int kSmem =
-      (kMaxN + 1) * CG + kNF + 32 * C + 3 * kTerms + 3 * kRS + 8 + kShares + kChainD + kStage;
+      (kMaxN + 1) * CG + kNF + 32 * C + 3 * kTerms + 3 * kRS + 8 + 2 * kShares + kChainD + kStage;
 };
 
 __device__ __forceinline__ bool nodata_value(float v, float nodata) {
@@ -74,12 +74,13 @@ __device__ __forceinline__ bool nodata_value(float v, float nodata) {
 // (scene s of region r is row rp[r] * S + s of the list, or pixel rp[r] of
 // scene s's grid), their count and the origin's slot.  A neighbour with a
 // nodata band in any scene is left out.
-__device__ __forceinline__ int regions_of(const RegionArgs &a, int64_t p, int64_t (&rp)[kMaxR],
+__device__ __noinline__ int regions_of(const RegionArgs &a, int64_t p, int64_t (&rp)[kMaxR],
                                           int &origin) {
   const int nb = a.fp.n_bands;
   if (a.list_R) {
     const int R = a.list_R[p];
     origin = a.list_origin[p];
+#pragma unroll 1
     for (int r = 0; r < kMaxR; r++) rp[r] = p * kMaxR + (r < R ? r : 0);
     return R;
   }
@@ -87,13 +88,17 @@ __device__ __forceinline__ int regions_of(const RegionArgs &a, int64_t p, int64_
   const int w = a.n_spatial - 1;
   int R = 0;
   origin = 0;
+#pragma unroll 1
   for (int ii = -w; ii <= w; ii++) {
     const int iii = i + ii < 0 ? 0 : (i + ii > a.nrows - 1 ? a.nrows - 1 : i + ii);
+#pragma unroll 1
     for (int jj = -w; jj <= w; jj++) {
       const int jjj = j + jj < 0 ? 0 : (j + jj > a.ncols - 1 ? a.ncols - 1 : j + jj);
       const int64_t q = (int64_t)iii * a.ncols + jjj;
       bool nodata = false;
+#pragma unroll 1
       for (int s = 0; s < a.n_scenes; s++)
+#pragma unroll 1
         for (int b = 0; b < nb; b++)
           if (nodata_value(a.grid[(s * a.npix + q) * nb + b], a.fp.nodata)) nodata = true;
       if (i == iii && j == jjj) origin = R;
@@ -107,6 +112,7 @@ __device__ __forceinline__ void write_masked(const photic_outputs &o, int64_t p,
                                              int32_t status) {
   if (o.depth) o.depth[p] = 0.0f;
   if (o.depth_f64) o.depth_f64[p] = 0.0;
+#pragma unroll 1
   for (int s = 0; s < S; s++) {
     if (o.P) o.P[p * S + s] = 0.0f;
     if (o.G) o.G[p * S + s] = 0.0f;
@@ -121,6 +127,7 @@ __device__ __forceinline__ void write_masked(const photic_outputs &o, int64_t p,
   if (o.evals_kept) o.evals_kept[p] = 0;
   if (o.status) o.status[p] = status;
   if (o.bottom_percent)
+#pragma unroll 1
     for (int k = 0; k < 3; k++) o.bottom_percent[p * 3 + k] = 0.0f;
   if (o.bottom_type) o.bottom_type[p] = 0.0f;
 }
@@ -147,6 +154,7 @@ constexpr double kMaxSkip = 0.9925;       // :880
 // pixel with an empirical depth, is 0 (every bottom type fitted).
 __device__ __forceinline__ void chain_begin(const RegionArgs &a, double *cst, double *cprev,
                                             int64_t c, int S) {
+#pragma unroll 1
   for (int k = 0; k < G_COUNT; k++) cst[k] = 0.0;
   const double m0 = 1.125 * (double)S;
   cst[G_MATCH] = m0 > kMinThreshold ? m0 : kMinThreshold;
@@ -155,6 +163,7 @@ __device__ __forceinline__ void chain_begin(const RegionArgs &a, double *cst, do
   cst[G_KBEG] = (double)(c * a.n_shallow / a.n_chains);
   cst[G_KEND] = (double)((c + 1) * a.n_shallow / a.n_chains);
   cst[G_K] = cst[G_KBEG];
+#pragma unroll 1
   for (int i = 0; i < 3 * kMaxScenes; i++) cprev[i] = 0.0;
 }
 
@@ -215,10 +224,13 @@ __device__ __forceinline__ float glut_diff(const double *meas, const double *rm,
                                            int nb) {
   double error = 0.0;
   int n_total = 0;
+#pragma unroll 1
   for (int k = 1; k <= 3; k++) {
     if (k >= nb) break;
     double current = 0.0, previous = 0.0, nobs = 0.0;
+#pragma unroll 1
     for (int s = 0; s < S; s++)
+#pragma unroll 1
       for (int r = 0; r < R; r++) {
         const double mv = meas[(s * R + r) * 3 + k - 1], lv = rm[(r * S + s) * 3 + k - 1];
         if ((float)mv != 0.0f && (float)lv != 0.0f) {
@@ -246,6 +258,7 @@ __device__ __forceinline__ float glut_diff(const double *meas, const double *rm,
 __device__ __noinline__ void serve_copy(const RegionArgs &a, int64_t p, int64_t src, float diff,
                                         int S, int lane) {
   const photic_outputs &o = a.out;
+#pragma unroll 1
   for (int f = lane; f < 15 + 3 * S; f += 32) {
     if (f == 0) { if (o.depth) o.depth[p] = o.depth[src]; }
     else if (f == 1) { if (o.depth_f64) o.depth_f64[p] = o.depth_f64[src]; }
@@ -289,7 +302,8 @@ __global__ void __launch_bounds__(BLOCK, 1) region_kernel(const __grid_constant_
          *kk = dd + kTerms, *io = kk + kTerms, *s490 = io + kTerms, *s550 = s490 + kRS,
          *s640 = s550 + kRS, *misc = s640 + kRS;
   double *share = misc + 8;
-  double *meas = share + kShares, *rmv = meas + 3 * kRS, *cprev = rmv + kTerms,
+  double *wB = share + kShares;  // q_k / sum(q) B_k of each (region, type)
+  double *meas = wB + kShares, *rmv = meas + 3 * kRS, *cprev = rmv + kTerms,
          *cst = cprev + 3 * kMaxScenes, *stg = cst + 24;
   const bool list = a.list_R != nullptr;
   // spectrum of scene s of region slot q (a pixel index of the grid, or a
@@ -356,6 +370,7 @@ __global__ void __launch_bounds__(BLOCK, 1) region_kernel(const __grid_constant_
           }
         }
         // measured bands 1..3 of every region and scene, scene-major
+#pragma unroll 1
         for (int t = lane; t < R * S * 3; t += 32) {
           const int s = t / (R * 3), r = (t / 3) % R, k = t % 3 + 1;
           meas[t] = k < nb ? (double)spec(rp[r], s)[k] : 0.0;
@@ -375,6 +390,7 @@ __global__ void __launch_bounds__(BLOCK, 1) region_kernel(const __grid_constant_
         const double *ring = a.ring + (size_t)c * a.cap * a.entry_stride;
         double bestd = 1.0e4;
         int64_t pos = 0;
+#pragma unroll 1
         for (int64_t j = lane; j < n_in; j += 32) {
           const double *e = ring + j * a.entry_stride;
           if ((int)e[0] == R && fabs(e[1] - dep) / (dep + kEps) < kContinuity &&
@@ -408,6 +424,7 @@ __global__ void __launch_bounds__(BLOCK, 1) region_kernel(const __grid_constant_
         const int64_t src = a.ring_src[(size_t)c * a.cap + pos];
         const double *e = ring + pos * a.entry_stride;
         serve_copy(a, p, src, (float)bestd, S, lane);
+#pragma unroll 1
         for (int i = lane; i < 3 * S; i += 32) cprev[i] = e[3 + i];
         __syncwarp();
         if (lane == 0) {
@@ -433,7 +450,9 @@ __global__ void __launch_bounds__(BLOCK, 1) region_kernel(const __grid_constant_
       // (model/samodel.c:933-947); samodel_optimise called directly has none
       if (!a.no_mask) {
         bool masked = false;
+#pragma unroll 1
         for (int s = 0; s < S; s++)
+#pragma unroll 1
           for (int b = 0; b < nb; b++) {
             const float v = spec(p, s)[b];
             if (nodata_value(v, fp.nodata) || v < 0.0f) masked = true;
@@ -471,36 +490,27 @@ __global__ void __launch_bounds__(BLOCK, 1) region_kernel(const __grid_constant_
     m.nrt = N;
     // term tau = ((r S + s) nb + b): region r, scene s, band b, in the order
     // samodel_error sums them (model/samodel.c:2465-2571)
-    double my_rrs[kHT], my_pw[kHT], my_sec[kHT];
-    int my_r[kHT], my_s[kHT], my_b[kHT];
-    bool my_on[kHT];
+    double my_rrs[kHT], my_pw[kHT];
+    int my_rsb[kHT];  // r | s << 8 | b << 16
+#pragma unroll 1
+    for (int h = 0, tau = lane; tau < nterm; h++, tau += 32) {
+      const int rs = tau / nb, b = tau % nb, r = rs / S, s = rs % S;
+      const float *sp = spec(rp[r], s);
+      double r8[kMaxBands];
 #pragma unroll
-    for (int h = 0; h < kHT; h++) {
-      const int tau = lane + 32 * h;
-      my_rrs[h] = my_pw[h] = my_sec[h] = 0.0;
-      my_r[h] = my_s[h] = my_b[h] = 0;
-      my_on[h] = tau < nterm;
-      if (my_on[h]) {
-        const int rs = tau / nb, b = tau % nb, r = rs / S, s = rs % S;
-        const float *sp = spec(rp[r], s);
-        double r8[kMaxBands];
-#pragma unroll
-        for (int c = 0; c < kMaxBands; c++) r8[c] = c < nb ? (double)sp[c] : 0.0;
-        double r440 = interp_plan<kMaxBands>(fp.plan[0], r8);
-        const double r490 = interp_plan<kMaxBands>(fp.plan[1], r8);
-        if (r440 < 0.0) r440 = 0.0001;
-        const double chi = r440 / r490;
-        double Y = 3.44 * (1.0 - 3.17 * fm::exp_t(-2.01 * chi));
-        if (Y < 0.0) Y = 0.0;
-        if (Y > 2.5) Y = 2.5;
-        my_rrs[h] = (double)sp[b];
-        my_pw[h] = pow(sc.ratio440[b], Y);
-        my_sec[h] = a.sec_sun[s];
-        my_r[h] = r;
-        my_s[h] = s;
-        my_b[h] = b;
-      }
+      for (int c = 0; c < kMaxBands; c++) r8[c] = c < nb ? (double)sp[c] : 0.0;
+      double r440 = interp_plan<kMaxBands>(fp.plan[0], r8);
+      const double r490 = interp_plan<kMaxBands>(fp.plan[1], r8);
+      if (r440 < 0.0) r440 = 0.0001;
+      const double chi = r440 / r490;
+      double Y = 3.44 * (1.0 - 3.17 * fm::exp_t(-2.01 * chi));
+      if (Y < 0.0) Y = 0.0;
+      if (Y > 2.5) Y = 2.5;
+      my_rrs[h] = (double)sp[b];
+      my_pw[h] = pow_call(sc.ratio440[b], Y);
+      my_rsb[h] = r | s << 8 | b << 16;
     }
+#pragma unroll 1
     for (int rs = lane; rs < R * S; rs += 32) {
       const float *sp = spec(rp[rs / S], rs % S);
       double r8[kMaxBands];
@@ -514,8 +524,11 @@ __global__ void __launch_bounds__(BLOCK, 1) region_kernel(const __grid_constant_
     // mean measured Rrs over all region-scene-bands, in the cost's order
     double tot = 0.0;
     if (lane == 0) {
+#pragma unroll 1
       for (int r = 0; r < R; r++)
+#pragma unroll 1
         for (int s = 0; s < S; s++)
+#pragma unroll 1
           for (int b = 0; b < nb; b++) tot = tot + (double)spec(rp[r], s)[b];
     }
     tot = __shfl_sync(kFull, tot, 0);
@@ -532,6 +545,7 @@ __global__ void __launch_bounds__(BLOCK, 1) region_kernel(const __grid_constant_
           sp = 1.25 * st;
         } else if (c < qo) {
           double m490 = 0.0;
+#pragma unroll 1
           for (int rs = 0; rs < R * S; rs++) m490 += s490[rs];
           m490 /= (double)R * S;
           st = 100.0 * 4.0 * m490;
@@ -542,6 +556,7 @@ __global__ void __launch_bounds__(BLOCK, 1) region_kernel(const __grid_constant_
         } else if (c < N) {
           const int s = (c - off) / 3, j = (c - off) % 3;
           double m490 = 0.0, m550 = 0.0, m640 = 0.0;
+#pragma unroll 1
           for (int r = 0; r < R; r++) {
             m490 += s490[r * S + s];
             m550 += s550[r * S + s];
@@ -550,7 +565,7 @@ __global__ void __launch_bounds__(BLOCK, 1) region_kernel(const __grid_constant_
           m490 /= (double)R;
           m550 /= (double)R;
           m640 /= (double)R;
-          const double P = 100.0 * 0.072 * pow(m490 / m550, -1.7);
+          const double P = cold_P(m490, m550);
           st = j == 0 ? P : j == 1 ? 1.5 * P : 100.0 * 30.0 * fp.aw640 * m640;
           sp = 2.0 * st;
         }
@@ -573,6 +588,7 @@ __global__ void __launch_bounds__(BLOCK, 1) region_kernel(const __grid_constant_
     for (int tt = 0; tt < C; tt++) best[tt] = 0.0;
     bool final_eval = eval_only, fitted = false;
     if (eval_only) {
+#pragma unroll 1
       for (int c = lane; c < N; c += 32) X[c] = a.eval_params[p * a.eval_stride + c];
     } else {
       cold(isnan(hemp) ? fp.hstarts[0] : hemp);
@@ -581,67 +597,46 @@ __global__ void __launch_bounds__(BLOCK, 1) region_kernel(const __grid_constant_
 
     for (;;) {
       __syncwarp();
+      // ---- each (region, type) on its own lane: the mixture's weight times
+      // albedo (model/samodel.c:2475-2496, 2878-2883), the share |100 B| |q| /
+      // sum |q| of the bottom-continuity term; each scene's ln P
+      if (lane < R * nbt) {
+        const int r = lane / nbt;
+        double qs = 0.0;
+#pragma unroll 1
+        for (int kb = 0; kb < nbt; kb++) qs += fabs(X[qo + r * nbt + kb]);
+        const double q = fabs(X[qo + lane]), B100 = fabs(X[R + lane]);
+        wB[lane] = div_call(q, qs) * (0.01 * B100);
+        share[lane] = div_call(B100 * q, qs);
+      }
+      double *lnps = stg + 64;
+      if (lane < S) lnps[lane] = log(0.01 * fabs(X[off + 3 * lane]));
+      __syncwarp();
       // ---- band terms at X
-#pragma unroll
-      for (int h = 0; h < kHT; h++) {
-        if (!my_on[h]) continue;
-        const int r = my_r[h], s = my_s[h], b = my_b[h], tau = lane + 32 * h;
+#pragma unroll 1
+      for (int h = 0, tau = lane; tau < nterm; h++, tau += 32) {
+        const int rsb = my_rsb[h], r = rsb & 255, s = (rsb >> 8) & 255, b = rsb >> 16;
+        const double pw = my_pw[h];
         const double H = fabs(X[r]);
         const double P = 0.01 * fabs(X[off + 3 * s]);
         const double Gg = 0.01 * fabs(X[off + 1 + 3 * s]);
         const double Xx = 0.01 * fabs(X[off + 2 + 3 * s]);
-        // bottom mixture of the region (model/samodel.c:2475-2496, 2878-2883);
-        // the loops over the (at most 3) types are unrolled so the values
-        // stay in registers
-        double Bk[3], qk[3], q_sum = 0.0, rho = 0.0;
-#pragma unroll
-        for (int k = 0; k < 3; k++) {
-          Bk[k] = k < nbt ? 0.01 * fabs(X[R + r * nbt + k]) : 0.0;
-          qk[k] = k < nbt ? fabs(X[qo + r * nbt + k]) : 0.0;
-        }
-#pragma unroll
-        for (int k = 0; k < 3; k++)
-          if (k < nbt) q_sum += qk[k];
-#pragma unroll
-        for (int k = 0; k < 3; k++)
-          if (k < nbt) qk[k] /= q_sum;
-#pragma unroll
-        for (int k = 0; k < 3; k++)
-          if (k < nbt) rho += qk[k] * Bk[k] * sc.refl_k[k][b];
-        const double lnP = log(P);
-        const double a_phi = (sc.a0[b] + sc.a1[b] * lnP) * P;
-        const double a_g = Gg * sc.eS[b];
-        const double aa = sc.aw[b] + a_phi + a_g;
-        const double bbk = sc.bbw[b] + Xx * my_pw[h];
-        const double u = bbk / (aa + bbk);
-        double Kb = aa + bbk;
-        if (Kb < 0.0) Kb = 0.0;
-        if (Kb > 2.5) Kb = 2.5;
-        const double rrs_dp = (0.084 + 0.170 * u) * u;
-        const double DuC = 1.03 * sqrt(1.0 + 2.4 * u);
-        const double DuB = 1.04 * sqrt(1.0 + 5.4 * u);
-        double M = my_sec[h] + DuC * sc.sec_view;
-        const double rrs_C = rrs_dp * (1.0 - fm::exp_t(-M * Kb * H));
-        M = my_sec[h] + DuB * sc.sec_view;
-        const double rrs_B = fm::div_by(rho, kPi, fm::kInvPi) * fm::exp_t(-M * Kb * H);
-        const double rrs = rrs_C + rrs_B;
-        const double Rm = 0.5 * rrs / (1.0 - 1.5 * rrs);
-        const double d = Rm - my_rrs[h];
-        dd[tau] = d * d;
-        kk[tau] = Kb;
+        const double lnP = lnps[s];
+        double rho = 0.0;
+#pragma unroll 1
+        for (int k = 0; k < nbt; k++) rho += wB[r * nbt + k] * sc.refl_k[k][b];
+        const bool near_x = sf::near_positive(H) && sf::near_positive(rho) &&
+                            sf::near_positive(P) && sf::near_positive(Gg) &&
+                            sf::near_positive(Xx) && sf::near(lnP) && sf::near_positive(pw);
+        BandTerm t;
+        band_term(sc, b, a.sec_sun[s], near_x, H, rho, P, lnP, Gg, Xx, pw, my_rrs[h], t);
+        dd[tau] = t.dd;
+        kk[tau] = t.K;
         if (final_eval) {
-          io[tau] = rrs_B / rrs;
-          if (eval_only && a.eval_rm) a.eval_rm[((p * kMaxR + r) * S + s) * nb + b] = Rm;
-          if (chained) rmv[tau] = Rm;
+          io[tau] = t.rrs_B / t.rrs;
+          if (eval_only && a.eval_rm) a.eval_rm[((p * kMaxR + r) * S + s) * nb + b] = t.Rm;
+          if (chained) rmv[tau] = t.Rm;
         }
-      }
-      // each (region, bottom) share |100 B| |q| / sum |q| on its own lane
-      // (the division is the costly part of the bottom-continuity term)
-      if (lane < R * nbt) {
-        const int r = lane / nbt, k = lane % nbt;
-        double qs = 0.0;
-        for (int kb = 0; kb < nbt; kb++) qs += fabs(X[qo + r * nbt + kb]);
-        share[lane] = fabs(X[R + r * nbt + k]) * fabs(X[qo + r * nbt + k]) / qs;
       }
       __syncwarp();
       // ---- the cost (model/samodel.c:2432-2759).  Every sum keeps the
@@ -656,9 +651,10 @@ __global__ void __launch_bounds__(BLOCK, 1) region_kernel(const __grid_constant_
       if (lane < R) habs[lane] = fabs(X[lane]);
       if (lane < S) {  // each scene's smallest K over the last region's bands (:2696-2701)
         double km = 1.0e4;
+#pragma unroll 1
         for (int b = 0; b < nb; b++) {
           const double Kb = kk[((R - 1) * S + lane) * nb + b];
-          if (__double2float_rn(Kb) != 0.0f && Kb < km) km = Kb;
+          if (k_counts(Kb) && sf::lt(Kb, km)) km = Kb;
         }
         kms[lane] = km;
       }
@@ -682,8 +678,8 @@ __global__ void __launch_bounds__(BLOCK, 1) region_kernel(const __grid_constant_
         for (int i = 0; i < cnt; i++) z = z + src[i * str];
       }
       const double err = __shfl_sync(kFull, z, 0);
-      const double dmean = __shfl_sync(kFull, z, 1) / (double)R;
-      if (lane >= 2 && lane < 2 + nbt) bmv[lane - 2] = z / (double)R;
+      const double dmean = div_call(__shfl_sync(kFull, z, 1), (double)R);
+      if (lane >= 2 && lane < 2 + nbt) bmv[lane - 2] = div_call(z, (double)R);
       const double thd = dmean < 4.0 ? 0.4 : dmean < 8.0 ? 0.2 : dmean < 12.0 ? 0.1 : 0.05;
       const double thb = dmean < 5.0 ? 0.25 : dmean < 10.0 ? 0.1 : dmean < 15.0 ? 0.05 : 0.01;
       bool outd = false, outb = false;
@@ -729,36 +725,52 @@ __global__ void __launch_bounds__(BLOCK, 1) region_kernel(const __grid_constant_
       double Ed = __shfl_sync(kFull, z2, 0), Eb = __shfl_sync(kFull, z2, 1);
       double Ke = __shfl_sync(kFull, z2, 2);
       const double btotal = __shfl_sync(kFull, z2, 3);
+      // 100 sqrt(sum / count) / mean of the residuals, the depths and the
+      // bottom shares, on lanes 0, 1 and 2
+      double rms;
+      {
+        const double num = lane == 1 ? Ed : lane == 2 ? Eb : err;
+        const double cnt = lane == 1 ? nd : lane == 2 ? nbo : (double)nterm;
+        double den = lane == 1 ? dmean : mean;
+        if (lane == 2) den = div_call(btotal, (double)nbt);
+        rms = div_call(100.0 * sf::sqrt(div_call(num, cnt)), den);
+        if (lane == 1 && nd == 0.0) rms = Ed;
+        if (lane == 2 && nbo == 0.0) rms = Eb;
+      }
+      Ed = __shfl_sync(kFull, rms, 1);
+      Eb = __shfl_sync(kFull, rms, 2);
       double y = 0.0;
       if (lane == 0) {
-        const double E = 100.0 * sqrt(fm::div_count(err, nterm)) / mean;
-        if (nd > 0.5) Ed = 100.0 * sqrt(Ed / nd) / dmean;
-        if (nbo > 0.5) {
-          const double bmean = btotal / ((double)nbt);
-          Eb = 100.0 * sqrt(Eb / nbo) / bmean;
-        }
+        const double E = rms;
         // the very-high-K term on the last scene's K (:2728-2732)
         const double km = kms[S - 1];
-        if (km > 0.7) {
+        if (sf::lt(0.7, km)) {
           const double dk = 4.0 * (km - 0.7);
           Ke = Ke + 100.0 * (dk * dk);
         }
         double model = 80.0 * E + 15.0 * Ed + 10.0 * Eb + 15.0 * Ke;
-        model = fm::div_by(model, 120.0, fm::kInv120);
+        model = fm::div_120(model);
         y = model;
         if (final_eval) {
           double iod = 0.0, Kall = 1.0e4;
+#pragma unroll 1
           for (int s = 0; s < S; s++)  // model/samodel.c:2051-2064
+#pragma unroll 1
             for (int r = 0; r < R; r++)
+#pragma unroll 1
               for (int b = 0; b < nb; b++) iod = iod + io[(r * S + s) * nb + b];
+#pragma unroll 1
           for (int s = 0; s < S; s++)  // min over md->K, model/samodel.c:1994
+#pragma unroll 1
             for (int b = 0; b < nb; b++) {
               const double Kb = kk[((R - 1) * S + s) * nb + b];
-              if (__double2float_rn(Kb) != 0.0f && Kb < Kall) Kall = Kb;
+              if (k_counts(Kb) && sf::lt(Kb, Kall)) Kall = Kb;
             }
           // bottom albedo of the last region, sum_k q_k B_k (model/samodel.c:2878-2881)
           double qs = 0.0, alb = 0.0;
+#pragma unroll 1
           for (int k = 0; k < nbt; k++) qs += fabs(X[qo + (R - 1) * nbt + k]);
+#pragma unroll 1
           for (int k = 0; k < nbt; k++)
             alb += (fabs(X[qo + (R - 1) * nbt + k]) / qs) * (0.01 * fabs(X[R + (R - 1) * nbt + k]));
           misc[0] = E;
@@ -790,6 +802,7 @@ __global__ void __launch_bounds__(BLOCK, 1) region_kernel(const __grid_constant_
         if (lane == 0) {
           const double ow = sqrt((double)R);
           double depth = 0.0;
+#pragma unroll 1
           for (int r = 0; r < R; r++) {
             const double h = fabs(X[r]);
             if (r == origin) depth += ow * h;
@@ -814,6 +827,7 @@ __global__ void __launch_bounds__(BLOCK, 1) region_kernel(const __grid_constant_
             }
           if (o.depth) o.depth[p] = (float)depth;
           if (o.depth_f64) o.depth_f64[p] = depth;
+#pragma unroll 1
           for (int s = 0; s < S; s++) {
             if (o.P) o.P[p * S + s] = (float)(0.01 * fabs(X[off + 3 * s]));
             if (o.G) o.G[p * S + s] = (float)(0.01 * fabs(X[off + 1 + 3 * s]));
@@ -827,6 +841,7 @@ __global__ void __launch_bounds__(BLOCK, 1) region_kernel(const __grid_constant_
           if (o.evals) o.evals[p] = total;
           if (o.evals_kept) o.evals_kept[p] = kept_evals;
           if (o.bottom_percent)
+#pragma unroll 1
             for (int k = 0; k < 3; k++) o.bottom_percent[p * 3 + k] = (float)pct[k];
           if (o.bottom_type) o.bottom_type[p] = (float)type;
           if (o.status)
@@ -834,6 +849,7 @@ __global__ void __launch_bounds__(BLOCK, 1) region_kernel(const __grid_constant_
                           (hot ? PHOTIC_PX_HOT : 0) | (kept_start << 16) | (R << 24);
         }
         if (a.list_params)
+#pragma unroll 1
           for (int c = lane; c < N; c += 32) a.list_params[p * a.eval_stride + c] = X[c];
         fitted = true;
         break;
@@ -866,10 +882,7 @@ __global__ void __launch_bounds__(BLOCK, 1) region_kernel(const __grid_constant_
             if (m.own(tt)) X[m.coord(tt)] = best[tt];  // re-evaluate at the kept optimum (:2413)
           final_eval = true;
         } else {
-          double hs = fp.hstarts[0];
-          for (int k = 1; k < kMaxHStarts; k++)
-            if (k == kst) hs = fp.hstarts[k];
-          cold(hs);
+          cold(fp.hstarts[kst]);
           m.begin(var_limit, fp.konvge, fp.kcount);
         }
       }
@@ -885,11 +898,14 @@ __global__ void __launch_bounds__(BLOCK, 1) region_kernel(const __grid_constant_
       const bool ins = fitted && me < cst[G_ENTRY] && depth < 32.0;
       const int64_t slot = (int64_t)cst[G_TOTLUT] % a.cap;
       if (fitted)
+#pragma unroll 1
         for (int i = lane; i < 3 * S; i += 32) cprev[i] = fabs(X[off + i]);
       __syncwarp();
       if (ins) {
         double *e = a.ring + ((size_t)c * a.cap + slot) * a.entry_stride;
+#pragma unroll 1
         for (int i = lane; i < 3 * S; i += 32) e[3 + i] = cprev[i];
+#pragma unroll 1
         for (int t = lane; t < R * S * 3; t += 32) {
           const int r = t / (S * 3), s = (t / 3) % S, k = t % 3 + 1;
           e[3 + 3 * S + t] = k < nb ? rmv[(r * S + s) * nb + k] : 0.0;
