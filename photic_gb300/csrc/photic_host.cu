@@ -278,6 +278,62 @@ int joint_fork(ForkSlot **out) {
 // kernel keeps 128.
 int default_invert_block(int precision) { return precision == PHOTIC_PREC_FP64 ? 256 : 128; }
 
+// Launch shape of the inversion for a queue of `positions`.  One FP64 warp
+// instruction keeps a quarter of an SM busy for 64 clocks whatever its live
+// lanes, so few positions go, a few lanes each, to one warp per quarter
+// (blocks of 128 threads, one per SM); more take the block that is fastest
+// for a full device.
+void invert_shape(const InvertArgs &a, int precision, int sms, int64_t positions, int &block,
+                  int &per_sm, int64_t &grid, int32_t &claim) {
+  const int64_t quarters = (int64_t)sms * 4;
+  const bool few = block == 0 && per_sm == 0 && positions <= quarters * 32;
+  if (few) {
+    block = 128;
+    per_sm = 1;
+  }
+  if (block == 0) block = default_invert_block(precision);
+  if (per_sm == 0) per_sm = invert_blocks_per_sm(a, precision, block);
+  grid = (int64_t)sms * per_sm;
+  const int64_t warps = grid * (block / 32);
+  const int64_t share = (positions + warps - 1) / (warps > 0 ? warps : 1);
+  claim = share < 1 ? 1 : share > 32 ? 32 : (int32_t)share;
+  const int64_t need = (positions + (int64_t)claim * (block / 32) - 1) / ((int64_t)claim * (block / 32));
+  if (grid > need) grid = need;
+}
+
+// Device memory for the starts' records: the last pixels of a larger scene
+// run start by start, the ones before them with their starts in sequence.
+constexpr int64_t kRecordBytesMax = 1ll << 30;
+
+// The batched inversion of prepared arguments: workspace (queue head, exits,
+// records), launch shape, launches.
+int run_invert(InvertArgs &a, int precision, int block, int per_sm, int sms, cudaStream_t s) {
+  const int64_t per_pixel = (int64_t)a.fp.n_hstarts * kStartRecordBytes + sizeof(int32_t);
+  a.n_par = a.fp.n_hstarts > 1 ? kRecordBytesMax / per_pixel : 0;
+  if (a.n_par > a.npix) a.n_par = a.npix;
+  a.n_seq = a.npix - a.n_par;
+  int64_t grid = 0;
+  invert_shape(a, precision, sms, a.n_seq + a.n_par * a.fp.n_hstarts, block, per_sm, grid, a.claim);
+  if (per_sm < 1) return fail(PHOTIC_ERR_CUDA, "kernel does not fit on the device");
+  const size_t off_rec = 256, rec_bytes = (size_t)a.n_par * a.fp.n_hstarts * kStartRecordBytes;
+  const size_t off_exit = off_rec + rec_bytes;
+  unsigned char *ws = nullptr;
+  cudaError_t e = cudaMallocAsync((void **)&ws, off_exit + (size_t)a.n_par * sizeof(int32_t), s);
+  if (e != cudaSuccess) return fail(PHOTIC_ERR_NOMEM, "workspace: %s", cudaGetErrorString(e));
+  a.queue = reinterpret_cast<unsigned long long *>(ws);
+  a.records = ws + off_rec;
+  a.exit_k = reinterpret_cast<int32_t *>(ws + off_exit);
+  e = cudaMemsetAsync(ws, 0, sizeof(unsigned long long), s);
+  // 0x7f7f7f7f: no start has met the early exit
+  if (e == cudaSuccess && a.n_par > 0)
+    e = cudaMemsetAsync(a.exit_k, 0x7f, (size_t)a.n_par * sizeof(int32_t), s);
+  if (e == cudaSuccess) e = launch_invert(a, precision, block, (int)grid, s);
+  cudaError_t e2 = cudaFreeAsync(ws, s);
+  if (e != cudaSuccess) return cuda_fail(e, "invert kernel launch");
+  if (e2 != cudaSuccess) return cuda_fail(e2, "cudaFreeAsync");
+  return PHOTIC_OK;
+}
+
 }  // namespace
 
 namespace photic {
@@ -425,15 +481,16 @@ int photic_invert_batch_ordered(const photic_config *cfg, const float *d_rrs, in
   a.error = err;
   a.early_exit = cfg->early_exit_per_scene * (double)(float)1;
 
-  const bool guarded = cfg->precision == PHOTIC_PREC_GUARDED;
-  int block = cfg->block_threads    ? cfg->block_threads
-              : guarded             ? 128
-                                    : default_invert_block(cfg->precision);
-  if (guarded && block == 64) block = 128;
+  a.counters = g_counter_ptr;
+  a.guard_stats = g_guard_stats_ptr;
+  if (cfg->precision != PHOTIC_PREC_GUARDED)
+    return run_invert(a, cfg->precision, cfg->block_threads, cfg->blocks_per_sm, sms, s);
+
+  int block = cfg->block_threads ? cfg->block_threads : 128;
+  if (block == 64) block = 128;
   int per_sm = cfg->blocks_per_sm;
   if (per_sm == 0) {
-    per_sm = guarded ? guarded_blocks_per_sm(a, block)
-                     : invert_blocks_per_sm(a, cfg->precision, block);
+    per_sm = guarded_blocks_per_sm(a, block);
     if (per_sm < 1) return fail(PHOTIC_ERR_CUDA, "kernel does not fit on the device");
   }
   int64_t grid = (int64_t)sms * per_sm;
@@ -446,10 +503,7 @@ int photic_invert_batch_ordered(const photic_config *cfg, const float *d_rrs, in
   e = cudaMemsetAsync(queue, 0, sizeof(unsigned long long), s);
   if (e != cudaSuccess) return cuda_fail(e, "cudaMemsetAsync");
   a.queue = queue;
-  a.counters = g_counter_ptr;
-  a.guard_stats = g_guard_stats_ptr;
-  e = guarded ? launch_guarded(a, block, (int)grid, s)
-              : launch_invert(a, cfg->precision, block, (int)grid, s);
+  e = launch_guarded(a, block, (int)grid, s);
   cudaError_t e2 = cudaFreeAsync(queue, s);
   if (e != cudaSuccess) return cuda_fail(e, "invert kernel launch");
   if (e2 != cudaSuccess) return cuda_fail(e2, "cudaFreeAsync");
@@ -1256,16 +1310,11 @@ extern "C" int photic_invert_batch_noalloc(const photic_config *cfg, const float
   a.error = reinterpret_cast<unsigned int *>(scratch + 1);
   a.early_exit = cfg->early_exit_per_scene * (double)(float)1;
 
-  const int block =
-      cfg->block_threads ? cfg->block_threads : default_invert_block(cfg->precision);
-  int per_sm = cfg->blocks_per_sm;
-  if (per_sm == 0) {
-    per_sm = invert_blocks_per_sm(a, cfg->precision, block);
-    if (per_sm < 1) return fail(PHOTIC_ERR_CUDA, "kernel does not fit on the device");
-  }
-  int64_t grid = (int64_t)sms * per_sm;
-  const int64_t need = (npix + block - 1) / block;
-  if (grid > need) grid = need;
+  a.n_seq = npix;  // no records without allocation: every pixel's starts in sequence
+  int block = cfg->block_threads, per_sm = cfg->blocks_per_sm;
+  int64_t grid = 0;
+  invert_shape(a, cfg->precision, sms, npix, block, per_sm, grid, a.claim);
+  if (per_sm < 1) return fail(PHOTIC_ERR_CUDA, "kernel does not fit on the device");
 
   // The previous call left its final queue position and error bits here.
   cudaError_t e = cudaMemsetAsync(scratch, 0, needed, s);
@@ -1355,20 +1404,7 @@ int invert_prepared(const photic_config &cfg, const FitParams &fp, const SceneCo
   a.error = err;
   a.early_exit = cfg.early_exit_per_scene * (double)(float)1;
   a.no_mask = 1;  // the mask test belongs to samodel()'s pixel loop
-  const int block = default_invert_block(PHOTIC_PREC_FP64);
-  int per_sm = invert_blocks_per_sm(a, PHOTIC_PREC_FP64, block);
-  if (per_sm < 1) return fail(PHOTIC_ERR_CUDA, "kernel does not fit on the device");
-  int64_t grid = (int64_t)sms * per_sm;
-  if (grid > (npix + block - 1) / block) grid = (npix + block - 1) / block;
-  unsigned long long *queue = nullptr;
-  cudaError_t e = cudaMallocAsync((void **)&queue, sizeof(unsigned long long), s);
-  if (e != cudaSuccess) return fail(PHOTIC_ERR_NOMEM, "queue head");
-  cudaMemsetAsync(queue, 0, sizeof(unsigned long long), s);
-  a.queue = queue;
-  e = launch_invert(a, PHOTIC_PREC_FP64, block, (int)grid, s);
-  cudaFreeAsync(queue, s);
-  if (e != cudaSuccess) return cuda_fail(e, "invert launch");
-  return PHOTIC_OK;
+  return run_invert(a, PHOTIC_PREC_FP64, 0, 0, sms, s);
 }
 
 // Cost with details at n parameter vectors, prepared constants.

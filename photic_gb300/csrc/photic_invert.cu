@@ -10,7 +10,10 @@
 // 32 pixels with one atomic and stages their spectra through shared memory
 // with coalesced (float4 when the layout allows) loads.  Ragged iteration
 // counts (a few hundred to several thousand evaluations per pixel) thus
-// never leave a lane idle while work remains.
+// never leave a lane idle while work remains.  A pixel's depth starts are
+// positions of the queue of their own while the scene is small enough to
+// keep their results (see invert_kernel): a launch then ends with single
+// starts of at most kcount evaluations instead of with pixels of eight.
 //
 // The arithmetic is a policy: PrecF64 (IEEE double, reference operation
 // order, --fmad=false), PrecF32 (the forward model in float with the
@@ -197,6 +200,68 @@ struct PrecDF {
   }
 };
 
+// One start's nelmin result, kept until the pixel's starts are compared.
+template <class P>
+struct StartRecord {
+  typename P::T y;
+  int32_t evals;  // -1: the start hit the defensive evaluation cap
+  int32_t fault;
+  typename P::T x[kN];
+};
+
+template <class P, int NB>
+__device__ __forceinline__ void write_fit(const photic_outputs &o, int64_t p,
+                                          const typename P::T *x,
+                                          const typename P::Details &det, int32_t total,
+                                          int32_t kept_evals, int32_t kept_start,
+                                          int32_t kept_fault) {
+  const double H = fabs(P::to_double(x[0]));
+  if (o.depth) o.depth[p] = (float)H;
+  if (o.depth_f64) o.depth_f64[p] = H;
+  if (o.P) o.P[p] = (float)(0.01 * fabs(P::to_double(x[3])));
+  if (o.G) o.G[p] = (float)(0.01 * fabs(P::to_double(x[4])));
+  if (o.X) o.X[p] = (float)(0.01 * fabs(P::to_double(x[5])));
+  if (o.bottom_albedo) o.bottom_albedo[p] = (float)det.bottom_albedo;
+  if (o.model_error) o.model_error[p] = (float)det.model_error;
+  if (o.rrs_error) o.rrs_error[p] = (float)det.rrs_error;
+  if (o.K_min) o.K_min[p] = (float)det.K_min;
+  if (o.iod) o.iod[p] = (float)det.iod;
+  if (o.evals) o.evals[p] = total;
+  if (o.evals_kept) o.evals_kept[p] = kept_evals;
+  if (o.params)
+    for (int i = 0; i < kN; i++) o.params[p * kN + i] = P::to_double(x[i]);
+  if (o.status)
+    o.status[p] = PHOTIC_PX_FITTED | (kept_fault == 0 ? PHOTIC_PX_CONVERGED : 0) |
+                  (kept_start << 16);
+}
+
+template <int NB>
+__device__ __forceinline__ void load_spectrum(const InvertArgs &args, int64_t p, float (&r)[NB]) {
+  if (NB == 4 && args.vec4) {
+    const float4 v4 = __ldg(reinterpret_cast<const float4 *>(args.rrs) + p);
+    r[0] = v4.x;
+    r[1] = v4.y;
+    r[2] = v4.z;
+    r[3] = v4.w;
+  } else {
+#pragma unroll
+    for (int b = 0; b < NB; b++)
+      r[b] = b < args.fp.n_bands ? __ldg(args.rrs + p * args.pixel_stride + b * args.band_stride)
+                                 : 0.0f;
+  }
+}
+
+// The queue's positions: the first n_seq are pixels, each lane running a
+// pixel's starts one after the other; then, for the other n_par pixels, every
+// start is a position of its own (start-major: the first starts of all these
+// pixels, then the second starts, ...), its result goes to a record, and
+// finish_kernel compares a pixel's records in the order of the starts.  The
+// result is the sequential one: a start is left out once an earlier start of
+// its pixel has met the early exit (exit_k), where the sequential loop would
+// have ended at that start or before.  A launch lasts at least as long as its
+// longest position, and a pixel whose starts all fail takes eight times a
+// start: 256 pixels 131 -> 34 ms, 20 011 eight-band pixels 470 -> 124 ms, a
+// 1024 x 320 scene 601 -> 443 ms, a 701 x 997 tile of seeds 382 -> 363 ms.
 template <class P, int NB, int BS>
 __global__ void __launch_bounds__(BS) invert_kernel(const __grid_constant__ InvertArgs args) {
   using T = typename P::T;
@@ -207,123 +272,135 @@ __global__ void __launch_bounds__(BS) invert_kernel(const __grid_constant__ Inve
   T *sbest = sf + (kN + 1) * BS;                    // [N][BS]
   using Px = typename P::template Pixel<NB>;
   Px *spx = reinterpret_cast<Px *>(sbest + kN * BS);  // [BS/32][32] set-ups of the chunk
-  float *schunk = reinterpret_cast<float *>(spx + BS);  // [BS/32][32][NB]
+  int64_t *spos = reinterpret_cast<int64_t *>(spx + BS);  // [BS/32][32] their positions
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  float *wchunk = schunk + warp * 32 * NB;
   Px *wpx = spx + warp * 32;
+  int64_t *wpos = spos + warp * 32;
   const unsigned lt_mask = (1u << lane) - 1u;
+  StartRecord<P> *const rec = reinterpret_cast<StartRecord<P> *>(args.records);
+  const int64_t total_pos = args.n_seq + args.n_par * fp.n_hstarts;
 
   NmLane<kN, P, BS> m;
   m.v = sv + tid;
   m.f = sf + tid;
   T *best = sbest + tid;
-  typename P::template Pixel<NB> px;
+  Px px;
   const T var_limit = P::var_limit(args);
   const photic_outputs &o = args.out;
 
-  int64_t pixel = -1;
+  int64_t pixel = -1, item = -1;  // item: pixel number within the n_par, or -1
   int32_t start_k = 0, n_starts = 0, total = 0, kept_evals = 0, kept_start = 0, kept_fault = 0;
   int32_t guard = 0;
   T lowest = P::zero();
 
   bool has = false, open = true;
-  int64_t chunk_base = 0, chunk_next = 0, chunk_end = 0;
+  int chunk_next = 0, chunk_end = 0;
   const int32_t guard_cap = (fp.n_hstarts + 1) * (fp.kcount + 8 * kN + 16);
 
   for (;;) {
-    // ---- hand out pixels to lanes that have none -------------------------
+    // ---- hand out positions to lanes that have none ----------------------
     unsigned need = __ballot_sync(kFull, !has && open);
     while (need) {
       if (chunk_next >= chunk_end) {
         unsigned long long base = 0;
-        if (lane == 0) base = atomicAdd(args.queue, 32ull);
+        if (lane == 0) base = atomicAdd(args.queue, (unsigned long long)args.claim);
         base = __shfl_sync(kFull, base, 0);
-        if (base >= (unsigned long long)args.npix) {
+        if (base >= (unsigned long long)total_pos) {
           open = false;
           break;
         }
-        chunk_base = (int64_t)base;
-        chunk_next = chunk_base;
-        chunk_end = min(chunk_base + 32, args.npix);
         __syncwarp();
-        const int64_t q = chunk_base + lane;
-        if (q < args.npix) {
-          const int64_t p = args.order ? (int64_t)args.order[q] : q;
-          if (NB == 4 && args.vec4) {
-            const float4 v4 = __ldg(reinterpret_cast<const float4 *>(args.rrs) + p);
-            wchunk[lane * NB + 0] = v4.x;
-            wchunk[lane * NB + 1] = v4.y;
-            wchunk[lane * NB + 2] = v4.z;
-            wchunk[lane * NB + 3] = v4.w;
-          } else {
+        // Every lane looks at one position of the chunk: masked pixels are
+        // written, starts that are not needed dropped, the others set up
+        // (interpolated Rrs, Y and (440/lambda)^Y, model/samodel.c:1783-1799,
+        // 2897-2902) with the whole warp, instead of each lane alone when it
+        // takes the pixel.
+        const int64_t w = (int64_t)base + lane;
+        bool live = lane < args.claim && w < total_pos;
+        int64_t p = 0;
+        float r[NB];
+        if (live) {
+          int64_t q = w;
+          int k = 0;
+          if (w >= args.n_seq) {
+            k = (int)((w - args.n_seq) / args.n_par);
+            q = args.n_seq + (w - args.n_seq) % args.n_par;
+          }
+          p = args.order ? (int64_t)args.order[q] : q;
+          if (k > 0)
+            live = __ldcg(args.exit_k + (q - args.n_seq)) >= k &&
+                   (args.seeds == nullptr || isnan(args.seeds[p * kN]));
+          if (live) {
+            load_spectrum<NB>(args, p, r);
+            bool masked = false;
 #pragma unroll
             for (int b = 0; b < NB; b++)
-              wchunk[lane * NB + b] =
-                  b < fp.n_bands ? __ldg(args.rrs + p * args.pixel_stride + b * args.band_stride)
-                                 : 0.0f;
-          }
-          // every lane sets up one pixel of the chunk (interpolated Rrs,
-          // Y and (440/lambda)^Y, model/samodel.c:1783-1799, 2897-2902)
-          // with the whole warp, instead of each lane alone when it takes
-          // the pixel; a masked pixel's set-up is never used
-          float r[NB];
-#pragma unroll
-          for (int b = 0; b < NB; b++) r[b] = wchunk[lane * NB + b];
-          P::template setup<NB>(args, r, wpx[lane]);
-        }
-        __syncwarp();
-      }
-      const int rank = __popc(need & lt_mask);
-      const int avail = (int)(chunk_end - chunk_next);
-      const bool mine = ((need >> lane) & 1u) && rank < avail;
-      const unsigned taken = __ballot_sync(kFull, mine);
-      bool masked = false;
-      if (mine) {
-        const int64_t q = chunk_next + rank;  // queue position -> pixel
-        const int64_t p = args.order ? (int64_t)args.order[q] : q;
-        float r[NB];
-#pragma unroll
-        for (int b = 0; b < NB; b++) r[b] = wchunk[(q - chunk_base) * NB + b];
-#pragma unroll
-        for (int b = 0; b < NB; b++)
-          if (b < fp.n_bands && !args.no_mask && band_masked(r[b], fp.nodata)) masked = true;
-        if (masked) {
-          write_masked(o, p);
-        } else {
-          px = wpx[q - chunk_base];
-          pixel = p;
-          total = kept_evals = kept_start = kept_fault = guard = 0;
-          lowest = P::from_double(1.0e4);
-          start_k = 0;
-          bool seeded = false;
-#pragma unroll
-          for (int i = 0; i < kN; i++) best[i * BS] = P::zero();
-          if (args.seeds != nullptr) {
-            const double *sd = args.seeds + p * kN;
-            if (!isnan(sd[0])) {
-              const double rel[kN] = {1.25, 1.5, 0.5, 2.0, 2.0, 2.0};
-              seeded = true;
-#pragma unroll
-              for (int i = 0; i < kN; i++) {
-                m.start[i] = P::from_double(sd[i]);
-                m.step[i] = P::from_double((rel[i] * fp.seed_step_scale) * sd[i]);
+              if (b < fp.n_bands && !args.no_mask && band_masked(r[b], fp.nodata)) masked = true;
+            if (masked) {
+              live = false;
+              if (k == 0) {
+                write_masked(o, p);
+                if (w >= args.n_seq) args.exit_k[q - args.n_seq] = -1;
               }
             }
           }
-          n_starts = seeded ? 1 : fp.n_hstarts;
-          if (!seeded) {
-            P::template cold_start<NB>(args, px, m.start, m.step);
-            m.start[0] = P::hstart(args, 0);
-            m.step[0] = P::h_step(m.start[0]);
-          }
-          m.begin(var_limit, fp.konvge, fp.kcount);
-          has = true;
         }
+        const unsigned alive = __ballot_sync(kFull, live);
+        if (live) {
+          const int slot = __popc(alive & lt_mask);
+          P::template setup<NB>(args, r, wpx[slot]);
+          wpos[slot] = w;
+        }
+        chunk_next = 0;
+        chunk_end = __popc(alive);
+        __syncwarp();
+        if (chunk_end == 0) continue;
+      }
+      const int rank = __popc(need & lt_mask);
+      const bool mine = ((need >> lane) & 1u) && rank < chunk_end - chunk_next;
+      const unsigned taken = __ballot_sync(kFull, mine);
+      if (mine) {
+        const int slot = chunk_next + rank;
+        const int64_t w = wpos[slot];
+        int64_t q = w;
+        start_k = 0;
+        item = -1;
+        if (w >= args.n_seq) {
+          item = (w - args.n_seq) % args.n_par;
+          start_k = (int32_t)((w - args.n_seq) / args.n_par);
+          q = args.n_seq + item;
+        }
+        pixel = args.order ? (int64_t)args.order[q] : q;
+        px = wpx[slot];
+        total = kept_evals = kept_start = kept_fault = guard = 0;
+        lowest = P::from_double(1.0e4);
+        bool seeded = false;
+#pragma unroll
+        for (int i = 0; i < kN; i++) best[i * BS] = P::zero();
+        if (args.seeds != nullptr) {
+          const double *sd = args.seeds + pixel * kN;
+          if (!isnan(sd[0])) {
+            const double rel[kN] = {1.25, 1.5, 0.5, 2.0, 2.0, 2.0};
+            seeded = true;
+#pragma unroll
+            for (int i = 0; i < kN; i++) {
+              m.start[i] = P::from_double(sd[i]);
+              m.step[i] = P::from_double((rel[i] * fp.seed_step_scale) * sd[i]);
+            }
+          }
+        }
+        n_starts = seeded ? 1 : fp.n_hstarts;
+        if (!seeded) {
+          P::template cold_start<NB>(args, px, m.start, m.step);
+          m.start[0] = P::hstart(args, start_k);
+          m.step[0] = P::h_step(m.start[0]);
+        }
+        m.begin(var_limit, fp.konvge, fp.kcount);
+        has = true;
       }
       chunk_next += __popc(taken);
       need &= ~taken;
-      need |= __ballot_sync(kFull, mine && masked);
     }
     if (!__any_sync(kFull, has)) break;
 
@@ -343,36 +420,31 @@ __global__ void __launch_bounds__(BS) invert_kernel(const __grid_constant__ Inve
         else y = P::template cost<NB>(args, px, m.x);
       }
       if (fin) {
-        const int64_t p = pixel;
-        const double H = fabs(P::to_double(m.x[0]));
-        if (o.depth) o.depth[p] = (float)H;
-        if (o.depth_f64) o.depth_f64[p] = H;
-        if (o.P) o.P[p] = (float)(0.01 * fabs(P::to_double(m.x[3])));
-        if (o.G) o.G[p] = (float)(0.01 * fabs(P::to_double(m.x[4])));
-        if (o.X) o.X[p] = (float)(0.01 * fabs(P::to_double(m.x[5])));
-        if (o.bottom_albedo) o.bottom_albedo[p] = (float)det.bottom_albedo;
-        if (o.model_error) o.model_error[p] = (float)det.model_error;
-        if (o.rrs_error) o.rrs_error[p] = (float)det.rrs_error;
-        if (o.K_min) o.K_min[p] = (float)det.K_min;
-        if (o.iod) o.iod[p] = (float)det.iod;
-        if (o.evals) o.evals[p] = total;
-        if (o.evals_kept) o.evals_kept[p] = kept_evals;
-        if (o.params)
-          for (int i = 0; i < kN; i++) o.params[p * kN + i] = P::to_double(m.x[i]);
-        if (o.status)
-          o.status[p] = PHOTIC_PX_FITTED | (kept_fault == 0 ? PHOTIC_PX_CONVERGED : 0) |
-                        (kept_start << 16);
+        write_fit<P, NB>(o, pixel, m.x, det, total, kept_evals, kept_start, kept_fault);
         has = false;
-      } else {
-        if (++guard > guard_cap) {
-          // Defensive cap: each nelmin call is bounded by kcount, so
-          // reaching this means a defect; flag it instead of spinning.
-          atomicOr(args.error, PHOTIC_DEVERR_EVAL_CAP);
-          if (o.status) o.status[pixel] = PHOTIC_PX_INVALID;
+      } else if (++guard > guard_cap) {
+        // Defensive cap: each nelmin call is bounded by kcount, so
+        // reaching this means a defect; flag it instead of spinning.
+        atomicOr(args.error, PHOTIC_DEVERR_EVAL_CAP);
+        if (item >= 0) rec[item * fp.n_hstarts + start_k].evals = -1;
+        else if (o.status) o.status[pixel] = PHOTIC_PX_INVALID;
+        has = false;
+      } else if (m.step_machine(y)) {
+        const T ynewlo = m.F(m.lo);
+        if (item >= 0) {
+          // a start on its own: its record, and the early exit for the
+          // pixel's later starts (model/samodel.c:2404)
+          StartRecord<P> &rc = rec[item * fp.n_hstarts + start_k];
+          rc.y = ynewlo;
+          rc.evals = m.icount;
+          rc.fault = m.ifault;
+#pragma unroll
+          for (int i = 0; i < kN; i++) rc.x[i] = m.xmin[i];
+          if (P::lt(ynewlo, P::from_double(args.early_exit)) && P::lt(ynewlo, P::from_double(1.0e4)))
+            atomicMin(args.exit_k + item, start_k);
           has = false;
-        } else if (m.step_machine(y)) {
+        } else {
           // nelmin returned: keep the best start (model/samodel.c:2380-2405)
-          const T ynewlo = m.F(m.lo);
           total += m.icount;
           bool finish = false;
           if (P::lt(ynewlo, lowest)) {
@@ -396,19 +468,76 @@ __global__ void __launch_bounds__(BS) invert_kernel(const __grid_constant__ Inve
             m.phase = PH_FINAL;
           }
         }
+      } else if (item >= 0 && start_k > 0 && (guard & 63) == 0 &&
+                 __ldcg(args.exit_k + item) < start_k) {
+        has = false;  // an earlier start has ended the pixel
       }
     }
   }
 }
 
+// The n_par pixels after their starts have run: the records compared in the
+// order of the starts, as the sequential loop does (model/samodel.c:
+// 2380-2405), and the products at the kept optimum.
+template <class P, int NB>
+__global__ void __launch_bounds__(128) finish_kernel(const __grid_constant__ InvertArgs args) {
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= args.n_par || args.exit_k[i] < 0) return;
+  const FitParams &fp = args.fp;
+  const int64_t q = args.n_seq + i;
+  const int64_t p = args.order ? (int64_t)args.order[q] : q;
+  const bool seeded = args.seeds != nullptr && !isnan(args.seeds[p * kN]);
+  const int n_starts = seeded ? 1 : fp.n_hstarts;
+  const StartRecord<P> *rec = reinterpret_cast<const StartRecord<P> *>(args.records) +
+                              i * fp.n_hstarts;
+  typename P::T lowest = P::from_double(1.0e4), x[kN];
+#pragma unroll
+  for (int c = 0; c < kN; c++) x[c] = P::zero();
+  int32_t total = 0, kept_evals = 0, kept_start = 0, kept_fault = 0;
+  for (int k = 0; k < n_starts; k++) {
+    if (rec[k].evals < 0) {
+      if (args.out.status) args.out.status[p] = PHOTIC_PX_INVALID;
+      return;
+    }
+    total += rec[k].evals;
+    if (P::lt(rec[k].y, lowest)) {
+      lowest = rec[k].y;
+#pragma unroll
+      for (int c = 0; c < kN; c++) x[c] = rec[k].x[c];
+      kept_evals = rec[k].evals;
+      kept_start = k;
+      kept_fault = rec[k].fault;
+      if (P::lt(lowest, P::from_double(args.early_exit))) break;
+    }
+  }
+  float r[NB];
+  load_spectrum<NB>(args, p, r);
+  typename P::template Pixel<NB> px;
+  P::template setup<NB>(args, r, px);
+  typename P::Details det;
+  if constexpr (P::kFused) {
+    typename P::template Keep<NB> keep;
+    keep.want = true;
+    const typename P::T y = P::template cost_keep<NB>(args, px, x, keep);
+    P::template details_from_keep<NB>(args, keep, y, det);
+  } else {
+    P::template details<NB>(args, px, x, det);
+  }
+  write_fit<P, NB>(args.out, p, x, det, total, kept_evals, kept_start, kept_fault);
+}
+
 template <class P, int NB, int BS>
 cudaError_t launch_one(const InvertArgs &a, int grid, cudaStream_t s, int *occupancy) {
-  const size_t smem = invert_smem_bytes(BS, NB) + (size_t)BS * sizeof(typename P::template Pixel<NB>);
+  const size_t smem =
+      invert_smem_bytes(BS) + (size_t)BS * sizeof(typename P::template Pixel<NB>);
   auto k = invert_kernel<P, NB, BS>;
   cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   if (occupancy) return cudaOccupancyMaxActiveBlocksPerMultiprocessor(occupancy, k, BS, smem);
+  static_assert(sizeof(StartRecord<P>) == kStartRecordBytes, "record size");
   k<<<grid, BS, smem, s>>>(a);
+  if (a.n_par > 0)
+    finish_kernel<P, NB><<<(unsigned)((a.n_par + 127) / 128), 128, 0, s>>>(a);
   return cudaGetLastError();
 }
 
@@ -429,12 +558,11 @@ cudaError_t launch_prec(const InvertArgs &a, int block, int grid, cudaStream_t s
 
 }  // namespace
 
-// Shared memory of the simplex and the staged spectra; launch_one adds the
+// Shared memory of the simplex and the staged positions; launch_one adds the
 // chunk's pixel set-ups, whose size depends on the precision policy.
-size_t invert_smem_bytes(int block, int nb) {
+size_t invert_smem_bytes(int block) {
   // double and double-float both take 8 bytes per value
-  return (size_t)block * 8 * ((kN + 1) * kN + (kN + 1) + kN) +
-         (size_t)(block / 32) * 32 * (nb <= 4 ? 4 : 8) * sizeof(float);
+  return (size_t)block * 8 * ((kN + 1) * kN + (kN + 1) + kN + 1);
 }
 
 cudaError_t launch_invert(const InvertArgs &a, int precision, int block, int grid,

@@ -35,9 +35,16 @@ struct InvertArgs {
   double early_exit;  // early-exit cost threshold (per-scene value * scenes)
   int32_t no_mask;    // fit every pixel: samodel_optimise has no mask test
   const int32_t *order;  // optional queue position -> pixel (e.g. long fits first)
+  // the queue: n_seq pixels with their starts in sequence, then the starts of
+  // the other n_par pixels one by one (photic_invert.cu)
+  int64_t n_seq, n_par;
+  void *records;         // [n_par][n_hstarts] results of the starts
+  int32_t *exit_k;       // [n_par] first start known to meet the early exit, -1 masked
+  int32_t claim;         // positions a warp claims at a time (1..32)
 };
 
-size_t invert_smem_bytes(int block, int nb);
+constexpr size_t kStartRecordBytes = 64;
+size_t invert_smem_bytes(int block);
 cudaError_t launch_invert(const InvertArgs &a, int precision, int block, int grid,
                           cudaStream_t s);
 // Resident blocks per SM of the kernel that launch_invert would use (0 on error).
