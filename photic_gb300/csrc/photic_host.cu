@@ -305,6 +305,15 @@ void invert_shape(const InvertArgs &a, int precision, int sms, int64_t positions
 // run start by start, the ones before them with their starts in sequence.
 constexpr int64_t kRecordBytesMax = 1ll << 30;
 
+// The records of `slots` pixels' starts in mem: none completed, no exit met.
+cudaError_t start_work_init(StartWork &w, unsigned char *mem, int64_t slots, int n_starts,
+                            int x_stride, cudaStream_t s) {
+  start_work_layout(w, mem, slots, n_starts, x_stride);
+  cudaError_t e = cudaMemsetAsync(w.done, 0, (size_t)slots * sizeof *w.done, s);
+  if (e == cudaSuccess) e = cudaMemsetAsync(w.exit_k, 0x7f, (size_t)slots * sizeof *w.exit_k, s);
+  return e;
+}
+
 // The batched inversion of prepared arguments: workspace (queue head, exits,
 // records), launch shape, launches.
 int run_invert(InvertArgs &a, int precision, int block, int per_sm, int sms, cudaStream_t s) {
@@ -674,19 +683,32 @@ int photic_joint_invert_batch(const photic_config *cfg, const int32_t *d_offsets
   a.out = *out;
   a.error = err;
 
-  // workspace: counts, starts, fills (8 x i32 each), queues (8 x u64), list
-  const size_t head = 3 * 8 * sizeof(int32_t) + 8 * sizeof(unsigned long long);
-  const size_t bytes = head + (size_t)npix * sizeof(int32_t);
+  // workspace: queues (2 x 8 x u64), counts, starts, fills, counts of the rest
+  // (8 x i32 each), the list and the rest's,
+  // and the records of the depth starts run one by one (the lane-group
+  // kernels, up to four bands) while they fit
+  const size_t head = 4 * 8 * sizeof(int32_t) + 16 * sizeof(unsigned long long);
+  const int xs = cfg->layout == PHOTIC_LAYOUT_REFERENCE ? 3 + 3 * kMaxScenes : 1 + 4 * kMaxScenes;
+  size_t bytes = head + 2 * (size_t)npix * sizeof(int32_t);
+  const size_t off_sw = (bytes + 255) / 256 * 256;
+  const size_t sw_bytes = start_work_bytes(npix, a.fp.n_hstarts, xs);
+  a.by_start = cfg->n_bands <= 4 && a.fp.n_hstarts > 1 && sw_bytes <= (size_t)kRecordBytesMax;
+  if (a.by_start) bytes = off_sw + sw_bytes;
   unsigned char *ws = nullptr;
   cudaError_t e = cudaMallocAsync((void **)&ws, bytes, s);
   if (e != cudaSuccess) return fail(PHOTIC_ERR_NOMEM, "joint workspace: %s", cudaGetErrorString(e));
   e = cudaMemsetAsync(ws, 0, head, s);
+  if (e == cudaSuccess && a.by_start)
+    e = start_work_init(a.sw, ws + off_sw, npix, a.fp.n_hstarts, xs, s);
   if (e != cudaSuccess) return cuda_fail(e, "cudaMemsetAsync");
   a.queues = reinterpret_cast<unsigned long long *>(ws);
-  a.bin_count = reinterpret_cast<int32_t *>(ws + 8 * sizeof(unsigned long long));
+  a.rest_queues = a.queues + 8;
+  a.bin_count = reinterpret_cast<int32_t *>(a.queues + 16);
   a.bin_start = a.bin_count + 8;
   int32_t *fill = a.bin_count + 16;
+  a.rest_count = a.bin_count + 24;
   a.list = reinterpret_cast<int32_t *>(ws + head);
+  a.rest = a.list + npix;
   const int per_sm = cfg->blocks_per_sm;
   ForkSlot *fs = nullptr;
   rc = joint_fork(&fs);
@@ -1435,13 +1457,21 @@ int run_region(RegionArgs &a, int max_params, int per_sm, cudaStream_t s) {
   int rc = device_state(&err, &sms);
   if (rc) return rc;
   a.error = err;
-  unsigned long long *queue = nullptr;
-  cudaError_t e = cudaMallocAsync((void **)&queue, sizeof(unsigned long long), s);
+  const int n_starts = a.fp.n_hstarts;
+  const size_t per_pixel = start_work_bytes(1, n_starts, max_params);
+  a.n_par = a.eval_params || n_starts < 2 ? 0 : kRecordBytesMax / (int64_t)per_pixel;
+  if (a.n_par > a.npix) a.n_par = a.npix;
+  a.n_seq = a.npix - a.n_par;
+  const size_t off = 256;
+  unsigned char *ws = nullptr;
+  cudaError_t e = cudaMallocAsync(
+      (void **)&ws, off + (a.n_par ? start_work_bytes(a.n_par, n_starts, max_params) : 0), s);
   if (e != cudaSuccess) return fail(PHOTIC_ERR_NOMEM, "queue head");
-  cudaMemsetAsync(queue, 0, sizeof(unsigned long long), s);
-  a.queue = queue;
-  e = launch_region(a, max_params, sms, per_sm, s);
-  cudaFreeAsync(queue, s);
+  a.queue = reinterpret_cast<unsigned long long *>(ws);
+  e = cudaMemsetAsync(ws, 0, off, s);
+  if (e == cudaSuccess && a.n_par > 0) e = start_work_init(a.sw, ws + off, a.n_par, n_starts, max_params, s);
+  if (e == cudaSuccess) e = launch_region(a, max_params, sms, per_sm, s);
+  cudaFreeAsync(ws, s);
   if (e != cudaSuccess) return cuda_fail(e, "region launch");
   return PHOTIC_OK;
 }

@@ -31,6 +31,7 @@
 #include "photic_kernels.h"
 #include "photic_nm.cuh"
 #include "photic_nmgroup.cuh"
+#include "photic_starts.cuh"
 
 namespace photic {
 
@@ -81,7 +82,7 @@ __device__ __forceinline__ void scene_shape(const JointArgs &a, int64_t o0, int 
 // Cold start (model/samodel.c:2249-2353) for the lane's own coordinates;
 // depth from hs.
 template <int LAYOUT, int K, int N, int C, int G>
-__device__ __forceinline__ void group_cold(const JointArgs &a, int64_t o0, int gl, double hs,
+__device__ __noinline__ void group_cold(const JointArgs &a, int64_t o0, int gl, double hs,
                                            double (&start)[C], double (&step)[C]) {
   const double c5 = 100.0 * 30.0 * a.fp.aw640;
 #pragma unroll
@@ -112,7 +113,7 @@ __device__ __forceinline__ void group_cold(const JointArgs &a, int64_t o0, int g
       } else {
         const int s = (i - 3) / 3, r = (i - 3) % 3;
         scene_shape(a, o0, s, r490, r550, r640);
-        const double P = 100.0 * 0.072 * pow(r490 / r550, -1.7);
+        const double P = 100.0 * 0.072 * pow_call(r490 / r550, -1.7);
         st = r == 0 ? P : r == 1 ? 1.5 * P : c5 * r640;
         sp = 2.0 * st;
       }
@@ -123,7 +124,7 @@ __device__ __forceinline__ void group_cold(const JointArgs &a, int64_t o0, int g
         st = 100.0 * 4.0 * r490;
         sp = 1.5 * st;
       } else {
-        const double P = 100.0 * 0.072 * pow(r490 / r550, -1.7);
+        const double P = 100.0 * 0.072 * pow_call(r490 / r550, -1.7);
         st = r == 1 ? P : r == 2 ? 1.5 * P : c5 * r640;
         sp = 2.0 * st;
       }
@@ -143,7 +144,8 @@ __global__ void __launch_bounds__(kBlock) joint_group_kernel(const __grid_consta
   const photic_outputs &o = a.out;
   const int nb = fp.n_bands;
   const int bin = K - 1;
-  const int32_t count = a.bin_count[bin];
+  const bool rest = a.by_start == 2;
+  const int32_t count = rest ? a.rest_count[bin] : a.bin_count[bin];
   const int32_t first = a.bin_start[bin];
 
   const int gid = threadIdx.x / G, gl = threadIdx.x % G;
@@ -180,7 +182,11 @@ __global__ void __launch_bounds__(kBlock) joint_group_kernel(const __grid_consta
   const int32_t guard_cap = (fp.n_hstarts + 1) * (fp.kcount + 8 * N + 16);
 
   bool has = false, exhausted = false, final_eval = false;
-  int64_t p = 0, o0 = 0;
+  int64_t p = 0, o0 = 0, slot = 0;
+  // the start of a queue position that is one, else -1
+  int item_k = a.by_start ? 0 : -1;
+  const unsigned long long tickets =
+      (unsigned long long)count * (unsigned long long)(rest ? fp.n_hstarts - 1 : 1);
   int32_t kst = 0, total = 0, kept_evals = 0, kept_start = 0, kept_fault = 0, guard = 0;
   double lowest = 0.0, mean = 0.0;
   double best[C];
@@ -189,20 +195,31 @@ __global__ void __launch_bounds__(kBlock) joint_group_kernel(const __grid_consta
   double my_rrs = 0.0, my_pw = 0.0, my_sec = 0.0;
 
   for (;;) {
-    // ---- refill: a group without a pixel takes the next one of its bin
-    unsigned long long tk = ~0ull;
-    if (!has && !exhausted && gl == 0) tk = atomicAdd(&a.queues[bin], 1ull);
-    tk = __shfl_sync(kFull, tk, 0, G);
+    // ---- refill: a group without a pixel takes the next one of its bin, or
+    // the next depth start that its pixel still wants
     bool fresh = false;
-    if (!has && !exhausted) {
-      if (tk < (unsigned long long)count) {
-        p = a.list[first + (int64_t)tk];
-        o0 = a.offsets[p];
-        fresh = true;
-      } else {
-        exhausted = true;
+    do {
+      unsigned long long tk = ~0ull;
+      const bool ask = !has && !exhausted && !fresh;
+      if (ask && gl == 0) tk = atomicAdd(rest ? &a.rest_queues[bin] : &a.queues[bin], 1ull);
+      tk = __shfl_sync(kFull, tk, 0, G);
+      if (ask) {
+        if (tk < tickets) {
+          if (rest) {
+            item_k = 1 + (int)(tk / (unsigned long long)count);
+            slot = a.rest[first + (int64_t)(tk % (unsigned long long)count)];
+            fresh = start_wanted(a.sw, slot, item_k);
+          } else {
+            slot = first + (int64_t)tk;
+            fresh = true;
+          }
+          p = a.list[slot];
+          o0 = a.offsets[p];
+        } else {
+          exhausted = true;
+        }
       }
-    }
+    } while (__any_sync(kFull, !has && !exhausted && !fresh));
     if (__all_sync(kFull, !has && !fresh)) break;
 
     // ---- set-up of fresh pixels: per-band inputs, per-scene shape
@@ -225,7 +242,7 @@ __global__ void __launch_bounds__(kBlock) joint_group_kernel(const __grid_consta
       double Y = 3.44 * (1.0 - 3.17 * fm::exp_t(-2.01 * chi));
       if (Y < 0.0) Y = 0.0;
       if (Y > 2.5) Y = 2.5;
-      my_pw = pow(sc.ratio440[bb], Y);
+      my_pw = pow_call(sc.ratio440[bb], Y);
       double th = a.theta_sun[o0 + bs];
       th *= 3.141592653589793 / 180.0;
       my_sec = 1.0 / cos(th);
@@ -242,7 +259,7 @@ __global__ void __launch_bounds__(kBlock) joint_group_kernel(const __grid_consta
     mtot = __shfl_sync(kFull, mtot, 0, G);
     if (fresh) {
       if (masked) {
-        if (gl == 0) {
+        if (gl == 0 && item_k <= 0) {
           if (o.depth) o.depth[p] = 0.0f;
           if (o.depth_f64) o.depth_f64[p] = 0.0;
           if (o.bottom_albedo) o.bottom_albedo[p] = 0.0f;
@@ -254,7 +271,7 @@ __global__ void __launch_bounds__(kBlock) joint_group_kernel(const __grid_consta
           if (o.evals_kept) o.evals_kept[p] = 0;
           if (o.status) o.status[p] = PHOTIC_PX_MASKED;
         }
-        if (band_lane && bb == 0) {
+        if (band_lane && bb == 0 && item_k <= 0) {
           if (o.P) o.P[o0 + bs] = 0.0f;
           if (o.G) o.G[o0 + bs] = 0.0f;
           if (o.X) o.X[o0 + bs] = 0.0f;
@@ -267,8 +284,8 @@ __global__ void __launch_bounds__(kBlock) joint_group_kernel(const __grid_consta
         final_eval = false;
 #pragma unroll
         for (int t = 0; t < C; t++) best[t] = 0.0;
-        kst = 0;
-        group_cold<LAYOUT, K, N, C, G>(a, o0, gl, fp.hstarts[0], m.start, m.step);
+        kst = item_k > 0 ? item_k : 0;
+        group_cold<LAYOUT, K, N, C, G>(a, o0, gl, fp.hstarts[kst], m.start, m.step);
         m.begin(var_limit, fp.konvge, fp.kcount);
       }
     }
@@ -334,7 +351,7 @@ __global__ void __launch_bounds__(kBlock) joint_group_kernel(const __grid_consta
         Ke = Ke + 100.0 * (dk * dk);
       }
       double model = 80.0 * E + 15.0 * Ke;
-      model = fm::div_by(model, 120.0, fm::kInv120);
+      model = fm::div_120(model);
       y = model;
       if (final_eval) {
         double qB;
@@ -381,37 +398,77 @@ __global__ void __launch_bounds__(kBlock) joint_group_kernel(const __grid_consta
       final_eval = false;
     } else if (has) {
       // ---- Nelder-Mead: consume y, stage the next point
-      if (++guard > guard_cap) {
-        // each nelmin call is bounded by kcount; reaching this is a defect
-        if (gl == 0) {
-          atomicOr(a.error, PHOTIC_DEVERR_EVAL_CAP);
-          if (o.status) o.status[p] = PHOTIC_PX_INVALID;
-        }
+      const bool capped = ++guard > guard_cap;
+      // each nelmin call is bounded by kcount; reaching the cap is a defect
+      if (capped && gl == 0) atomicOr(a.error, PHOTIC_DEVERR_EVAL_CAP);
+      if (capped && item_k < 0) {
+        if (gl == 0 && o.status) o.status[p] = PHOTIC_PX_INVALID;
         has = false;
-      } else if (m.step_machine(y)) {
-        // nelmin returned: keep the best start (model/samodel.c:2380-2405)
+      } else if (item_k > 0 && (guard & 63) == 0 && !start_wanted(a.sw, slot, item_k)) {
+        has = false;  // an earlier start has ended the pixel
+      } else if (capped || m.step_machine(y)) {
         const double ynewlo = m.F(m.lo);
+        if (item_k >= 0) {
+          // a start on its own: its record; the group that completes the
+          // pixel's starts compares them and evaluates the kept optimum
+          const int64_t it = slot * fp.n_hstarts + item_k;
+#pragma unroll
+          for (int t = 0; t < C; t++)
+            if (m.own(t)) a.sw.x[it * a.sw.x_stride + m.coord(t)] = m.xmin[t];
+          if (gl == 0) {
+            a.sw.y[it] = ynewlo;
+            a.sw.evals[it] = capped ? -1 : m.icount;
+            a.sw.fault[it] = m.ifault;
+          }
+          __threadfence();
+          __syncwarp(gmask);
+          int mine = 0;
+          if (gl == 0) mine = start_done(a.sw, slot, item_k, fp.n_hstarts, ynewlo, early);
+          mine = __shfl_sync(gmask, mine, 0, G);
+          has = false;
+          if (!rest && !mine && gl == 0)  // the pixel's other starts run in the next launch
+            a.rest[first + atomicAdd(a.rest_count + bin, 1)] = (int32_t)slot;
+          if (mine) {
+            const StartChoice c = choose_start(a.sw, slot, fp.n_hstarts, early);
+            if (c.invalid) {
+              if (gl == 0 && o.status) o.status[p] = PHOTIC_PX_INVALID;
+            } else {
+              total = c.total;
+              kept_evals = c.kept_evals;
+              kept_start = c.kept_start < 0 ? 0 : c.kept_start;
+              kept_fault = c.kept_fault;
+              const double *bx = a.sw.x + (slot * fp.n_hstarts + kept_start) * a.sw.x_stride;
+#pragma unroll
+              for (int t = 0; t < C; t++) {
+                best[t] = 0.0;
+                if (c.kept_start >= 0 && m.own(t)) best[t] = __ldcg(bx + m.coord(t));
+              }
+              m.set_x_from(best);  // re-evaluate at the kept optimum (:2413)
+              final_eval = true;
+              has = true;
+            }
+          }
+        } else {
+        // nelmin returned: keep the best start (model/samodel.c:2380-2405)
         total += m.icount;
         bool finish = false;
-        if (ynewlo < lowest) {
+        if (sf::lt(ynewlo, lowest)) {
           lowest = ynewlo;
 #pragma unroll
           for (int t = 0; t < C; t++) best[t] = m.xmin[t];
           kept_evals = m.icount;
           kept_start = kst;
           kept_fault = m.ifault;
-          if (lowest < early) finish = true;  // model/samodel.c:2404
+          if (sf::lt(lowest, early)) finish = true;  // model/samodel.c:2404
         }
         kst++;
         if (finish || kst >= fp.n_hstarts) {
           m.set_x_from(best);  // re-evaluate at the kept optimum (:2413)
           final_eval = true;
         } else {
-          double h = fp.hstarts[0];
-          for (int i = 1; i < kMaxHStarts; i++)
-            if (i == kst) h = fp.hstarts[i];
-          group_cold<LAYOUT, K, N, C, G>(a, o0, gl, h, m.start, m.step);
+          group_cold<LAYOUT, K, N, C, G>(a, o0, gl, fp.hstarts[kst], m.start, m.step);
           m.begin(var_limit, fp.konvge, fp.kcount);
+        }
         }
       }
     }
@@ -433,6 +490,11 @@ cudaError_t launch_group_k(const JointArgs &a, int per_sm, int sms, cudaStream_t
   if (occ < 1) return cudaErrorInvalidConfiguration;
   const int use = per_sm > 0 && per_sm < occ ? per_sm : occ;
   joint_group_kernel<LAYOUT, K><<<sms * use, kBlock, bytes, s>>>(a);
+  if (a.by_start) {
+    JointArgs b = a;
+    b.by_start = 2;
+    joint_group_kernel<LAYOUT, K><<<sms * use, kBlock, bytes, s>>>(b);
+  }
   return cudaGetLastError();
 }
 

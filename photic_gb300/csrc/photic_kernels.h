@@ -43,6 +43,32 @@ struct InvertArgs {
   int32_t claim;         // positions a warp claims at a time (1..32)
 };
 
+// Records of depth starts run as work items (photic_starts.cuh): item
+// slot * n_starts + k is start k of the pixel in `slot`.
+struct StartWork {
+  double *y;                  // [items] cost reached
+  double *x;                  // [items][x_stride] minimiser
+  int32_t *evals, *fault;     // [items] (evals -1: the defensive cap)
+  int32_t *exit_k;            // [slots] first start known to meet the early exit
+  unsigned long long *done;   // [slots] starts completed; bit 63: being compared
+  int32_t x_stride;
+};
+// Bytes of the arrays of `slots` pixels, and their addresses within `mem`.
+inline size_t start_work_bytes(int64_t slots, int n_starts, int x_stride) {
+  return (size_t)slots * ((size_t)n_starts * (16 + 8 * (size_t)x_stride) + 16) + 256;
+}
+inline void start_work_layout(StartWork &w, unsigned char *mem, int64_t slots, int n_starts,
+                              int x_stride) {
+  const int64_t items = slots * n_starts;
+  w.x_stride = x_stride;
+  w.done = reinterpret_cast<unsigned long long *>(mem);
+  w.y = reinterpret_cast<double *>(w.done + slots);
+  w.x = w.y + items;
+  w.evals = reinterpret_cast<int32_t *>(w.x + items * x_stride);
+  w.fault = w.evals + items;
+  w.exit_k = w.fault + items;
+}
+
 constexpr size_t kStartRecordBytes = 64;
 size_t invert_smem_bytes(int block);
 cudaError_t launch_invert(const InvertArgs &a, int precision, int block, int grid,
@@ -127,6 +153,14 @@ struct JointArgs {
   unsigned long long *queues; // [8] work-queue heads
   photic_outputs out;
   unsigned int *error;
+  // depth starts as queue positions (photic_starts.cuh; the slots are
+  // positions of the list): 0 no, 1 this launch runs first starts, 2 the
+  // other starts of the pixels that the first did not end
+  int32_t by_start;
+  StartWork sw;
+  int32_t *rest;              // [npix] per bin, from bin_start: slots left after start 0
+  int32_t *rest_count;        // [8]
+  unsigned long long *rest_queues;  // [8] their queue heads
 };
 // Bins pixels by scene count and runs one persistent kernel per count.
 // Streams and events for running the per-k joint kernels side by side.
@@ -293,6 +327,10 @@ struct RegionArgs {
                                 // scene's K_min (the cost's), IOD, K_min over all
                                 // scenes (the post-fit product's)
   unsigned long long *queue;    // work-queue head (zeroed): pixels, or chains
+  // pixels beyond the first n_seq: one queue position per depth start
+  // (photic_starts.cuh); n_par = 0 in the chain and evaluation modes
+  int64_t n_seq, n_par;
+  StartWork sw;
   photic_outputs out;           // per pixel (P, G, X: [npix][n_scenes]); status carries
                                 // the region count << 24
   unsigned int *error;

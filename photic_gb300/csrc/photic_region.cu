@@ -34,6 +34,7 @@
 #include "photic_fp64.cuh"
 #include "photic_kernels.h"
 #include "photic_nmgroup.cuh"
+#include "photic_starts.cuh"
 
 namespace photic {
 
@@ -333,7 +334,8 @@ __global__ void __launch_bounds__(BLOCK, 1) region_kernel(const __grid_constant_
   }
 
   for (;;) {
-    int64_t p = 0;
+    int64_t p = 0, slot = 0;  // slot: of the pixel's records
+    int item_k = -1;          // the start of a position that is one, else -1
     int64_t rp[kMaxR];
     int origin = 0, R = 0;
     bool hot = false;
@@ -443,8 +445,14 @@ __global__ void __launch_bounds__(BLOCK, 1) region_kernel(const __grid_constant_
       unsigned long long t = 0;
       if (lane == 0) t = atomicAdd(a.queue, 1ull);
       t = __shfl_sync(kFull, t, 0);
-      if (t >= (unsigned long long)a.npix) break;
+      if (t >= (unsigned long long)(a.n_seq + a.n_par * fp.n_hstarts)) break;
       p = (int64_t)t;
+      if (p >= a.n_seq) {
+        item_k = (int)((p - a.n_seq) / a.n_par);
+        slot = (p - a.n_seq) % a.n_par;
+        p = a.n_seq + slot;
+        if (item_k > 0 && !start_wanted(a.sw, slot, item_k)) continue;
+      }
 
       // the pixel loop's mask test on the centre, every scene
       // (model/samodel.c:933-947); samodel_optimise called directly has none
@@ -458,12 +466,16 @@ __global__ void __launch_bounds__(BLOCK, 1) region_kernel(const __grid_constant_
             if (nodata_value(v, fp.nodata) || v < 0.0f) masked = true;
           }
         if (masked) {
-          if (lane == 0) write_masked(o, p, S, PHOTIC_PX_MASKED);
+          if (lane == 0 && item_k <= 0) write_masked(o, p, S, PHOTIC_PX_MASKED);
           continue;
         }
       }
       R = regions_of(a, p, rp, origin);
       if (a.h_emp) hemp = hbot = a.h_emp[p];
+      if (item_k >= 0 && !isnan(hemp)) {  // a single start
+        if (item_k > 0) continue;
+        item_k = -1;
+      }
     }
 
     // ---- set-up: bottom types, per-term inputs
@@ -474,7 +486,7 @@ __global__ void __launch_bounds__(BLOCK, 1) region_kernel(const __grid_constant_
     if (R < 1 && a.list_R) {
       // a problem without regions (md->n_regions == 0: the reference's
       // loops skip it, model/samodel.c:951-953, 1428-1430)
-      if (lane == 0) write_masked(o, p, S, PHOTIC_PX_MASKED);
+      if (lane == 0 && item_k <= 0) write_masked(o, p, S, PHOTIC_PX_MASKED);
       __syncwarp();
       continue;
     }
@@ -591,7 +603,8 @@ __global__ void __launch_bounds__(BLOCK, 1) region_kernel(const __grid_constant_
 #pragma unroll 1
       for (int c = lane; c < N; c += 32) X[c] = a.eval_params[p * a.eval_stride + c];
     } else {
-      cold(isnan(hemp) ? fp.hstarts[0] : hemp);
+      if (item_k > 0) kst = item_k;
+      cold(isnan(hemp) ? fp.hstarts[kst] : hemp);
       m.begin(var_limit, fp.konvge, fp.kcount);
     }
 
@@ -854,26 +867,61 @@ __global__ void __launch_bounds__(BLOCK, 1) region_kernel(const __grid_constant_
         fitted = true;
         break;
       }
-      if (++guard > guard_cap) {
-        if (lane == 0) {
-          atomicOr(a.error, PHOTIC_DEVERR_EVAL_CAP);
-          if (o.status) o.status[p] = PHOTIC_PX_INVALID;
-        }
+      const bool capped = ++guard > guard_cap;
+      if (capped && lane == 0) atomicOr(a.error, PHOTIC_DEVERR_EVAL_CAP);
+      if (capped && item_k < 0) {
+        if (lane == 0 && o.status) o.status[p] = PHOTIC_PX_INVALID;
         break;
       }
-      if (m.step_machine(y)) {
+      if (item_k > 0 && (guard & 63) == 0 && !start_wanted(a.sw, slot, item_k)) break;
+      if (capped || m.step_machine(y)) {
         // nelmin returned: keep the best start (model/samodel.c:2380-2405)
         const double ynewlo = m.F(m.lo);
+        if (item_k >= 0) {
+          // a start on its own: its record; the warp that completes the
+          // pixel's starts compares them and evaluates the kept optimum
+          const int64_t it = slot * n_starts + item_k;
+#pragma unroll
+          for (int tt = 0; tt < C; tt++)
+            if (m.own(tt)) a.sw.x[it * a.sw.x_stride + m.coord(tt)] = m.xmin[tt];
+          if (lane == 0) {
+            a.sw.y[it] = capped ? kNaN : ynewlo;
+            a.sw.evals[it] = capped ? -1 : m.icount;
+            a.sw.fault[it] = m.ifault;
+          }
+          __threadfence();
+          __syncwarp();
+          int mine = 0;
+          if (lane == 0)
+            mine = start_done(a.sw, slot, item_k, n_starts, capped ? kNaN : ynewlo, early);
+          mine = __shfl_sync(kFull, mine, 0);
+          if (!mine) break;
+          const StartChoice c = choose_start(a.sw, slot, n_starts, early);
+          if (c.invalid) {
+            if (lane == 0 && o.status) o.status[p] = PHOTIC_PX_INVALID;
+            break;
+          }
+          total = c.total;
+          kept_evals = c.kept_evals;
+          kept_start = c.kept_start < 0 ? 0 : c.kept_start;
+          kept_fault = c.kept_fault;
+          const double *bx = a.sw.x + (slot * n_starts + kept_start) * a.sw.x_stride;
+#pragma unroll
+          for (int tt = 0; tt < C; tt++)
+            if (m.own(tt)) X[m.coord(tt)] = c.kept_start < 0 ? 0.0 : __ldcg(bx + m.coord(tt));
+          final_eval = true;
+          continue;
+        }
         total += m.icount;
         bool finish = false;
-        if (ynewlo < lowest) {
+        if (sf::lt(ynewlo, lowest)) {
           lowest = ynewlo;
 #pragma unroll
           for (int tt = 0; tt < C; tt++) best[tt] = m.xmin[tt];
           kept_evals = m.icount;
           kept_start = kst;
           kept_fault = m.ifault;
-          if (lowest < early) finish = true;  // model/samodel.c:2404
+          if (sf::lt(lowest, early)) finish = true;  // model/samodel.c:2404
         }
         kst++;
         if (finish || kst >= n_starts) {
@@ -958,7 +1006,8 @@ cudaError_t launch_shape(const RegionArgs &a, int sms, int per_sm, cudaStream_t 
     *warps = grid * (BLOCK / 32);
     return cudaSuccess;
   }
-  const int64_t units = a.order ? a.n_chains : a.npix;  // chains, or pixels
+  // chains, or queue positions
+  const int64_t units = a.order ? a.n_chains : a.n_seq + a.n_par * a.fp.n_hstarts;
   const int64_t need = (units + BLOCK / 32 - 1) / (BLOCK / 32);
   if (grid > need) grid = need;
   k<<<(int)grid, BLOCK, bytes, s>>>(a);
