@@ -166,7 +166,9 @@ static __device__ PHOTIC_NOINLINE void band_term_general(const SceneConsts &sc, 
 // X, pw and ln P are, the band's constants' bit in sc.near_mask that those
 // are, and the tests below cover the intermediates; a term that fails one
 // (an exact zero, an absurd exponent, NaN) is evaluated again above.
+// `want_B`: t.rrs_B is used, not only t.rrs.
 __device__ __forceinline__ void band_term(const SceneConsts &sc, int b, double sec_sun, bool near_x,
+                                          bool want_B,
                                           double H, double rho, double P, double lnP, double G,
                                           double X, double pw, double r, BandTerm &t) {
   const double c = sc.a0[b] + sf::mul_mid(sc.a1[b], lnP);
@@ -185,12 +187,20 @@ __device__ __forceinline__ void band_term(const SceneConsts &sc, int b, double s
     DuB = sf::mul_mid(DuB, sc.sec_view);
   }
   const double MC = sec_sun + DuC, MB = sec_sun + DuB;
-  const double xC = -sf::mul_mid(sf::mul_mid(MC, K), H);
-  const double xB = -sf::mul_mid(sf::mul_mid(MB, K), H);
-  const double eC = fm::exp_t(xC), eB = fm::exp_t(xB);
+  // Beyond 200 optical depths the exponentials change no bit of the sums
+  // below (the columns' part is 1 - 0, the bottom's share is lost in rrs):
+  // -200 stands for every such depth, unless the bottom's part itself is
+  // asked for.  (One lane in eight warps was that deep, and took its warp
+  // through the general term.)
+  double dC = sf::mul_mid(sf::mul_mid(MC, K), H), dB = sf::mul_mid(sf::mul_mid(MB, K), H);
+  const bool deepC = fm::bits(dC) > 0x4069000000000000LL, deepB = fm::bits(dB) > 0x4069000000000000LL;
+  const double xC = deepC ? -200.0 : -dC, xB = deepB ? -200.0 : -dB;
+  bool ok = near_x && ((sc.near_mask >> b) & 1) && !(deepB && want_B);
+  const double eC = sf::exp_neg(xC, ok), eB = sf::exp_neg(xB, ok);
   const double oC = 1.0 - eC;
   const double rrs_C = sf::mul_mid(rrs_dp, oC);
-  const double rrs_B = sf::mul_mid(fma(rho, fm::kPiHi, rho * fm::kPiLo), eB);
+  const double rho_pi = fma(rho, fm::kPiHi, rho * fm::kPiLo);
+  const double rrs_B = sf::mul_mid(rho_pi, eB);
   const double rrs = rrs_C + rrs_B;
   const double den = 1.0 - sf::mul_mid(1.5, rrs);
   const double Rm = sf::div_mid(sf::half_mid(rrs), den);
@@ -200,9 +210,11 @@ __device__ __forceinline__ void band_term(const SceneConsts &sc, int b, double s
   t.rrs = rrs;
   t.Rm = Rm;
   t.dd = sf::mul_mid(d, d);
-  const bool ok = near_x && ((sc.near_mask >> b) & 1) && sf::near(c) && sf::near_positive(ab) &&
-                  sf::near_positive(u) && sf::near_positive(MC) && sf::near_positive(MB) &&
-                  sf::near_positive(oC) && sf::mid_positive(eB) && sf::near_positive(rrs) && sf::near(den) && sf::near(d);
+  ok = ok && sf::near(c) && sf::near_positive(ab) && sf::near_positive(u) &&
+       sf::near_positive(MC) && sf::near_positive(MB) && sf::near_positive(oC) &&
+       sf::near_positive(rrs) && sf::near(den) && sf::near(d);
+  // (deep: rrs_B at most 2^90 2^-288, below half an ulp of rrs above 2^-90)
+  if (deepB) ok = ok && sf::lt(rho_pi, 0x1p90) && sf::lt(0x1p-90, rrs);
   if (!ok) {
     BandTerm g;
     band_term_general(sc, b, sec_sun, H, rho, P, lnP, G, X, pw, r, &g);
@@ -253,8 +265,10 @@ __device__ __forceinline__ double cost_f64(const FitParams &fp, const SceneConst
 #pragma unroll 1
   for (int b = 0; b < nb; b++) {
     BandTerm t;
-    band_term(sc, b, sc.sec_sun, near_x && sf::near_positive(px.pw[b]), H, qB * sc.refl[b], P, lnP,
-              G, X, px.pw[b], px.rrs[b], t);
+    bool want_B = kDetails;
+    if constexpr (kKeep) want_B = keep->want;
+    band_term(sc, b, sc.sec_sun, near_x && sf::near_positive(px.pw[b]), want_B, H,
+              qB * sc.refl[b], P, lnP, G, X, px.pw[b], px.rrs[b], t);
     err = err + t.dd;
     if (k_counts(t.K) && sf::lt(t.K, K_min)) K_min = t.K;
     if (kDetails) {

@@ -158,6 +158,8 @@ struct PrecDF {
   static __device__ __forceinline__ T mul2(T a) { return df64{2.0f * a.hi, 2.0f * a.lo}; }
   static __device__ __forceinline__ T half(T a) { return df64{0.5f * a.hi, 0.5f * a.lo}; }
   static __device__ __forceinline__ T scale2(T a, float c) { return df64{c * a.hi, c * a.lo}; }
+  static __device__ __forceinline__ T add_scaled2(T a, T b, float c) { return add(a, scale2(b, c)); }
+  static __device__ __forceinline__ bool sum_less_one(const T *, int, int, int, T &) { return false; }
   static __device__ __forceinline__ T div_n(T a, int n) { return df_div_f(a, (float)n); }
   static __device__ __forceinline__ bool lt(T a, T b) { return df_lt(a, b); }
   static __device__ __forceinline__ bool le(T a, T b) { return df_le(a, b); }
@@ -168,10 +170,7 @@ struct PrecDF {
   static __device__ __forceinline__ double to_double(T a) { return df_to_double(a); }
   static __device__ __forceinline__ T var_limit(const InvertArgs &a) { return dp(a.ds.reqmin_n); }
   static __device__ __forceinline__ T hstart(const InvertArgs &a, int k) {
-    DfPair h = a.ds.hstarts[0];
-    for (int i = 1; i < kMaxHStarts; i++)
-      if (i == k) h = a.ds.hstarts[i];
-    return dp(h);
+    return dp(a.ds.hstarts[k]);
   }
   static __device__ __forceinline__ T h_step(T h) { return df_mul_f(h, 1.25f); }
   template <int NB>
@@ -267,9 +266,8 @@ __global__ void __launch_bounds__(BS) invert_kernel(const __grid_constant__ Inve
   using T = typename P::T;
   const FitParams &fp = args.fp;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  T *sv = reinterpret_cast<T *>(smem_raw);          // [(N+1)*N][BS]
-  T *sf = sv + (kN + 1) * kN * BS;                  // [N+1][BS]
-  T *sbest = sf + (kN + 1) * BS;                    // [N][BS]
+  T *snm = reinterpret_cast<T *>(smem_raw);          // [NmPixel's slots][BS]
+  T *sbest = snm + NmPixel<P, BS>::kSlots * BS;      // [N][BS]
   using Px = typename P::template Pixel<NB>;
   Px *spx = reinterpret_cast<Px *>(sbest + kN * BS);  // [BS/32][32] set-ups of the chunk
   int64_t *spos = reinterpret_cast<int64_t *>(spx + BS);  // [BS/32][32] their positions
@@ -281,9 +279,9 @@ __global__ void __launch_bounds__(BS) invert_kernel(const __grid_constant__ Inve
   StartRecord<P> *const rec = reinterpret_cast<StartRecord<P> *>(args.records);
   const int64_t total_pos = args.n_seq + args.n_par * fp.n_hstarts;
 
-  NmLane<kN, P, BS> m;
-  m.v = sv + tid;
-  m.f = sf + tid;
+  NmPixel<P, BS> m;
+  m.w = snm + tid;
+  m.phase = PH_INIT_BASE;
   T *best = sbest + tid;
   Px px;
   const T var_limit = P::var_limit(args);
@@ -376,6 +374,7 @@ __global__ void __launch_bounds__(BS) invert_kernel(const __grid_constant__ Inve
         total = kept_evals = kept_start = kept_fault = guard = 0;
         lowest = P::from_double(1.0e4);
         bool seeded = false;
+        T start[kN], step[kN];
 #pragma unroll
         for (int i = 0; i < kN; i++) best[i * BS] = P::zero();
         if (args.seeds != nullptr) {
@@ -385,17 +384,18 @@ __global__ void __launch_bounds__(BS) invert_kernel(const __grid_constant__ Inve
             seeded = true;
 #pragma unroll
             for (int i = 0; i < kN; i++) {
-              m.start[i] = P::from_double(sd[i]);
-              m.step[i] = P::from_double((rel[i] * fp.seed_step_scale) * sd[i]);
+              start[i] = P::from_double(sd[i]);
+              step[i] = P::from_double((rel[i] * fp.seed_step_scale) * sd[i]);
             }
           }
         }
         n_starts = seeded ? 1 : fp.n_hstarts;
         if (!seeded) {
-          P::template cold_start<NB>(args, px, m.start, m.step);
-          m.start[0] = P::hstart(args, start_k);
-          m.step[0] = P::h_step(m.start[0]);
+          P::template cold_start<NB>(args, px, start, step);
+          start[0] = P::hstart(args, start_k);
+          step[0] = P::h_step(start[0]);
         }
+        m.set_start(start, step);
         m.begin(var_limit, fp.konvge, fp.kcount);
         has = true;
       }
@@ -408,19 +408,21 @@ __global__ void __launch_bounds__(BS) invert_kernel(const __grid_constant__ Inve
     if (has) {
       const bool fin = m.phase == PH_FINAL;
       typename P::Details det;
-      T y = P::zero();
+      T y = P::zero(), x[kN];
+#pragma unroll
+      for (int i = 0; i < kN; i++) x[i] = m.x(i);
       if constexpr (P::kFused) {
         // the kept optimum is evaluated together with the other lanes' points
         typename P::template Keep<NB> keep;
         keep.want = fin;
-        y = P::template cost_keep<NB>(args, px, m.x, keep);
+        y = P::template cost_keep<NB>(args, px, x, keep);
         if (fin) P::template details_from_keep<NB>(args, keep, y, det);
       } else {
-        if (fin) P::template details<NB>(args, px, m.x, det);
-        else y = P::template cost<NB>(args, px, m.x);
+        if (fin) P::template details<NB>(args, px, x, det);
+        else y = P::template cost<NB>(args, px, x);
       }
       if (fin) {
-        write_fit<P, NB>(o, pixel, m.x, det, total, kept_evals, kept_start, kept_fault);
+        write_fit<P, NB>(o, pixel, x, det, total, kept_evals, kept_start, kept_fault);
         has = false;
       } else if (++guard > guard_cap) {
         // Defensive cap: each nelmin call is bounded by kcount, so
@@ -439,7 +441,7 @@ __global__ void __launch_bounds__(BS) invert_kernel(const __grid_constant__ Inve
           rc.evals = m.icount;
           rc.fault = m.ifault;
 #pragma unroll
-          for (int i = 0; i < kN; i++) rc.x[i] = m.xmin[i];
+          for (int i = 0; i < kN; i++) rc.x[i] = m.x(i);
           if (P::lt(ynewlo, P::from_double(args.early_exit)) && P::lt(ynewlo, P::from_double(1.0e4)))
             atomicMin(args.exit_k + item, start_k);
           has = false;
@@ -450,7 +452,7 @@ __global__ void __launch_bounds__(BS) invert_kernel(const __grid_constant__ Inve
           if (P::lt(ynewlo, lowest)) {
             lowest = ynewlo;
 #pragma unroll
-            for (int i = 0; i < kN; i++) best[i * BS] = m.xmin[i];
+            for (int i = 0; i < kN; i++) best[i * BS] = m.x(i);
             kept_evals = m.icount;
             kept_start = start_k;
             kept_fault = m.ifault;
@@ -458,13 +460,15 @@ __global__ void __launch_bounds__(BS) invert_kernel(const __grid_constant__ Inve
           }
           start_k++;
           if (!finish && start_k < n_starts) {
-            P::template cold_start<NB>(args, px, m.start, m.step);
-            m.start[0] = P::hstart(args, start_k);
-            m.step[0] = P::h_step(m.start[0]);
+            T start[kN], step[kN];
+            P::template cold_start<NB>(args, px, start, step);
+            start[0] = P::hstart(args, start_k);
+            step[0] = P::h_step(start[0]);
+            m.set_start(start, step);
             m.begin(var_limit, fp.konvge, fp.kcount);
           } else {
 #pragma unroll
-            for (int i = 0; i < kN; i++) m.x[i] = best[i * BS];
+            for (int i = 0; i < kN; i++) m.x(i) = best[i * BS];
             m.phase = PH_FINAL;
           }
         }
@@ -562,7 +566,7 @@ cudaError_t launch_prec(const InvertArgs &a, int block, int grid, cudaStream_t s
 // chunk's pixel set-ups, whose size depends on the precision policy.
 size_t invert_smem_bytes(int block) {
   // double and double-float both take 8 bytes per value
-  return (size_t)block * 8 * ((kN + 1) * kN + (kN + 1) + kN + 1);
+  return (size_t)block * 8 * (NmPixel<PrecF64, 32>::kSlots + kN + 1);
 }
 
 cudaError_t launch_invert(const InvertArgs &a, int precision, int block, int grid,

@@ -311,7 +311,7 @@ __global__ void __launch_bounds__(kBlock) joint_group_kernel(const __grid_consta
                           sf::near_positive(Gg) && sf::near_positive(Xx) && sf::near(lnP) &&
                           sf::near_positive(my_pw);
       BandTerm t;
-      band_term(sc, bb, my_sec, near_x, H, qB * sc.refl[bb], P, lnP, Gg, Xx, my_pw, my_rrs, t);
+      band_term(sc, bb, my_sec, near_x, final_eval, H, qB * sc.refl[bb], P, lnP, Gg, Xx, my_pw, my_rrs, t);
       g.dd[gl] = t.dd;
       g.kk[gl] = t.K;
       if (final_eval) g.io[gl] = t.rrs_B / t.rrs;

@@ -223,7 +223,7 @@ struct ChainSmem {
 };
 
 size_t lut_smem_bytes() {
-  return sizeof(ChainSmem) + (size_t)kLutBlock * 8 * ((kN + 1) * kN + (kN + 1) + kN);
+  return sizeof(ChainSmem) + (size_t)kLutBlock * 8 * (NmPixel<P, kLutBlock>::kSlots + kN);
 }
 
 // Ring field k of chain c, slot j: ring[(c * 8 + k) * cap + j]
@@ -309,14 +309,13 @@ __global__ void __launch_bounds__(kLutBlock) lut_kernel(const __grid_constant__ 
   const FitParams &fp = ia.fp;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   ChainSmem &S = *reinterpret_cast<ChainSmem *>(smem_raw);
-  double *sv = reinterpret_cast<double *>(smem_raw + sizeof(ChainSmem));  // [(N+1)*N][BS]
-  double *sf = sv + (kN + 1) * kN * BS;                                     // [N+1][BS]
-  double *sbest = sf + (kN + 1) * BS;                                       // [N][BS]
+  double *snm = reinterpret_cast<double *>(smem_raw + sizeof(ChainSmem));  // NmPixel's slots
+  double *sbest = snm + NmPixel<P, BS>::kSlots * BS;                        // [N][BS]
 
   const int tid = threadIdx.x, lane = tid & 31, wbase = tid & ~31;
-  NmLane<kN, P, BS> m;
-  m.v = sv + tid;
-  m.f = sf + tid;
+  NmPixel<P, BS> m;
+  m.w = snm + tid;
+  m.phase = PH_INIT_BASE;
   double *best = sbest + tid;
   PixelF64<NB> px;
   const double var_limit = P::var_limit(ia);
@@ -479,7 +478,8 @@ __global__ void __launch_bounds__(kLutBlock) lut_kernel(const __grid_constant__ 
       start_k = 0;
 #pragma unroll
       for (int i = 0; i < kN; i++) best[i * BS] = 0.0;
-      P::template cold_start<NB>(ia, px, m.start, m.step);
+      double start[kN], step[kN];
+      P::template cold_start<NB>(ia, px, start, step);
       // the pixel's empirical depth (:955-979): its single start, hot
       // or cold; a pixel without one is fitted cold
       bool emp_present = false;
@@ -494,23 +494,24 @@ __global__ void __launch_bounds__(kLutBlock) lut_kernel(const __grid_constant__ 
       hot_fit = S.s[CS_HOT][tid] && (args.emp == nullptr || emp_present);
       if (hot_fit) {  // :2234-2241, 2285-2305
         const double h = emp_present ? h_emp : S.d[CD_DPREV][tid];
-        m.start[0] = h;
-        m.step[0] = P::h_step(h);
-        m.start[3] = S.d[CD_PREV0][tid];
-        m.start[4] = S.d[CD_PREV1][tid];
-        m.start[5] = S.d[CD_PREV2][tid];
+        start[0] = h;
+        step[0] = P::h_step(h);
+        start[3] = S.d[CD_PREV0][tid];
+        start[4] = S.d[CD_PREV1][tid];
+        start[5] = S.d[CD_PREV2][tid];
 #pragma unroll
-        for (int i = 3; i < 6; i++) m.step[i] = __dmul_rn(2.0, m.start[i]);
+        for (int i = 3; i < 6; i++) step[i] = __dmul_rn(2.0, start[i]);
         n_starts = 1;
       } else if (emp_present) {  // :2221-2223
-        m.start[0] = h_emp;
-        m.step[0] = P::h_step(h_emp);
+        start[0] = h_emp;
+        step[0] = P::h_step(h_emp);
         n_starts = 1;
       } else {
-        m.start[0] = P::hstart(ia, 0);
-        m.step[0] = P::h_step(m.start[0]);
+        start[0] = P::hstart(ia, 0);
+        step[0] = P::h_step(start[0]);
         n_starts = fp.n_hstarts;
       }
+      m.set_start(start, step);
       m.begin(var_limit, fp.konvge, fp.kcount);
       has = true;
     }
@@ -521,19 +522,22 @@ __global__ void __launch_bounds__(kLutBlock) lut_kernel(const __grid_constant__ 
       // one evaluation for every lane; at the kept optimum its kept band
       // values give the products (the final point is evaluated together
       // with the other lanes' trial points)
+      double x[kN];
+#pragma unroll
+      for (int i = 0; i < kN; i++) x[i] = m.x(i);
       BandKeep<NB> keep;
       keep.want = m.phase == PH_FINAL;
-      const double y = P::template cost_keep<NB>(ia, px, m.x, keep);
+      const double y = P::template cost_keep<NB>(ia, px, x, keep);
       if (m.phase == PH_FINAL) {
         typename P::Details det;
         P::template details_from_keep<NB>(ia, keep, y, det);
         const int64_t p = pixel;
-        const double H = fabs(m.x[0]);
+        const double H = fabs(x[0]);
         if (o.depth) o.depth[p] = (float)H;
         if (o.depth_f64) o.depth_f64[p] = H;
-        if (o.P) o.P[p] = (float)(0.01 * fabs(m.x[3]));
-        if (o.G) o.G[p] = (float)(0.01 * fabs(m.x[4]));
-        if (o.X) o.X[p] = (float)(0.01 * fabs(m.x[5]));
+        if (o.P) o.P[p] = (float)(0.01 * fabs(x[3]));
+        if (o.G) o.G[p] = (float)(0.01 * fabs(x[4]));
+        if (o.X) o.X[p] = (float)(0.01 * fabs(x[5]));
         if (o.bottom_albedo) o.bottom_albedo[p] = (float)det.bottom_albedo;
         if (o.model_error) o.model_error[p] = (float)det.model_error;
         if (o.rrs_error) o.rrs_error[p] = (float)det.rrs_error;
@@ -542,7 +546,7 @@ __global__ void __launch_bounds__(kLutBlock) lut_kernel(const __grid_constant__ 
         if (o.evals) o.evals[p] = total;
         if (o.evals_kept) o.evals_kept[p] = kept_evals;
         if (o.params)
-          for (int i = 0; i < kN; i++) o.params[p * kN + i] = m.x[i];
+          for (int i = 0; i < kN; i++) o.params[p * kN + i] = x[i];
         if (o.status)
           o.status[p] = PHOTIC_PX_FITTED | (kept_fault == 0 ? PHOTIC_PX_CONVERGED : 0) |
                         (hot_fit ? PHOTIC_PX_HOT : 0) | (kept_start << 16);
@@ -551,9 +555,9 @@ __global__ void __launch_bounds__(kLutBlock) lut_kernel(const __grid_constant__ 
         const double me = det.model_error;
         S.d[CD_DEPTH][tid] = H;
         S.d[CD_KMIN][tid] = det.K_min;
-        S.d[CD_PREV0][tid] = fabs(m.x[3]);
-        S.d[CD_PREV1][tid] = fabs(m.x[4]);
-        S.d[CD_PREV2][tid] = fabs(m.x[5]);
+        S.d[CD_PREV0][tid] = fabs(x[3]);
+        S.d[CD_PREV1][tid] = fabs(x[4]);
+        S.d[CD_PREV2][tid] = fabs(x[5]);
         S.s[CS_NOPT][tid]++;
         if (!((float)me == 0.0f)) {  // vec_mean2_double skips zeros
           S.d[CD_ERRTOT][tid] = __dadd_rn(S.d[CD_ERRTOT][tid], me);
@@ -569,9 +573,9 @@ __global__ void __launch_bounds__(kLutBlock) lut_kernel(const __grid_constant__ 
           R[RG_RM1 * cap + slot] = fp.n_bands > 1 ? keep.Rm[1] : 0.0;
           R[RG_RM2 * cap + slot] = fp.n_bands > 2 ? keep.Rm[2] : 0.0;
           R[RG_RM3 * cap + slot] = fp.n_bands > 3 ? keep.Rm[3] : 0.0;
-          R[RG_PREV0 * cap + slot] = fabs(m.x[3]);
-          R[RG_PREV1 * cap + slot] = fabs(m.x[4]);
-          R[RG_PREV2 * cap + slot] = fabs(m.x[5]);
+          R[RG_PREV0 * cap + slot] = fabs(x[3]);
+          R[RG_PREV1 * cap + slot] = fabs(x[4]);
+          R[RG_PREV2 * cap + slot] = fabs(x[5]);
           args.ring_src[(size_t)c * cap + slot] = p;
           S.i[CI_TOTLUT][tid] = tl + 1;
         }
@@ -594,7 +598,7 @@ __global__ void __launch_bounds__(kLutBlock) lut_kernel(const __grid_constant__ 
           if (ynewlo < lowest) {
             lowest = ynewlo;
 #pragma unroll
-            for (int i = 0; i < kN; i++) best[i * BS] = m.xmin[i];
+            for (int i = 0; i < kN; i++) best[i * BS] = m.x(i);
             kept_evals = m.icount;
             kept_start = start_k;
             kept_fault = m.ifault;
@@ -602,13 +606,15 @@ __global__ void __launch_bounds__(kLutBlock) lut_kernel(const __grid_constant__ 
           }
           start_k++;
           if (!finish && start_k < n_starts) {
-            P::template cold_start<NB>(ia, px, m.start, m.step);
-            m.start[0] = P::hstart(ia, start_k);
-            m.step[0] = P::h_step(m.start[0]);
+            double start[kN], step[kN];
+            P::template cold_start<NB>(ia, px, start, step);
+            start[0] = P::hstart(ia, start_k);
+            step[0] = P::h_step(start[0]);
+            m.set_start(start, step);
             m.begin(var_limit, fp.konvge, fp.kcount);
           } else {
 #pragma unroll
-            for (int i = 0; i < kN; i++) m.x[i] = best[i * BS];
+            for (int i = 0; i < kN; i++) m.x(i) = best[i * BS];
             m.phase = PH_FINAL;
           }
         }

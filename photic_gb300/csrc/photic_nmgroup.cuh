@@ -40,6 +40,12 @@ struct NmGroup {
   double ck[C][kCk];
   int32_t ck_valid;
 
+  static __device__ __forceinline__ bool lt(double a, double b) {
+    return kSharedF ? sf::lt(a, b) : sf::lt_call(a, b);
+  }
+  static __device__ __forceinline__ bool le(double a, double b) {
+    return kSharedF ? sf::le(a, b) : sf::le_call(a, b);
+  }
   __device__ __forceinline__ int dim() const { return NT > 0 ? NT : nrt; }
   __device__ __forceinline__ int coord(int t) const { return gl + t * G; }
   __device__ __forceinline__ bool own(int t) const { return coord(t) < dim(); }
@@ -136,7 +142,7 @@ struct NmGroup {
 #pragma unroll 1
     for (int j = 1; j <= dim(); j++) {
       const double fj = F(j);
-      if (sf::lt(fj, ylo)) {
+      if (lt(fj, ylo)) {
         ylo = fj;
         lo = j;
       }
@@ -158,7 +164,7 @@ struct NmGroup {
 #pragma unroll 1
       for (int j = gl; j <= dim(); j += G) {
         const double f = F(j);
-        if (f == f && (idx == 0x7fffffff || sf::lt(v, f))) {
+        if (f == f && (idx == 0x7fffffff || lt(v, f))) {
           v = f;
           idx = j;
         }
@@ -168,7 +174,7 @@ struct NmGroup {
         const double ov = __shfl_xor_sync(gmask, v, o);
         const int oi = __shfl_xor_sync(gmask, idx, o);
         if (oi != 0x7fffffff &&
-            (idx == 0x7fffffff || sf::lt(v, ov) || (!sf::lt(ov, v) && oi < idx))) {
+            (idx == 0x7fffffff || lt(v, ov) || (!lt(ov, v) && oi < idx))) {
           v = ov;
           idx = oi;
         }
@@ -181,7 +187,7 @@ struct NmGroup {
 #pragma unroll 1
     for (int j = 1; j <= dim(); j++) {
       const double fj = F(j);
-      if (sf::lt(yhi, fj)) {
+      if (lt(yhi, fj)) {
         yhi = fj;
         h = j;
       }
@@ -197,14 +203,14 @@ struct NmGroup {
       int c = 0;
 #pragma unroll 1
       for (int j = gl; j <= dim(); j += G)
-        if (sf::lt(fr_, F(j))) c++;
+        if (lt(fr_, F(j))) c++;
       return (int)__reduce_add_sync(gmask, (unsigned)c);
 #endif
     }
     int worse = 0;
 #pragma unroll 1
     for (int j = 0; j <= dim(); j++)
-      if (sf::lt(fr_, F(j))) worse++;
+      if (lt(fr_, F(j))) worse++;
     return worse;
   }
 
@@ -274,7 +280,7 @@ struct NmGroup {
 
   __device__ __forceinline__ bool iteration_end() {
     const double fh = F(hi);
-    if (sf::lt(fh, ylo)) {
+    if (lt(fh, ylo)) {
       ylo = fh;
       lo = hi;
     }
@@ -292,7 +298,7 @@ struct NmGroup {
         const double d = F(j) - mean;
         z = z + d * d;
       }
-      if (sf::le(z, var_limit)) return true;
+      if (le(z, var_limit)) return true;
     }
     return false;
   }
@@ -338,7 +344,7 @@ struct NmGroup {
         break;
       case PH_REFLECT:
         fr = y;
-        if (sf::lt(fr, ylo)) {
+        if (lt(fr, ylo)) {
           pk = PK_EXPAND;
           phase = PH_EXPAND;
         } else {
@@ -355,11 +361,11 @@ struct NmGroup {
         }
         break;
       case PH_EXPAND:
-        rep = sf::lt(fr, y) ? 1 : 2;
+        rep = lt(fr, y) ? 1 : 2;
         break;
       case PH_CONTRACT_IN:
         // shrink every vertex towards the best (model/asa047.c:331-351)
-        if (sf::lt(F(hi), y)) shr = 0;
+        if (lt(F(hi), y)) shr = 0;
         else rep = 2;
         break;
       case PH_SHRINK:
@@ -368,7 +374,7 @@ struct NmGroup {
         else cs = CS_READY;
         break;
       case PH_CONTRACT_OUT:
-        rep = sf::le(y, fr) ? 2 : 1;
+        rep = le(y, fr) ? 2 : 1;
         break;
       case PH_PROBE_PLUS:
       case PH_PROBE_MINUS:

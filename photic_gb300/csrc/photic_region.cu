@@ -642,7 +642,7 @@ __global__ void __launch_bounds__(BLOCK, 1) region_kernel(const __grid_constant_
                             sf::near_positive(P) && sf::near_positive(Gg) &&
                             sf::near_positive(Xx) && sf::near(lnP) && sf::near_positive(pw);
         BandTerm t;
-        band_term(sc, b, a.sec_sun[s], near_x, H, rho, P, lnP, Gg, Xx, pw, my_rrs[h], t);
+        band_term(sc, b, a.sec_sun[s], near_x, final_eval, H, rho, P, lnP, Gg, Xx, pw, my_rrs[h], t);
         dd[tau] = t.dd;
         kk[tau] = t.K;
         if (final_eval) {

@@ -96,6 +96,8 @@ PHOTIC_FM_HD float f_rsqrt(float x) {
 // The rare operands: the compiled operations, out of line.
 PHOTIC_SF_NOINLINE double div_rare(double a, double b) { return a / b; }
 PHOTIC_SF_NOINLINE double sqrt_rare(double a) { return ::sqrt(a); }
+PHOTIC_SF_NOINLINE bool lt_rare(double a, double b) { return a < b; }
+PHOTIC_SF_NOINLINE bool le_rare(double a, double b) { return a <= b; }
 
 // The significand m in [2^52, 2^53) of a double as two floats: the leading
 // 24 bits in [1, 2), and 23 of the other 29 as a value below 2^-23.
@@ -242,23 +244,167 @@ PHOTIC_FM_HD double sqrt_mid(double x) {
 // sqrt(x), correctly rounded.
 PHOTIC_FM_HD double sqrt(double x) { return mid_positive(x) ? sqrt_mid(x) : sqrt_rare(x); }
 
-// a < b.  Of doubles without a sign bit the bits compare as integers (a NaN
-// is above every number); a sign bit on either side takes the compiled
-// comparison.
+// a < b and a <= b.  Of doubles without a sign bit the bits compare as
+// integers (a NaN is above every number); a sign bit on either side takes the
+// compiled comparison.  The compiler runs that one beside the integer one;
+// the _call forms keep it off the FP64 pipe at the price of a branch: faster
+// where that pipe is the bound (8 009 temporal stacks 224 -> 207 ms), slower
+// in the single-scene kernels (1024 x 320 scene 346 -> 363 ms).
 PHOTIC_FM_HD bool lt(double a, double b) {
   const int64_t ia = bits(a), ib = bits(b);
   if ((ia | ib) < 0) return a < b;
   return ia < ib && ib <= 0x7ff0000000000000LL;
 }
-// a <= b.
 PHOTIC_FM_HD bool le(double a, double b) {
   const int64_t ia = bits(a), ib = bits(b);
   if ((ia | ib) < 0) return a <= b;
   return ia <= ib && ib <= 0x7ff0000000000000LL;
 }
+PHOTIC_FM_HD bool lt_call(double a, double b) {
+  const int64_t ia = bits(a), ib = bits(b);
+  if ((ia | ib) < 0) return lt_rare(a, b);
+  return ia < ib && ib <= 0x7ff0000000000000LL;
+}
+PHOTIC_FM_HD bool le_call(double a, double b) {
+  const int64_t ia = bits(a), ib = bits(b);
+  if ((ia | ib) < 0) return le_rare(a, b);
+  return ia <= ib && ib <= 0x7ff0000000000000LL;
+}
 
 // a / 2, exactly, for a normal a of twice the least normal's size or more.
 PHOTIC_FM_HD double half_mid(double a) { return from_bits(bits(a) - (1ll << 52)); }
+
+PHOTIC_FM_HD uint64_t mulhi(uint64_t a, uint64_t b) {
+#if defined(__CUDA_ARCH__)
+  return __umul64hi(a, b);
+#else
+  return (uint64_t)(((unsigned __int128)a * b) >> 64);
+#endif
+}
+
+// (v >> s) rounded to nearest, for s in [1, 63]; the value v is the floor of
+// never lies half way (see exp_neg).
+PHOTIC_FM_HD uint64_t shift_round(uint64_t v, uint32_t s) { return ((v >> (s - 1)) + 1) >> 1; }
+
+// fm::exp_t(x), bit for bit, for x in (-354, 0): `ok` is cleared where this
+// cannot tell (the argument's multiple of ln2/64 nearly half way between two,
+// a remainder below 2^-40 or of at most 21 significant bits), with the result
+// then undefined.
+//
+// exp_t spends eleven FP64 operations.  Here the multiple n comes from the
+// single-precision pipe; the polynomial's three fused multiply-adds
+// c1 = r/120 + 1/24, c2 = c1 r + 1/6, c = c2 r + 1/2, whose results lie in
+// known binades, are fixed-point products rounded to the grid of the double;
+// r r is mul_mid; five FP64 operations remain.  A product of a 53-bit and a
+// 53-bit significand that is shifted down by s >= 62 places could only lie
+// half way between two grid points with 61 trailing zeros; with fewer than 21
+// in r and fewer than 32 in c1 and c2 it never does.
+PHOTIC_FM_HD double exp_neg(double x, bool &ok) {
+  const double kL1 = 0x1.62e4200000000p-7, kL2 = 0x1.fdf473de6af28p-28;  // as in exp_t
+  const float kInvH = 0x1.715476p+6f, kInvL = 0x1.4ae0cp-20f;            // 64 / ln 2
+  const uint64_t u = (uint64_t)bits(x);
+  const uint32_t h = (uint32_t)(u >> 32) & 0x7fffffffu, l = (uint32_t)u;
+  ok = ok && h - 0x3c300000u < 0x40762000u - 0x3c300000u;  // 2^-60 <= |x| < 354
+  // |x| as two floats
+  const uint32_t fb = ((h << 3) | (l >> 29)) + 0x40000000u;
+  const float xh = f_bits(fb);
+  const uint32_t fe = (fb & 0x7f800000u) - (23u << 23);
+  const float xl = f_bits(((l >> 6) & 0x7fffffu) | fe) - f_bits(fe);
+  float t = f_fma(xh, kInvH, kMagic);
+  float nf = t - kMagic;
+  float fr = f_fma(xh, kInvH, -nf);
+  fr = f_fma(xh, kInvL, fr);
+  fr = f_fma(xl, kInvH, fr);
+  t = fr + kMagic;  // the first rounding of a large product may be off by one
+  t = t - kMagic;
+  fr = fr - t;
+  nf = nf + t;
+  ok = ok && fabsf(fr) < 0.5f - 0x1p-18f;
+  const int32_t N = (int32_t)(u_bits(nf + kMagic) - kMagicBits);  // -n
+  const uint32_t nb = u_bits(nf);
+  // N as a double (2^-127 for 0, which leaves x unchanged below)
+  const double nd = from_bits(((int64_t)((nb >> 3) + 0x38000000u) << 32) | (uint32_t)(nb << 29));
+  double r = fma(nd, kL1, x);
+  r = fma(nd, kL2, r);
+  const uint64_t ur = (uint64_t)bits(r);
+  const uint32_t rh = (uint32_t)(ur >> 32), rl = (uint32_t)ur;
+  const int32_t er = 1023 - (int32_t)((rh >> 20) & 0x7ff);  // |r| in [2^-er, 2^(1-er))
+  ok = ok && er <= 40 && (rl << 11) != 0;
+  const bool neg = (int32_t)rh < 0;
+  const uint64_t mr = ((((uint64_t)((rh & 0xfffffu) | 0x100000u)) << 32) | rl) << 11;
+  // c1 on the grid 2^-57, c2 on 2^-55, c on 2^-53 (2^-54 below 1/2)
+  uint64_t v = shift_round(mulhi(mr, 0x8888888888888800ull), 12 + er);
+  const uint64_t c1 = 0x15555555555555ull + (neg ? 0 - v : v);
+  v = shift_round(mulhi(mr, c1), 1 + er);
+  const uint64_t c2 = 0x15555555555555ull + (neg ? 0 - v : v);
+  v = shift_round(mulhi(mr, c2), neg ? er : 1 + er);
+  ok = ok && (uint32_t)c1 != 0 && (uint32_t)c2 != 0;
+  const double c = from_bits((int64_t)(0x3fe0000000000000ull + (neg ? 0 - v : v)));
+  const double p = fma(mul_mid(r, r), c, r);
+  const int j = -N & 63;
+#if defined(__CUDA_ARCH__)
+  const double2 T = __ldg(reinterpret_cast<const double2 *>(fm::kExp2TabDev) + j);
+  const double th = T.x, tl = T.y;
+#else
+  const double th = fm::kExp2TabHost[2 * j], tl = fm::kExp2TabHost[2 * j + 1];
+#endif
+  const double y = fma(th, p, tl) + th;
+  return from_bits(bits(y) + fm::shl52(-N >> 6));
+}
+
+PHOTIC_FM_HD int clz(uint32_t x) {
+#if defined(__CUDA_ARCH__)
+  return __clz((int)x);
+#else
+  return x ? __builtin_clz(x) : 32;
+#endif
+}
+
+// s rounded to 53 significant bits, nearest even.
+PHOTIC_FM_HD int64_t round53(int64_t s) {
+  const int32_t h = (int32_t)(s >> 32);
+  const int c = clz((uint32_t)(h ^ (h >> 31)));
+  const uint32_t k = c < 11 ? 11u - (uint32_t)c : 0u;
+  const uint32_t mask = (1u << k) - 1u;
+  const uint32_t lo = (uint32_t)s;
+  s += (mask >> 1) + ((lo >> k) & mask & 1u);
+  return s & ~(int64_t)mask;
+}
+
+// ((0 + v[0]) + v[1]) + ... + v[n-1], then minus v[h], each operation rounded
+// as in double, v[j] = p[j * stride] for n <= 7: the doubles as integers on
+// the finest one's grid, the running sum rounded to 53 bits after every
+// step.  False, with nothing done, for a zero, subnormal or special value or
+// where the exponents span more than seven (the sum would leave 63 bits).
+PHOTIC_FM_HD bool sum_less_one(const double *p, int stride, int n, int h, double &z) {
+  uint32_t emin = 0x7ff, emax = 0;
+  for (int j = 0; j < n; j++) {
+    const uint32_t e = (uint32_t)((uint64_t)bits(p[j * stride]) >> 52) & 0x7ffu;
+    emin = e < emin ? e : emin;
+    emax = e > emax ? e : emax;
+  }
+  if (emin < 256u || emax > 1790u || emax - emin > 7u) return false;
+  int64_t acc = 0;
+  for (int j = 0; j <= n; j++) {
+    const uint64_t u = (uint64_t)bits(p[(j < n ? j : h) * stride]);
+    const uint32_t e = (uint32_t)(u >> 52) & 0x7ffu;
+    int64_t m = (int64_t)(((u & 0xfffffffffffffull) | 0x10000000000000ull) << (e - emin));
+    if (((int64_t)u < 0) != (j == n)) m = -m;
+    acc = round53(acc + m);
+  }
+  const bool neg = acc < 0;
+  const uint64_t a = (uint64_t)(neg ? -acc : acc);
+  if (a == 0) {
+    z = 0.0;
+    return true;
+  }
+  const uint32_t ah = (uint32_t)(a >> 32);
+  const int lz = ah ? clz(ah) : 32 + clz((uint32_t)a);
+  const uint64_t m = lz >= 11 ? a << (lz - 11) : a >> (11 - lz);  // exact
+  const uint64_t e = (uint64_t)emin + (uint64_t)(11 - lz);
+  z = from_bits((int64_t)((m - 0x10000000000000ull) + (e << 52) + (neg ? 1ull << 63 : 0)));
+  return true;
+}
 
 }  // namespace sf
 }  // namespace photic

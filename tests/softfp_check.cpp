@@ -35,7 +35,7 @@ using namespace photic;
 
 namespace {
 
-long g_bad = 0;
+long g_bad = 0, g_exp = 0, g_exp_rare = 0;
 
 void same(double got, double want, const char *what, double a, double b) {
   if (memcmp(&got, &want, 8) == 0 || (got != got && want != want)) return;
@@ -96,8 +96,17 @@ int main(int argc, char **argv) {
     same(fm::div_pi(a), a / 3.141592653589793, "pi", a, 0);
     same(fm::div_120(a), a / 120.0, "120", a, 0);
     same(fm::div_6(a), a / 6.0, "6", a, 0);
+    {  // the exponential over the range and the scale the cost meets
+      const double e = -fabs(i & 1 ? sample(-62, 8) : sample(-8, 6));
+      bool ok = true;
+      const double got = sf::exp_neg(e, ok);
+      g_exp++;
+      if (ok) same(got, fm::exp_t(e), "exp", e, 0);
+      else g_exp_rare += e < -0x1p-30 && e > -350.0;
+    }
     if (sf::lt(a, b) != (a < b) || sf::lt(b, a) != (b < a) || sf::le(a, b) != (a <= b) ||
-        !sf::le(a, a) || sf::lt(a, a))
+        !sf::le(a, a) || sf::lt(a, a) || sf::lt_call(a, b) != (a < b) ||
+        sf::le_call(a, b) != (a <= b))
       g_bad++, printf("comparison of %a and %a\n", a, b);
   }
   const double special[] = {0.0, -0.0, 1.0, -1.0, 2.0, INFINITY, -INFINITY, NAN, -NAN, 5e-324,
@@ -109,10 +118,18 @@ int main(int argc, char **argv) {
     same(fm::div_120(a), a / 120.0, "120", a, 0);
     for (double b : special) {
       same(sf::div(a, b), a / b, "div", a, b);
-      if (sf::lt(a, b) != (a < b) || sf::le(a, b) != (a <= b))
+      if (sf::lt(a, b) != (a < b) || sf::le(a, b) != (a <= b) || sf::lt_call(a, b) != (a < b) ||
+          sf::le_call(a, b) != (a <= b))
         g_bad++, printf("comparison of %a and %a\n", a, b);
     }
   }
-  printf("mismatches %ld\n", g_bad);
+  const double refused[] = {-0.0, 0.0, -5e-324, -354.0, -400.0, -1e300, -INFINITY, NAN};
+  for (double e : refused) {
+    bool ok = true;
+    (void)sf::exp_neg(e, ok);
+    if (ok) g_bad++, printf("exp takes %a\n", e);
+  }
+  printf("mismatches %ld, exponentials left to the general path %ld of %ld\n", g_bad, g_exp_rare,
+         g_exp);
   return g_bad != 0;
 }
