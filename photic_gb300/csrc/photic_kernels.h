@@ -10,6 +10,11 @@
 
 namespace photic {
 
+// Stream-ordered workspace from the library's pool (photic_host.cu), freed
+// with cudaFreeAsync; ws_trim gives the current device's unused part back.
+cudaError_t ws_alloc(void **p, size_t bytes, cudaStream_t s);
+void ws_trim();
+
 // Device error bits accumulated in the per-call error word.
 enum : unsigned {
   PHOTIC_DEVERR_EVAL_CAP = 1u,     // a pixel exceeded the defensive evaluation cap

@@ -665,14 +665,14 @@ cudaError_t lut_order(LutKeyArgs ka, int64_t *order, int64_t *n_shallow, cudaStr
     e = cub::DeviceRadixSort::SortPairs(nullptr, b_sort, sel_keys, sorted_keys, sel_idx, order,
                                         npix, 0, 32, s);
   const size_t b_temp = b_sel > b_sort ? b_sel : b_sort;
-  if (e == cudaSuccess) e = cudaMallocAsync((void **)&keys, npix * sizeof(float), s);
-  if (e == cudaSuccess) e = cudaMallocAsync((void **)&sel_keys, npix * sizeof(float), s);
-  if (e == cudaSuccess) e = cudaMallocAsync((void **)&sorted_keys, npix * sizeof(float), s);
-  if (e == cudaSuccess) e = cudaMallocAsync((void **)&flags, npix, s);
-  if (e == cudaSuccess) e = cudaMallocAsync((void **)&idx, npix * sizeof(int64_t), s);
-  if (e == cudaSuccess) e = cudaMallocAsync((void **)&sel_idx, npix * sizeof(int64_t), s);
-  if (e == cudaSuccess) e = cudaMallocAsync((void **)&d_count, sizeof(int64_t), s);
-  if (e == cudaSuccess) e = cudaMallocAsync(&temp, b_temp, s);
+  if (e == cudaSuccess) e = ws_alloc((void **)&keys, npix * sizeof(float), s);
+  if (e == cudaSuccess) e = ws_alloc((void **)&sel_keys, npix * sizeof(float), s);
+  if (e == cudaSuccess) e = ws_alloc((void **)&sorted_keys, npix * sizeof(float), s);
+  if (e == cudaSuccess) e = ws_alloc((void **)&flags, npix, s);
+  if (e == cudaSuccess) e = ws_alloc((void **)&idx, npix * sizeof(int64_t), s);
+  if (e == cudaSuccess) e = ws_alloc((void **)&sel_idx, npix * sizeof(int64_t), s);
+  if (e == cudaSuccess) e = ws_alloc((void **)&d_count, sizeof(int64_t), s);
+  if (e == cudaSuccess) e = ws_alloc(&temp, b_temp, s);
   if (e == cudaSuccess) {
     ka.keys = keys;
     ka.flags = flags;

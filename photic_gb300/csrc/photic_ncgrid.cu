@@ -30,11 +30,13 @@
 
 namespace photic {
 int report_error(int code, const char *message);
+cudaError_t ws_alloc(void **p, size_t bytes, cudaStream_t s);
 }
 
 namespace {
 
 using photic::report_error;
+using photic::ws_alloc;
 
 int io_fail(const std::string &path, const char *what) {
   return report_error(PHOTIC_ERR_IO, (path + ": " + what).c_str());
@@ -919,7 +921,7 @@ cudaError_t pack_general(const float *d_grid, int64_t n, float fspv, int64_t nti
   unsigned char *ws = nullptr;
   const size_t off_pref = ((size_t)ntiles * 4 + 255) / 256 * 256;
   const size_t off_st = off_pref + ((size_t)ntiles * 4 + 255) / 256 * 256;
-  cudaError_t e = cudaMallocAsync((void **)&ws, off_st + sizeof(PackState), s);
+  cudaError_t e = ws_alloc((void **)&ws, off_st + sizeof(PackState), s);
   if (e != cudaSuccess) return cudaErrorMemoryAllocation;
   float *tmin = (float *)ws, *tpre = (float *)(ws + off_pref);
   PackState *st = (PackState *)(ws + off_st);
@@ -1049,7 +1051,7 @@ int photic_nc_pack(const float *d_grid, int64_t n, double spval, void *d_packed_
   if (ntiles > 0x7FFFFFFFLL) return report_error(PHOTIC_ERR_INVALID, "grid too large");
   const float fspv = (float)spval;  // model/nc.c:278
   PackState *st = nullptr;
-  cudaError_t e = cudaMallocAsync((void **)&st, sizeof(PackState), s);
+  cudaError_t e = ws_alloc((void **)&st, sizeof(PackState), s);
   if (e != cudaSuccess) return report_error(PHOTIC_ERR_NOMEM, "pack workspace");
   PackState h{};
   e = cudaMemsetAsync(st, 0, sizeof *st, s);
@@ -1100,7 +1102,7 @@ int photic_nc_read_bands(const char *const *paths, int32_t n_bands, float *d_rrs
   unsigned char *d = nullptr;
   cudaError_t e = cudaMallocHost(&h, band_bytes * n_bands);
   if (e != cudaSuccess) return report_error(PHOTIC_ERR_NOMEM, "pinned staging");
-  e = cudaMallocAsync((void **)&d, band_bytes * n_bands, s);
+  e = ws_alloc((void **)&d, band_bytes * n_bands, s);
   if (e != cudaSuccess) {
     cudaFreeHost(h);
     return report_error(PHOTIC_ERR_NOMEM, "device staging");
@@ -1133,7 +1135,7 @@ int photic_nc_write_grid(const char *path, const float *d_grid, int32_t ncols, i
   const int64_t n = (int64_t)ncols * nrows;
   cudaStream_t s = (cudaStream_t)stream;
   void *dpk = nullptr, *hpk = nullptr;
-  cudaError_t e = cudaMallocAsync(&dpk, (size_t)n * 2, s);
+  cudaError_t e = ws_alloc(&dpk, (size_t)n * 2, s);
   if (e != cudaSuccess) return report_error(PHOTIC_ERR_NOMEM, "pack output");
   e = cudaMallocHost(&hpk, (size_t)n * 2);
   if (e != cudaSuccess) {
