@@ -685,6 +685,21 @@ int photic_lut_invert_batch(const photic_config *cfg, const photic_lut_config *l
     const int64_t lanes = (int64_t)sms * per_sm * block;
     int64_t C = lut->n_chains ? lut->n_chains : kLutChainsPerLane * lanes;
     if (C > S) C = S;
+    if (C == S && !d_empirical) {
+      // a chain for every pixel: plain cold fits, their starts in parallel
+      a.inv.pixels = order;
+      a.inv.npix = S;
+      a.inv.no_mask = 1;
+      a.inv.source = d_source;
+      a.inv.chain_stats = d_chain_stats;
+      a.inv.vec4 = nb == 4 && ((uintptr_t)d_rrs & 15u) == 0;
+      rc = run_invert(a.inv, PHOTIC_PREC_FP64, 0, 0, sms, s);
+      if (!d_order) cudaFreeAsync(order, s);
+      if (rc) return rc;
+      if (n_chains_used) *n_chains_used = C;
+      if (n_shallow) *n_shallow = S;
+      return PHOTIC_OK;
+    }
     const int64_t per_chain = (S + C - 1) / C;
     const int64_t cap = per_chain < lut->n_lut ? per_chain : (int64_t)lut->n_lut;
     a.order = order;
@@ -2776,7 +2791,7 @@ void region_args(const photic_config *cfg, const float *d_grid, int32_t n_scenes
   a.grid = d_grid;
   a.nrows = nrows;
   a.ncols = ncols;
-  a.npix = (int64_t)nrows * ncols;
+  a.npix = a.grid_npix = (int64_t)nrows * ncols;
   a.n_scenes = n_scenes;
   a.n_spatial = n_spatial;
   a.n_bottoms = n_bottoms;
@@ -2898,6 +2913,18 @@ extern "C" int photic_region_lut_invert_batch(
     }
     int64_t C = lut->n_chains ? lut->n_chains : kRegionChainsPerWarp * warps;
     if (C > S) C = S;
+    if (C == S && !d_empirical) {
+      // a chain for every pixel: the plain general fit, its starts in parallel
+      a.pixels = order;
+      a.npix = S;
+      a.no_mask = 1;
+      rc = run_region(a, nmax, cfg->blocks_per_sm, s);
+      if (!d_order) cudaFreeAsync(order, s);
+      if (rc) return rc;
+      if (n_chains_used) *n_chains_used = C;
+      if (n_shallow) *n_shallow = S;
+      return PHOTIC_OK;
+    }
     const int64_t per_chain = (S + C - 1) / C;
     const int64_t cap = per_chain < lut->n_lut ? per_chain : (int64_t)lut->n_lut;
     a.order = order;

@@ -234,6 +234,17 @@ __device__ __forceinline__ void write_fit(const photic_outputs &o, int64_t p,
                   (kept_start << 16);
 }
 
+__device__ __forceinline__ int64_t pixel_at(const InvertArgs &args, int64_t q) {
+  return args.order ? (int64_t)args.order[q] : args.pixels ? args.pixels[q] : q;
+}
+
+// What the lookup-table loop reports of the pixel at position q.
+__device__ __forceinline__ void write_single_chain(const InvertArgs &args, int64_t q, int64_t p,
+                                                   double model_error) {
+  if (args.source) args.source[p] = -1;
+  if (args.chain_stats) single_chain_stats(args.chain_stats + q * 4, 1.5, model_error);
+}
+
 template <int NB>
 __device__ __forceinline__ void load_spectrum(const InvertArgs &args, int64_t p, float (&r)[NB]) {
   if (NB == 4 && args.vec4) {
@@ -288,6 +299,7 @@ __global__ void __launch_bounds__(BS) invert_kernel(const __grid_constant__ Inve
   const photic_outputs &o = args.out;
 
   int64_t pixel = -1, item = -1;  // item: pixel number within the n_par, or -1
+  int64_t position = 0;
   int32_t start_k = 0, n_starts = 0, total = 0, kept_evals = 0, kept_start = 0, kept_fault = 0;
   int32_t guard = 0;
   T lowest = P::zero();
@@ -325,7 +337,7 @@ __global__ void __launch_bounds__(BS) invert_kernel(const __grid_constant__ Inve
             k = (int)((w - args.n_seq) / args.n_par);
             q = args.n_seq + (w - args.n_seq) % args.n_par;
           }
-          p = args.order ? (int64_t)args.order[q] : q;
+          p = pixel_at(args, q);
           if (k > 0)
             live = __ldcg(args.exit_k + (q - args.n_seq)) >= k &&
                    (args.seeds == nullptr || isnan(args.seeds[p * kN]));
@@ -369,7 +381,8 @@ __global__ void __launch_bounds__(BS) invert_kernel(const __grid_constant__ Inve
           start_k = (int32_t)((w - args.n_seq) / args.n_par);
           q = args.n_seq + item;
         }
-        pixel = args.order ? (int64_t)args.order[q] : q;
+        position = q;
+        pixel = pixel_at(args, q);
         px = wpx[slot];
         total = kept_evals = kept_start = kept_fault = guard = 0;
         lowest = P::from_double(1.0e4);
@@ -423,6 +436,7 @@ __global__ void __launch_bounds__(BS) invert_kernel(const __grid_constant__ Inve
       }
       if (fin) {
         write_fit<P, NB>(o, pixel, x, det, total, kept_evals, kept_start, kept_fault);
+        if (args.pixels) write_single_chain(args, position, pixel, det.model_error);
         has = false;
       } else if (++guard > guard_cap) {
         // Defensive cap: each nelmin call is bounded by kcount, so
@@ -489,7 +503,7 @@ __global__ void __launch_bounds__(128) finish_kernel(const __grid_constant__ Inv
   if (i >= args.n_par || args.exit_k[i] < 0) return;
   const FitParams &fp = args.fp;
   const int64_t q = args.n_seq + i;
-  const int64_t p = args.order ? (int64_t)args.order[q] : q;
+  const int64_t p = pixel_at(args, q);
   const bool seeded = args.seeds != nullptr && !isnan(args.seeds[p * kN]);
   const int n_starts = seeded ? 1 : fp.n_hstarts;
   const StartRecord<P> *rec = reinterpret_cast<const StartRecord<P> *>(args.records) +
@@ -528,6 +542,7 @@ __global__ void __launch_bounds__(128) finish_kernel(const __grid_constant__ Inv
     P::template details<NB>(args, px, x, det);
   }
   write_fit<P, NB>(args.out, p, x, det, total, kept_evals, kept_start, kept_fault);
+  if (args.pixels) write_single_chain(args, q, p, det.model_error);
 }
 
 template <class P, int NB, int BS>

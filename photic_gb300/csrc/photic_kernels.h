@@ -46,6 +46,11 @@ struct InvertArgs {
   void *records;         // [n_par][n_hstarts] results of the starts
   int32_t *exit_k;       // [n_par] first start known to meet the early exit, -1 masked
   int32_t claim;         // positions a warp claims at a time (1..32)
+  // the lookup-table loop with a chain for every pixel: position -> pixel,
+  // and what the loop reports of a fitted pixel and of its chain
+  const int64_t *pixels;
+  int64_t *source;       // optional [npix]: -1
+  double *chain_stats;   // optional [positions][4]
 };
 
 // Records of depth starts run as work items (photic_starts.cuh): item
@@ -84,6 +89,21 @@ int invert_blocks_per_sm(const InvertArgs &a, int precision, int block);
 // FP64-faithful inversion with double-float screening (photic_guarded.cu).
 cudaError_t launch_guarded(const InvertArgs &a, int block, int grid, cudaStream_t s);
 int guarded_blocks_per_sm(const InvertArgs &a, int block);
+
+// A chain of one pixel (model/samodel.c:871-1211): its empty table serves
+// nothing, the pixel is fitted cold, and the thresholds move once, from m0 by
+// the fit's model error (error_mean is a float, model/common.c:877-891, and
+// leaves a zero out).
+__device__ __forceinline__ void single_chain_stats(double *cs, double m0, double me) {
+  const double mean = (float)me != 0.0f ? (double)(float)me : 0.0;
+  double match = m0 + (0.75 * mean + (0.25 * me) / 1.0);
+  match = match / 2.0;
+  match = 1.5 > match ? 1.5 : match;
+  cs[0] = 0.0;
+  cs[1] = 1.0;
+  cs[2] = match;
+  cs[3] = match;
+}
 
 // samodel()'s pixel loop with the dynamic lookup table (photic_lut.cu).
 struct LutKeyArgs {
@@ -309,7 +329,8 @@ struct RegionArgs {
   SceneConsts sc;
   const float *grid;            // grid mode: [nrows][ncols][n_bands]
   int nrows, ncols;
-  int64_t npix;                 // problems (grid: nrows * ncols)
+  int64_t npix;                 // problems (grid: nrows * ncols, or the listed pixels)
+  int64_t grid_npix;            // nrows * ncols
   int32_t n_scenes;             // scenes of the same bands; grid: [S][nrows][ncols][n_bands]
   double sec_sun[kMaxScenes];   // per-scene secant of the subsurface sun zenith
   int32_t n_spatial;            // 1: each pixel alone, 2: 3 x 3 regions
@@ -343,6 +364,7 @@ struct RegionArgs {
   // the sorted shallow pixels cut into n_chains contiguous slices, one warp
   // per slice at a time
   const int64_t *order;         // [n_shallow]; NULL: every pixel from the queue
+  const int64_t *pixels;        // every chain one pixel: queue position -> pixel (order NULL)
   int64_t n_shallow, n_chains, cap;  // cap: table slots per chain
   int32_t entry_stride;         // doubles per table entry
   double *ring;                 // [n_chains][cap][entry_stride]

@@ -101,7 +101,7 @@ __device__ __noinline__ int regions_of(const RegionArgs &a, int64_t p, int64_t (
       for (int s = 0; s < a.n_scenes; s++)
 #pragma unroll 1
         for (int b = 0; b < nb; b++)
-          if (nodata_value(a.grid[(s * a.npix + q) * nb + b], a.fp.nodata)) nodata = true;
+          if (nodata_value(a.grid[(s * a.grid_npix + q) * nb + b], a.fp.nodata)) nodata = true;
       if (i == iii && j == jjj) origin = R;
       if (!nodata) rp[R++] = q;
     }
@@ -310,7 +310,7 @@ __global__ void __launch_bounds__(BLOCK, 1) region_kernel(const __grid_constant_
   // spectrum of scene s of region slot q (a pixel index of the grid, or a
   // region row of the list)
   auto spec = [&](int64_t q, int s) -> const float * {
-    return list ? a.list_rrs + (q * S + s) * nb : a.grid + ((int64_t)s * a.npix + q) * nb;
+    return list ? a.list_rrs + (q * S + s) * nb : a.grid + ((int64_t)s * a.grid_npix + q) * nb;
   };
 
   NmGroup<0, C, 32, CG, true> m;
@@ -334,7 +334,7 @@ __global__ void __launch_bounds__(BLOCK, 1) region_kernel(const __grid_constant_
   }
 
   for (;;) {
-    int64_t p = 0, slot = 0;  // slot: of the pixel's records
+    int64_t p = 0, slot = 0, position = 0;  // slot: of the pixel's records
     int item_k = -1;          // the start of a position that is one, else -1
     int64_t rp[kMaxR];
     int origin = 0, R = 0;
@@ -453,6 +453,8 @@ __global__ void __launch_bounds__(BLOCK, 1) region_kernel(const __grid_constant_
         p = a.n_seq + slot;
         if (item_k > 0 && !start_wanted(a.sw, slot, item_k)) continue;
       }
+      position = p;
+      if (a.pixels) p = a.pixels[p];
 
       // the pixel loop's mask test on the centre, every scene
       // (model/samodel.c:933-947); samodel_optimise called directly has none
@@ -860,6 +862,13 @@ __global__ void __launch_bounds__(BLOCK, 1) region_kernel(const __grid_constant_
           if (o.status)
             o.status[p] = PHOTIC_PX_FITTED | (kept_fault == 0 ? PHOTIC_PX_CONVERGED : 0) |
                           (hot ? PHOTIC_PX_HOT : 0) | (kept_start << 16) | (R << 24);
+        }
+        if (a.pixels && lane == 0) {
+          if (a.source) a.source[p] = -1;
+          const double m0 = 1.125 * (double)S;
+          if (a.chain_stats)
+            single_chain_stats(a.chain_stats + position * 4,
+                               m0 > kMinThreshold ? m0 : kMinThreshold, misc[1]);
         }
         if (a.list_params)
 #pragma unroll 1
