@@ -353,6 +353,7 @@ struct RegionArgs {
                                 // scene's K_min (the cost's), IOD, K_min over all
                                 // scenes (the post-fit product's)
   unsigned long long *queue;    // work-queue head (zeroed): pixels, or chains
+  double *simplex;              // the resident warps' simplexes (launch_region)
   // pixels beyond the first n_seq: one queue position per depth start
   // (photic_starts.cuh); n_par = 0 in the chain and evaluation modes
   int64_t n_seq, n_par;

@@ -51,17 +51,25 @@ constexpr int kChainD = 3 * kRS + kTerms + 3 * kMaxScenes + 24;
 constexpr int kStage = 72;
 
 // Launch shapes: C coordinates per lane, vertex row stride CG.
+//
+// With more than a coordinate a lane the simplex (35 KB at n = 66) lies in
+// global memory, a slab for every resident warp, 59 MB in all and so in L2:
+// in shared memory it held an SM to five warps, with the FP64 pipe half idle;
+// eleven are resident now.  A lane reads and writes only its own columns.
 template <int C, int CG>
 struct Shape {
   static constexpr int kMaxN = C == 1 ? 32 : CG;
   static constexpr int kNF = kMaxN + 2;
-  // doubles of shared memory per warp: vertices (n+1) x CG, the vertex
+  static constexpr bool kGlobalV = C > 1;
+  static constexpr int kV = (kMaxN + 1) * CG;  // doubles of a simplex
+  // doubles of shared memory per warp: vertices (n+1) x CG where they are
+  // there, the vertex
   // costs (one copy for the warp), the evaluation point, band terms (residual^2, K, bottom share of
   // the reflectance), per-region Rrs(490/550/640), final details and
   // per-(region, bottom) shares of the bottom-continuity term, and the
   // chain mode's arrays
   static constexpr int kSmem =
-      (kMaxN + 1) * CG + kNF + 32 * C + 3 * kTerms + 3 * kRS + 8 + 2 * kShares + kChainD + kStage;
+      (kGlobalV ? 0 : kV) + kNF + 32 * C + 3 * kTerms + 3 * kRS + 8 + 2 * kShares + kChainD + kStage;
 };
 
 __device__ __forceinline__ bool nodata_value(float v, float nodata) {
@@ -299,7 +307,12 @@ __global__ void __launch_bounds__(BLOCK, 1) region_kernel(const __grid_constant_
   const int nb = fp.n_bands, S = a.n_scenes;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   double *base = smem + warp * Sh::kSmem;
-  double *V = base, *Fb = V + (kMaxN + 1) * CG, *X = Fb + kNF, *dd = X + 32 * C,
+  // (a slab's rows end beyond the last coordinate's column: a lane without a
+  // coordinate in a slot reads the slot's first)
+  double *V = Sh::kGlobalV
+                  ? a.simplex + ((int64_t)blockIdx.x * (BLOCK / 32) + warp) * Sh::kV
+                  : base;
+  double *Fb = base + (Sh::kGlobalV ? 0 : Sh::kV), *X = Fb + kNF, *dd = X + 32 * C,
          *kk = dd + kTerms, *io = kk + kTerms, *s490 = io + kTerms, *s550 = s490 + kRS,
          *s640 = s550 + kRS, *misc = s640 + kRS;
   double *share = misc + 8;
@@ -997,11 +1010,20 @@ __global__ void __launch_bounds__(BLOCK, 1) region_kernel(const __grid_constant_
   }
 }
 
-// warps: when non-NULL, only the number of resident warps is returned.
-template <int C, int CG, int BLOCK>
-cudaError_t launch_shape(const RegionArgs &a, int sms, int per_sm, cudaStream_t s,
+// warps: when non-NULL, only the number of warps that the default chain count
+// follows is returned: kRefBlocks blocks an SM, whatever is resident today.
+// The count of chains decides which pixels a chain's table serves, so it is a
+// constant of the shape.
+template <int C, int CG, int BLOCK, int kRefBlocks>
+cudaError_t launch_shape(const RegionArgs &args, int sms, int per_sm, cudaStream_t s,
                          int64_t *warps) {
-  const size_t bytes = (size_t)(BLOCK / 32) * Shape<C, CG>::kSmem * sizeof(double);
+  using Sh = Shape<C, CG>;
+  if (warps) {
+    const int use = per_sm > 0 && per_sm < kRefBlocks ? per_sm : kRefBlocks;
+    *warps = (int64_t)sms * use * (BLOCK / 32);
+    return cudaSuccess;
+  }
+  const size_t bytes = (size_t)(BLOCK / 32) * Sh::kSmem * sizeof(double);
   auto k = region_kernel<C, CG, BLOCK>;
   cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
   if (e != cudaSuccess) return e;
@@ -1011,16 +1033,24 @@ cudaError_t launch_shape(const RegionArgs &a, int sms, int per_sm, cudaStream_t 
   if (occ < 1) return cudaErrorInvalidConfiguration;
   const int use = per_sm > 0 && per_sm < occ ? per_sm : occ;
   int64_t grid = (int64_t)sms * use;
-  if (warps) {
-    *warps = grid * (BLOCK / 32);
-    return cudaSuccess;
-  }
+  RegionArgs a = args;
   // chains, or queue positions
   const int64_t units = a.order ? a.n_chains : a.n_seq + a.n_par * a.fp.n_hstarts;
   const int64_t need = (units + BLOCK / 32 - 1) / (BLOCK / 32);
   if (grid > need) grid = need;
+  void *simplex = nullptr;
+  if (Sh::kGlobalV) {
+    e = ws_alloc(&simplex, (size_t)grid * (BLOCK / 32) * Sh::kV * sizeof(double), s);
+    if (e != cudaSuccess) return e;
+    a.simplex = static_cast<double *>(simplex);
+  }
   k<<<(int)grid, BLOCK, bytes, s>>>(a);
-  return cudaGetLastError();
+  e = cudaGetLastError();
+  if (simplex) {
+    const cudaError_t e2 = cudaFreeAsync(simplex, s);
+    if (e == cudaSuccess) e = e2;
+  }
+  return e;
 }
 
 // One thread per sample: the sampled pixel's regions in extract_Rrs_data's
@@ -1081,10 +1111,12 @@ int region_max_params(int max_regions, int n_bottoms, int n_scenes) {
 
 cudaError_t launch_region(const RegionArgs &a, int max_params, int sms, int per_sm,
                           cudaStream_t s, int64_t *warps) {
-  if (max_params <= Shape<1, 32>::kMaxN) return launch_shape<1, 32, 128>(a, sms, per_sm, s, warps);
+  if (max_params <= Shape<1, 32>::kMaxN)
+    return launch_shape<1, 32, 128, 2>(a, sms, per_sm, s, warps);
   if (max_params <= Shape<3, kRegionMaxParams>::kMaxN)
-    return launch_shape<3, kRegionMaxParams, 32>(a, sms, per_sm, s, warps);
-  if (max_params <= Shape<3, 96>::kMaxN) return launch_shape<3, 96, 32>(a, sms, per_sm, s, warps);
+    return launch_shape<3, kRegionMaxParams, 32, 5>(a, sms, per_sm, s, warps);
+  if (max_params <= Shape<3, 96>::kMaxN)
+    return launch_shape<3, 96, 32, 2>(a, sms, per_sm, s, warps);
   return cudaErrorInvalidValue;
 }
 
