@@ -158,61 +158,58 @@ static __device__ PHOTIC_NOINLINE void band_term_general(const SceneConsts &sc, 
   t->dd = d * d;
 }
 
-// The same bits with the divisions, square roots, products and comparisons on
-// the integer and FP32 pipes (photic_softfp.cuh), the additions and the
-// exponentials' polynomials on the FP64 pipe, so that the pipes share the
-// work.  A product by the unit secant of a nadir view is skipped (exact).
-// The soft operations need normal operands: `near_x` says that H, rho, P, G,
-// X, pw and ln P are, the band's constants' bit in sc.near_mask that those
-// are, and the tests below cover the intermediates; a term that fails one
-// (an exact zero, an absurd exponent, NaN) is evaluated again above.
+// The same bits with the divisions, square roots, comparisons and most of the
+// exponentials on the integer and FP32 pipes (photic_softfp.cuh).  The
+// products stay on the FP64 pipe: thirty integer instructions each beside it
+// cost more in instruction fetch than they saved (1024 x 320 scene 346 -> 325
+// ms without them, 41 x 29 general fit 335 -> 299, 8 009 stacks 217 -> 201).
+// A product by the unit secant of a nadir view is skipped (exact).
+// The soft operations need normal operands of moderate exponent: the tests
+// below cover each, and a term that fails one (an exact zero, an absurd
+// exponent, NaN) is evaluated again above.
 // `want_B`: t.rrs_B is used, not only t.rrs.
-__device__ __forceinline__ void band_term(const SceneConsts &sc, int b, double sec_sun, bool near_x,
-                                          bool want_B,
-                                          double H, double rho, double P, double lnP, double G,
-                                          double X, double pw, double r, BandTerm &t) {
-  const double c = sc.a0[b] + sf::mul_mid(sc.a1[b], lnP);
-  const double a_phi = sf::mul_mid(c, P);
-  const double a_g = sf::mul_mid(G, sc.eS[b]);
+__device__ __forceinline__ void band_term(const SceneConsts &sc, int b, double sec_sun,
+                                          bool want_B, double H, double rho, double P, double lnP,
+                                          double G, double X, double pw, double r, BandTerm &t) {
+  const double a_phi = (sc.a0[b] + sc.a1[b] * lnP) * P;
+  const double a_g = G * sc.eS[b];
   const double a = sc.aw[b] + a_phi + a_g;
-  const double bb = sc.bbw[b] + sf::mul_mid(X, pw);
+  const double bb = sc.bbw[b] + X * pw;
   const double ab = a + bb;
   const double u = sf::div_mid(bb, ab);
   const double K = fm::bits(ab) > 0x4004000000000000LL ? 2.5 : ab;  // > 2.5 (positive here)
-  const double rrs_dp = sf::mul_mid(0.084 + sf::mul_mid(0.170, u), u);
-  double DuC = sf::mul_mid(1.03, sf::sqrt_mid(1.0 + sf::mul_mid(2.4, u)));
-  double DuB = sf::mul_mid(1.04, sf::sqrt_mid(1.0 + sf::mul_mid(5.4, u)));
+  const double rrs_dp = (0.084 + 0.170 * u) * u;
+  double DuC = 1.03 * sf::sqrt_mid(1.0 + 2.4 * u);
+  double DuB = 1.04 * sf::sqrt_mid(1.0 + 5.4 * u);
   if (sc.sec_view != 1.0) {
-    DuC = sf::mul_mid(DuC, sc.sec_view);
-    DuB = sf::mul_mid(DuB, sc.sec_view);
+    DuC = DuC * sc.sec_view;
+    DuB = DuB * sc.sec_view;
   }
-  const double MC = sec_sun + DuC, MB = sec_sun + DuB;
   // Beyond 200 optical depths the exponentials change no bit of the sums
   // below (the columns' part is 1 - 0, the bottom's share is lost in rrs):
   // -200 stands for every such depth, unless the bottom's part itself is
   // asked for.  (One lane in eight warps was that deep, and took its warp
   // through the general term.)
-  double dC = sf::mul_mid(sf::mul_mid(MC, K), H), dB = sf::mul_mid(sf::mul_mid(MB, K), H);
+  const double dC = (sec_sun + DuC) * K * H, dB = (sec_sun + DuB) * K * H;
   const bool deepC = fm::bits(dC) > 0x4069000000000000LL, deepB = fm::bits(dB) > 0x4069000000000000LL;
-  const double xC = deepC ? -200.0 : -dC, xB = deepB ? -200.0 : -dB;
-  bool ok = near_x && ((sc.near_mask >> b) & 1) && !(deepB && want_B);
-  const double eC = sf::exp_neg(xC, ok), eB = sf::exp_neg(xB, ok);
-  const double oC = 1.0 - eC;
-  const double rrs_C = sf::mul_mid(rrs_dp, oC);
+  bool ok = !(deepB && want_B);
+  const double eC = sf::exp_neg(deepC ? -200.0 : -dC, ok);
+  const double eB = sf::exp_neg(deepB ? -200.0 : -dB, ok);
+  const double rrs_C = rrs_dp * (1.0 - eC);
   const double rho_pi = fma(rho, fm::kPiHi, rho * fm::kPiLo);
-  const double rrs_B = sf::mul_mid(rho_pi, eB);
+  const double rrs_B = rho_pi * eB;
   const double rrs = rrs_C + rrs_B;
-  const double den = 1.0 - sf::mul_mid(1.5, rrs);
+  const double den = 1.0 - 1.5 * rrs;
   const double Rm = sf::div_mid(sf::half_mid(rrs), den);
   const double d = Rm - r;
   t.K = K;
   t.rrs_B = rrs_B;
   t.rrs = rrs;
   t.Rm = Rm;
-  t.dd = sf::mul_mid(d, d);
-  ok = ok && sf::near(c) && sf::near_positive(ab) && sf::near_positive(u) &&
-       sf::near_positive(MC) && sf::near_positive(MB) && sf::near_positive(oC) &&
-       sf::near_positive(rrs) && sf::near(den) && sf::near(d);
+  t.dd = d * d;
+  ok = ok && sf::near_positive(bb) && sf::near_positive(ab) && sf::near_positive(u) &&
+       sf::near_positive(dC) && sf::near_positive(dB) && sf::near_positive(rho) &&
+       sf::near_positive(rrs) && sf::near(den);
   // (deep: rrs_B at most 2^90 2^-288, below half an ulp of rrs above 2^-90)
   if (deepB) ok = ok && sf::lt(rho_pi, 0x1p90) && sf::lt(0x1p-90, rrs);
   if (!ok) {
@@ -259,16 +256,13 @@ __device__ __forceinline__ double cost_f64(const FitParams &fp, const SceneConst
   const double X = 0.01 * fabs(x[5]);
   const double lnP = log(P);
   const double qB = q * B;
-  const bool near_x = sf::near_positive(H) && sf::near_positive(qB) && sf::near_positive(P) &&
-                      sf::near_positive(G) && sf::near_positive(X) && sf::near(lnP);
   double err = 0.0, K_min = 1.0e4, iod = 0.0;
 #pragma unroll 1
   for (int b = 0; b < nb; b++) {
     BandTerm t;
     bool want_B = kDetails;
     if constexpr (kKeep) want_B = keep->want;
-    band_term(sc, b, sc.sec_sun, near_x && sf::near_positive(px.pw[b]), want_B, H,
-              qB * sc.refl[b], P, lnP, G, X, px.pw[b], px.rrs[b], t);
+    band_term(sc, b, sc.sec_sun, want_B, H, qB * sc.refl[b], P, lnP, G, X, px.pw[b], px.rrs[b], t);
     err = err + t.dd;
     if (k_counts(t.K) && sf::lt(t.K, K_min)) K_min = t.K;
     if (kDetails) {

@@ -19,7 +19,6 @@
 #include "../../include/photic.h"
 #include "../../include/photic_nc.h"
 #include "photic_kernels.h"
-#include "photic_softfp.cuh"
 #include "photic_params.h"
 #include "photic_tables.h"
 
@@ -169,15 +168,6 @@ double table_at(const double *tab, double x) {
   return interp_apply(resolve_interp(tables::wl, tables::kNRef, x), tab);
 }
 
-// Bands whose constants band_term's soft operations take (photic_fp64.cuh).
-void set_near_mask(SceneConsts &sc, int nb) {
-  sc.near_mask = 0;
-  for (int b = 0; b < nb; b++)
-    if (sf::near(sc.a1[b]) && sf::near_positive(sc.eS[b]) && sf::near_positive(sc.refl[b]) &&
-        sf::near_positive(sc.sec_view) && sc.bbw[b] >= 0.0)
-      sc.near_mask |= 1u << b;
-}
-
 // Scene constants for a subsurface sun zenith (samodel():521-618).
 void make_scene(const photic_config &cfg, double theta_sun_deg, SceneConsts &sc) {
   memset(&sc, 0, sizeof sc);
@@ -201,7 +191,6 @@ void make_scene(const photic_config &cfg, double theta_sun_deg, SceneConsts &sc)
     sc.eS[b] = exp(-S * (l - 440.0));
     sc.ratio440[b] = 440.0 / l;
   }
-  set_near_mask(sc, cfg.n_bands);
 }
 
 void make_fit(const photic_config &cfg, FitParams &fp) {
@@ -1478,7 +1467,6 @@ int from_md(const photic_model_data *md, int s, photic_config &cfg, FitParams &f
   sc.sec_sun = md->sec_theta_sun[s];
   sc.sec_view = md->sec_theta_view[s];
   sc.h_tide = cfg.h_tide;
-  set_near_mask(sc, nb);
   return PHOTIC_OK;
 }
 

@@ -124,15 +124,13 @@ __device__ __forceinline__ double jcost(const JointArgs &a, const JPixel<K, NB> 
       X = 0.01 * fabs(x[4 + 4 * s]);
     }
     const double lnP = log(P);
-    const bool near_x = sf::near_positive(H) && sf::near_positive(qB) && sf::near_positive(P) &&
-                        sf::near_positive(G) && sf::near_positive(X) && sf::near(lnP);
     double km = 1.0e4;
 #pragma unroll 1  // the pixel is in local memory; one copy of the band term
     for (int b = 0; b < NB; b++) {
       if (b < nb) {
         BandTerm t;
-        band_term(sc, b, px.sec_sun[s], near_x && sf::near_positive(px.pw[s][b]), kDetails, H,
-                  qB * sc.refl[b], P, lnP, G, X, px.pw[s][b], px.rrs[s][b], t);
+        band_term(sc, b, px.sec_sun[s], kDetails, H, qB * sc.refl[b], P, lnP, G, X, px.pw[s][b],
+                  px.rrs[s][b], t);
         err = err + t.dd;
         const double Kb = t.K;
         if (k_counts(Kb) && sf::lt(Kb, km)) km = Kb;

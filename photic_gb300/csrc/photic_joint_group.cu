@@ -307,11 +307,8 @@ __global__ void __launch_bounds__(kBlock) joint_group_kernel(const __grid_consta
       const double Gg = 0.01 * fabs(x[cP + 1]);
       const double Xx = 0.01 * fabs(x[cP + 2]);
       const double lnP = log(P);
-      const bool near_x = sf::near_positive(H) && sf::near_positive(qB) && sf::near_positive(P) &&
-                          sf::near_positive(Gg) && sf::near_positive(Xx) && sf::near(lnP) &&
-                          sf::near_positive(my_pw);
       BandTerm t;
-      band_term(sc, bb, my_sec, near_x, final_eval, H, qB * sc.refl[bb], P, lnP, Gg, Xx, my_pw, my_rrs, t);
+      band_term(sc, bb, my_sec, final_eval, H, qB * sc.refl[bb], P, lnP, Gg, Xx, my_pw, my_rrs, t);
       g.dd[gl] = t.dd;
       g.kk[gl] = t.K;
       if (final_eval) g.io[gl] = t.rrs_B / t.rrs;

@@ -78,7 +78,7 @@ struct NmPixel {
     if (kcount <= icount) return false;
     T yhi = F(0);
     hi = 0;
-#pragma unroll
+#pragma unroll 1
     for (int j = 1; j <= N; j++) {
       const T fj = F(j);
       if (P::lt(yhi, fj)) {
@@ -150,7 +150,7 @@ struct NmPixel {
           phase = PH_EXPAND;
         } else {
           int worse = 0;
-#pragma unroll
+#pragma unroll 1
           for (int j = 0; j <= N; j++)
             if (P::lt(fr, F(j))) worse++;
           if (worse > 1) {

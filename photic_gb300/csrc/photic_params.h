@@ -32,8 +32,6 @@ struct SceneConsts {
   double eS[kMaxBands];       // exp(-0.015 * (lambda - 440)), host libm
   double ratio440[kMaxBands]; // 440 / lambda
   double sec_sun, sec_view, h_tide;
-  uint32_t near_mask;         // bands whose constants (and both secants) the cost's soft
-                              // operations take: not zero, of moderate exponent
 };
 
 // K-penalty constants of samodel_error (model/samodel.c:2696-2732):

@@ -653,11 +653,8 @@ __global__ void __launch_bounds__(BLOCK, 1) region_kernel(const __grid_constant_
         double rho = 0.0;
 #pragma unroll 1
         for (int k = 0; k < nbt; k++) rho += wB[r * nbt + k] * sc.refl_k[k][b];
-        const bool near_x = sf::near_positive(H) && sf::near_positive(rho) &&
-                            sf::near_positive(P) && sf::near_positive(Gg) &&
-                            sf::near_positive(Xx) && sf::near(lnP) && sf::near_positive(pw);
         BandTerm t;
-        band_term(sc, b, a.sec_sun[s], near_x, final_eval, H, rho, P, lnP, Gg, Xx, pw, my_rrs[h], t);
+        band_term(sc, b, a.sec_sun[s], final_eval, H, rho, P, lnP, Gg, Xx, pw, my_rrs[h], t);
         dd[tau] = t.dd;
         kk[tau] = t.K;
         if (final_eval) {

@@ -295,7 +295,7 @@ PHOTIC_FM_HD uint64_t shift_round(uint64_t v, uint32_t s) { return ((v >> (s - 1
 // single-precision pipe; the polynomial's three fused multiply-adds
 // c1 = r/120 + 1/24, c2 = c1 r + 1/6, c = c2 r + 1/2, whose results lie in
 // known binades, are fixed-point products rounded to the grid of the double;
-// r r is mul_mid; five FP64 operations remain.  A product of a 53-bit and a
+// six FP64 operations remain.  A product of a 53-bit and a
 // 53-bit significand that is shifted down by s >= 62 places could only lie
 // half way between two grid points with 61 trailing zeros; with fewer than 21
 // in r and fewer than 32 in c1 and c2 it never does.
@@ -340,7 +340,7 @@ PHOTIC_FM_HD double exp_neg(double x, bool &ok) {
   v = shift_round(mulhi(mr, c2), neg ? er : 1 + er);
   ok = ok && (uint32_t)c1 != 0 && (uint32_t)c2 != 0;
   const double c = from_bits((int64_t)(0x3fe0000000000000ull + (neg ? 0 - v : v)));
-  const double p = fma(mul_mid(r, r), c, r);
+  const double p = fma(r * r, c, r);
   const int j = -N & 63;
 #if defined(__CUDA_ARCH__)
   const double2 T = __ldg(reinterpret_cast<const double2 *>(fm::kExp2TabDev) + j);
