@@ -4,15 +4,22 @@
 // the building block of the surrogate MLP (photic_mlp.cu): forward layers
 // (bias + SiLU), input gradients (times SiLU') and weight gradients.
 //
-// One CTA (4 warps) owns a 128 x BN output tile (or, split-K, one slice of
+// One CTA (8 warps) owns a 128 x BN output tile (or, split-K, one slice of
 // K of it: the weight-gradient products have 128 x 128 outputs and K = the
 // batch, so their K is spread over CTAs and the partial sums are added in a
-// fixed order by a second kernel).  K is consumed in chunks
-// of 64: all threads stage the A and B chunks into shared memory in the
-// canonical no-swizzle core-matrix layout (16-byte vector loads), one
-// thread issues four K=16 MMAs and commits them to an mbarrier, everyone
-// waits (bounded), and the epilogue reads the accumulator back with
-// tcgen05.ld, one TMEM lane (= output row) per thread.
+// fixed order by a second kernel).  K is consumed in chunks of 64 through two
+// buffers: all threads stage the A and B chunks into shared memory in the
+// canonical no-swizzle core-matrix layout (16-byte vector loads; an operand
+// stored with K as its rows is transposed 8 x 8 in registers on the way), one
+// thread issues four K=16 MMAs and commits them to the buffer's mbarrier while
+// the others stage the next chunk, every wait is bounded, and the epilogue
+// reads the accumulator back with tcgen05.ld, one TMEM lane (= output row) per
+// thread, sixteen columns at a time in 16-byte accesses.
+//
+// At the MLP's sizes (8 192 x 128 x 128) the products are bound by the
+// epilogue's and the staging's memory instructions, not by the tensor cores:
+// with four warps and an element per access a forward layer took 49 us, now 15
+// (from cold caches; half-width tiles on twice the SMs took as long).
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -25,6 +32,7 @@ namespace photic {
 namespace {
 
 constexpr int kBM = 128, kBN = 128, kBK = 64;
+constexpr int kThreads = 256;
 constexpr uint32_t kTmemCols = 256;        // >= any N the descriptor can name here
 constexpr uint32_t kWaitLimit = 1u << 26;  // bounded mbarrier spin
 
@@ -50,23 +58,141 @@ __device__ __forceinline__ void stage(const __nv_bfloat16 *src, int ld, int nrow
   }
 }
 
-__global__ void __launch_bounds__(128) tn_gemm_kernel(const __grid_constant__ GemmArgs g) {
+// The same from a matrix stored with K as its rows (element (r, k) at
+// src[k * ld + r]): eight rows of eight values a thread, transposed in
+// registers.  ld and r0 are multiples of 8 and the rows 16-byte aligned.
+__device__ __forceinline__ void stage_k_rows(const __nv_bfloat16 *src, int ld, int nrows_total,
+                                             int r0, int rows, int k0, int K, unsigned char *dst,
+                                             int thread, int threads) {
+  const int blocks = rows >> 3;
+  for (int v = thread; v < blocks * (kBK / 8); v += threads) {
+    const int rb = v % blocks, c = v / blocks;
+    uint4 a[8];
+#pragma unroll
+    for (int k = 0; k < 8; k++) {
+      const int gk = k0 + c * 8 + k;
+      a[k] = make_uint4(0u, 0u, 0u, 0u);
+      if (gk < K && r0 + rb * 8 < nrows_total)
+        a[k] = *reinterpret_cast<const uint4 *>(src + (size_t)gk * ld + r0 + rb * 8);
+    }
+#pragma unroll
+    for (int m = 0; m < 8; m++) {
+      uint32_t w[4];
+#pragma unroll
+      for (int i = 0; i < 4; i++) {
+        const uint4 &lo = a[2 * i], &hi = a[2 * i + 1];
+        const uint32_t x = m < 2 ? lo.x : m < 4 ? lo.y : m < 6 ? lo.z : lo.w;
+        const uint32_t y = m < 2 ? hi.x : m < 4 ? hi.y : m < 6 ? hi.z : hi.w;
+        w[i] = __byte_perm(x, y, (m & 1) ? 0x7632 : 0x5410);
+      }
+      *reinterpret_cast<uint4 *>(dst + (rb * 8 + c) * 128 + m * 16) =
+          make_uint4(w[0], w[1], w[2], w[3]);
+    }
+  }
+}
+
+__device__ __forceinline__ uint32_t pack_bf16(float a, float b) {
+  const __nv_bfloat162 h = __halves2bfloat162(__float2bfloat16(a), __float2bfloat16(b));
+  return *reinterpret_cast<const uint32_t *>(&h);
+}
+
+// Columns [col, col + 16) of a row, 16-byte accesses.
+__device__ __forceinline__ void store16(float *dst, const float (&v)[16]) {
+#pragma unroll
+  for (int j = 0; j < 4; j++)
+    reinterpret_cast<float4 *>(dst)[j] =
+        make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+}
+__device__ __forceinline__ void store16(__nv_bfloat16 *dst, const float (&v)[16]) {
+#pragma unroll
+  for (int j = 0; j < 2; j++)
+    reinterpret_cast<uint4 *>(dst)[j] =
+        make_uint4(pack_bf16(v[8 * j], v[8 * j + 1]), pack_bf16(v[8 * j + 2], v[8 * j + 3]),
+                   pack_bf16(v[8 * j + 4], v[8 * j + 5]), pack_bf16(v[8 * j + 6], v[8 * j + 7]));
+}
+__device__ __forceinline__ void epilogue16(const GemmArgs &g, __nv_bfloat16 *gO, int64_t row,
+                                           int col, float (&v)[16]) {
+  switch (g.epi) {
+    case EPI_F32:
+      store16(g.C + row * g.ldc + col, v);
+      break;
+    case EPI_BIAS_F32:
+#pragma unroll
+      for (int j = 0; j < 16; j++) v[j] = v[j] + g.bias[col + j];
+      store16(g.C + row * g.ldc + col, v);
+      break;
+    case EPI_BIAS_SILU:
+#pragma unroll
+      for (int j = 0; j < 16; j++) v[j] = v[j] + g.bias[col + j];
+      if (g.Z) store16(g.Z + row * g.ldz + col, v);
+#pragma unroll
+      for (int j = 0; j < 16; j++) v[j] = silu(v[j]);
+      store16(gO + row * g.ldo + col, v);
+      break;
+    case EPI_DSILU: {
+      float z[16];
+#pragma unroll
+      for (int j = 0; j < 4; j++) {
+        const float4 t = reinterpret_cast<const float4 *>(g.Z + row * g.ldz + col)[j];
+        z[4 * j] = t.x;
+        z[4 * j + 1] = t.y;
+        z[4 * j + 2] = t.z;
+        z[4 * j + 3] = t.w;
+      }
+#pragma unroll
+      for (int j = 0; j < 16; j++) v[j] = v[j] * dsilu(z[j]);
+      store16(gO + row * g.ldo + col, v);
+      break;
+    }
+    default:
+      break;
+  }
+}
+__device__ __forceinline__ void epilogue1(const GemmArgs &g, __nv_bfloat16 *gO, int64_t row,
+                                          int col, float acc) {
+  switch (g.epi) {
+    case EPI_F32:
+      g.C[row * g.ldc + col] = acc;
+      break;
+    case EPI_BIAS_F32:
+      g.C[row * g.ldc + col] = acc + g.bias[col];
+      break;
+    case EPI_BIAS_SILU: {
+      const float z = acc + g.bias[col];
+      if (g.Z) g.Z[row * g.ldz + col] = z;
+      gO[row * g.ldo + col] = __float2bfloat16(silu(z));
+      break;
+    }
+    case EPI_DSILU:
+      gO[row * g.ldo + col] = __float2bfloat16(acc * dsilu(g.Z[row * g.ldz + col]));
+      break;
+    default:
+      break;
+  }
+}
+
+// blockIdx.z: the product of the batch, and its slice of K.
+__global__ void __launch_bounds__(kThreads) tn_gemm_kernel(const __grid_constant__ GemmBatch b) {
+  const GemmArgs &g = b.g[blockIdx.z / b.slices];
+  const int slice = blockIdx.z % b.slices;
   const __nv_bfloat16 *gA = reinterpret_cast<const __nv_bfloat16 *>(g.A);
   const __nv_bfloat16 *gB = reinterpret_cast<const __nv_bfloat16 *>(g.B);
   __nv_bfloat16 *gO = reinterpret_cast<__nv_bfloat16 *>(g.O);
   extern __shared__ __align__(1024) unsigned char smem[];
-  unsigned char *sA = smem;                      // kBM x kBK
-  unsigned char *sB = smem + kBM * kBK * 2;      // kBN x kBK
-  __shared__ __align__(8) uint64_t mbar;
+  constexpr int kBufBytes = (kBM + kBN) * kBK * 2;  // a chunk of A, then of B
+  __shared__ __align__(8) uint64_t mbar[2];
   __shared__ uint32_t tmem_slot;
 
   const int m0 = blockIdx.x * kBM, n0 = blockIdx.y * kBN;
   const int ncols = min(kBN, g.N - n0);          // valid output columns of this tile
   const int mma_n = (ncols + 15) / 16 * 16;      // MMA N: multiple of 16, <= 128
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 
   if (warp == 0) tc::tmem_alloc(&tmem_slot, kTmemCols);
-  if (threadIdx.x == 0) tc::mbar_init(&mbar, 1);
+  if (tid == 0) {
+    tc::mbar_init(&mbar[0], 1);
+    tc::mbar_init(&mbar[1], 1);
+  }
   tc::fence_before_sync();
   __syncthreads();
   tc::fence_after_sync();
@@ -77,15 +203,39 @@ __global__ void __launch_bounds__(128) tn_gemm_kernel(const __grid_constant__ Ge
   // split-K: CTA z takes chunks [c0, c1) of K and writes a partial sum
   const int nchunks = (g.K + kBK - 1) / kBK;
   const int per = g.ksplit > 1 ? (nchunks + g.ksplit - 1) / g.ksplit : nchunks;
-  const int c0 = (int)blockIdx.z * per;
+  const int c0 = slice * per;
   const int c1 = min(nchunks, c0 + per);
-  for (int kc = c0; kc < c1 && ok; kc++) {
+  // Wait for the MMAs of chunk kc (the n-th use of its buffer).  A wait that
+  // runs out records the error and gives the tensor core a second bounded
+  // chance to finish before the shared memory and TMEM go away.
+  auto finished = [&](int kc) {
+    const int u = kc - c0;
+    const uint32_t parity = (uint32_t)(u >> 1) & 1u;
+    if (tc::mbar_wait(&mbar[u & 1], parity, kWaitLimit)) return true;
+    if (tid == 0) atomicOr(g.error, PHOTIC_DEVERR_MMA_TIMEOUT);
+    tc::mbar_wait(&mbar[u & 1], parity, kWaitLimit);
+    return false;
+  };
+  int issued = 0;  // chunks whose MMAs are committed
+  for (int kc = c0; kc < c1; kc++) {
     const int k0 = kc * kBK;
-    stage(gA, g.lda, g.M, m0, kBM, k0, g.K, sA);
-    stage(gB, g.ldb, g.N, n0, kBN, k0, g.K, sB);
+    unsigned char *sA = smem + ((kc - c0) & 1) * kBufBytes, *sB = sA + kBM * kBK * 2;
+    if (kc - c0 >= 2 && ok) ok = finished(kc - 2);
+    if (!__syncthreads_and(ok)) {
+      ok = false;
+      break;
+    }
+    if (g.k_rows) {
+      stage_k_rows(gA, g.lda, g.M, m0, kBM, k0, g.K, sA, tid, kThreads / 2);
+      if (tid >= kThreads / 2)
+        stage_k_rows(gB, g.ldb, g.N, n0, mma_n, k0, g.K, sB, tid - kThreads / 2, kThreads / 2);
+    } else {
+      stage(gA, g.lda, g.M, m0, kBM, k0, g.K, sA);
+      stage(gB, g.ldb, g.N, n0, mma_n, k0, g.K, sB);
+    }
     tc::fence_smem_async();
     __syncthreads();
-    if (threadIdx.x == 0) {
+    if (tid == 0) {
       tc::fence_after_sync();
       const uint32_t a0 = tc::smem_u32(sA), b0 = tc::smem_u32(sB);
 #pragma unroll
@@ -96,63 +246,42 @@ __global__ void __launch_bounds__(128) tn_gemm_kernel(const __grid_constant__ Ge
           tc::mma_bf16(tmem, ad, bd, idesc, (kc > c0 || kk > 0) ? 1u : 0u);
         }
       }
-      tc::mma_commit(&mbar);
+      tc::mma_commit(&mbar[(kc - c0) & 1]);
     }
-    if (!tc::mbar_wait(&mbar, (uint32_t)((kc - c0) & 1), kWaitLimit)) {
-      ok = false;
-      if (threadIdx.x == 0) atomicOr(g.error, PHOTIC_DEVERR_MMA_TIMEOUT);
-      // give the tensor core a second bounded chance to finish before the
-      // shared memory and TMEM go away
-      tc::mbar_wait(&mbar, (uint32_t)((kc - c0) & 1), kWaitLimit);
-    }
-    tc::fence_after_sync();
-    __syncthreads();
+    issued++;
   }
+  // no MMA stays in flight on any exit
+  for (int u = issued > 2 ? issued - 2 : 0; u < issued; u++)
+    if (!finished(c0 + u)) ok = false;
+  ok = __syncthreads_and(ok) != 0;
+  tc::fence_after_sync();
 
+  const int64_t row = m0 + (warp & 3) * 32 + lane;
   if (ok && c1 <= c0) {
     // an empty split contributes zeros
-    const int row = m0 + warp * 32 + lane;
-    if (row < g.M)
+    if (row < g.M && warp < 4)
       for (int j = 0; j < ncols; j++)
-        g.partial[((size_t)blockIdx.z * g.M + row) * g.N + n0 + j] = 0.0f;
+        g.partial[((size_t)slice * g.M + row) * g.N + n0 + j] = 0.0f;
   } else if (ok) {
-    const int row = m0 + warp * 32 + lane;
-    for (int cc = 0; cc < mma_n; cc += 16) {
+    // warps 0-3 and 4-7 share the TMEM lanes and take every other 16 columns
+    for (int cc = (warp >> 2) * 16; cc < mma_n; cc += 32) {
       float v[16];
-      tc::tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)cc, v);
+      tc::tmem_ld16(tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)cc, v);
+      const int col = n0 + cc;
       if (row < g.M) {
+        if (g.vec && cc + 16 <= ncols) {
+          if (g.partial) store16(g.partial + ((size_t)slice * g.M + row) * g.N + col, v);
+          else epilogue16(g, gO, row, col, v);
+        } else {
 #pragma unroll
-        for (int j = 0; j < 16; j++) {
-          const int col = n0 + cc + j;
-          if (cc + j >= ncols) break;
-          float acc = v[j];
-          if (g.partial) {
-            g.partial[((size_t)blockIdx.z * g.M + row) * g.N + col] = acc;
-            continue;
-          }
-          switch (g.epi) {
-            case EPI_F32:
-              g.C[(size_t)row * g.ldc + col] = acc;
-              break;
-            case EPI_BIAS_F32:
-              g.C[(size_t)row * g.ldc + col] = acc + g.bias[col];
-              break;
-            case EPI_BIAS_SILU: {
-              const float z = acc + g.bias[col];
-              if (g.Z) g.Z[(size_t)row * g.ldz + col] = z;
-              gO[(size_t)row * g.ldo + col] = __float2bfloat16(silu(z));
-              break;
-            }
-            case EPI_DSILU: {
-              const float z = g.Z[(size_t)row * g.ldz + col];
-              gO[(size_t)row * g.ldo + col] = __float2bfloat16(acc * dsilu(z));
-              break;
-            }
-            default:
-              break;
+          for (int j = 0; j < 16; j++) {
+            if (cc + j >= ncols) break;
+            if (g.partial) g.partial[((size_t)slice * g.M + row) * g.N + col + j] = v[j];
+            else epilogue1(g, gO, row, col + j, v[j]);
           }
         }
       }
+      __syncwarp();
     }
   }
   tc::fence_before_sync();
@@ -168,6 +297,7 @@ __global__ void splitk_reduce_kernel(const float *partial, int S, int M, int N, 
   if (i >= (int64_t)M * N) return;
   const int r = (int)(i / N), c = (int)(i % N);
   float s = 0.0f;
+#pragma unroll 16  // the loads of sixteen splits in flight; the additions in order
   for (int z = 0; z < S; z++) s += partial[(size_t)z * M * N + i];
   C[(size_t)r * ldc + c] = s;
 }
@@ -178,14 +308,38 @@ __global__ void splitk_reduce_kernel(const float *partial, int S, int M, int N, 
 // TMEM of resident CTAs (2 x 256 of 512 columns) never over-subscribes.
 size_t gemm_smem_bytes() { return 96 * 1024; }
 
-cudaError_t launch_gemm(const GemmArgs &g, cudaStream_t s) {
-  if (g.M <= 0 || g.N <= 0) return cudaSuccess;
+namespace {
+
+// 16-byte accesses of the epilogue: every row of every array that it touches
+// on a 16-byte boundary.
+int epilogue_vec(const GemmArgs &a) {
+  auto rows16 = [](const void *p, int64_t row_bytes) {
+    return p == nullptr || (((uintptr_t)p | (uintptr_t)row_bytes) & 15u) == 0;
+  };
+  return a.partial ? rows16(a.partial, (int64_t)a.N * 4)
+                   : rows16(a.C, (int64_t)a.ldc * 4) && rows16(a.Z, (int64_t)a.ldz * 4) &&
+                         rows16(a.O, (int64_t)a.ldo * 2);
+}
+
+cudaError_t launch_batch(const GemmBatch &b, int n, int M, int N, cudaStream_t s) {
   const size_t smem = gemm_smem_bytes();
   cudaError_t e = cudaFuncSetAttribute(tn_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)smem);
   if (e != cudaSuccess) return e;
+  dim3 grid((unsigned)((M + kBM - 1) / kBM), (unsigned)((N + kBN - 1) / kBN),
+            (unsigned)(b.slices * n));
+  tn_gemm_kernel<<<grid, kThreads, smem, s>>>(b);
+  return cudaGetLastError();
+}
+
+}  // namespace
+
+cudaError_t launch_gemm(const GemmArgs &g, cudaStream_t s) {
+  if (g.M <= 0 || g.N <= 0) return cudaSuccess;
   const int nchunks = (g.K + kBK - 1) / kBK;
-  GemmArgs a = g;
+  GemmBatch b{};
+  GemmArgs &a = b.g[0];
+  a = g;
   int S = 1;
   if (g.ksplit > 1 && g.partial && g.epi == EPI_F32 && nchunks > 1) {
     const int per = (nchunks + g.ksplit - 1) / g.ksplit;
@@ -195,14 +349,34 @@ cudaError_t launch_gemm(const GemmArgs &g, cudaStream_t s) {
     a.ksplit = 1;
     a.partial = nullptr;
   }
-  dim3 grid((unsigned)((g.M + kBM - 1) / kBM), (unsigned)((g.N + kBN - 1) / kBN), (unsigned)S);
-  tn_gemm_kernel<<<grid, 128, smem, s>>>(a);
-  if (S > 1) {
+  a.vec = epilogue_vec(a);
+  b.slices = S;
+  cudaError_t e = launch_batch(b, 1, g.M, g.N, s);
+  if (e == cudaSuccess && S > 1) {
     const int64_t n = (int64_t)g.M * g.N;
-    splitk_reduce_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(a.partial, S, g.M, g.N, g.C,
+    splitk_reduce_kernel<<<(unsigned)((n + 127) / 128), 128, 0, s>>>(a.partial, S, g.M, g.N, g.C,
                                                                      g.ldc);
+    e = cudaGetLastError();
   }
-  return cudaGetLastError();
+  return e;
+}
+
+// Split-K products of one M and K in one launch, the partial sums left in
+// their scratch: [slices][M][N] each.  Returns the slices.
+cudaError_t launch_gemm_partials(const GemmArgs *g, int n, int *slices, cudaStream_t s) {
+  GemmBatch b{};
+  const int nchunks = (g[0].K + kBK - 1) / kBK;
+  const int per = (nchunks + g[0].ksplit - 1) / g[0].ksplit;
+  b.slices = (nchunks + per - 1) / per;
+  int N = 0;
+  for (int i = 0; i < n; i++) {
+    b.g[i] = g[i];
+    b.g[i].ksplit = b.slices;
+    b.g[i].vec = epilogue_vec(b.g[i]);
+    N = g[i].N > N ? g[i].N : N;
+  }
+  *slices = b.slices;
+  return launch_batch(b, n, g[0].M, N, s);
 }
 
 }  // namespace photic

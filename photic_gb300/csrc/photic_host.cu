@@ -973,14 +973,18 @@ struct WorkAlloc {
     const size_t bfH = (size_t)Rpad * kMlpH * 2, fH = (size_t)Rpad * kMlpH * 4;
     size_t oX0 = take((size_t)Rpad * kMlpIn * 2), oA1 = take(bfH), oA2 = take(bfH), oA3 = take(bfH);
     size_t oY = take((size_t)Rpad * kMlpOut * 4);
-    size_t oZ1 = 0, oZ2 = 0, oZ3 = 0, odY = 0, odZ = 0, odZ2 = 0, oT1 = 0, oT2 = 0, oG4 = 0, oG = 0,
-           oSK = 0;
+    size_t oZ1 = 0, oZ2 = 0, oZ3 = 0, odY = 0, odZ1 = 0, odZ2 = 0, odZ3 = 0, oG = 0, oP[4] = {},
+           oC[4] = {};
+    const int nW[4] = {kMlpIn, kMlpH, kMlpH, kMlpOut}, nC[4] = {kMlpH, kMlpH, kMlpH, kMlpOut};
     if (train) {
       oZ1 = take(fH); oZ2 = take(fH); oZ3 = take(fH);
-      odY = take((size_t)Rpad * kMlpOut * 2); odZ = take(bfH); odZ2 = take(bfH);
-      oT1 = take(bfH); oT2 = take(bfH);
-      oG4 = take((size_t)kMlpH * kMlpOut * 4); oG = take((size_t)kMlpParams * 4);
-      oSK = take((size_t)kMlpSplitK * kMlpH * kMlpH * 4);
+      odY = take((size_t)Rpad * kMlpOut * 2);
+      odZ1 = take(bfH); odZ2 = take(bfH); odZ3 = take(bfH);
+      oG = take((size_t)kMlpParams * 4);
+      for (int l = 0; l < 4; l++) {
+        oP[l] = take((size_t)kMlpSplitK * kMlpH * nW[l] * 4);
+        oC[l] = take((size_t)256 * nC[l] * 4);
+      }
     }
     cudaError_t e = ws_alloc(&mem, off, s);
     if (e != cudaSuccess) return e;
@@ -992,10 +996,13 @@ struct WorkAlloc {
     w.Y = (float *)(b + oY);
     if (train) {
       w.Z1 = (float *)(b + oZ1); w.Z2 = (float *)(b + oZ2); w.Z3 = (float *)(b + oZ3);
-      w.dY = (__nv_bfloat16 *)(b + odY); w.dZ = (__nv_bfloat16 *)(b + odZ);
-      w.dZ2 = (__nv_bfloat16 *)(b + odZ2); w.T1 = (__nv_bfloat16 *)(b + oT1);
-      w.T2 = (__nv_bfloat16 *)(b + oT2); w.G4t = (float *)(b + oG4); w.grad = (float *)(b + oG);
-      w.splitk = (float *)(b + oSK);
+      w.dY = (__nv_bfloat16 *)(b + odY); w.dZ1 = (__nv_bfloat16 *)(b + odZ1);
+      w.dZ2 = (__nv_bfloat16 *)(b + odZ2); w.dZ3 = (__nv_bfloat16 *)(b + odZ3);
+      w.grad = (float *)(b + oG);
+      for (int l = 0; l < 4; l++) {
+        w.part[l] = (float *)(b + oP[l]);
+        w.cols[l] = (float *)(b + oC[l]);
+      }
     }
     return cudaSuccess;
   }

@@ -232,10 +232,18 @@ struct GemmArgs {
   unsigned int *error;
   int lbo, sbo;    // core-matrix strides of the shared-memory layout (bytes)
   int epi;
+  int k_rows;      // A and B are stored [K][lda], [K][ldb] (lda, ldb multiples of 8)
+  int vec;         // set by launch_gemm: the epilogue's rows allow 16-byte accesses
   int ksplit;      // > 1: split K over this many CTAs (EPI_F32 only) ...
   float *partial;  // ... with partial sums in [ksplit][M][N] scratch
 };
+constexpr int kGemmBatch = 4;
+struct GemmBatch {
+  GemmArgs g[kGemmBatch];
+  int slices;  // K slices of each product
+};
 cudaError_t launch_gemm(const GemmArgs &g, cudaStream_t s);
+cudaError_t launch_gemm_partials(const GemmArgs *g, int n, int *slices, cudaStream_t s);
 
 // Surrogate MLP (photic_mlp.cu): 6 (padded 16) -> 128 -> 128 -> 128 -> 5
 // (padded 16).  FP32 master parameters, flat, in this order.
@@ -257,9 +265,12 @@ struct MlpState {
 };
 constexpr int kMlpSplitK = 64;  // K splits of the weight-gradient products
 struct MlpWork {
-  __nv_bfloat16 *X0, *A1, *A2, *A3, *dY, *dZ, *dZ2, *T1, *T2;
-  float *Z1, *Z2, *Z3, *Y, *G4t, *grad;
-  float *splitk;  // [kMlpSplitK][128][128] partial sums (training)
+  __nv_bfloat16 *X0, *A1, *A2, *A3, *dY, *dZ3, *dZ2, *dZ1;
+  float *Z1, *Z2, *Z3, *Y, *grad;
+  // training: the weight gradients' partial sums, per layer [slices][128][N]
+  // with N = 16, 128, 128, 16 (kMlpSplitK slices at most), and the biases'
+  // [256][C] with C = 128, 128, 128, 16
+  float *part[4], *cols[4];
 };
 // Band constants in single precision, for the seed polish.
 struct SceneF32 {

@@ -12,8 +12,8 @@
 // Backward (MSE on standardised targets):
 //   dW_l = dZ_l^T A_{l-1},  db_l = colsum(dZ_l),
 //   dZ_{l-1} = (dZ_l W_l) * SiLU'(Z_{l-1}).
-// Every product is one TN GEMM; the transposed operands it needs are
-// formed by small transpose kernels.  Adam keeps FP32 master weights and
+// Every product is one GEMM of photic_gemm.cu, which transposes the weight
+// gradients' operands as it stages them.  Adam keeps FP32 master weights and
 // refreshes the BF16 copies (and their transposes) after each step.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -41,21 +41,6 @@ __global__ void featurize_kernel(const float *x, int R, int Rpad, const float *i
   }
 }
 
-// dst[c][r] = src[r][c] (BF16), rows padded with zeros up to Rpad.
-__global__ void transpose_kernel(const bf16 *src, int R, int C, int Rpad, bf16 *dst) {
-  __shared__ bf16 tile[32][33];
-  const int r0 = blockIdx.x * 32, c0 = blockIdx.y * 32;
-  for (int i = threadIdx.y; i < 32; i += blockDim.y) {
-    const int r = r0 + i, c = c0 + threadIdx.x;
-    tile[i][threadIdx.x] = (r < R && c < C) ? src[(size_t)r * C + c] : __float2bfloat16(0.0f);
-  }
-  __syncthreads();
-  for (int i = threadIdx.y; i < 32; i += blockDim.y) {
-    const int c = c0 + i, r = r0 + threadIdx.x;
-    if (c < C && r < Rpad) dst[(size_t)c * Rpad + r] = tile[threadIdx.x][i];
-  }
-}
-
 // MSE on standardised targets; dY = 2 (Y - t) / (R * 5) as BF16, padding 0.
 __global__ void loss_grad_kernel(const float *Y, const float *t, int R, int Rpad,
                                  const float *out_mean, const float *out_std, bf16 *dY,
@@ -80,27 +65,83 @@ __global__ void loss_grad_kernel(const float *Y, const float *t, int R, int Rpad
   if ((threadIdx.x & 31) == 0 && loss) atomicAdd(loss, l / (float)(R * 5));
 }
 
-// colsum over rows of a [R][C] BF16 matrix into FP32 g[C].
-__global__ void colsum_kernel(const bf16 *m, int R, int C, float *g) {
-  const int c = blockIdx.x;
-  float s = 0.0f;
-  for (int r = threadIdx.x; r < R; r += blockDim.x) s += __bfloat162float(m[(size_t)r * C + c]);
-  __shared__ float red[256];
-  red[threadIdx.x] = s;
-  __syncthreads();
-  for (int w = blockDim.x / 2; w > 0; w >>= 1) {
-    if (threadIdx.x < w) red[threadIdx.x] += red[threadIdx.x + w];
-    __syncthreads();
+// Bias gradients: column sums of the four [R][C] BF16 matrices dZ_l, first as
+// 256 partial sums a column, of rows t, t + 256, ..., the rows read along the
+// columns (a block per column read 2 of every 256 bytes, 25 us for 8 192 x
+// 128), then by a tree over t in grads_finish_kernel.
+constexpr int kColParts = 256;
+struct ColsumArgs {
+  const bf16 *m[4];
+  float *parts[4];
+  int C[4], R;
+};
+__global__ void colsum_parts_kernel(const __grid_constant__ ColsumArgs a) {
+  const int l = blockIdx.y, C = a.C[l];
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;  // t * C / 2 + column pair
+  const int t = i / (C / 2), c = i % (C / 2);
+  if (t >= kColParts) return;
+  const bf16 *m = a.m[l];
+  float s0 = 0.0f, s1 = 0.0f;
+#pragma unroll 8
+  for (int r = t; r < a.R; r += kColParts) {
+    const __nv_bfloat162 v = *reinterpret_cast<const __nv_bfloat162 *>(m + (size_t)r * C + 2 * c);
+    s0 += __bfloat162float(v.x);
+    s1 += __bfloat162float(v.y);
   }
-  if (threadIdx.x == 0) g[c] = red[0];
+  a.parts[l][t * C + 2 * c] = s0;
+  a.parts[l][t * C + 2 * c + 1] = s1;
 }
 
-// out[i][o] = in[o][i] for a small FP32 matrix (weight-gradient layouts).
-__global__ void transpose_f32_kernel(const float *in, int rows, int cols, float *out) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= rows * cols) return;
-  const int r = i / cols, c = i % cols;
-  out[(size_t)c * rows + r] = in[i];
+// The gradients from their partial sums: a thread per weight adds its
+// slices in order, a warp per bias adds its column's 256 partial sums as a
+// tree (t with t + 128, t + 64, ...).  dW4 comes as (A3^T dY), transposed.
+struct GradsFinishArgs {
+  const float *part[4], *cols[4];
+  float *grad;
+  int slices;
+};
+constexpr int kWeights = 2 * kMlpH * kMlpIn + 2 * kMlpH * kMlpH, kBiases = 3 * kMlpH + kMlpOut;
+constexpr int kWeightBlocks = kWeights / 128, kBiasBlocks = kBiases / 4;
+static_assert(kMlpIn == kMlpOut && kWeights % 128 == 0 && kBiases % 4 == 0, "grid");
+__global__ void __launch_bounds__(128) grads_finish_kernel(const __grid_constant__ GradsFinishArgs a) {
+  constexpr int kSmall = kMlpH * kMlpIn, kBig = kMlpH * kMlpH;
+  if (blockIdx.x < kWeightBlocks) {
+    int i = blockIdx.x * 128 + threadIdx.x, l, out;
+    if (i < kSmall) {
+      l = 0;
+      out = kOffW1 + i;
+    } else if ((i -= kSmall) < kBig) {
+      l = 1;
+      out = kOffW2 + i;
+    } else if ((i -= kBig) < kBig) {
+      l = 2;
+      out = kOffW3 + i;
+    } else {
+      i -= kBig;
+      l = 3;
+      out = kOffW4 + (i % kMlpOut) * kMlpH + i / kMlpOut;
+    }
+    const float *p = a.part[l] + i;
+    const size_t stride = l == 0 || l == 3 ? kSmall : kBig;
+    float s = 0.0f;
+#pragma unroll 16
+    for (int z = 0; z < a.slices; z++) s += p[(size_t)z * stride];
+    a.grad[out] = s;
+    return;
+  }
+  const int w = (blockIdx.x - kWeightBlocks) * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  const int l = w / kMlpH, c = w % kMlpH, C = l < 3 ? kMlpH : kMlpOut;
+  const int off[4] = {kOffB1, kOffB2, kOffB3, kOffB4};
+  float r[8];
+#pragma unroll
+  for (int j = 0; j < 8; j++) r[j] = a.cols[l][(lane + 32 * j) * C + c];
+#pragma unroll
+  for (int h = 4; h > 0; h >>= 1)
+#pragma unroll
+    for (int j = 0; j < h; j++) r[j] += r[j + h];
+#pragma unroll
+  for (int h = 16; h > 0; h >>= 1) r[0] += __shfl_down_sync(0xffffffffu, r[0], h);
+  if (lane == 0) a.grad[off[l] + c] = r[0];
 }
 
 // Adam (Kingma & Ba 2015) on the FP32 master parameters.
@@ -417,10 +458,9 @@ __global__ void features_from_rrs_kernel(const float *rrs, int64_t npix, int nb,
 
 static int gemm(const void *A, int lda, const void *B, int ldb, int M, int N, int K, int epi,
                 float *C, int ldc, void *O, int ldo, float *Z, int ldz, const float *bias,
-                unsigned int *err, cudaStream_t s, float *splitk = nullptr) {
+                unsigned int *err, cudaStream_t s) {
   GemmArgs g{};
-  g.ksplit = splitk ? kMlpSplitK : 1;
-  g.partial = splitk;
+  g.ksplit = 1;
   g.A = A;
   g.B = B;
   g.lda = lda;
@@ -465,11 +505,6 @@ cudaError_t mlp_forward(const MlpState &st, const float *x, int R, int Rpad, Mlp
   return cudaGetLastError();
 }
 
-static void tr(const bf16 *src, int R, int C, int Rpad, bf16 *dst, cudaStream_t s) {
-  dim3 grid((unsigned)((Rpad + 31) / 32), (unsigned)((C + 31) / 32));
-  transpose_kernel<<<grid, dim3(32, 8), 0, s>>>(src, R, C, Rpad, dst);
-}
-
 // Forward + backward; gradients (same layout as the parameters) into w.grad.
 cudaError_t mlp_backward(const MlpState &st, const float *x, const float *t, int R, int Rpad,
                          MlpWork &w, float *loss, unsigned int *err, cudaStream_t s) {
@@ -479,39 +514,47 @@ cudaError_t mlp_backward(const MlpState &st, const float *x, const float *t, int
   loss_grad_kernel<<<(Rpad + 255) / 256, 256, 0, s>>>(w.Y, t, R, Rpad, st.out_mean, st.out_std,
                                                       w.dY, loss);
   int bad = 0;
-  // layer 4: dW4 = dY^T A3 (computed as (A3^T dY)^T), db4 = colsum(dY)
-  tr(w.A3, Rpad, kMlpH, Rpad, w.T1, s);
-  tr(w.dY, Rpad, kMlpOut, Rpad, w.T2, s);
-  bad |= gemm(w.T1, Rpad, w.T2, Rpad, kMlpH, kMlpOut, Rpad, EPI_F32, w.G4t, kMlpOut, nullptr, 0,
-              nullptr, 0, nullptr, err, s, w.splitk);
-  transpose_f32_kernel<<<(kMlpH * kMlpOut + 255) / 256, 256, 0, s>>>(w.G4t, kMlpH, kMlpOut,
-                                                                     g + kOffW4);
-  colsum_kernel<<<kMlpOut, 256, 0, s>>>(w.dY, Rpad, kMlpOut, g + kOffB4);
-  // dZ3 = (dY W4) * SiLU'(Z3)
+  // dZ_{l-1} = (dZ_l W_l) * SiLU'(Z_{l-1})
   bad |= gemm(w.dY, kMlpOut, st.W4t, kMlpOut, Rpad, kMlpH, kMlpOut, EPI_DSILU, nullptr, 0,
-              w.dZ, kMlpH, w.Z3, kMlpH, nullptr, err, s);
-  // layer 3
-  tr(w.dZ, Rpad, kMlpH, Rpad, w.T2, s);
-  tr(w.A2, Rpad, kMlpH, Rpad, w.T1, s);
-  bad |= gemm(w.T2, Rpad, w.T1, Rpad, kMlpH, kMlpH, Rpad, EPI_F32, g + kOffW3, kMlpH, nullptr, 0,
-              nullptr, 0, nullptr, err, s, w.splitk);
-  colsum_kernel<<<kMlpH, 256, 0, s>>>(w.dZ, Rpad, kMlpH, g + kOffB3);
-  bad |= gemm(w.dZ, kMlpH, st.W3t, kMlpH, Rpad, kMlpH, kMlpH, EPI_DSILU, nullptr, 0, w.dZ2,
+              w.dZ3, kMlpH, w.Z3, kMlpH, nullptr, err, s);
+  bad |= gemm(w.dZ3, kMlpH, st.W3t, kMlpH, Rpad, kMlpH, kMlpH, EPI_DSILU, nullptr, 0, w.dZ2,
               kMlpH, w.Z2, kMlpH, nullptr, err, s);
-  // layer 2
-  tr(w.dZ2, Rpad, kMlpH, Rpad, w.T2, s);
-  tr(w.A1, Rpad, kMlpH, Rpad, w.T1, s);
-  bad |= gemm(w.T2, Rpad, w.T1, Rpad, kMlpH, kMlpH, Rpad, EPI_F32, g + kOffW2, kMlpH, nullptr, 0,
-              nullptr, 0, nullptr, err, s, w.splitk);
-  colsum_kernel<<<kMlpH, 256, 0, s>>>(w.dZ2, Rpad, kMlpH, g + kOffB2);
-  bad |= gemm(w.dZ2, kMlpH, st.W2t, kMlpH, Rpad, kMlpH, kMlpH, EPI_DSILU, nullptr, 0, w.dZ,
+  bad |= gemm(w.dZ2, kMlpH, st.W2t, kMlpH, Rpad, kMlpH, kMlpH, EPI_DSILU, nullptr, 0, w.dZ1,
               kMlpH, w.Z1, kMlpH, nullptr, err, s);
-  // layer 1 (no input gradient needed)
-  tr(w.dZ, Rpad, kMlpH, Rpad, w.T2, s);
-  tr(w.X0, Rpad, kMlpIn, Rpad, w.T1, s);
-  bad |= gemm(w.T2, Rpad, w.T1, Rpad, kMlpH, kMlpIn, Rpad, EPI_F32, g + kOffW1, kMlpIn, nullptr,
-              0, nullptr, 0, nullptr, err, s, w.splitk);
-  colsum_kernel<<<kMlpH, 256, 0, s>>>(w.dZ, Rpad, kMlpH, g + kOffB1);
+  // dW_l = dZ_l^T A_{l-1}, every layer's slices in one launch; both operands
+  // have the product's K as their rows; layer 4 as A3^T dY
+  const bf16 *a[4] = {w.dZ1, w.dZ2, w.dZ3, w.A3}, *b[4] = {w.X0, w.A1, w.A2, w.dY};
+  const int n[4] = {kMlpIn, kMlpH, kMlpH, kMlpOut};
+  GemmArgs ga[4];
+  GradsFinishArgs f{};
+  ColsumArgs ca{};
+  const bf16 *dz[4] = {w.dZ1, w.dZ2, w.dZ3, w.dY};
+  ca.R = Rpad;
+  f.grad = g;
+  for (int l = 0; l < 4; l++) {
+    ga[l] = GemmArgs{};
+    ga[l].A = a[l];
+    ga[l].B = b[l];
+    ga[l].lda = kMlpH;
+    ga[l].ldb = n[l];
+    ga[l].M = kMlpH;
+    ga[l].N = n[l];
+    ga[l].K = Rpad;
+    ga[l].error = err;
+    ga[l].lbo = 128;
+    ga[l].sbo = 1024;
+    ga[l].epi = EPI_F32;
+    ga[l].k_rows = 1;
+    ga[l].ksplit = kMlpSplitK;
+    ga[l].partial = w.part[l];
+    f.part[l] = w.part[l];
+    f.cols[l] = ca.parts[l] = w.cols[l];
+    ca.m[l] = dz[l];
+    ca.C[l] = l < 3 ? kMlpH : kMlpOut;
+  }
+  if (launch_gemm_partials(ga, 4, &f.slices, s) != cudaSuccess) bad = 1;
+  colsum_parts_kernel<<<dim3(kColParts * (kMlpH / 2) / 128, 4), 128, 0, s>>>(ca);
+  grads_finish_kernel<<<kWeightBlocks + kBiasBlocks, 128, 0, s>>>(f);
   if (bad) return cudaErrorLaunchFailure;
   return cudaGetLastError();
 }

@@ -48,8 +48,8 @@ struct PrecF64 {
   static __device__ __forceinline__ T div_n(T a, int n) {
     return n == 6 ? fm::div_6(a) : fm::div_by(a, (double)n, 1.0 / (double)n);
   }
-  static __device__ __forceinline__ bool lt(T a, T b) { return sf::lt(a, b); }
-  static __device__ __forceinline__ bool le(T a, T b) { return sf::le(a, b); }
+  static __device__ __forceinline__ bool lt(T a, T b) { return sf::lt_call(a, b); }
+  static __device__ __forceinline__ bool le(T a, T b) { return sf::le_call(a, b); }
   static __device__ __forceinline__ T eps_step(T s) { return s * 1.0e-6; }
   static __device__ __forceinline__ T eps_scale() { return 1.0e-6; }
   static __device__ __forceinline__ long long trunc10(T y) { return photic::trunc10(y); }

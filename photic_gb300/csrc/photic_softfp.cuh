@@ -248,8 +248,8 @@ PHOTIC_FM_HD double sqrt(double x) { return mid_positive(x) ? sqrt_mid(x) : sqrt
 // integers (a NaN is above every number); a sign bit on either side takes the
 // compiled comparison.  The compiler runs that one beside the integer one;
 // the _call forms keep it off the FP64 pipe at the price of a branch: faster
-// where that pipe is the bound (8 009 temporal stacks 224 -> 207 ms), slower
-// in the single-scene kernels (1024 x 320 scene 346 -> 363 ms).
+// where that pipe is the bound (8 009 temporal stacks 224 -> 207 ms,
+// 1024 x 320 scene 316 -> 313), not in the general fit.
 PHOTIC_FM_HD bool lt(double a, double b) {
   const int64_t ia = bits(a), ib = bits(b);
   if ((ia | ib) < 0) return a < b;
