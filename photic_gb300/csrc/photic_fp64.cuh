@@ -64,10 +64,10 @@ __device__ __forceinline__ double interp_plan(const InterpPlan &p, const double 
 }
 
 // Per-pixel set-up: Rrs at 440..640 nm with the negative-440 guard
-// (model/samodel.c:1785-1799), Y and the spectral mean.
+// (model/samodel.c:1785-1799), Y and the spectral mean; and the bands' powers.
 template <int NB>
-__device__ __forceinline__ void pixel_setup_f64(const FitParams &fp, const SceneConsts &sc,
-                                                const double *r, PixelF64<NB> &px) {
+__device__ __forceinline__ double pixel_shape_f64(const FitParams &fp, const double *r,
+                                                  PixelF64<NB> &px) {
   const int nb = fp.n_bands;
   double tot = 0.0;
 #pragma unroll
@@ -87,9 +87,15 @@ __device__ __forceinline__ void pixel_setup_f64(const FitParams &fp, const Scene
   double Y = 3.44 * (1.0 - 3.17 * fm::exp_t(-2.01 * chi));
   if (Y < 0.0) Y = 0.0;
   if (Y > 2.5) Y = 2.5;
-#pragma unroll 1
-  for (int b = 0; b < nb; b++) px.pw[b] = pow_call(sc.ratio440[b], Y);
   px.mean = tot / (double)nb;
+  return Y;
+}
+template <int NB>
+__device__ __forceinline__ void pixel_setup_f64(const FitParams &fp, const SceneConsts &sc,
+                                                const double *r, PixelF64<NB> &px) {
+  const double Y = pixel_shape_f64<NB>(fp, r, px);
+#pragma unroll 1
+  for (int b = 0; b < fp.n_bands; b++) px.pw[b] = pow_call(sc.ratio440[b], Y);
 }
 
 // Whether a K takes part in the minimum: the reference compares it, cast to
@@ -237,6 +243,20 @@ struct BandKeep {
   double E, K_min, qB;
 };
 
+// The cost of one scene and region from its squared residuals' sum and least
+// K (model/samodel.c:2696-2744).
+__device__ __forceinline__ double cost_total_f64(const FitParams &fp, double err, double K_min,
+                                                 double mean, double H, double &E) {
+  E = sf::div(100.0 * sf::sqrt(fm::div_count(err, fp.n_bands)), mean);
+  double Ke = k_penalty_f64(fp.kp, H, K_min);
+  if (sf::lt(0.7, K_min)) {
+    double d = 4.0 * (K_min - 0.7);
+    Ke = Ke + 100.0 * (d * d);
+  }
+  const double model = 80.0 * E + 15.0 * Ke;
+  return fm::div_120(model);
+}
+
 // Cost of x = (H, 100B, q, 100P, 100G, 100X) for one scene, one region,
 // one bottom type: samodel_error (model/samodel.c:2432-2759) over
 // samodel_Rrs (model/samodel.c:2846-2949).  With one region the depth and
@@ -276,14 +296,8 @@ __device__ __forceinline__ double cost_f64(const FitParams &fp, const SceneConst
       }
     }
   }
-  const double E = sf::div(100.0 * sf::sqrt(fm::div_count(err, nb)), px.mean);
-  double Ke = k_penalty_f64(fp.kp, H, K_min);
-  if (sf::lt(0.7, K_min)) {
-    double d = 4.0 * (K_min - 0.7);
-    Ke = Ke + 100.0 * (d * d);
-  }
-  double model = 80.0 * E + 15.0 * Ke;
-  model = fm::div_120(model);
+  double E;
+  const double model = cost_total_f64(fp, err, K_min, px.mean, H, E);
   if constexpr (kKeep) {
     keep->E = E;
     keep->K_min = K_min;

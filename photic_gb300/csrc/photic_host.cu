@@ -367,11 +367,24 @@ cudaError_t start_work_init(StartWork &w, unsigned char *mem, int64_t slots, int
   return e;
 }
 
+// Whether a group of lanes a start (invert_few_kernel) is faster than a lane:
+// up to 512 starts an SM with four bands, twice that with eight, where a lane
+// has twice the terms.  Measured on 152 SMs, milliseconds with groups / with
+// lanes: 256 pixels of four bands 14.6 / 34.8, 2 400 30 / 38, 9 600 54.0 /
+// 54.3, 20 000 81 / 66; eight bands 256 15.7 / 54, 20 000 106 / 111, 40 000
+// 168 / 148.  A seeded pixel is one start and some fallbacks, counted as two:
+// 3 000 16.5 / 39, 40 000 54.9 / 54.5, 80 000 87 / 62.
+bool few_starts(const InvertArgs &a, int precision, int sms) {
+  const int64_t starts = a.npix * (a.seeds && a.fp.n_hstarts > 2 ? 2 : a.fp.n_hstarts);
+  return precision == PHOTIC_PREC_FP64 && starts <= (int64_t)sms * (a.fp.n_bands > 4 ? 1024 : 512);
+}
+
 // The batched inversion of prepared arguments: workspace (queue head, exits,
 // records), launch shape, launches.
 int run_invert(InvertArgs &a, int precision, int block, int per_sm, int sms, cudaStream_t s) {
   const int64_t per_pixel = (int64_t)a.fp.n_hstarts * kStartRecordBytes + sizeof(int32_t);
-  a.n_par = a.fp.n_hstarts > 1 ? kRecordBytesMax / per_pixel : 0;
+  const bool few = block == 0 && per_sm == 0 && few_starts(a, precision, sms);
+  a.n_par = few || a.fp.n_hstarts > 1 ? kRecordBytesMax / per_pixel : 0;
   if (a.n_par > a.npix) a.n_par = a.npix;
   a.n_seq = a.npix - a.n_par;
   int64_t grid = 0;
@@ -389,7 +402,8 @@ int run_invert(InvertArgs &a, int precision, int block, int per_sm, int sms, cud
   // 0x7f7f7f7f: no start has met the early exit
   if (e == cudaSuccess && a.n_par > 0)
     e = cudaMemsetAsync(a.exit_k, 0x7f, (size_t)a.n_par * sizeof(int32_t), s);
-  if (e == cudaSuccess) e = launch_invert(a, precision, block, (int)grid, s);
+  if (e == cudaSuccess)
+    e = few ? launch_invert_few(a, sms, s) : launch_invert(a, precision, block, (int)grid, s);
   cudaError_t e2 = cudaFreeAsync(ws, s);
   if (e != cudaSuccess) return cuda_fail(e, "invert kernel launch");
   if (e2 != cudaSuccess) return cuda_fail(e2, "cudaFreeAsync");

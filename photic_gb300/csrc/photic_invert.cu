@@ -29,6 +29,7 @@
 #include "photic_fp64.cuh"
 #include "photic_kernels.h"
 #include "photic_nm.cuh"
+#include "photic_nmgroup.cuh"
 #include "photic_prec64.cuh"
 
 namespace photic {
@@ -494,6 +495,165 @@ __global__ void __launch_bounds__(BS) invert_kernel(const __grid_constant__ Inve
   }
 }
 
+// The same queue of starts for few positions: a group of eight lanes a start,
+// band b on lane b, coordinate i of the simplex on lane i (NmGroup).  A launch
+// of few positions lasts as long as one start's chain of up to kcount
+// evaluations, and one lane's evaluation takes four times a band's FP64
+// instructions and six coordinates' (342 a trip, here about 130, at 64 clocks
+// each for a warp alone on its SM quarter): 256 pixels 35 -> 14.6 ms.  A full
+// device is better used by a lane a start (few_starts, photic_host.cu).
+constexpr int kFewLanes = 8, kFewBlock = 128;
+template <int NB>
+__global__ void __launch_bounds__(kFewBlock) invert_few_kernel(const __grid_constant__ InvertArgs args) {
+  constexpr int G = kFewLanes;
+  using Nm = NmGroup<kN, 1, G, G>;
+  constexpr int kV = (kN + 1) * G, kF = (kN + 2) * G;
+  __shared__ double smem[kFewBlock / G][kV + kF + 3 * G];
+  const FitParams &fp = args.fp;
+  const SceneConsts &sc = args.sc;
+  const int nb = fp.n_bands;
+  const int gl = threadIdx.x % G;
+  double *base = smem[threadIdx.x / G];
+  double *X = base + kV + kF, *dd = X + G, *kk = dd + G;
+  Nm m;
+  m.V = base;
+  m.Fv = base + kV + gl;
+  m.X = X;
+  m.gl = gl;
+  m.clear();
+  const unsigned gmask = ((1u << G) - 1u) << ((threadIdx.x & 31) & ~(G - 1));
+  m.gmask = gmask;
+  StartRecord<PrecF64> *const rec = reinterpret_cast<StartRecord<PrecF64> *>(args.records);
+  const int64_t total_pos = args.n_par * fp.n_hstarts;
+  const double var_limit = fp.reqmin * (double)kN;
+  const int32_t guard_cap = (fp.n_hstarts + 1) * (fp.kcount + 8 * kN + 16);
+
+  bool has = false, open = true;
+  int64_t item = 0;
+  int32_t start_k = 0, guard = 0;
+  double my_rrs = 0.0, my_pw = 0.0, mean = 0.0;
+
+  for (;;) {
+    bool fresh = false;
+    int64_t p = 0;
+    float r[NB];
+    do {
+      unsigned long long w = ~0ull;
+      const bool ask = !has && open && !fresh;
+      if (ask && gl == 0) w = atomicAdd(args.queue, 1ull);
+      w = __shfl_sync(kFull, w, 0, G);
+      if (ask) {
+        if (w < (unsigned long long)total_pos) {
+          start_k = (int32_t)((int64_t)w / args.n_par);
+          item = (int64_t)w % args.n_par;
+          p = pixel_at(args, item);
+          fresh = start_k == 0 || (__ldcg(args.exit_k + item) >= start_k &&
+                                   (args.seeds == nullptr || isnan(args.seeds[p * kN])));
+          if (fresh) {
+            load_spectrum<NB>(args, p, r);
+#pragma unroll
+            for (int b = 0; b < NB; b++)
+              if (b < nb && !args.no_mask && band_masked(r[b], fp.nodata)) fresh = false;
+            if (!fresh && start_k == 0 && gl == 0) {
+              write_masked(args.out, p);
+              args.exit_k[item] = -1;
+            }
+          }
+        } else {
+          open = false;
+        }
+      }
+    } while (__any_sync(kFull, !has && open && !fresh));
+    if (!__any_sync(kFull, has || fresh)) break;
+
+    if (fresh) {
+      PixelF64<NB> px;
+      double rd[NB];
+#pragma unroll
+      for (int b = 0; b < NB; b++) rd[b] = (double)r[b];
+      const double Y = pixel_shape_f64<NB>(fp, rd, px);
+      mean = px.mean;
+#pragma unroll
+      for (int b = 0; b < NB; b++)
+        if (b == gl) my_rrs = px.rrs[b];
+      my_pw = pow_call(sc.ratio440[gl < nb ? gl : 0], Y);
+      double start[kN], step[kN];
+      bool seeded = false;
+      if (args.seeds != nullptr) {
+        const double *sd = args.seeds + p * kN;
+        if (!isnan(sd[0])) {
+          const double rel[kN] = {1.25, 1.5, 0.5, 2.0, 2.0, 2.0};
+          seeded = true;
+#pragma unroll
+          for (int i = 0; i < kN; i++) {
+            start[i] = sd[i];
+            step[i] = (rel[i] * fp.seed_step_scale) * sd[i];
+          }
+        }
+      }
+      if (!seeded) {
+        cold_start_f64<NB>(fp, px, start, step);
+        start[0] = fp.hstarts[start_k];
+        step[0] = PrecF64::h_step(start[0]);
+      }
+      m.start[0] = 0.0;
+      m.step[0] = 0.0;
+#pragma unroll
+      for (int i = 0; i < kN; i++)
+        if (i == gl) {
+          m.start[0] = start[i];
+          m.step[0] = step[i];
+        }
+      guard = 0;
+      m.begin(var_limit, fp.konvge, fp.kcount);
+      has = true;
+    }
+    __syncwarp();
+    // ---- one evaluation per group at X: a band a lane, then the sum and the
+    // rest of the cost on every lane
+    if (has && gl < nb) {
+      const double H = fabs(X[0]), B = 0.01 * fabs(X[1]);
+      const double qB = fm::self_ratio(fabs(X[2])) * B;
+      const double P = 0.01 * fabs(X[3]), Gg = 0.01 * fabs(X[4]), Xx = 0.01 * fabs(X[5]);
+      BandTerm t;
+      band_term(sc, gl, sc.sec_sun, false, H, qB * sc.refl[gl], P, log(P), Gg, Xx, my_pw, my_rrs, t);
+      dd[gl] = t.dd;
+      kk[gl] = t.K;
+    }
+    __syncwarp();
+    if (has) {
+      double err = 0.0, K_min = 1.0e4, E;
+#pragma unroll
+      for (int b = 0; b < NB; b++)
+        if (b < nb) {
+          err = err + dd[b];
+          const double K = kk[b];
+          if (k_counts(K) && sf::lt(K, K_min)) K_min = K;
+        }
+      const double y = cost_total_f64(fp, err, K_min, mean, fabs(X[0]), E);
+      __syncwarp(gmask);  // every lane has read X, dd and kk
+      const bool capped = ++guard > guard_cap;
+      if (capped && gl == 0) atomicOr(args.error, PHOTIC_DEVERR_EVAL_CAP);
+      if (start_k > 0 && (guard & 63) == 0 && __ldcg(args.exit_k + item) < start_k) {
+        has = false;  // an earlier start has ended the pixel
+      } else if (capped || m.step_machine(y)) {
+        const double ynewlo = m.F(m.lo);
+        StartRecord<PrecF64> &rc = rec[item * fp.n_hstarts + start_k];
+        if (gl < kN) rc.x[gl] = m.xmin[0];
+        if (gl == 0) {
+          rc.y = ynewlo;
+          rc.evals = capped ? -1 : m.icount;
+          rc.fault = m.ifault;
+          if (!capped && sf::lt(ynewlo, args.early_exit) && sf::lt(ynewlo, 1.0e4))
+            atomicMin(args.exit_k + item, start_k);
+        }
+        has = false;
+      }
+    }
+    __syncwarp();
+  }
+}
+
 // The n_par pixels after their starts have run: the records compared in the
 // order of the starts, as the sequential loop does (model/samodel.c:
 // 2380-2405), and the products at the kept optimum.
@@ -582,6 +742,33 @@ cudaError_t launch_prec(const InvertArgs &a, int block, int grid, cudaStream_t s
 size_t invert_smem_bytes(int block) {
   // double and double-float both take 8 bytes per value
   return (size_t)block * 8 * (NmPixel<PrecF64, 32>::kSlots + kN + 1);
+}
+
+namespace {
+
+template <int NB>
+cudaError_t launch_few(const InvertArgs &a, int sms, cudaStream_t s) {
+  int occ = 0;
+  cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, invert_few_kernel<NB>,
+                                                                kFewBlock, 0);
+  if (e != cudaSuccess) return e;
+  if (occ < 1) return cudaErrorInvalidConfiguration;
+  // one block (a warp a quarter) per SM first
+  constexpr int kGroups = kFewBlock / kFewLanes;
+  const int64_t positions = a.n_par * a.fp.n_hstarts;
+  int64_t per_sm = (positions + (int64_t)sms * kGroups - 1) / ((int64_t)sms * kGroups);
+  if (per_sm > occ) per_sm = occ;
+  const int64_t need = (positions + kGroups - 1) / kGroups;
+  const int64_t grid = per_sm * sms < need ? per_sm * sms : need;
+  invert_few_kernel<NB><<<(unsigned)grid, kFewBlock, 0, s>>>(a);
+  finish_kernel<PrecF64, NB><<<(unsigned)((a.n_par + 127) / 128), 128, 0, s>>>(a);
+  return cudaGetLastError();
+}
+
+}  // namespace
+
+cudaError_t launch_invert_few(const InvertArgs &a, int sms, cudaStream_t s) {
+  return a.fp.n_bands <= 4 ? launch_few<4>(a, sms, s) : launch_few<8>(a, sms, s);
 }
 
 cudaError_t launch_invert(const InvertArgs &a, int precision, int block, int grid,

@@ -83,6 +83,8 @@ constexpr size_t kStartRecordBytes = 64;
 size_t invert_smem_bytes(int block);
 cudaError_t launch_invert(const InvertArgs &a, int precision, int block, int grid,
                           cudaStream_t s);
+// FP64, every position a start (n_seq = 0): a group of lanes each.
+cudaError_t launch_invert_few(const InvertArgs &a, int sms, cudaStream_t s);
 // Resident blocks per SM of the kernel that launch_invert would use (0 on error).
 int invert_blocks_per_sm(const InvertArgs &a, int precision, int block);
 

@@ -243,7 +243,7 @@ struct NmGroup {
     for (int t = 0; t < C; t++)
       if (slot_used(t)) {
         z[t] = z[t] - Vv(hi, column(t));
-        cen[t] = fm::div_by(z[t], (double)dim(), inv_n);
+        cen[t] = NT == 6 ? fm::div_6(z[t]) : fm::div_by(z[t], (double)dim(), inv_n);
       }
     phase = PH_REFLECT;
     return true;

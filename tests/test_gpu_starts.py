@@ -1,5 +1,6 @@
 """The inversion with every depth start a queue position of its own (the
-allocating entry points) against the sequential loop over a pixel's starts
+allocating entry points: a group of lanes a start, or a lane a start for
+more) against the sequential loop over a pixel's starts
 (the allocation-free one): the same bits, at sizes around a warp and a block,
 with seeds, an early exit at the first start, one that is never met, and the
 largest number of starts."""
@@ -11,6 +12,7 @@ import torch
 
 pytestmark = pytest.mark.gpu
 
+WL8 = (412.5, 442.5, 490.0, 510.0, 560.0, 620.0, 665.0, 708.75)
 FIELDS = ("depth_f64", "P", "G", "X", "bottom_albedo", "model_error", "rrs_error", "K_min", "iod",
           "evals", "evals_kept", "status", "params")
 
@@ -37,6 +39,11 @@ def _noalloc(gpu, rrs, cfg, seeds):
     (300, {"hstarts": tuple(0.7 * (i + 1) for i in range(32)), "kcount": 120}, False),
     (3001, {"seed_step_scale": 0.1}, True),
     (2000, {"precision": "df64"}, False),
+    # two and eight bands, a lane a start beyond the groups' sizes
+    (90, {"wavelengths": (482.0, 561.0)}, False),
+    (130, {"wavelengths": WL8}, False),
+    (11003, {}, False),
+    (40, {"block_threads": 64}, False),
 ])
 def test_starts_in_parallel_match_the_sequence(gpu, npix, kw, seeded):
     cfg = gpu.Config(**kw)
