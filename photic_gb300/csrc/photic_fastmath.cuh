@@ -36,8 +36,10 @@
 
 #if defined(__CUDACC__)
 #define PHOTIC_FM_HD __host__ __device__ __forceinline__
+#define PHOTIC_FM_OUT static __host__ __device__ __noinline__
 #else
 #define PHOTIC_FM_HD inline
+#define PHOTIC_FM_OUT inline
 #endif
 
 namespace photic {
@@ -150,6 +152,10 @@ PHOTIC_FM_HD int ilog2(int n) {
 #endif
 }
 
+// The compiled division, out of line: the divisions below take it for
+// operands that the fits do not meet.
+PHOTIC_FM_OUT double div_out(double a, double b) { return a / b; }
+
 // a / b for a positive normal b fixed in advance, inv = RN(1 / b)
 // (Markstein's correction, see the file header).  A quotient that is zero,
 // subnormal, infinite or NaN -- outside the correction's hypotheses, and
@@ -157,7 +163,7 @@ PHOTIC_FM_HD int ilog2(int n) {
 PHOTIC_FM_HD double div_by(double a, double b, double inv) {
   const double q = a * inv;
   const int64_t e = (bits(q) >> 52) & 0x7ff;
-  if (e == 0 || e == 0x7ff) return a / b;
+  if (e == 0 || e == 0x7ff) return div_out(a, b);
   const double r = fma(-q, b, a);
   return fma(r, inv, q);
 }
@@ -174,7 +180,7 @@ PHOTIC_FM_HD double div_by(double a, double b, double inv) {
 // divided.
 PHOTIC_FM_HD double div_const(double a, double b, double hi, double lo) {
   const int64_t e = (bits(a) >> 52) & 0x7ff;
-  if (e < 256 || e > 1790) return a / b;
+  if (e < 256 || e > 1790) return div_out(a, b);
   return fma(a, hi, a * lo);
 }
 constexpr double kPiHi = 0x1.45f306dc9c883p-2, kPiLo = -0x1.0c3b15964a2c2p-57;
@@ -198,7 +204,7 @@ constexpr double kInv120 = 1.0 / 120.0;
 // divided.
 PHOTIC_FM_HD double div_count(double a, int n) {
   if ((n & (n - 1)) == 0) return a * from_bits(shl52(1023 - ilog2(n)));
-  return a / (double)n;
+  return div_out(a, (double)n);
 }
 
 }  // namespace fm
