@@ -183,8 +183,11 @@ PHOTIC_FM_HD double div_const(double a, double b, double hi, double lo) {
   if (e < 256 || e > 1790) return div_out(a, b);
   return fma(a, hi, a * lo);
 }
+// RN(1/n - hi) for hi = RN(1/n): the remainder 1 - n hi is exact.
+PHOTIC_FM_HD double recip_lo(double n, double hi) { return fma(-hi, n, 1.0) / n; }
 constexpr double kPiHi = 0x1.45f306dc9c883p-2, kPiLo = -0x1.0c3b15964a2c2p-57;
 constexpr double k120Hi = 0x1.1111111111111p-7, k120Lo = 0x1.1111111111111p-63;
+constexpr double k3Hi = 0x1.5555555555555p-2, k3Lo = 0x1.5555555555555p-56;
 constexpr double k6Hi = 0x1.5555555555555p-3, k6Lo = 0x1.5555555555555p-57;
 PHOTIC_FM_HD double div_pi(double a) { return div_const(a, 3.141592653589793, kPiHi, kPiLo); }
 PHOTIC_FM_HD double div_120(double a) { return div_const(a, 120.0, k120Hi, k120Lo); }

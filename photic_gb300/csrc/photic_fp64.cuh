@@ -247,7 +247,10 @@ struct BandKeep {
 // K (model/samodel.c:2696-2744).
 __device__ __forceinline__ double cost_total_f64(const FitParams &fp, double err, double K_min,
                                                  double mean, double H, double &E) {
-  E = sf::div(100.0 * sf::sqrt(fm::div_count(err, fp.n_bands)), mean);
+  const int nb = fp.n_bands;
+  const double ms = (nb & (nb - 1)) == 0 ? fm::div_count(err, nb)
+                                         : fm::div_const(err, (double)nb, fp.inv_nb, fp.inv_nb_lo);
+  E = sf::div(100.0 * sf::sqrt(ms), mean);
   double Ke = k_penalty_f64(fp.kp, H, K_min);
   if (sf::lt(0.7, K_min)) {
     double d = 4.0 * (K_min - 0.7);

@@ -18,6 +18,7 @@
 
 #include "../../include/photic.h"
 #include "../../include/photic_nc.h"
+#include "photic_fastmath.cuh"
 #include "photic_kernels.h"
 #include "photic_params.h"
 #include "photic_tables.h"
@@ -196,6 +197,8 @@ void make_scene(const photic_config &cfg, double theta_sun_deg, SceneConsts &sc)
 void make_fit(const photic_config &cfg, FitParams &fp) {
   memset(&fp, 0, sizeof fp);
   fp.n_bands = cfg.n_bands;
+  fp.inv_nb = 1.0 / (double)cfg.n_bands;
+  fp.inv_nb_lo = fm::recip_lo((double)cfg.n_bands, fp.inv_nb);
   fp.kcount = cfg.kcount;
   fp.konvge = cfg.konvge;
   fp.n_hstarts = cfg.n_hstarts;

@@ -178,6 +178,7 @@ __global__ void __launch_bounds__(kBlock) joint_group_kernel(const __grid_consta
   const int cP = LAYOUT == PHOTIC_LAYOUT_REFERENCE ? 3 + 3 * bs : 2 + 4 * bs;
 
   const double var_limit = fp.reqmin * (double)N;
+  const double inv_t = 1.0 / (double)(K * nb), inv_t_lo = fm::recip_lo((double)(K * nb), inv_t);
   const double early = fp.early_exit_per_scene * (double)(float)K;
   const int32_t guard_cap = (fp.n_hstarts + 1) * (fp.kcount + 8 * N + 16);
 
@@ -332,7 +333,9 @@ __global__ void __launch_bounds__(kBlock) joint_group_kernel(const __grid_consta
       double err = 0.0, Ke = 0.0, Kall = 1.0e4, iod = 0.0;
       for (int tau = 0; tau < K * 4; tau++)
         if ((tau & 3) < nb) err = err + g.dd[tau];
-      for (int s = 0; s < K; s++) Ke = Ke + g.kpen[s];
+      // (a scene without a penalty adds +0)
+      for (int s = 0; s < K; s++)
+        if (fm::bits(g.kpen[s]) != 0) Ke = Ke + g.kpen[s];
       if (final_eval) {
         for (int s = 0; s < K; s++)
           for (int b = 0; b < nb; b++) {
@@ -342,7 +345,7 @@ __global__ void __launch_bounds__(kBlock) joint_group_kernel(const __grid_consta
           }
       }
       const double km = g.kmin[K - 1];
-      const double E = sf::div(100.0 * sf::sqrt(fm::div_count(err, K * nb)), mean);
+      const double E = sf::div(100.0 * sf::sqrt(fm::div_const(err, (double)(K * nb), inv_t, inv_t_lo)), mean);
       if (sf::lt(0.7, km)) {  // the last scene's K_min (model/samodel.c:2726-2732)
         const double dk = 4.0 * (km - 0.7);
         Ke = Ke + 100.0 * (dk * dk);

@@ -27,7 +27,9 @@ struct NmGroup {
   unsigned gmask;      // the group's lanes
   double cen[C], refl[C], trial[C], xmin[C], start[C], step[C];
   double ylo, fr, scale, var_limit;
-  double inv_n, inv_n1;  // RN(1 / n), RN(1 / (n + 1)) for the centroid and the variance test
+  // 1 / n as hi + lo for the centroid's division, RN(1 / (n + 1)) for the
+  // variance test's
+  double inv_n, inv_n_lo, inv_n1;
   long long floor_lo;
   int32_t phase, jj, hi, lo, icount, numres, ifault, countdown, kcount, konvge;
   // The centroid sums every coordinate over the vertices in order, and an
@@ -91,6 +93,7 @@ struct NmGroup {
     }
     ylo = fr = 0.0;
     inv_n = inv_n1 = 1.0;
+    inv_n_lo = 0.0;
     scale = 1.0;
     floor_lo = 0;
     phase = jj = hi = lo = icount = numres = ifault = countdown = ck_valid = 0;
@@ -106,6 +109,7 @@ struct NmGroup {
     scale = 1.0;
     var_limit = var_limit_;
     inv_n = 1.0 / (double)dim();
+    inv_n_lo = fm::recip_lo((double)dim(), inv_n);
     inv_n1 = 1.0 / (double)(dim() + 1);
     restart_simplex();
   }
@@ -152,33 +156,26 @@ struct NmGroup {
   // The worst vertex: the first index of the largest cost, a NaN cost
   // never replacing the running one (a NaN at index 0 is kept, model/
   // asa047.c:221-231).  With one cost copy for the warp, each lane scans
-  // the vertices j = lane, lane + 32, ... and the warp combines the lanes'
-  // (cost, index) by the larger cost, the smaller index on a tie.
+  // the vertices j = lane, lane + 32, ..., and the warp reduces the costs'
+  // order keys, then the indices that have the largest.
   __device__ __forceinline__ int worst_vertex() {
     if constexpr (kSharedF) {
 #if defined(__CUDA_ARCH__)
-      const double f0 = F(0);
-      if (f0 != f0) return 0;
-      double v = 0.0;
+      if (sf::order_key(F(0)) == 0) return 0;
+      uint64_t v = 0;
       int idx = 0x7fffffff;
 #pragma unroll 1
       for (int j = gl; j <= dim(); j += G) {
-        const double f = F(j);
-        if (f == f && (idx == 0x7fffffff || lt(v, f))) {
+        const uint64_t f = sf::order_key(F(j));
+        if (f > v) {
           v = f;
           idx = j;
         }
       }
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        const double ov = __shfl_xor_sync(gmask, v, o);
-        const int oi = __shfl_xor_sync(gmask, idx, o);
-        if (oi != 0x7fffffff &&
-            (idx == 0x7fffffff || lt(v, ov) || (!lt(ov, v) && oi < idx))) {
-          v = ov;
-          idx = oi;
-        }
-      }
+      const uint32_t h = __reduce_max_sync(gmask, (uint32_t)(v >> 32));
+      const uint32_t l = __reduce_max_sync(gmask, (uint32_t)(v >> 32) == h ? (uint32_t)v : 0u);
+      if (v != ((uint64_t)h << 32 | l)) idx = 0x7fffffff;
+      idx = __reduce_min_sync(gmask, idx);
       return idx;
 #endif
     }
@@ -201,9 +198,10 @@ struct NmGroup {
     if constexpr (kSharedF) {
 #if defined(__CUDA_ARCH__)
       int c = 0;
+      const uint64_t kf = sf::order_key(fr_);
 #pragma unroll 1
       for (int j = gl; j <= dim(); j += G)
-        if (lt(fr_, F(j))) c++;
+        if (kf != 0 && kf < sf::order_key(F(j))) c++;
       return (int)__reduce_add_sync(gmask, (unsigned)c);
 #endif
     }
@@ -243,7 +241,7 @@ struct NmGroup {
     for (int t = 0; t < C; t++)
       if (slot_used(t)) {
         z[t] = z[t] - Vv(hi, column(t));
-        cen[t] = NT == 6 ? fm::div_6(z[t]) : fm::div_by(z[t], (double)dim(), inv_n);
+        cen[t] = fm::div_const(z[t], (double)dim(), inv_n, inv_n_lo);
       }
     phase = PH_REFLECT;
     return true;
@@ -264,14 +262,14 @@ struct NmGroup {
   // The pending point of the iteration, cen + c (a - b) (photic_nm.cuh): the
   // reflection, the expansion or a contraction, written once.
   __device__ __forceinline__ void make_point(int pk) {
-    const double c = pk == PK_EXPAND ? 2.0 : (pk == PK_REFL ? 1.0 : 0.5);
+    const float c = pk == PK_EXPAND ? 2.0f : (pk == PK_REFL ? 1.0f : 0.5f);
 #pragma unroll
     for (int t = 0; t < C; t++)
       if (slot_used(t)) {
         const double w = Vv(hi, column(t));
         const double a = pk == PK_REFL ? cen[t] : (pk == PK_CONTRACT_IN ? w : refl[t]);
         const double b = pk == PK_REFL ? w : cen[t];
-        const double p = cen[t] + c * (a - b);
+        const double p = sf::add_scaled2(cen[t], a - b, c);
         if (pk == PK_REFL) refl[t] = p;
         else trial[t] = p;
         if (own(t)) X[coord(t)] = p;

@@ -70,6 +70,7 @@ struct FitParams {
   double reqmin;
   double early_exit_per_scene;
   double aw640;
+  double inv_nb, inv_nb_lo;  // 1 / n_bands as hi + lo (fm::div_const)
   double seed_step_scale;
   double hstarts[kMaxHStarts];
   InterpPlan plan[kNRefTargets];

@@ -31,16 +31,7 @@ struct PrecF64 {
   static __device__ __forceinline__ T half(T a) { return a * 0.5; }
   // a * c for c in {1/2, 1, 2}: exact
   static __device__ __forceinline__ T scale2(T a, float c) { return a * (double)c; }
-  // a + b * c for c in {1/2, 1, 2}: the product is exact (but for half the
-  // least exponents and twice the largest, which are multiplied on their
-  // own), so the fused sum rounds as the separate one
-  static __device__ __forceinline__ T add_scaled2(T a, T b, float c) {
-    const double cd = fm::from_bits((int64_t)(0x3fe00000u + (c > 0.5f ? 0x100000u : 0u) +
-                                              (c > 1.0f ? 0x100000u : 0u)) << 32);
-    const uint32_t e = (uint32_t)((uint64_t)fm::bits(b) >> 52) & 0x7ffu;
-    if (e - 2u > 2042u) return a + b * cd;
-    return fma(b, cd, a);
-  }
+  static __device__ __forceinline__ T add_scaled2(T a, T b, float c) { return sf::add_scaled2(a, b, c); }
   static __device__ __forceinline__ bool sum_less_one(const T *p, int stride, int n, int h, T &z) {
     return sf::sum_less_one(p, stride, n, h, z);
   }

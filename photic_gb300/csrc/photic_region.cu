@@ -47,8 +47,8 @@ constexpr int kMaxR = kRegionMaxR, kTerms = 128, kHT = kTerms / 32, kShares = 32
 constexpr int kChainD = 3 * kRS + kTerms + 3 * kMaxScenes + 24;
 // the cost's staging, per warp: |H| and depth deviations per region, bottom
 // deviations per (type, region), K penalty and smallest K per scene, mean
-// share per type, ln P per scene
-constexpr int kStage = 72;
+// share per type, ln P and P, G, X per scene, reciprocals of 1..31
+constexpr int kStage = 72 + 3 * kMaxScenes + 64;
 
 // Launch shapes: C coordinates per lane, vertex row stride CG.
 //
@@ -337,6 +337,14 @@ __global__ void __launch_bounds__(BLOCK, 1) region_kernel(const __grid_constant_
 
   const double early = fp.early_exit_per_scene * (double)(float)S;
   const double kNaN = __longlong_as_double(0x7ff8000000000000LL);
+  // 1 / n as hi + lo for the divisions by small counts (fm::div_const)
+  double *rec_hi = stg + 72 + 3 * kMaxScenes, *rec_lo = rec_hi + 32;
+  {
+    const double n = lane > 0 ? (double)lane : 1.0;
+    rec_hi[lane] = 1.0 / n;
+    rec_lo[lane] = fm::recip_lo(n, 1.0 / n);
+  }
+  __syncwarp();
   const bool chained = a.order != nullptr;
   if (chained) {
     if (lane == 0) {
@@ -560,6 +568,7 @@ __global__ void __launch_bounds__(BLOCK, 1) region_kernel(const __grid_constant_
     }
     tot = __shfl_sync(kFull, tot, 0);
     const double mean = tot / (double)nterm;
+    const double inv_t = 1.0 / (double)nterm, inv_t_lo = fm::recip_lo((double)nterm, inv_t);
 
     // cold start of the lane's coordinates (model/samodel.c:2249-2353)
     auto cold = [&](double hs) {
@@ -633,12 +642,24 @@ __global__ void __launch_bounds__(BLOCK, 1) region_kernel(const __grid_constant_
         double qs = 0.0;
 #pragma unroll 1
         for (int kb = 0; kb < nbt; kb++) qs += fabs(X[qo + r * nbt + kb]);
-        const double q = fabs(X[qo + lane]), B100 = fabs(X[R + lane]);
-        wB[lane] = div_call(q, qs) * (0.01 * B100);
-        share[lane] = div_call(B100 * q, qs);
+        const double q = fabs(X[qo + lane]), B100 = fabs(X[R + lane]), Bq = B100 * q;
+        double w, sh;  // the two divisions side by side
+        if (sf::mid(q) && sf::mid(qs) && sf::mid(Bq)) {
+          w = sf::div_mid(q, qs);
+          sh = sf::div_mid(Bq, qs);
+        } else {
+          w = fm::div_out(q, qs);
+          sh = fm::div_out(Bq, qs);
+        }
+        wB[lane] = w * (0.01 * B100);
+        share[lane] = sh;
       }
-      double *lnps = stg + 64;
-      if (lane < S) lnps[lane] = log(0.01 * fabs(X[off + 3 * lane]));
+      double *lnps = stg + 64, *pgx = stg + 72;
+      if (lane < 3 * S) {
+        const double v = 0.01 * fabs(X[off + lane]);
+        pgx[lane] = v;
+        if (lane % 3 == 0) lnps[lane / 3] = log(v);
+      }
       __syncwarp();
       // ---- band terms at X
 #pragma unroll 1
@@ -646,13 +667,11 @@ __global__ void __launch_bounds__(BLOCK, 1) region_kernel(const __grid_constant_
         const int rsb = my_rsb[h], r = rsb & 255, s = (rsb >> 8) & 255, b = rsb >> 16;
         const double pw = my_pw[h];
         const double H = fabs(X[r]);
-        const double P = 0.01 * fabs(X[off + 3 * s]);
-        const double Gg = 0.01 * fabs(X[off + 1 + 3 * s]);
-        const double Xx = 0.01 * fabs(X[off + 2 + 3 * s]);
+        const double P = pgx[3 * s], Gg = pgx[3 * s + 1], Xx = pgx[3 * s + 2];
         const double lnP = lnps[s];
-        double rho = 0.0;
+        double rho = wB[r * nbt] * sc.refl_k[0][b];  // (0 + the first, which is not -0)
 #pragma unroll 1
-        for (int k = 0; k < nbt; k++) rho += wB[r * nbt + k] * sc.refl_k[k][b];
+        for (int k = 1; k < nbt; k++) rho += wB[r * nbt + k] * sc.refl_k[k][b];
         BandTerm t;
         band_term(sc, b, a.sec_sun[s], final_eval, H, rho, P, lnP, Gg, Xx, pw, my_rrs[h], t);
         dd[tau] = t.dd;
@@ -703,8 +722,10 @@ __global__ void __launch_bounds__(BLOCK, 1) region_kernel(const __grid_constant_
         for (int i = 0; i < cnt; i++) z = z + src[i * str];
       }
       const double err = __shfl_sync(kFull, z, 0);
-      const double dmean = div_call(__shfl_sync(kFull, z, 1), (double)R);
-      if (lane >= 2 && lane < 2 + nbt) bmv[lane - 2] = div_call(z, (double)R);
+      // (1 on the lanes without a sum: a zero takes the compiled division)
+      const double zR = fm::div_const(lane < 2 + nbt ? z : 1.0, (double)R, rec_hi[R], rec_lo[R]);
+      const double dmean = __shfl_sync(kFull, zR, 1);
+      if (lane >= 2 && lane < 2 + nbt) bmv[lane - 2] = zR;
       const double thd = dmean < 4.0 ? 0.4 : dmean < 8.0 ? 0.2 : dmean < 12.0 ? 0.1 : 0.05;
       const double thb = dmean < 5.0 ? 0.25 : dmean < 10.0 ? 0.1 : dmean < 15.0 ? 0.05 : 0.01;
       bool outd = false, outb = false;
@@ -723,8 +744,8 @@ __global__ void __launch_bounds__(BLOCK, 1) region_kernel(const __grid_constant_
         dv2b[lane] = outb ? dv * dv : 0.0;
       }
       if (lane < S) kpen[lane] = k_penalty_f64(fp.kp, habs[origin], kms[lane]);
-      const double nd = (double)__popc(__ballot_sync(kFull, outd));
-      const double nbo = (double)__popc(__ballot_sync(kFull, outb));
+      const unsigned outs_d = __ballot_sync(kFull, outd), outs_b = __ballot_sync(kFull, outb);
+      const double nd = (double)__popc(outs_d), nbo = (double)__popc(outs_b);
       __syncwarp();
       // ordered sums: lane 0 the depth deviations, lane 1 the bottom
       // deviations (type-major), lane 2 the scenes' K penalties, lane 3 the
@@ -754,13 +775,17 @@ __global__ void __launch_bounds__(BLOCK, 1) region_kernel(const __grid_constant_
       // bottom shares, on lanes 0, 1 and 2
       double rms;
       {
-        const double num = lane == 1 ? Ed : lane == 2 ? Eb : err;
-        const double cnt = lane == 1 ? nd : lane == 2 ? nbo : (double)nterm;
-        double den = lane == 1 ? dmean : mean;
-        if (lane == 2) den = div_call(btotal, (double)nbt);
-        rms = div_call(100.0 * sf::sqrt(div_call(num, cnt)), den);
-        if (lane == 1 && nd == 0.0) rms = Ed;
-        if (lane == 2 && nbo == 0.0) rms = Eb;
+        const bool d = lane == 1 && outs_d != 0, bt = lane == 2 && outs_b != 0;
+        const int ci = __popc(d ? outs_d : outs_b);
+        const double num = d ? Ed : bt ? Eb : err, cnt = d ? nd : bt ? nbo : (double)nterm;
+        const double hi = d || bt ? rec_hi[ci] : inv_t, lo = d || bt ? rec_lo[ci] : inv_t_lo;
+        const double bmean = nbt == 1   ? btotal
+                             : nbt == 2 ? btotal * 0.5
+                                        : fm::div_const(btotal, 3.0, fm::k3Hi, fm::k3Lo);
+        const double den = d ? dmean : bt ? bmean : mean;
+        rms = div_call(100.0 * sf::sqrt(fm::div_const(num, cnt, hi, lo)), den);
+        if (lane == 1 && !d) rms = Ed;
+        if (lane == 2 && !bt) rms = Eb;
       }
       Ed = __shfl_sync(kFull, rms, 1);
       Eb = __shfl_sync(kFull, rms, 2);

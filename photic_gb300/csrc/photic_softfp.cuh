@@ -271,6 +271,26 @@ PHOTIC_FM_HD bool le_call(double a, double b) {
   return ia <= ib && ib <= 0x7ff0000000000000LL;
 }
 
+// Unsigned keys that order as the doubles do, both zeros alike; 0 for a NaN,
+// below every number's.
+PHOTIC_FM_HD uint64_t order_key(double a) {
+  const uint64_t u = (uint64_t)bits(a), sign = 1ull << 63;
+  if ((u & ~sign) > 0x7ff0000000000000ull) return 0;
+  if (u == sign) return sign;
+  return u & sign ? ~u : u | sign;
+}
+
+// a + b * c for c in {1/2, 1, 2}: the product is exact (but for half the
+// least exponents and twice the largest, which are multiplied on their
+// own), so the fused sum rounds as the separate one.
+PHOTIC_FM_HD double add_scaled2(double a, double b, float c) {
+  const double cd = from_bits(
+      (int64_t)(0x3fe00000u + (c > 0.5f ? 0x100000u : 0u) + (c > 1.0f ? 0x100000u : 0u)) << 32);
+  const uint32_t e = (uint32_t)((uint64_t)bits(b) >> 52) & 0x7ffu;
+  if (e - 2u > 2042u) return a + b * cd;
+  return fma(b, cd, a);
+}
+
 // a / 2, exactly, for a normal a of twice the least normal's size or more.
 PHOTIC_FM_HD double half_mid(double a) { return from_bits(bits(a) - (1ll << 52)); }
 

@@ -104,6 +104,13 @@ int main(int argc, char **argv) {
       if (ok) same(got, fm::exp_t(e), "exp", e, 0);
       else g_exp_rare += e < -0x1p-30 && e > -350.0;
     }
+    {  // small counts: as hi + lo
+      const double k = (double)(1 + i % 128), hi = 1.0 / k;
+      same(fm::div_const(a, k, hi, fm::recip_lo(k, hi)), a / k, "count", a, k);
+      const float c = i % 3 == 0 ? 0.5f : i % 3 == 1 ? 1.0f : 2.0f;
+      same(sf::add_scaled2(a, b, c), a + b * (double)c, "point", a, b);
+      if ((sf::order_key(a) < sf::order_key(b)) != (a < b)) g_bad++, printf("key %a %a\n", a, b);
+    }
     if (sf::lt(a, b) != (a < b) || sf::lt(b, a) != (b < a) || sf::le(a, b) != (a <= b) ||
         !sf::le(a, a) || sf::lt(a, a) || sf::lt_call(a, b) != (a < b) ||
         sf::le_call(a, b) != (a <= b))
@@ -118,6 +125,10 @@ int main(int argc, char **argv) {
     same(fm::div_120(a), a / 120.0, "120", a, 0);
     for (double b : special) {
       same(sf::div(a, b), a / b, "div", a, b);
+      same(sf::add_scaled2(a, b, 0.5f), a + b * 0.5, "point", a, b);
+      same(sf::add_scaled2(a, b, 2.0f), a + b * 2.0, "point", a, b);
+      if ((sf::order_key(a) != 0 && sf::order_key(a) < sf::order_key(b)) != (a < b))
+        g_bad++, printf("key %a %a\n", a, b);
       if (sf::lt(a, b) != (a < b) || sf::le(a, b) != (a <= b) || sf::lt_call(a, b) != (a < b) ||
           sf::le_call(a, b) != (a <= b))
         g_bad++, printf("comparison of %a and %a\n", a, b);
