@@ -506,8 +506,8 @@ constexpr int kFewLanes = 8, kFewBlock = 128;
 template <int NB>
 __global__ void __launch_bounds__(kFewBlock) invert_few_kernel(const __grid_constant__ InvertArgs args) {
   constexpr int G = kFewLanes;
-  using Nm = NmGroup<kN, 1, G, G>;
-  constexpr int kV = (kN + 1) * G, kF = (kN + 2) * G;
+  using Nm = NmGroup<kN, 1, G, G, true>;
+  constexpr int kV = (kN + 1) * G, kF = kN + 2;
   __shared__ double smem[kFewBlock / G][kV + kF + 3 * G];
   const FitParams &fp = args.fp;
   const SceneConsts &sc = args.sc;
@@ -517,7 +517,7 @@ __global__ void __launch_bounds__(kFewBlock) invert_few_kernel(const __grid_cons
   double *X = base + kV + kF, *dd = X + G, *kk = dd + G;
   Nm m;
   m.V = base;
-  m.Fv = base + kV + gl;
+  m.Fv = base + kV;
   m.X = X;
   m.gl = gl;
   m.clear();

@@ -52,10 +52,10 @@ struct JG {
   static_assert(C == 1 || G == 32, "a second coordinate slot only with a warp per pixel");
   static constexpr int CG = C * G;            // row length of a vertex
   static constexpr int NF = (N + 2) & ~1;     // vertex costs, padded
-  // doubles of shared memory per group: vertices, per-lane vertex costs,
+  // doubles of shared memory per group: vertices, vertex costs,
   // the evaluation point, band terms (squared residual, K, bottom share)
   // and the final cost details
-  static constexpr int kSmem = (N + 1) * CG + NF * G + CG + 3 * G + 8 + 16;
+  static constexpr int kSmem = (N + 1) * CG + NF + CG + 3 * G + 8 + 16;
   static constexpr int kGroups = kBlock / G;
 };
 
@@ -154,7 +154,7 @@ __global__ void __launch_bounds__(kBlock) joint_group_kernel(const __grid_consta
     double *base = smem + gid * D::kSmem;
     g.V = base;
     g.F = g.V + (N + 1) * CG;
-    g.X = g.F + D::NF * G;
+    g.X = g.F + D::NF;
     g.dd = g.X + CG;
     g.kk = g.dd + G;
     g.io = g.kk + G;
@@ -162,12 +162,13 @@ __global__ void __launch_bounds__(kBlock) joint_group_kernel(const __grid_consta
     g.kmin = g.misc + 8;
     g.kpen = g.kmin + 8;
   }
-  NmGroup<N, C, G, CG> m;
+  NmGroup<N, C, G, CG, true> m;
   m.V = g.V;
-  m.Fv = g.F + gl;
+  m.Fv = g.F;
   m.X = g.X;
   m.gl = gl;
   m.clear();
+  g.dd[gl] = 0.0;  // the slots of bands beyond nb stay zero
   const unsigned gmask = (G == 32 ? kFull : ((1u << G) - 1u) << ((threadIdx.x & 31) & ~(G - 1)));
   m.gmask = gmask;
 
@@ -331,8 +332,9 @@ __global__ void __launch_bounds__(kBlock) joint_group_kernel(const __grid_consta
     double y = 0.0;
     if (has && gl == 0) {
       double err = 0.0, Ke = 0.0, Kall = 1.0e4, iod = 0.0;
-      for (int tau = 0; tau < K * 4; tau++)
-        if ((tau & 3) < nb) err = err + g.dd[tau];
+      // on the integer pipe: the FP64 pipe is this kernel's bound (fewer bands
+      // than four leave zeros, which add nothing)
+      err = sf::sum_positive(g.dd, 1, 4 * K);
       // (a scene without a penalty adds +0)
       for (int s = 0; s < K; s++)
         if (fm::bits(g.kpen[s]) != 0) Ke = Ke + g.kpen[s];

@@ -43,10 +43,10 @@ struct NmGroup {
   int32_t ck_valid;
 
   static __device__ __forceinline__ bool lt(double a, double b) {
-    return kSharedF ? sf::lt(a, b) : sf::lt_call(a, b);
+    return NT > 0 ? sf::lt_call(a, b) : sf::lt(a, b);
   }
   static __device__ __forceinline__ bool le(double a, double b) {
-    return kSharedF ? sf::le(a, b) : sf::le_call(a, b);
+    return NT > 0 ? sf::le_call(a, b) : sf::le(a, b);
   }
   __device__ __forceinline__ int dim() const { return NT > 0 ? NT : nrt; }
   __device__ __forceinline__ int coord(int t) const { return gl + t * G; }

@@ -426,5 +426,53 @@ PHOTIC_FM_HD bool sum_less_one(const double *p, int stride, int n, int h, double
   return true;
 }
 
+// ((0 + p[0]) + p[stride]) + ..., n terms, each addition rounded as in double,
+// for terms that are not negative: the running sum as a significand and an
+// exponent, about thirty integer instructions an addition against one FP64
+// instruction, for the ordered sums that one lane of a warp forms where the
+// FP64 pipe is the bound.  Subnormal, infinite and NaN terms and negative ones
+// are added in double.
+PHOTIC_FM_HD double sum_positive(const double *p, int stride, int n) {
+  uint64_t m = 0;  // significand, leading bit 61, nine bits of room below
+  int32_t ez = 0;
+  bool plain = true;
+#if defined(__CUDA_ARCH__)
+#pragma unroll 1
+#endif
+  for (int i = 0; i < n; i++) {
+    const uint64_t u = (uint64_t)bits(p[i * stride]);
+    const uint32_t h = (uint32_t)(u >> 32);
+    const int32_t e = (int32_t)(h >> 20);  // sign and exponent
+    const uint64_t t = (((uint64_t)((h & 0xfffffu) | 0x100000u) << 32) | (uint32_t)u) << 9;
+    if (u == 0) continue;
+    plain = plain && (uint32_t)(e - 1) < 0x7feu;
+    // the larger exponent's term stays (equal ones in either order)
+    const bool swap = e > ez;
+    const uint64_t a = swap ? t : m;
+    const uint64_t b = swap ? m : t;
+    int32_t d = swap ? e - ez : ez - e;
+    ez = swap ? e : ez;
+    d = d > 63 ? 63 : d;
+    const uint64_t c = b >> d;
+    const uint64_t s = (a + c) | ((c << d) != b ? 1u : 0u);
+    const uint32_t k = (uint32_t)(s >> 62);  // carry
+    uint64_t r = s + ((0x100ull << k) - 1u) + ((s >> (9 + k)) & 1u);
+    r >>= 9 + k;
+    const uint32_t o = (uint32_t)(r >> 53);  // rounded up to the next power
+    m = (r >> o) << 9;
+    ez += (int32_t)(k + o);
+  }
+  if (!plain || ez >= 0x7ff) {
+    double z = 0.0;
+#if defined(__CUDA_ARCH__)
+#pragma unroll 1
+#endif
+    for (int i = 0; i < n; i++) z = z + p[i * stride];
+    return z;
+  }
+  if (m == 0) return 0.0;
+  return from_bits((int64_t)((m >> 9) - (1ull << 52) + ((uint64_t)ez << 52)));
+}
+
 }  // namespace sf
 }  // namespace photic

@@ -134,6 +134,16 @@ int main(int argc, char **argv) {
         g_bad++, printf("comparison of %a and %a\n", a, b);
     }
   }
+  for (long i = 0; i < n / 20; i++) {  // ordered sums of terms that are not negative
+    double v[40];
+    const int m = (int)(next() % 40), span = i % 4 == 0 ? 0 : i % 4 == 1 ? 3 : i % 4 == 2 ? 30 : 900;
+    for (int j = 0; j < m; j++) v[j] = next() % 9 == 0 ? 0.0 : fabs(sample(-span, span));
+    if (m && i % 97 == 0) v[next() % m] = i % 2 ? NAN : i % 3 ? INFINITY : 3e-310;
+    if (m && i % 89 == 0) v[next() % m] = -1.0;
+    double want = 0.0;
+    for (int j = 0; j < m; j++) want = want + v[j];
+    same(sf::sum_positive(v, 1, m), want, "sum", m, 0);
+  }
   const double refused[] = {-0.0, 0.0, -5e-324, -354.0, -400.0, -1e300, -INFINITY, NAN};
   for (double e : refused) {
     bool ok = true;
