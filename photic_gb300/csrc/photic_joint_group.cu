@@ -13,7 +13,7 @@
 //   * the Nelder-Mead bookkeeping is split by coordinate: lane l owns
 //     coordinate l (and l + 32 for the one n = 33 shape) of every vertex, centroid and
 //     trial point, so the O(n^2) centroid becomes O(n) per lane; the
-//     vertex costs (one copy per lane) and the decisions taken on them are
+//     vertex costs (one copy per group) and the decisions taken on them are
 //     replicated in every lane of the group;
 //   * vertices live in shared memory in lane-owned columns; the point to
 //     evaluate is staged there for the band lanes.

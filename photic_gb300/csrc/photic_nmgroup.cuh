@@ -4,8 +4,8 @@
 // coordinate l (and l + G, ... up to C slots) of every vertex, the centroid
 // and the trial points; the vertex costs and every decision taken on them
 // are replicated in all lanes of the group, each lane keeping its own copy
-// of the costs -- or, with kSharedF (a group of a whole warp), one copy
-// that every write reaches between two warp barriers.  The simplex size is a
+// of the costs -- or, with kSharedF, one copy for the group, which every
+// write reaches between two barriers of the group's lanes.  The simplex size is a
 // template constant (NT > 0) or set at run time (NT = 0, member nrt), for
 // pixels whose parameter count varies.
 #pragma once

@@ -129,35 +129,6 @@ PHOTIC_FM_HD bool near_positive(double a) {
   return (hi - 0x34100000u) < 0x17d00000u;
 }
 
-// a * b, correctly rounded, for normal operands with a normal product: the
-// 106-bit product of the significands, its leading 53 bits rounded to
-// nearest even.
-PHOTIC_FM_HD double mul_mid(double a, double b) {
-  const uint64_t ua = (uint64_t)bits(a), ub = (uint64_t)bits(b);
-  const uint32_t ah = (uint32_t)(ua >> 32), al = (uint32_t)ua;
-  const uint32_t bh = (uint32_t)(ub >> 32), bl = (uint32_t)ub;
-  const uint32_t Ah = (ah & 0xfffffu) | 0x100000u, Bh = (bh & 0xfffffu) | 0x100000u;
-  const uint64_t p0 = (uint64_t)al * bl;
-  uint64_t m = (uint64_t)al * Bh + (p0 >> 32);
-  m = (uint64_t)Ah * bl + m;
-  const uint64_t h = (uint64_t)Ah * Bh + (m >> 32);
-  const uint32_t h1 = (uint32_t)(h >> 32), h0 = (uint32_t)h, m0 = (uint32_t)m;
-  const uint32_t top = h1 >> 9;  // 1: the product is at least 2 (bit 105)
-  const uint32_t k = 20u + top;
-  // (h : m0) >> k and the bits below
-  const uint64_t q = (((uint64_t)h1 << 32) | h0) << (32u - k);
-  uint32_t r0 = (uint32_t)q | (m0 >> k);
-  uint32_t r1 = (uint32_t)(q >> 32);
-  const uint32_t rest = m0 << (32u - k);
-  const uint32_t t = rest | ((uint32_t)p0 != 0u ? 1u : 0u);
-  const uint32_t up = t > 0x80000000u - (r0 & 1u) ? 1u : 0u;
-  const uint32_t e =
-      (ah & 0x7ff00000u) + (bh & 0x7ff00000u) - 0x40000000u + ((top + 0u) << 20);
-  uint64_t out = ((((uint64_t)r1 << 32) | r0) + up) + ((uint64_t)e << 32);
-  out |= (uint64_t)((ah ^ bh) & 0x80000000u) << 32;
-  return from_bits((int64_t)out);
-}
-
 // a / b, correctly rounded, for operands in mid; y: 1 / (leading 24 bits of
 // b's significand) to 22 bits.
 PHOTIC_FM_HD double div_mid(double a, double b, float y) {
