@@ -25,6 +25,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <type_traits>
+
 #include "photic_dfcost.cuh"
 #include "photic_fp64.cuh"
 #include "photic_kernels.h"
@@ -262,6 +264,124 @@ __device__ __forceinline__ void load_spectrum(const InvertArgs &args, int64_t p,
   }
 }
 
+// The end of a launch.  Starts run for 100 to 2 000 evaluations, so once the
+// queue is empty warps thin out, and a warp with one start left takes as long
+// a trip as a full one.  A warp therefore first takes up starts that others
+// have handed on, and one that still has no more than args.give hands on its
+// own and ends; when no more than args.few_left are left in all, every warp
+// does, and groups of lanes finish them (invert_few_kernel).  Nothing waits:
+// a warp takes the next records in order that are ready, or none.  1024 x 320
+// pixels 307 -> 299 ms, 20 011 of eight bands 112 -> 83, a 701 x 997 tile of
+// seeds 278 -> 264, the lookup-table loop over 509 x 400 91 -> 86.
+// counted: the warp's starts in LeftStarts::live, -1 before its first call.
+// true: the warp ends.
+template <int BS, class Px>
+__device__ __forceinline__ bool hand_on(const InvertArgs &args, NmPixel<PrecF64, BS> &m, Px &px,
+                                        int lane, double var_limit, bool &has, int64_t &item,
+                                        int32_t &start_k, int32_t &guard, int &counted) {
+  using Nm = NmPixel<PrecF64, BS>;
+  constexpr int kPx = 2 * (int)(sizeof px.rrs / sizeof(double)) + 1;
+  LeftStarts &q = *args.left;
+  unsigned char *const mem = reinterpret_cast<unsigned char *>(args.left);
+  int32_t *const ready = reinterpret_cast<int32_t *>(mem + left_ready_offset());
+  LeftStart *const rec = reinterpret_cast<LeftStart *>(mem + left_record_offset(args.left_slots));
+  double *const mine = reinterpret_cast<double *>(&px);
+
+  int n = __popc(__ballot_sync(kFull, has));
+  unsigned head = 0;
+  bool few = false;
+  if (lane == 0) {
+    if (counted < 0) {
+      atomicAdd(&q.live, n);
+      __threadfence();
+      atomicAdd(&q.warps_out, 1);
+    } else if (n != counted) {
+      atomicSub(&q.live, counted - n);
+    }
+    few = __ldcg(&q.warps_out) == (int)(gridDim.x * (BS / 32)) && __ldcg(&q.live) <= args.few_left;
+    head = __ldcg(&q.taken);
+  }
+  head = __shfl_sync(kFull, head, 0);
+  few = __shfl_sync(kFull, few, 0);
+
+  if (n < 32 && !few) {
+    const unsigned at = head + lane;
+    const bool full = at < (unsigned)args.left_slots && __ldcg(ready + at) != 0;
+    const unsigned waiting = __ballot_sync(kFull, full);
+    const int run = waiting == kFull ? 32 : __ffs(~waiting) - 1;
+    const int k = run < 32 - n ? run : 32 - n;
+    if (k > 0) {
+      __threadfence();
+      bool won = false;
+      if (lane == 0) won = atomicCAS(&q.taken, head, head + k) == head;
+      won = __shfl_sync(kFull, won, 0);
+      const unsigned idle = __ballot_sync(kFull, !has);
+      const int rank = __popc(idle & ((1u << lane) - 1u));
+      if (won && !has && rank < k) {
+        const LeftStart &d = rec[head + rank];
+#pragma unroll 1
+        for (int i = 0; i < Nm::kSlots; i++) m.w[i * BS] = __ldcg(d.slots + i);
+#pragma unroll
+        for (int i = 0; i < kPx; i++) mine[i] = __ldcg(d.px + i);
+        m.ylo = __ldcg(&d.ylo);
+        m.fr = __ldcg(&d.fr);
+        m.scale = __ldcg(&d.scale);
+        m.floor_lo = __ldcg(&d.floor_lo);
+        m.phase = __ldcg(&d.phase);
+        m.jj = __ldcg(&d.jj);
+        m.hi = __ldcg(&d.hi);
+        m.lo = __ldcg(&d.lo);
+        m.icount = __ldcg(&d.icount);
+        m.numres = __ldcg(&d.numres);
+        m.ifault = __ldcg(&d.ifault);
+        m.countdown = __ldcg(&d.countdown);
+        m.var_limit = var_limit;
+        m.konvge = args.fp.konvge;
+        m.kcount = args.fp.kcount;
+        item = __ldcg(&d.item);
+        start_k = __ldcg(&d.start_k);
+        guard = __ldcg(&d.guard);
+        has = true;
+      }
+      if (won) n += k;
+    }
+  }
+  counted = n;
+
+  // starts in sequence (item < 0) stay with their warp
+  if ((n > args.give && !few) || __any_sync(kFull, has && item < 0)) return false;
+  unsigned base = 0;
+  if (lane == 0 && n > 0) base = atomicAdd(&q.given, (unsigned)n);
+  base = __shfl_sync(kFull, base, 0);
+  const unsigned busy = __ballot_sync(kFull, has);
+  const unsigned at = base + __popc(busy & ((1u << lane) - 1u));
+  if (has && at < (unsigned)args.left_slots) {
+    LeftStart &d = rec[at];
+#pragma unroll 1
+    for (int i = 0; i < Nm::kSlots; i++) d.slots[i] = m.w[i * BS];
+#pragma unroll
+    for (int i = 0; i < kPx; i++) d.px[i] = mine[i];
+    d.ylo = m.ylo;
+    d.fr = m.fr;
+    d.scale = m.scale;
+    d.floor_lo = m.floor_lo;
+    d.item = item;
+    d.phase = m.phase;
+    d.jj = m.jj;
+    d.hi = m.hi;
+    d.lo = m.lo;
+    d.icount = m.icount;
+    d.numres = m.numres;
+    d.ifault = m.ifault;
+    d.countdown = m.countdown;
+    d.start_k = start_k;
+    d.guard = guard;
+    __threadfence();
+    atomicExch(ready + at, 1);
+  }
+  return true;
+}
+
 // The queue's positions: the first n_seq are pixels, each lane running a
 // pixel's starts one after the other; then, for the other n_par pixels, every
 // start is a position of its own (start-major: the first starts of all these
@@ -306,7 +426,7 @@ __global__ void __launch_bounds__(BS) invert_kernel(const __grid_constant__ Inve
   T lowest = P::zero();
 
   bool has = false, open = true;
-  int chunk_next = 0, chunk_end = 0;
+  int chunk_next = 0, chunk_end = 0, counted = -1;
   const int32_t guard_cap = (fp.n_hstarts + 1) * (fp.kcount + 8 * kN + 16);
 
   for (;;) {
@@ -416,6 +536,11 @@ __global__ void __launch_bounds__(BS) invert_kernel(const __grid_constant__ Inve
       chunk_next += __popc(taken);
       need &= ~taken;
     }
+    if constexpr (std::is_same<P, PrecF64>::value) {
+      if (!open && args.left != nullptr) {
+        if (hand_on(args, m, px, lane, var_limit, has, item, start_k, guard, counted)) break;
+      }
+    }
     if (!__any_sync(kFull, has)) break;
 
     // ---- one cost evaluation per lane, then the bookkeeping --------------
@@ -502,8 +627,11 @@ __global__ void __launch_bounds__(BS) invert_kernel(const __grid_constant__ Inve
 // instructions and six coordinates' (342 a trip, here about 130, at 64 clocks
 // each for a warp alone on its SM quarter): 256 pixels 35 -> 14.6 ms.  A full
 // device is better used by a lane a start (few_starts, photic_host.cu).
+//
+// kLeft: the starts that the warps of the lane kernel have handed on and none
+// has taken up, each from the state it was left in.
 constexpr int kFewLanes = 8, kFewBlock = 128;
-template <int NB>
+template <int NB, bool kLeft>
 __global__ void __launch_bounds__(kFewBlock) invert_few_kernel(const __grid_constant__ InvertArgs args) {
   constexpr int G = kFewLanes;
   using Nm = NmGroup<kN, 1, G, G, true>;
@@ -524,7 +652,7 @@ __global__ void __launch_bounds__(kFewBlock) invert_few_kernel(const __grid_cons
   const unsigned gmask = ((1u << G) - 1u) << ((threadIdx.x & 31) & ~(G - 1));
   m.gmask = gmask;
   StartRecord<PrecF64> *const rec = reinterpret_cast<StartRecord<PrecF64> *>(args.records);
-  const int64_t total_pos = args.n_par * fp.n_hstarts;
+  const int64_t total_pos = kLeft ? (int64_t)__ldcg(&args.left->given) : args.n_par * fp.n_hstarts;
   const double var_limit = fp.reqmin * (double)kN;
   const int32_t guard_cap = (fp.n_hstarts + 1) * (fp.kcount + 8 * kN + 16);
 
@@ -536,14 +664,24 @@ __global__ void __launch_bounds__(kFewBlock) invert_few_kernel(const __grid_cons
   for (;;) {
     bool fresh = false;
     int64_t p = 0;
+    const LeftStart *left = nullptr;
     float r[NB];
     do {
       unsigned long long w = ~0ull;
       const bool ask = !has && open && !fresh;
-      if (ask && gl == 0) w = atomicAdd(args.queue, 1ull);
+      if (ask && gl == 0)
+        w = kLeft ? (unsigned long long)atomicAdd(&args.left->taken, 1u)
+                  : atomicAdd(args.queue, 1ull);
       w = __shfl_sync(kFull, w, 0, G);
       if (ask) {
-        if (w < (unsigned long long)total_pos) {
+        if (kLeft && w < (unsigned long long)total_pos) {
+          left = reinterpret_cast<const LeftStart *>(
+                     reinterpret_cast<const unsigned char *>(args.left) +
+                     left_record_offset(args.left_slots)) + w;
+          start_k = left->start_k;
+          item = left->item;
+          fresh = __ldcg(args.exit_k + item) >= start_k;
+        } else if (w < (unsigned long long)total_pos) {
           start_k = (int32_t)((int64_t)w / args.n_par);
           item = (int64_t)w % args.n_par;
           p = pixel_at(args, item);
@@ -566,7 +704,40 @@ __global__ void __launch_bounds__(kFewBlock) invert_few_kernel(const __grid_cons
     } while (__any_sync(kFull, !has && open && !fresh));
     if (!__any_sync(kFull, has || fresh)) break;
 
-    if (fresh) {
+    if (kLeft && fresh) {
+      using Px = NmPixel<PrecF64, 1>;
+      const int i = gl < kN ? gl : 0;  // a lane without a coordinate holds the first's
+      mean = left->px[2 * NB];
+      my_rrs = left->px[gl < NB ? gl : 0];
+      my_pw = left->px[NB + (gl < NB ? gl : 0)];
+      m.start[0] = left->slots[Px::kV + kN * kN + i];  // vertex N while the simplex is set up
+      m.begin(var_limit, fp.konvge, fp.kcount);
+      __syncwarp(gmask);
+      if (gl < kN) {
+#pragma unroll 1
+        for (int j = 0; j <= kN; j++) m.V[j * G + gl] = left->slots[Px::kV + j * kN + gl];
+        X[gl] = left->slots[Px::kX + gl];
+      }
+      if (gl <= kN) m.Fv[gl] = left->slots[Px::kF + gl];
+      m.step[0] = left->slots[Px::kStep + i];
+      m.refl[0] = left->slots[Px::kRefl + i];
+      m.cen[0] = left->slots[Px::kCen + i];
+      m.xmin[0] = m.trial[0] = left->slots[Px::kX + i];
+      m.ylo = left->ylo;
+      m.fr = left->fr;
+      m.scale = left->scale;
+      m.floor_lo = left->floor_lo;
+      m.phase = left->phase;
+      m.jj = left->jj;
+      m.hi = left->hi;
+      m.lo = left->lo;
+      m.icount = left->icount;
+      m.numres = left->numres;
+      m.ifault = left->ifault;
+      m.countdown = left->countdown;
+      guard = left->guard;
+      has = true;
+    } else if (fresh) {
       PixelF64<NB> px;
       double rd[NB];
 #pragma unroll
@@ -705,6 +876,26 @@ __global__ void __launch_bounds__(128) finish_kernel(const __grid_constant__ Inv
   if (args.pixels) write_single_chain(args, q, p, det.model_error);
 }
 
+// Groups of lanes for up to `positions` starts.
+template <int NB, bool kLeft>
+cudaError_t launch_few_kernel(const InvertArgs &a, int64_t positions, cudaStream_t s) {
+  auto k = invert_few_kernel<NB, kLeft>;
+  int occ = 0, dev = 0, sms = 0;
+  cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k, kFewBlock, 0);
+  if (e == cudaSuccess) e = cudaGetDevice(&dev);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  if (e != cudaSuccess) return e;
+  if (occ < 1) return cudaErrorInvalidConfiguration;
+  // one block (a warp a quarter) per SM first
+  constexpr int kGroups = kFewBlock / kFewLanes;
+  int64_t per_sm = (positions + (int64_t)sms * kGroups - 1) / ((int64_t)sms * kGroups);
+  if (per_sm > occ) per_sm = occ;
+  const int64_t need = (positions + kGroups - 1) / kGroups;
+  const int64_t grid = per_sm * sms < need ? per_sm * sms : need;
+  k<<<(unsigned)grid, kFewBlock, 0, s>>>(a);
+  return cudaGetLastError();
+}
+
 template <class P, int NB, int BS>
 cudaError_t launch_one(const InvertArgs &a, int grid, cudaStream_t s, int *occupancy) {
   const size_t smem =
@@ -715,6 +906,12 @@ cudaError_t launch_one(const InvertArgs &a, int grid, cudaStream_t s, int *occup
   if (occupancy) return cudaOccupancyMaxActiveBlocksPerMultiprocessor(occupancy, k, BS, smem);
   static_assert(sizeof(StartRecord<P>) == kStartRecordBytes, "record size");
   k<<<grid, BS, smem, s>>>(a);
+  if constexpr (std::is_same<P, PrecF64>::value) {
+    if (a.left != nullptr) {
+      e = launch_few_kernel<NB, true>(a, (int64_t)grid * BS, s);
+      if (e != cudaSuccess) return e;
+    }
+  }
   if (a.n_par > 0)
     finish_kernel<P, NB><<<(unsigned)((a.n_par + 127) / 128), 128, 0, s>>>(a);
   return cudaGetLastError();
@@ -747,28 +944,17 @@ size_t invert_smem_bytes(int block) {
 namespace {
 
 template <int NB>
-cudaError_t launch_few(const InvertArgs &a, int sms, cudaStream_t s) {
-  int occ = 0;
-  cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, invert_few_kernel<NB>,
-                                                                kFewBlock, 0);
+cudaError_t launch_few(const InvertArgs &a, cudaStream_t s) {
+  cudaError_t e = launch_few_kernel<NB, false>(a, a.n_par * a.fp.n_hstarts, s);
   if (e != cudaSuccess) return e;
-  if (occ < 1) return cudaErrorInvalidConfiguration;
-  // one block (a warp a quarter) per SM first
-  constexpr int kGroups = kFewBlock / kFewLanes;
-  const int64_t positions = a.n_par * a.fp.n_hstarts;
-  int64_t per_sm = (positions + (int64_t)sms * kGroups - 1) / ((int64_t)sms * kGroups);
-  if (per_sm > occ) per_sm = occ;
-  const int64_t need = (positions + kGroups - 1) / kGroups;
-  const int64_t grid = per_sm * sms < need ? per_sm * sms : need;
-  invert_few_kernel<NB><<<(unsigned)grid, kFewBlock, 0, s>>>(a);
   finish_kernel<PrecF64, NB><<<(unsigned)((a.n_par + 127) / 128), 128, 0, s>>>(a);
   return cudaGetLastError();
 }
 
 }  // namespace
 
-cudaError_t launch_invert_few(const InvertArgs &a, int sms, cudaStream_t s) {
-  return a.fp.n_bands <= 4 ? launch_few<4>(a, sms, s) : launch_few<8>(a, sms, s);
+cudaError_t launch_invert_few(const InvertArgs &a, cudaStream_t s) {
+  return a.fp.n_bands <= 4 ? launch_few<4>(a, s) : launch_few<8>(a, s);
 }
 
 cudaError_t launch_invert(const InvertArgs &a, int precision, int block, int grid,

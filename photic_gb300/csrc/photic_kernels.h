@@ -46,6 +46,10 @@ struct InvertArgs {
   void *records;         // [n_par][n_hstarts] results of the starts
   int32_t *exit_k;       // [n_par] first start known to meet the early exit, -1 masked
   int32_t claim;         // positions a warp claims at a time (1..32)
+  struct LeftStarts *left;  // starts that warps hand on at the launch's end, or NULL
+  int32_t give;             // a warp with at most this many starts hands them on
+  int32_t few_left;         // so does every warp once no more than these are left
+  int32_t left_slots;       // records in left: one for every lane of the launch
   // the lookup-table loop with a chain for every pixel: position -> pixel,
   // and what the loop reports of a fitted pixel and of its chain
   const int64_t *pixels;
@@ -80,11 +84,35 @@ inline void start_work_layout(StartWork &w, unsigned char *mem, int64_t slots, i
 }
 
 constexpr size_t kStartRecordBytes = 64;
+
+// A start in progress: the pixel and the state of photic_nmpixel.cuh between
+// two evaluations.
+struct LeftStart {
+  double px[17];     // PixelF64's reflectances, powers and mean
+  double slots[73];  // NmPixel's
+  double ylo, fr, scale;
+  long long floor_lo, item;
+  int32_t phase, jj, hi, lo, icount, numres, ifault, countdown, start_k, guard;
+};
+// Starts handed on, followed in memory by int32_t ready[slots] and
+// LeftStart[slots] (zero up to the latter before the launch).
+struct LeftStarts {
+  unsigned int given, taken;     // records reserved, records taken up (in order)
+  int32_t live;                  // starts running or waiting, of the warps below
+  int32_t warps_out;             // warps that have seen the queue empty
+};
+__host__ __device__ inline size_t left_ready_offset() { return 64; }
+__host__ __device__ inline size_t left_record_offset(int64_t slots) {
+  return (left_ready_offset() + (size_t)slots * sizeof(int32_t) + 255) / 256 * 256;
+}
+inline size_t left_bytes(int64_t slots) {
+  return left_record_offset(slots) + (size_t)slots * sizeof(LeftStart);
+}
 size_t invert_smem_bytes(int block);
 cudaError_t launch_invert(const InvertArgs &a, int precision, int block, int grid,
                           cudaStream_t s);
 // FP64, every position a start (n_seq = 0): a group of lanes each.
-cudaError_t launch_invert_few(const InvertArgs &a, int sms, cudaStream_t s);
+cudaError_t launch_invert_few(const InvertArgs &a, cudaStream_t s);
 // Resident blocks per SM of the kernel that launch_invert would use (0 on error).
 int invert_blocks_per_sm(const InvertArgs &a, int precision, int block);
 

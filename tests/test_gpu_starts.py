@@ -44,6 +44,11 @@ def _noalloc(gpu, rrs, cfg, seeds):
     (130, {"wavelengths": WL8}, False),
     (11003, {}, False),
     (40, {"block_threads": 64}, False),
+    # starts that warps hand on at the end of a launch: eight bands, seeds,
+    # and a scene whose first pixels run their starts in sequence
+    (20011, {"wavelengths": WL8}, False),
+    (60007, {"seed_step_scale": 0.1}, True),
+    (530001, {"hstarts": tuple(0.7 * (i + 1) for i in range(32)), "kcount": 30}, False),
 ])
 def test_starts_in_parallel_match_the_sequence(gpu, npix, kw, seeded):
     cfg = gpu.Config(**kw)
