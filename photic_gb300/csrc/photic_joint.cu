@@ -366,6 +366,9 @@ template <int LAYOUT, int NB>
 cudaError_t launch_all_k(const JointArgs &a, int sms, int per_sm, cudaStream_t s,
                          const JointFork *f) {
   cudaError_t e;
+  if constexpr (NB <= 4) {
+    if ((e = load_joint_groups(a)) != cudaSuccess) return e;
+  }
   if (f && (e = cudaEventRecord(f->fork, s)) != cudaSuccess) return e;
   for (int k = kMaxScenes; k >= 1; k--) {
     cudaStream_t t = f ? f->side[k - 1] : s;

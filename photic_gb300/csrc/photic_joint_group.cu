@@ -27,6 +27,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <utility>
+
 #include "photic_fp64.cuh"
 #include "photic_kernels.h"
 #include "photic_nm.cuh"
@@ -39,6 +41,7 @@ namespace {
 
 constexpr unsigned kFull = 0xffffffffu;
 constexpr int kBlock = 128;
+constexpr int kSmemMax = 227 * 1024;  // shared memory of a block, at most
 
 template <int LAYOUT, int K>
 struct JG {
@@ -478,16 +481,46 @@ __global__ void __launch_bounds__(kBlock) joint_group_kernel(const __grid_consta
   }
 }
 
+// Loads the kernels and lets them use all of a block's shared memory (the
+// same limit from every thread).  A kernel that is first loaded while others
+// run waits for them: loaded one by one, the first call of a process ran its
+// sixteen kernels one after the other, 321 ms instead of 165.
+template <int LAYOUT, int... K>
+cudaError_t load_groups(std::integer_sequence<int, K...>) {
+  cudaError_t e = cudaSuccess;
+  ((e = e != cudaSuccess ? e
+                         : cudaFuncSetAttribute(joint_group_kernel<LAYOUT, K + 1>,
+                                                cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                kSmemMax)),
+   ...);
+  return e;
+}
+
 template <int LAYOUT, int K>
 cudaError_t launch_group_k(const JointArgs &a, int per_sm, int sms, cudaStream_t s) {
   using D = JG<LAYOUT, K>;
-  const size_t bytes = (size_t)D::kGroups * D::kSmem * sizeof(double);
-  cudaError_t e = cudaFuncSetAttribute(joint_group_kernel<LAYOUT, K>,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-  if (e != cudaSuccess) return e;
+  // Blocks resident together on an SM, bounded by shared memory that nothing
+  // uses.  A start runs up to kcount evaluations in sequence, on a full SM at
+  // the rate that the FP64 pipe shares out among its warps, and a launch ends
+  // with the last of them: with eight warps the pipe is nearly as busy as
+  // with twenty and each start is twice as fast.  Milliseconds with no bound
+  // / 3 / 2 / 1 blocks, n = 3 + 3k: 512 pixels 71 / 51 / 48 / 38, 1 024 79 /
+  // 64 / 58 / 57, 4 096 138 / 117 / 105 / 114, 8 009 185 / 162 / 164 / 206,
+  // 16 000 272 / 252 / 277 / 370, 65 536 834 / 862 / 969 / 1 351; n = 1 + 4k:
+  // 512 70 / 57 / 49 / 37, 3 001 134 / 103 / 90 / 98, 4 096 144 / 120 / 109 / 125, 8 009 192 / 170 / 175
+  // / 221, 65 536 931 / 950 / 1 075 / 1 518.
+  size_t bytes = (size_t)D::kGroups * D::kSmem * sizeof(double);
+  if (per_sm <= 0) {
+    const int bound = a.npix <= (int64_t)sms * 5     ? 1
+                      : a.npix <= (int64_t)sms * 48  ? 2
+                      : a.npix <= (int64_t)sms * 160 ? 3
+                                                     : 0;
+    const size_t share = bound ? kSmemMax / bound - 1024 : 0;
+    if (bytes < share) bytes = share;
+  }
   int occ = 0;
-  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, joint_group_kernel<LAYOUT, K>, kBlock,
-                                                    bytes);
+  cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+      &occ, joint_group_kernel<LAYOUT, K>, kBlock, bytes);
   if (e != cudaSuccess) return e;
   if (occ < 1) return cudaErrorInvalidConfiguration;
   const int use = per_sm > 0 && per_sm < occ ? per_sm : occ;
@@ -516,6 +549,12 @@ cudaError_t launch_group_layout(const JointArgs &a, int k, int per_sm, int sms, 
 }
 
 }  // namespace
+
+cudaError_t load_joint_groups(const JointArgs &a) {
+  using Ks = std::make_integer_sequence<int, kMaxScenes>;
+  return a.fp.layout == PHOTIC_LAYOUT_REFERENCE ? load_groups<PHOTIC_LAYOUT_REFERENCE>(Ks())
+                                                : load_groups<PHOTIC_LAYOUT_SCENE_B>(Ks());
+}
 
 cudaError_t launch_joint_group(const JointArgs &a, int k, int per_sm, int sms, cudaStream_t s) {
   return a.fp.layout == PHOTIC_LAYOUT_REFERENCE

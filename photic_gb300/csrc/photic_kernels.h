@@ -229,6 +229,7 @@ struct JointFork {
 cudaError_t launch_joint(const JointArgs &a, int32_t *fill, int sms, int per_sm, cudaStream_t s,
                          const JointFork *f);
 // One per-k lane-group kernel (photic_joint_group.cu), n_bands <= 4.
+cudaError_t load_joint_groups(const JointArgs &a);
 cudaError_t launch_joint_group(const JointArgs &a, int k, int per_sm, int sms, cudaStream_t s);
 
 struct JointGenArgs {
