@@ -173,34 +173,35 @@ static __device__ PHOTIC_NOINLINE void band_term_general(const SceneConsts &sc, 
 // The soft operations need normal operands of moderate exponent: the tests
 // below cover each, and a term that fails one (an exact zero, an absurd
 // exponent, NaN) is evaluated again above.
-// `want_B`: t.rrs_B is used, not only t.rrs.
-__device__ __forceinline__ void band_term(const SceneConsts &sc, int b, double sec_sun,
-                                          bool want_B, double H, double rho, double P, double lnP,
-                                          double G, double X, double pw, double r, BandTerm &t) {
+
+// The band's medium: u and K, and whether its operands are moderate.
+__device__ __forceinline__ bool band_medium(const SceneConsts &sc, int b, double P, double lnP,
+                                            double G, double X, double pw, double &u, double &K) {
   const double a_phi = (sc.a0[b] + sc.a1[b] * lnP) * P;
   const double a_g = G * sc.eS[b];
   const double a = sc.aw[b] + a_phi + a_g;
   const double bb = sc.bbw[b] + X * pw;
   const double ab = a + bb;
-  const double u = sf::div_mid(bb, ab);
-  const double K = fm::bits(ab) > 0x4004000000000000LL ? 2.5 : ab;  // > 2.5 (positive here)
+  u = sf::div_mid(bb, ab);
+  K = fm::bits(ab) > 0x4004000000000000LL ? 2.5 : ab;  // > 2.5 (positive here)
+  return sf::near_positive(bb) && sf::near_positive(ab) && sf::near_positive(u);
+}
+
+// exp(-d) of a light path of d optical depths.  Beyond 200 of them the
+// exponentials change no bit of band_close's sums (the columns' part is 1 - 0,
+// the bottom's share is lost in rrs): -200 stands for every such depth,
+// unless the bottom's part itself is asked for.  (One lane in eight warps was
+// that deep, and took its warp through the general term.)
+__device__ __forceinline__ double path_loss(double d, bool &deep, bool &ok) {
+  deep = fm::bits(d) > 0x4069000000000000LL;
+  ok = ok && sf::near_positive(d);
+  return sf::exp_neg(deep ? -200.0 : -d, ok);
+}
+
+// The term from the two paths' losses; false if it has to be evaluated again.
+__device__ __forceinline__ bool band_close(double u, double K, double eC, double eB, bool deepB,
+                                           double rho, double r, BandTerm &t) {
   const double rrs_dp = (0.084 + 0.170 * u) * u;
-  double DuC = 1.03 * sf::sqrt_mid(1.0 + 2.4 * u);
-  double DuB = 1.04 * sf::sqrt_mid(1.0 + 5.4 * u);
-  if (sc.sec_view != 1.0) {
-    DuC = DuC * sc.sec_view;
-    DuB = DuB * sc.sec_view;
-  }
-  // Beyond 200 optical depths the exponentials change no bit of the sums
-  // below (the columns' part is 1 - 0, the bottom's share is lost in rrs):
-  // -200 stands for every such depth, unless the bottom's part itself is
-  // asked for.  (One lane in eight warps was that deep, and took its warp
-  // through the general term.)
-  const double dC = (sec_sun + DuC) * K * H, dB = (sec_sun + DuB) * K * H;
-  const bool deepC = fm::bits(dC) > 0x4069000000000000LL, deepB = fm::bits(dB) > 0x4069000000000000LL;
-  bool ok = !(deepB && want_B);
-  const double eC = sf::exp_neg(deepC ? -200.0 : -dC, ok);
-  const double eB = sf::exp_neg(deepB ? -200.0 : -dB, ok);
   const double rrs_C = rrs_dp * (1.0 - eC);
   const double rho_pi = fma(rho, fm::kPiHi, rho * fm::kPiLo);
   const double rrs_B = rho_pi * eB;
@@ -213,11 +214,51 @@ __device__ __forceinline__ void band_term(const SceneConsts &sc, int b, double s
   t.rrs = rrs;
   t.Rm = Rm;
   t.dd = d * d;
-  ok = ok && sf::near_positive(bb) && sf::near_positive(ab) && sf::near_positive(u) &&
-       sf::near_positive(dC) && sf::near_positive(dB) && sf::near_positive(rho) &&
-       sf::near_positive(rrs) && sf::near(den);
+  bool ok = sf::near_positive(rho) && sf::near_positive(rrs) && sf::near(den);
   // (deep: rrs_B at most 2^90 2^-288, below half an ulp of rrs above 2^-90)
   if (deepB) ok = ok && sf::lt(rho_pi, 0x1p90) && sf::lt(0x1p-90, rrs);
+  return ok;
+}
+
+// `want_B`: t.rrs_B is used, not only t.rrs.
+__device__ __forceinline__ void band_term(const SceneConsts &sc, int b, double sec_sun,
+                                          bool want_B, double H, double rho, double P, double lnP,
+                                          double G, double X, double pw, double r, BandTerm &t) {
+  double u, K;
+  bool ok = band_medium(sc, b, P, lnP, G, X, pw, u, K);
+  double DuC = 1.03 * sf::sqrt_mid(1.0 + 2.4 * u);
+  double DuB = 1.04 * sf::sqrt_mid(1.0 + 5.4 * u);
+  if (sc.sec_view != 1.0) {
+    DuC = DuC * sc.sec_view;
+    DuB = DuB * sc.sec_view;
+  }
+  bool deepC, deepB;
+  const double eC = path_loss((sec_sun + DuC) * K * H, deepC, ok);
+  const double eB = path_loss((sec_sun + DuB) * K * H, deepB, ok);
+  ok = band_close(u, K, eC, eB, deepB, rho, r, t) && ok && !(deepB && want_B);
+  if (!ok) {
+    BandTerm g;
+    band_term_general(sc, b, sec_sun, H, rho, P, lnP, G, X, pw, r, &g);
+    t = g;
+  }
+}
+
+// The same term from two lanes of the group `mask`: a lane with `bottom` set
+// evaluates the bottom's path, the lane `apart` below it the columns' and the
+// term (valid there).
+__device__ __forceinline__ void band_term_pair(const SceneConsts &sc, int b, double sec_sun,
+                                               bool bottom, int apart, unsigned mask, double H,
+                                               double rho, double P, double lnP, double G, double X,
+                                               double pw, double r, BandTerm &t) {
+  double u, K;
+  bool ok = band_medium(sc, b, P, lnP, G, X, pw, u, K), deep;
+  double Du = (bottom ? 1.04 : 1.03) * sf::sqrt_mid(1.0 + (bottom ? 5.4 : 2.4) * u);
+  if (sc.sec_view != 1.0) Du = Du * sc.sec_view;
+  const double e = path_loss((sec_sun + Du) * K * H, deep, ok);
+  const double eB = __shfl_down_sync(mask, e, apart);
+  const int fB = __shfl_down_sync(mask, (ok ? 1 : 0) | (deep ? 2 : 0), apart);
+  if (bottom) return;
+  ok = band_close(u, K, e, eB, (fB & 2) != 0, rho, r, t) && ok && (fB & 1) != 0;
   if (!ok) {
     BandTerm g;
     band_term_general(sc, b, sec_sun, H, rho, P, lnP, G, X, pw, r, &g);

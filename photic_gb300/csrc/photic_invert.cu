@@ -621,7 +621,7 @@ __global__ void __launch_bounds__(BS) invert_kernel(const __grid_constant__ Inve
 }
 
 // The same queue of starts for few positions: a group of eight lanes a start,
-// band b on lane b, coordinate i of the simplex on lane i (NmGroup).  A launch
+// band b on lane b (and, of four, its bottom path on lane b + 4), coordinate i of the simplex on lane i (NmGroup).  A launch
 // of few positions lasts as long as one start's chain of up to kcount
 // evaluations, and one lane's evaluation takes four times a band's FP64
 // instructions and six coordinates' (342 a trip, here about 130, at 64 clocks
@@ -636,11 +636,15 @@ __global__ void __launch_bounds__(kFewBlock) invert_few_kernel(const __grid_cons
   constexpr int G = kFewLanes;
   using Nm = NmGroup<kN, 1, G, G, true>;
   constexpr int kV = (kN + 1) * G, kF = kN + 2;
+  // up to four bands: band gl % 4, the lanes from 4 on its bottom path
+  constexpr int kPaths = G / 2;
+  constexpr bool kPair = NB <= kPaths;
   __shared__ double smem[kFewBlock / G][kV + kF + 3 * G];
   const FitParams &fp = args.fp;
   const SceneConsts &sc = args.sc;
   const int nb = fp.n_bands;
   const int gl = threadIdx.x % G;
+  const int band = kPair ? (gl % kPaths < nb ? gl % kPaths : 0) : (gl < nb ? gl : 0);
   double *base = smem[threadIdx.x / G];
   double *X = base + kV + kF, *dd = X + G, *kk = dd + G;
   Nm m;
@@ -708,8 +712,8 @@ __global__ void __launch_bounds__(kFewBlock) invert_few_kernel(const __grid_cons
       using Px = NmPixel<PrecF64, 1>;
       const int i = gl < kN ? gl : 0;  // a lane without a coordinate holds the first's
       mean = left->px[2 * NB];
-      my_rrs = left->px[gl < NB ? gl : 0];
-      my_pw = left->px[NB + (gl < NB ? gl : 0)];
+      my_rrs = left->px[band];
+      my_pw = left->px[NB + band];
       m.start[0] = left->slots[Px::kV + kN * kN + i];  // vertex N while the simplex is set up
       m.begin(var_limit, fp.konvge, fp.kcount);
       __syncwarp(gmask);
@@ -746,8 +750,8 @@ __global__ void __launch_bounds__(kFewBlock) invert_few_kernel(const __grid_cons
       mean = px.mean;
 #pragma unroll
       for (int b = 0; b < NB; b++)
-        if (b == gl) my_rrs = px.rrs[b];
-      my_pw = pow_call(sc.ratio440[gl < nb ? gl : 0], Y);
+        if (b == band) my_rrs = px.rrs[b];
+      my_pw = pow_call(sc.ratio440[band], Y);
       double start[kN], step[kN];
       bool seeded = false;
       if (args.seeds != nullptr) {
@@ -782,14 +786,21 @@ __global__ void __launch_bounds__(kFewBlock) invert_few_kernel(const __grid_cons
     __syncwarp();
     // ---- one evaluation per group at X: a band a lane, then the sum and the
     // rest of the cost on every lane
-    if (has && gl < nb) {
+    if (has && (kPair || gl < nb)) {
       const double H = fabs(X[0]), B = 0.01 * fabs(X[1]);
       const double qB = fm::self_ratio(fabs(X[2])) * B;
       const double P = 0.01 * fabs(X[3]), Gg = 0.01 * fabs(X[4]), Xx = 0.01 * fabs(X[5]);
       BandTerm t;
-      band_term(sc, gl, sc.sec_sun, false, H, qB * sc.refl[gl], P, log(P), Gg, Xx, my_pw, my_rrs, t);
-      dd[gl] = t.dd;
-      kk[gl] = t.K;
+      if constexpr (kPair)
+        band_term_pair(sc, band, sc.sec_sun, gl >= kPaths, kPaths, gmask, H, qB * sc.refl[band], P,
+                       log(P), Gg, Xx, my_pw, my_rrs, t);
+      else
+        band_term(sc, gl, sc.sec_sun, false, H, qB * sc.refl[gl], P, log(P), Gg, Xx, my_pw, my_rrs,
+                  t);
+      if (gl < nb) {
+        dd[gl] = t.dd;
+        kk[gl] = t.K;
+      }
     }
     __syncwarp();
     if (has) {
