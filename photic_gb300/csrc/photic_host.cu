@@ -370,16 +370,18 @@ cudaError_t start_work_init(StartWork &w, unsigned char *mem, int64_t slots, int
   return e;
 }
 
-// Whether a group of lanes a start (invert_few_kernel) is faster than a lane:
-// up to 512 starts an SM with four bands, twice that with eight, where a lane
-// has twice the terms.  Measured on 152 SMs, milliseconds with groups / with
-// lanes: 256 pixels of four bands 14.6 / 34.8, 2 400 30 / 38, 9 600 54.0 /
-// 54.3, 20 000 81 / 66; eight bands 256 15.7 / 54, 20 000 106 / 111, 40 000
-// 168 / 148.  A seeded pixel is one start and some fallbacks, counted as two:
-// 3 000 16.5 / 39, 40 000 54.9 / 54.5, 80 000 87 / 62.
+// Whether a group of lanes a start (invert_few_kernel) is faster than a lane
+// with the launch's end packed: up to 96 starts an SM with four bands, 256
+// with eight, where a lane has twice the terms.  Measured on 152 SMs,
+// milliseconds with groups / with lanes, eight starts a pixel: 600 pixels of
+// four bands 13.8 / 15.6, 1 200 18.3 / 18.7, 1 800 22.7 / 23.9, 2 400 26.6 /
+// 24.8, 9 600 48 / 38, 20 000 73 / 51; eight bands 600 17.0 / 23.9, 1 200 23.4
+// / 26.1, 4 800 47.9 / 48.1, 9 600 69 / 63, 20 000 108 / 87.  A seeded pixel is
+// one start and a few fallbacks, counted as one: 5 000 19.5 / 24.9, 15 000 30.2
+// / 31.1, 20 000 34.7 / 33.2, 40 000 51 / 41.
 bool few_starts(const InvertArgs &a, int precision, int sms) {
-  const int64_t starts = a.npix * (a.seeds && a.fp.n_hstarts > 2 ? 2 : a.fp.n_hstarts);
-  return precision == PHOTIC_PREC_FP64 && starts <= (int64_t)sms * (a.fp.n_bands > 4 ? 1024 : 512);
+  const int64_t starts = a.npix * (a.seeds ? 1 : a.fp.n_hstarts);
+  return precision == PHOTIC_PREC_FP64 && starts <= (int64_t)sms * (a.fp.n_bands > 4 ? 256 : 96);
 }
 
 // The batched inversion of prepared arguments: workspace (queue head, exits,

@@ -621,12 +621,14 @@ __global__ void __launch_bounds__(BS) invert_kernel(const __grid_constant__ Inve
 }
 
 // The same queue of starts for few positions: a group of eight lanes a start,
-// band b on lane b (and, of four, its bottom path on lane b + 4), coordinate i of the simplex on lane i (NmGroup).  A launch
-// of few positions lasts as long as one start's chain of up to kcount
-// evaluations, and one lane's evaluation takes four times a band's FP64
-// instructions and six coordinates' (342 a trip, here about 130, at 64 clocks
-// each for a warp alone on its SM quarter): 256 pixels 35 -> 14.6 ms.  A full
-// device is better used by a lane a start (few_starts, photic_host.cu).
+// band b on lane b (of up to four bands its bottom path on lane b + 4),
+// coordinate i of the simplex on lane i (NmGroup).  A launch of few positions
+// lasts as long as one start's chain of up to kcount evaluations, and one
+// lane's evaluation takes four times a band's FP64 instructions and six
+// coordinates' (342 a trip, here about 115, at 64 clocks each for a warp alone
+// on its SM quarter): 256 pixels 35 -> 14.6 ms, and with the bottom path on its
+// own lane 12.9.  A full device is better used by a lane a start (few_starts,
+// photic_host.cu).
 //
 // kLeft: the starts that the warps of the lane kernel have handed on and none
 // has taken up, each from the state it was left in.

@@ -44,6 +44,11 @@ def _noalloc(gpu, rrs, cfg, seeds):
     (130, {"wavelengths": WL8}, False),
     (11003, {}, False),
     (40, {"block_threads": 64}, False),
+    # both sides of the line between groups of lanes and lanes (152 SMs)
+    (1824, {}, False),
+    (1825, {}, False),
+    (4865, {"wavelengths": WL8}, False),
+    (14593, {"seed_step_scale": 0.1}, True),
     # starts that warps hand on at the end of a launch: eight bands, seeds,
     # and a scene whose first pixels run their starts in sequence
     (20011, {"wavelengths": WL8}, False),
