@@ -1008,7 +1008,7 @@ def ncgrid_leg(args, dev, rrs):
     container, GPU unpacking), and the two kernels timed alone against the
     measured HBM copy rate.  Algorithmic bytes: unpacking reads 2 B and
     writes 4 B per cell and band; packing reads 4 B and writes 2 B per cell
-    (its three passes read the grid three times).  Parity: the unpacked
+    (one pass for the extremes, one to quantise: the grid read twice).  Parity: the unpacked
     bands and the packed grid against the CPU oracle on a sample."""
     import tempfile
     import torch
@@ -1085,7 +1085,9 @@ def ncgrid_leg(args, dev, rrs):
                 "pack": {"ms": t_pk * 1e3, "algorithmic_bytes_per_cell": 6,
                          "achieved_gbs": pk_gbs,
                          "frac_of_measured_hbm": pk_gbs / peak if peak else None,
-                         "note": "three passes read the grid three times (14 B/cell moved)"},
+                         "note": "extremes, then quantisation: the grid read twice, the second "
+                                 "time partly from L2 (up to 10 B/cell moved); the time includes the "
+                                 "host's wait for the two extremes"},
                 "oracle_sample": {"cells": k, "pack_identical": pack_ok,
                                   "unpack_identical": bool(unpack_ok)}}
     finally:

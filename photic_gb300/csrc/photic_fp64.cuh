@@ -243,29 +243,6 @@ __device__ __forceinline__ void band_term(const SceneConsts &sc, int b, double s
   }
 }
 
-// The same term from two lanes of the group `mask`: a lane with `bottom` set
-// evaluates the bottom's path, the lane `apart` below it the columns' and the
-// term (valid there).
-__device__ __forceinline__ void band_term_pair(const SceneConsts &sc, int b, double sec_sun,
-                                               bool bottom, int apart, unsigned mask, double H,
-                                               double rho, double P, double lnP, double G, double X,
-                                               double pw, double r, BandTerm &t) {
-  double u, K;
-  bool ok = band_medium(sc, b, P, lnP, G, X, pw, u, K), deep;
-  double Du = (bottom ? 1.04 : 1.03) * sf::sqrt_mid(1.0 + (bottom ? 5.4 : 2.4) * u);
-  if (sc.sec_view != 1.0) Du = Du * sc.sec_view;
-  const double e = path_loss((sec_sun + Du) * K * H, deep, ok);
-  const double eB = __shfl_down_sync(mask, e, apart);
-  const int fB = __shfl_down_sync(mask, (ok ? 1 : 0) | (deep ? 2 : 0), apart);
-  if (bottom) return;
-  ok = band_close(u, K, e, eB, (fB & 2) != 0, rho, r, t) && ok && (fB & 1) != 0;
-  if (!ok) {
-    BandTerm g;
-    band_term_general(sc, b, sec_sun, H, rho, P, lnP, G, X, pw, r, &g);
-    t = g;
-  }
-}
-
 struct CostDetailsF64 {
   double rrs_error, model_error, bottom_albedo, K_min, iod;
   double Rm[kMaxBands];

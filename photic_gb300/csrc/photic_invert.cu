@@ -620,6 +620,29 @@ __global__ void __launch_bounds__(BS) invert_kernel(const __grid_constant__ Inve
   }
 }
 
+// A band's term (band_term) from two lanes of the group `mask`: a lane with
+// `bottom` set evaluates the bottom's path, the lane `apart` below it the
+// columns' and the term (valid there).
+__device__ __forceinline__ void band_term_pair(const SceneConsts &sc, int b, double sec_sun,
+                                               bool bottom, int apart, unsigned mask, double H,
+                                               double rho, double P, double lnP, double G, double X,
+                                               double pw, double r, BandTerm &t) {
+  double u, K;
+  bool ok = band_medium(sc, b, P, lnP, G, X, pw, u, K), deep;
+  double Du = (bottom ? 1.04 : 1.03) * sf::sqrt_mid(1.0 + (bottom ? 5.4 : 2.4) * u);
+  if (sc.sec_view != 1.0) Du = Du * sc.sec_view;
+  const double e = path_loss((sec_sun + Du) * K * H, deep, ok);
+  const double eB = __shfl_down_sync(mask, e, apart);
+  const int fB = __shfl_down_sync(mask, (ok ? 1 : 0) | (deep ? 2 : 0), apart);
+  if (bottom) return;
+  ok = band_close(u, K, e, eB, (fB & 2) != 0, rho, r, t) && ok && (fB & 1) != 0;
+  if (!ok) {
+    BandTerm g;
+    band_term_general(sc, b, sec_sun, H, rho, P, lnP, G, X, pw, r, &g);
+    t = g;
+  }
+}
+
 // The same queue of starts for few positions: a group of eight lanes a start,
 // band b on lane b (of up to four bands its bottom path on lane b + 4),
 // coordinate i of the simplex on lane i (NmGroup).  A launch of few positions
