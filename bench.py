@@ -1121,21 +1121,21 @@ def serving_leg(args, net):
 # 43 per band (photic_fp64.cuh cost_f64) + 9 in the tail.
 FLOPS_PER_EVAL_F64 = 4 * 43 + 9
 
-# FP64 thread instructions per cost evaluation of the seeded headline fit
-# (cost + Nelder-Mead bookkeeping): 160.6 G over 307.75 M evaluations in the
-# ncu capture of invert_kernel<PrecF64, 4, 256> on a 1024 x 1024 tile
-# (profiles/invert_kernel_warm_1024x1024_full.md); issued as 741 lane-slots
-# of FP64 warp instructions (70 % of lanes live).
-FP64_INST_PER_EVAL = 522
+# FP64 thread instructions per cost evaluation of a seeded fit (cost +
+# Nelder-Mead bookkeeping): 125.0 G over 413.9 M evaluations in the ncu
+# capture of invert_kernel<PrecF64, 4, 256> on a 1024 x 1024 tile
+# (profiles/fit_kernels_seeds1024_regions48_stacks16384.md); issued as 375
+# lane-slots of FP64 warp instructions (81 % of lanes live).
+FP64_INST_PER_EVAL = 302
 
 # dram__bytes_read.sum + dram__bytes_write.sum of the same capture
-# (76.75 MB + 5.47 MB over 1 048 576 seeded pixels), per pixel: the spectra
-# (16 B) and seed vector (48 B) read, depth, status and evaluation count
-# (16 B) written -- the algorithm's 80 B, no re-reads.
-TRAFFIC_BYTES_PER_PIXEL = (76.754688e6 + 5.472256e6) / 1048576
+# (115.0 MB + 64.0 MB over 1 048 576 seeded pixels), per pixel: the spectra
+# (16 B), seed vector (48 B) and queue order read, a record per start (64 B)
+# written, depth, status and evaluation count (16 B) written.
+TRAFFIC_BYTES_PER_PIXEL = (115.002112e6 + 63.977472e6) / 1048576
 TRAFFIC_NOTE = ("DRAM bytes per launch scaled by pixels from an ncu capture of this kernel on a "
-                "1048576-pixel seeded tile (78.2 B/pixel, against the 80 B/pixel the algorithm "
-                "moves: 16 B spectra + 48 B seed read, 16 B written)")
+                "1048576-pixel seeded tile (170.7 B/pixel: 16 B spectra + 48 B seed read, 16 B of "
+                "products and a 64 B record per start written, the records partly read back)")
 
 
 if __name__ == "__main__":
