@@ -554,40 +554,30 @@ __global__ void __launch_bounds__(256) nc_unpack_kernel(const __grid_constant__ 
 }
 
 // Four bands, two pixels a thread: one 4-byte load a band and one 32-byte
-// store, full sectors both.  Bound by HBM; with a pixel a thread the 2-byte
-// loads left too few bytes in flight (4096 x 4096 scene, 24 B a pixel: 91 us
-// before, 67 us now).  Needs packed grids on 4-byte and `out` on 32-byte
-// boundaries; anything else, and other band counts, take nc_unpack_kernel.
+// store, full sectors both.  Bound by HBM, and fastest with a thread for every
+// pair: 4096 x 4096 cells (24 B a pixel) 79 us with a pixel a thread on a grid
+// of eight blocks an SM, 73 with a pair a thread on that grid, 63 (6.4 TB/s)
+// with as many blocks as pairs ask for; four pairs in flight a thread 84.
+// Needs packed grids on 4-byte and `out` on 32-byte boundaries; anything else,
+// and other band counts, take nc_unpack_kernel.
 __device__ __forceinline__ float unpack_cell(const UnpackBand &u, uint32_t w) {
   const int16_t c = (int16_t)(uint16_t)w;
   return c == (int16_t)u.missing ? u.spval
                                  : __fadd_rn(__fmul_rn((float)c, u.scale_factor), u.add_offset);
 }
 __global__ void __launch_bounds__(256) nc_unpack4_kernel(const __grid_constant__ UnpackArgs a) {
-  const int64_t pairs = a.npix >> 1, stride = (int64_t)gridDim.x * blockDim.x;
-  constexpr int kAhead = 4;
-  int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  for (; i < pairs; i += kAhead * stride) {
-    uint32_t w[kAhead][4];
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < a.npix >> 1) {
+    float v[8];
 #pragma unroll
-    for (int k = 0; k < kAhead; k++)
-#pragma unroll
-      for (int b = 0; b < 4; b++)
-        if (i + k * stride < pairs)
-          w[k][b] = __byte_perm(
-              __ldcs(reinterpret_cast<const uint32_t *>(a.band[b].packed) + i + k * stride), 0,
-              0x2301);  // both shorts to host order
-#pragma unroll
-    for (int k = 0; k < kAhead; k++)
-      if (i + k * stride < pairs) {
-        float v[8];
-#pragma unroll
-        for (int b = 0; b < 4; b++) {
-          v[b] = unpack_cell(a.band[b], w[k][b] & 0xFFFFu);
-          v[4 + b] = unpack_cell(a.band[b], w[k][b] >> 16);
-        }
-        store8(a.out + 8 * (i + k * stride), v);
-      }
+    for (int b = 0; b < 4; b++) {
+      const uint32_t w = __byte_perm(
+          __ldcs(reinterpret_cast<const uint32_t *>(a.band[b].packed) + i), 0,
+          0x2301);  // both shorts to host order
+      v[b] = unpack_cell(a.band[b], w & 0xFFFFu);
+      v[4 + b] = unpack_cell(a.band[b], w >> 16);
+    }
+    store8(a.out + 8 * i, v);
   }
   if ((a.npix & 1) && blockIdx.x == 0 && threadIdx.x < 4) {  // the odd last pixel
     const UnpackBand &u = a.band[threadIdx.x];
@@ -946,8 +936,9 @@ cudaError_t launch_unpack(const UnpackArgs &a, cudaStream_t s) {
 cudaError_t unpack(const UnpackArgs &a, int nb, cudaStream_t s) {
   uintptr_t packed = 0;
   for (int b = 0; b < nb; b++) packed |= (uintptr_t)a.band[b].packed;
-  if (nb == 4 && ((uintptr_t)a.out & 31u) == 0 && (packed & 3u) == 0) {
-    nc_unpack4_kernel<<<streaming_grid((a.npix + 1) / 2), 256, 0, s>>>(a);
+  // (2^39 pixels are 2^30 blocks)
+  if (nb == 4 && ((uintptr_t)a.out & 31u) == 0 && (packed & 3u) == 0 && a.npix < (1ll << 39)) {
+    nc_unpack4_kernel<<<(unsigned)((a.npix + 511) / 512), 256, 0, s>>>(a);
     return cudaGetLastError();
   }
   switch (nb) {
