@@ -312,6 +312,7 @@ __device__ __forceinline__ bool hand_on(const InvertArgs &args, NmPixel<PrecF64,
     const int k = run < 32 - n ? run : 32 - n;
     if (k > 0) {
       __threadfence();
+      __syncwarp();  // another lane reads the record than saw its flag: votes order no memory
       bool won = false;
       if (lane == 0) won = atomicCAS(&q.taken, head, head + k) == head;
       won = __shfl_sync(kFull, won, 0);
