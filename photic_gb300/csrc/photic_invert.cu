@@ -33,6 +33,7 @@
 #include "photic_nm.cuh"
 #include "photic_nmgroup.cuh"
 #include "photic_prec64.cuh"
+#include "photic_starts.cuh"
 
 namespace photic {
 
@@ -710,12 +711,12 @@ __global__ void __launch_bounds__(kFewBlock) invert_few_kernel(const __grid_cons
                      left_record_offset(args.left_slots)) + w;
           start_k = left->start_k;
           item = left->item;
-          fresh = __ldcg(args.exit_k + item) >= start_k;
+          fresh = start_wanted(args.exit_k + item, start_k, gmask, G, gl);
         } else if (w < (unsigned long long)total_pos) {
           start_k = (int32_t)((int64_t)w / args.n_par);
           item = (int64_t)w % args.n_par;
           p = pixel_at(args, item);
-          fresh = start_k == 0 || (__ldcg(args.exit_k + item) >= start_k &&
+          fresh = start_k == 0 || (start_wanted(args.exit_k + item, start_k, gmask, G, gl) &&
                                    (args.seeds == nullptr || isnan(args.seeds[p * kN])));
           if (fresh) {
             load_spectrum<NB>(args, p, r);
@@ -842,7 +843,8 @@ __global__ void __launch_bounds__(kFewBlock) invert_few_kernel(const __grid_cons
       __syncwarp(gmask);  // every lane has read X, dd and kk
       const bool capped = ++guard > guard_cap;
       if (capped && gl == 0) atomicOr(args.error, PHOTIC_DEVERR_EVAL_CAP);
-      if (start_k > 0 && (guard & 63) == 0 && __ldcg(args.exit_k + item) < start_k) {
+      if (start_k > 0 && (guard & 63) == 0 &&
+          !start_wanted(args.exit_k + item, start_k, gmask, G, gl)) {
         has = false;  // an earlier start has ended the pixel
       } else if (capped || m.step_machine(y)) {
         const double ynewlo = m.F(m.lo);

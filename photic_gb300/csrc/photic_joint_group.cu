@@ -213,7 +213,7 @@ __global__ void __launch_bounds__(kBlock) joint_group_kernel(const __grid_consta
           if (rest) {
             item_k = 1 + (int)(tk / (unsigned long long)count);
             slot = a.rest[first + (int64_t)(tk % (unsigned long long)count)];
-            fresh = start_wanted(a.sw, slot, item_k);
+            fresh = start_wanted(a.sw.exit_k + slot, item_k, gmask, G, gl);
           } else {
             slot = first + (int64_t)tk;
             fresh = true;
@@ -409,7 +409,8 @@ __global__ void __launch_bounds__(kBlock) joint_group_kernel(const __grid_consta
       if (capped && item_k < 0) {
         if (gl == 0 && o.status) o.status[p] = PHOTIC_PX_INVALID;
         has = false;
-      } else if (item_k > 0 && (guard & 63) == 0 && !start_wanted(a.sw, slot, item_k)) {
+      } else if (item_k > 0 && (guard & 63) == 0 &&
+                 !start_wanted(a.sw.exit_k + slot, item_k, gmask, G, gl)) {
         has = false;  // an earlier start has ended the pixel
       } else if (capped || m.step_machine(y)) {
         const double ynewlo = m.F(m.lo);

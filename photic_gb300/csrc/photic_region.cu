@@ -473,7 +473,7 @@ __global__ void __launch_bounds__(BLOCK, C > 1 ? 12 : 1) region_kernel(const __g
         item_k = (int)((p - a.n_seq) / a.n_par);
         slot = (p - a.n_seq) % a.n_par;
         p = a.n_seq + slot;
-        if (item_k > 0 && !start_wanted(a.sw, slot, item_k)) continue;
+        if (item_k > 0 && !start_wanted(a.sw.exit_k + slot, item_k, kFull, 32, lane)) continue;
       }
       position = p;
       if (a.pixels) p = a.pixels[p];
@@ -920,7 +920,9 @@ __global__ void __launch_bounds__(BLOCK, C > 1 ? 12 : 1) region_kernel(const __g
         if (lane == 0 && o.status) o.status[p] = PHOTIC_PX_INVALID;
         break;
       }
-      if (item_k > 0 && (guard & 63) == 0 && !start_wanted(a.sw, slot, item_k)) break;
+      if (item_k > 0 && (guard & 63) == 0 &&
+          !start_wanted(a.sw.exit_k + slot, item_k, kFull, 32, lane))
+        break;
       if (capped || m.step_machine(y)) {
         // nelmin returned: keep the best start (model/samodel.c:2380-2405)
         const double ynewlo = m.F(m.lo);

@@ -37,9 +37,16 @@ __device__ __forceinline__ bool start_done(const StartWork &w, int64_t slot, int
   return mine;
 }
 
-// Whether start k of the pixel is still wanted.
-__device__ __forceinline__ bool start_wanted(const StartWork &w, int64_t slot, int k) {
-  return __ldcg(w.exit_k + slot) >= k;
+// Whether start k of the pixel whose word is *exit_k is still wanted: one
+// answer for the `width` lanes of `mask`, of which gl is the caller's rank.
+// Other warps lower the word meanwhile, so lanes that each loaded it could
+// disagree, and the exchanges and barriers that follow would then be met by a
+// part of the group: the first lane reads it and hands the rest its word.
+__device__ __forceinline__ bool start_wanted(const int32_t *exit_k, int k, unsigned mask, int width,
+                                             int gl) {
+  int32_t ex = 0;
+  if (gl == 0) ex = __ldcg(exit_k);
+  return __shfl_sync(mask, ex, 0, width) >= k;
 }
 
 struct StartChoice {
