@@ -2947,7 +2947,11 @@ extern "C" int photic_region_lut_invert_batch(
       a.pixels = order;
       a.npix = S;
       a.no_mask = 1;
-      rc = run_region(a, nmax, cfg->blocks_per_sm, s);
+      // (an invalid pixel leaves its chain's at zero)
+      if (d_chain_stats)
+        e = cudaMemsetAsync(d_chain_stats, 0, (size_t)C * 4 * sizeof(double), s);
+      rc = e == cudaSuccess ? run_region(a, nmax, cfg->blocks_per_sm, s)
+                            : cuda_fail(e, "cudaMemsetAsync");
       if (!d_order) cudaFreeAsync(order, s);
       if (rc) return rc;
       if (n_chains_used) *n_chains_used = C;

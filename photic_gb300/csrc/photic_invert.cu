@@ -249,6 +249,17 @@ __device__ __forceinline__ void write_single_chain(const InvertArgs &args, int64
   if (args.chain_stats) single_chain_stats(args.chain_stats + q * 4, 1.5, model_error);
 }
 
+// A pixel that ended invalid: no fit, and in the loop a chain that moved no
+// threshold.
+__device__ __forceinline__ void write_invalid(const InvertArgs &args, int64_t q, int64_t p) {
+  if (args.out.status) args.out.status[p] = PHOTIC_PX_INVALID;
+  if (args.pixels && args.chain_stats) {
+    double *const cs = args.chain_stats + q * 4;
+    cs[0] = cs[1] = 0.0;
+    cs[2] = cs[3] = 1.5;
+  }
+}
+
 template <int NB>
 __device__ __forceinline__ void load_spectrum(const InvertArgs &args, int64_t p, float (&r)[NB]) {
   if (NB == 4 && args.vec4) {
@@ -571,7 +582,7 @@ __global__ void __launch_bounds__(BS) invert_kernel(const __grid_constant__ Inve
         // reaching this means a defect; flag it instead of spinning.
         atomicOr(args.error, PHOTIC_DEVERR_EVAL_CAP);
         if (item >= 0) rec[item * fp.n_hstarts + start_k].evals = -1;
-        else if (o.status) o.status[pixel] = PHOTIC_PX_INVALID;
+        else write_invalid(args, position, pixel);
         has = false;
       } else if (m.step_machine(y)) {
         const T ynewlo = m.F(m.lo);
@@ -884,7 +895,7 @@ __global__ void __launch_bounds__(128) finish_kernel(const __grid_constant__ Inv
   int32_t total = 0, kept_evals = 0, kept_start = 0, kept_fault = 0;
   for (int k = 0; k < n_starts; k++) {
     if (rec[k].evals < 0) {
-      if (args.out.status) args.out.status[p] = PHOTIC_PX_INVALID;
+      write_invalid(args, q, p);
       return;
     }
     total += rec[k].evals;
