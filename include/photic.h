@@ -411,6 +411,13 @@ int photic_autotune(photic_config *cfg, int32_t kind, int64_t sample_npix, doubl
  * (bounded-wait timeouts, invalid inputs) since the previous call. */
 int photic_sync(void *stream);
 
+/* The batched calls take their scratch from a stream-ordered pool of the
+ * library's own, which keeps up to 512 MiB per device between calls.  Gives
+ * the current device's unused part back to the driver, for a caller that
+ * needs the memory otherwise; scratch of calls that have not completed stays
+ * (wait for them first to release it all).  Calls made later take new scratch. */
+int photic_release_workspace(void);
+
 /* Measured pipe throughput of the current device, for roofline
  * denominators of the compute-bound kernels: FP64 and FP32 FMA (TFLOP/s,
  * 2 flops per FMA) and MUFU ex2 (T ops/s).  Synchronous; ~0.1 s. */

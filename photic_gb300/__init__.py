@@ -8,4 +8,4 @@ from . import ncgrid  # noqa: F401
 from .api import (Config, JointGraph, PhoticError, alloc_outputs, cost,  # noqa: F401
                   depth_sigma, fallbacks_first, generate_field, generate_joint, generate_scene,
                   invert, joint_invert, lut_invert, region_depth_sigma, region_fit, region_invert,
-                  region_lut_invert, sync, version)
+                  region_lut_invert, release_workspace, sync, version)

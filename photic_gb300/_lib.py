@@ -137,6 +137,7 @@ _SIGS = {
                                       C.c_double]),
     "photic_band_constants": (C.c_int, [C.POINTER(photic_config), C.POINTER(C.c_double)]),
     "photic_sync": (C.c_int, [C.c_void_p]),
+    "photic_release_workspace": (C.c_int, []),
     "photic_forward_batch": (C.c_int, [C.POINTER(photic_config), C.c_void_p, C.c_void_p,
                                        C.c_void_p, C.c_int64, C.c_void_p, C.c_void_p,
                                        C.c_void_p]),

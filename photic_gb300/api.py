@@ -556,6 +556,13 @@ def sync(stream: Optional[torch.cuda.Stream] = None) -> None:
     L.check(L.lib().photic_sync(_stream_handle(stream)))
 
 
+def release_workspace() -> None:
+    """Give the scratch memory that the library keeps between calls (up to
+    512 MiB per device) back to the driver; the scratch of calls that have not
+    completed stays, so :func:`sync` first to release all of it."""
+    L.check(L.lib().photic_release_workspace())
+
+
 class JointGraph:
     """The temporal joint fit captured once as a CUDA graph for a fixed
     pixel count and observation count.  One replay runs the binning by

@@ -34,7 +34,8 @@ namespace photic {
 // library's own per device keeps up to kPoolKeepBytes between calls.  The
 // runtime's pools order reuse by stream and are safe between threads; memory
 // above the bound goes back at a synchronisation, all of it when an
-// allocation fails and when a surrogate is destroyed.  A capturing stream
+// allocation fails, when a surrogate is destroyed and when the caller asks
+// (photic_release_workspace).  A capturing stream
 // keeps to the default pool, whose allocations become the graph's.
 constexpr uint64_t kPoolKeepBytes = 512ull << 20;
 namespace {
@@ -80,11 +81,13 @@ cudaError_t ws_alloc(void **p, size_t bytes, cudaStream_t s) {
   return e;
 }
 
-void ws_trim() {
+cudaError_t ws_trim() {
   int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess) return;
+  const cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
   std::lock_guard<std::mutex> lk(g_pool_mu);
-  if ((int)g_pools.size() > dev && g_pools[dev]) cudaMemPoolTrimTo(g_pools[dev], 0);
+  return (int)g_pools.size() > dev && g_pools[dev] ? cudaMemPoolTrimTo(g_pools[dev], 0)
+                                                   : cudaSuccess;
 }
 
 }  // namespace photic
@@ -1141,7 +1144,7 @@ int photic_surrogate_create(photic_surrogate **out, uint64_t seed) {
 int photic_surrogate_destroy(photic_surrogate *s) {
   if (!s) return PHOTIC_OK;
   cudaFree(s->block);
-  ws_trim();  // its passes' workspace is the largest that the library keeps
+  (void)ws_trim();  // its passes' workspace is the largest that the library keeps
   delete s;
   return PHOTIC_OK;
 }
@@ -1324,6 +1327,11 @@ int photic_measure_peaks(double *fp64_tflops, double *fp32_tflops, double *mufu_
   cudaError_t e = measure_peaks(fp64_tflops, fp32_tflops, mufu_tops);
   if (e != cudaSuccess) return cuda_fail(e, "peak probes");
   return PHOTIC_OK;
+}
+
+int photic_release_workspace(void) {
+  const cudaError_t e = ws_trim();
+  return e == cudaSuccess ? PHOTIC_OK : cuda_fail(e, "cudaMemPoolTrimTo");
 }
 
 int photic_sync(void *stream) {

@@ -13,7 +13,7 @@ namespace photic {
 // Stream-ordered workspace from the library's pool (photic_host.cu), freed
 // with cudaFreeAsync; ws_trim gives the current device's unused part back.
 cudaError_t ws_alloc(void **p, size_t bytes, cudaStream_t s);
-void ws_trim();
+cudaError_t ws_trim();
 
 // Device error bits accumulated in the per-call error word.
 enum : unsigned {
