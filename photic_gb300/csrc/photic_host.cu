@@ -22,6 +22,7 @@
 #include "photic_kernels.h"
 #include "photic_params.h"
 #include "photic_tables.h"
+#include "photic_workspace.h"
 
 using namespace photic;
 
@@ -71,13 +72,13 @@ cudaError_t ws_alloc(void **p, size_t bytes, cudaStream_t s) {
   const cudaError_t c = cudaStreamIsCapturing(s, &cs);
   if (c != cudaSuccess) return c;
   cudaMemPool_t pool = cs == cudaStreamCaptureStatusNone ? device_pool() : nullptr;
-  if (!pool) return cudaMallocAsync(p, bytes, s);
-  cudaError_t e = cudaMallocFromPoolAsync(p, bytes, pool, s);
-  if (e == cudaErrorMemoryAllocation) {
-    (void)cudaGetLastError();
+  cudaError_t e = pool ? cudaMallocFromPoolAsync(p, bytes, pool, s) : cudaMallocAsync(p, bytes, s);
+  if (pool && e == cudaErrorMemoryAllocation) {
     cudaMemPoolTrimTo(pool, 0);
     e = cudaMallocFromPoolAsync(p, bytes, pool, s);
   }
+  // reported here, not by the launch of a call that then does with less
+  if (e != cudaSuccess) (void)cudaGetLastError();
   return e;
 }
 
@@ -363,6 +364,9 @@ void invert_shape(const InvertArgs &a, int precision, int sms, int64_t positions
 // Device memory for the starts' records: the last pixels of a larger scene
 // run start by start, the ones before them with their starts in sequence.
 constexpr int64_t kRecordBytesMax = 1ll << 30;
+// Where memory is short a call takes fewer (photic_workspace.h), but not fewer
+// than this, about what a stream-ordered pool takes from the driver at a time.
+constexpr int64_t kRecordBytesMin = 4ll << 20;
 
 // The records of `slots` pixels' starts in mem: none completed, no exit met.
 cudaError_t start_work_init(StartWork &w, unsigned char *mem, int64_t slots, int n_starts,
@@ -396,37 +400,51 @@ bool few_starts(const InvertArgs &a, int precision, int sms) {
 // 298 / 83.
 int run_invert(InvertArgs &a, int precision, int block, int per_sm, int sms, cudaStream_t s) {
   const int64_t per_pixel = (int64_t)a.fp.n_hstarts * kStartRecordBytes + sizeof(int32_t);
-  const bool few = block == 0 && per_sm == 0 && few_starts(a, precision, sms);
-  a.n_par = few || a.fp.n_hstarts > 1 ? kRecordBytesMax / per_pixel : 0;
-  if (a.n_par > a.npix) a.n_par = a.npix;
-  a.n_seq = a.npix - a.n_par;
+  const bool few_wanted = block == 0 && per_sm == 0 && few_starts(a, precision, sms);
+  int64_t n_par = few_wanted || a.fp.n_hstarts > 1 ? kRecordBytesMax / per_pixel : 0;
+  if (n_par > a.npix) n_par = a.npix;
+  // (groups of lanes need a record for every start; with one start a pixel
+  // they are all that records are for)
+  const int64_t least = a.fp.n_hstarts > 1 ? kRecordBytesMin / per_pixel : INT64_MAX;
+  bool few = false;
+  int threads = 0;
   int64_t grid = 0;
-  invert_shape(a, precision, sms, a.n_seq + a.n_par * a.fp.n_hstarts, block, per_sm, grid, a.claim);
-  if (per_sm < 1) return fail(PHOTIC_ERR_CUDA, "kernel does not fit on the device");
-  const size_t off_rec = 256, rec_bytes = (size_t)a.n_par * a.fp.n_hstarts * kStartRecordBytes;
-  const size_t off_exit = off_rec + rec_bytes;
-  const size_t off_left = (off_exit + (size_t)a.n_par * sizeof(int32_t) + 255) / 256 * 256;
-  const bool hand_on = precision == PHOTIC_PREC_FP64 && !few && a.n_par > 0;
-  const int64_t lanes = hand_on ? grid * block : 0;
-  a.give = 16;
-  a.left_slots = (int32_t)lanes;
-  a.few_left = sms * 80;
+  size_t off_left = 0;
   unsigned char *ws = nullptr;
-  cudaError_t e = ws_alloc((void **)&ws, off_left + (hand_on ? left_bytes(lanes) : 0), s);
-  if (e != cudaSuccess) return fail(PHOTIC_ERR_NOMEM, "workspace: %s", cudaGetErrorString(e));
-  a.queue = reinterpret_cast<unsigned long long *>(ws);
-  a.records = ws + off_rec;
-  a.exit_k = reinterpret_cast<int32_t *>(ws + off_exit);
+  cudaError_t e = cudaSuccess;
+  const WsTry t = take_less(n_par, least, [&](int64_t n) {
+    a.n_par = n;
+    a.n_seq = a.npix - n;
+    few = few_wanted && n == a.npix;
+    threads = block;
+    int blocks = per_sm;
+    invert_shape(a, precision, sms, a.n_seq + n * a.fp.n_hstarts, threads, blocks, grid, a.claim);
+    if (blocks < 1) return WsTry::kFailed;
+    const size_t off_rec = 256, rec_bytes = (size_t)n * a.fp.n_hstarts * kStartRecordBytes;
+    const size_t off_exit = off_rec + rec_bytes;
+    off_left = (off_exit + (size_t)n * sizeof(int32_t) + 255) / 256 * 256;
+    const bool hand_on = precision == PHOTIC_PREC_FP64 && !few && n > 0;
+    a.left_slots = (int32_t)(hand_on ? grid * threads : 0);
+    e = ws_alloc((void **)&ws, off_left + (hand_on ? left_bytes(a.left_slots) : 0), s);
+    if (e != cudaSuccess) return WsTry::kNoMemory;
+    a.queue = reinterpret_cast<unsigned long long *>(ws);
+    a.records = ws + off_rec;
+    a.exit_k = reinterpret_cast<int32_t *>(ws + off_exit);
+    a.left = hand_on ? reinterpret_cast<LeftStarts *>(ws + off_left) : nullptr;
+    return WsTry::kDone;
+  });
+  if (t == WsTry::kFailed) return fail(PHOTIC_ERR_CUDA, "kernel does not fit on the device");
+  if (t == WsTry::kNoMemory)
+    return fail(PHOTIC_ERR_NOMEM, "workspace: %s", cudaGetErrorString(e));
+  a.give = 16;
+  a.few_left = sms * 80;
   e = cudaMemsetAsync(ws, 0, sizeof(unsigned long long), s);
-  if (e == cudaSuccess && hand_on) {
-    a.left = reinterpret_cast<LeftStarts *>(ws + off_left);
-    e = cudaMemsetAsync(a.left, 0, left_record_offset(lanes), s);
-  }
+  if (e == cudaSuccess && a.left) e = cudaMemsetAsync(a.left, 0, left_record_offset(a.left_slots), s);
   // 0x7f7f7f7f: no start has met the early exit
   if (e == cudaSuccess && a.n_par > 0)
     e = cudaMemsetAsync(a.exit_k, 0x7f, (size_t)a.n_par * sizeof(int32_t), s);
   if (e == cudaSuccess)
-    e = few ? launch_invert_few(a, s) : launch_invert(a, precision, block, (int)grid, s);
+    e = few ? launch_invert_few(a, s) : launch_invert(a, precision, threads, (int)grid, s);
   cudaError_t e2 = cudaFreeAsync(ws, s);
   if (e != cudaSuccess) return cuda_fail(e, "invert kernel launch");
   if (e2 != cudaSuccess) return cuda_fail(e2, "cudaFreeAsync");
@@ -794,14 +812,21 @@ int photic_joint_invert_batch(const photic_config *cfg, const int32_t *d_offsets
   // kernels, up to four bands) while they fit
   const size_t head = 4 * 8 * sizeof(int32_t) + 16 * sizeof(unsigned long long);
   const int xs = cfg->layout == PHOTIC_LAYOUT_REFERENCE ? 3 + 3 * kMaxScenes : 1 + 4 * kMaxScenes;
-  size_t bytes = head + 2 * (size_t)npix * sizeof(int32_t);
+  const size_t bytes = head + 2 * (size_t)npix * sizeof(int32_t);
   const size_t off_sw = (bytes + 255) / 256 * 256;
   const size_t sw_bytes = start_work_bytes(npix, a.fp.n_hstarts, xs);
-  a.by_start = cfg->n_bands <= 4 && a.fp.n_hstarts > 1 && sw_bytes <= (size_t)kRecordBytesMax;
-  if (a.by_start) bytes = off_sw + sw_bytes;
+  // (all the records or none)
+  int64_t by_start =
+      cfg->n_bands <= 4 && a.fp.n_hstarts > 1 && sw_bytes <= (size_t)kRecordBytesMax ? 1 : 0;
   unsigned char *ws = nullptr;
-  cudaError_t e = ws_alloc((void **)&ws, bytes, s);
-  if (e != cudaSuccess) return fail(PHOTIC_ERR_NOMEM, "joint workspace: %s", cudaGetErrorString(e));
+  cudaError_t e = cudaSuccess;
+  const WsTry t = take_less(by_start, 1, [&](int64_t records) {
+    e = ws_alloc((void **)&ws, records ? off_sw + sw_bytes : bytes, s);
+    return e == cudaSuccess ? WsTry::kDone : WsTry::kNoMemory;
+  });
+  if (t != WsTry::kDone)
+    return fail(PHOTIC_ERR_NOMEM, "joint workspace: %s", cudaGetErrorString(e));
+  a.by_start = (int32_t)by_start;
   e = cudaMemsetAsync(ws, 0, head, s);
   if (e == cudaSuccess && a.by_start)
     e = start_work_init(a.sw, ws + off_sw, npix, a.fp.n_hstarts, xs, s);
@@ -1576,20 +1601,29 @@ int run_region(RegionArgs &a, int max_params, int per_sm, cudaStream_t s) {
   a.error = err;
   const int n_starts = a.fp.n_hstarts;
   const size_t per_pixel = start_work_bytes(1, n_starts, max_params);
-  a.n_par = a.eval_params || n_starts < 2 ? 0 : kRecordBytesMax / (int64_t)per_pixel;
-  if (a.n_par > a.npix) a.n_par = a.npix;
-  a.n_seq = a.npix - a.n_par;
+  int64_t n_par = a.eval_params || n_starts < 2 ? 0 : kRecordBytesMax / (int64_t)per_pixel;
+  if (n_par > a.npix) n_par = a.npix;
   const size_t off = 256;
-  unsigned char *ws = nullptr;
-  cudaError_t e = ws_alloc(
-      (void **)&ws, off + (a.n_par ? start_work_bytes(a.n_par, n_starts, max_params) : 0), s);
-  if (e != cudaSuccess) return fail(PHOTIC_ERR_NOMEM, "queue head");
-  a.queue = reinterpret_cast<unsigned long long *>(ws);
-  e = cudaMemsetAsync(ws, 0, off, s);
-  if (e == cudaSuccess && a.n_par > 0) e = start_work_init(a.sw, ws + off, a.n_par, n_starts, max_params, s);
-  if (e == cudaSuccess) e = launch_region(a, max_params, sms, per_sm, s);
-  cudaFreeAsync(ws, s);
-  if (e != cudaSuccess) return cuda_fail(e, "region launch");
+  cudaError_t e = cudaSuccess;
+  // launch_region takes workspace too, before it launches anything
+  const WsTry t = take_less(n_par, kRecordBytesMin / (int64_t)per_pixel, [&](int64_t n) {
+    a.n_par = n;
+    a.n_seq = a.npix - n;
+    unsigned char *ws = nullptr;
+    e = ws_alloc((void **)&ws, off + (n ? start_work_bytes(n, n_starts, max_params) : 0), s);
+    if (e != cudaSuccess) return WsTry::kNoMemory;
+    a.queue = reinterpret_cast<unsigned long long *>(ws);
+    e = cudaMemsetAsync(ws, 0, off, s);
+    if (e == cudaSuccess && n > 0) e = start_work_init(a.sw, ws + off, n, n_starts, max_params, s);
+    if (e == cudaSuccess) e = launch_region(a, max_params, sms, per_sm, s);
+    cudaFreeAsync(ws, s);
+    return e == cudaSuccess                 ? WsTry::kDone
+           : e == cudaErrorMemoryAllocation ? WsTry::kNoMemory
+                                            : WsTry::kFailed;
+  });
+  if (t == WsTry::kNoMemory)
+    return fail(PHOTIC_ERR_NOMEM, "region workspace: %s", cudaGetErrorString(e));
+  if (t == WsTry::kFailed) return cuda_fail(e, "region launch");
   return PHOTIC_OK;
 }
 

@@ -1067,8 +1067,13 @@ cudaError_t launch_shape(const RegionArgs &args, int sms, int per_sm, cudaStream
   if (grid > need) grid = need;
   void *simplex = nullptr;
   if (Sh::kGlobalV) {
-    e = ws_alloc(&simplex, (size_t)grid * (BLOCK / 32) * Sh::kV * sizeof(double), s);
-    if (e != cudaSuccess) return e;
+    // where memory is short: fewer records first (the caller's), then fewer
+    // warps at a time
+    while ((e = ws_alloc(&simplex, (size_t)grid * (BLOCK / 32) * Sh::kV * sizeof(double), s)) !=
+           cudaSuccess) {
+      if (a.n_par > 0 || grid == 1) return cudaErrorMemoryAllocation;
+      grid = (grid + 1) / 2;
+    }
     a.simplex = static_cast<double *>(simplex);
   }
   k<<<(int)grid, BLOCK, bytes, s>>>(a);
