@@ -37,6 +37,21 @@ import numpy as np
 
 TILE_BANDS = 4
 
+# Device bytes per pixel held by an admitted tile: spectra (16), their copy in
+# the batch (16), seeds (48) and residual (4), outputs (8), the network's
+# features and outputs (44) and the queue's order (8); ...
+STATE_BYTES_PER_PIXEL = 144
+# ... and the inversion's workspace while its batch runs: a record (64) for
+# every depth start and a word, up to a bound per call (photic_host.cu).
+RECORD_BYTES, RECORD_BYTES_MAX = 64, 1 << 30
+
+
+def tile_footprint(npix: int, n_starts: int) -> int:
+    """Device bytes of an admitted tile.  The tiles of a batch share one
+    call's records, so their footprints together cover the batch's."""
+    records = npix * (n_starts * RECORD_BYTES + 4)
+    return npix * STATE_BYTES_PER_PIXEL + min(records, RECORD_BYTES_MAX)
+
 
 @dataclass
 class TileRequest:
@@ -188,10 +203,8 @@ class GpuTileExecutor:
     """Device side of the serving loop (one CUDA device, one compute
     stream, one stream for tile creation)."""
 
-    # device bytes per pixel held by an admitted tile: spectra (16), their
-    # copy in the batch (16), seeds (48) and residual (4), outputs (8), the
-    # network's features and outputs (44) and the inversion's work queue
-    BYTES_PER_PIXEL = 144
+    # with the default eight starts, the records below their bound
+    BYTES_PER_PIXEL = tile_footprint(1, 8)
 
     def __init__(self, config=None, surrogate=None, mask_frac: float = 0.15,
                  device=None, n_streams: int = 2, polish_iters: int = 25,
@@ -211,7 +224,7 @@ class GpuTileExecutor:
         self.n_launched = 0
 
     def footprint(self, npix: int) -> int:
-        return npix * self.BYTES_PER_PIXEL
+        return tile_footprint(npix, len(self.cfg.hstarts))
 
     def admit(self, r: TileRequest) -> None:
         torch = self.torch
