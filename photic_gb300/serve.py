@@ -258,12 +258,12 @@ class GpuTileExecutor:
             st = out["status"]
             fitted = (st & 0xFF) == 0
             conv = fitted & ((st >> 8) & 1).bool()
+            # (sums of slices: an index built on the host would be copied from
+            # pageable memory, behind the inversion, and the host would wait
+            # for the batch here)
             offs = np.cumsum([0] + [r.npix for r in reqs])
-            seg = torch.tensor(np.repeat(np.arange(len(reqs)), [r.npix for r in reqs]),
-                               device=self.device)
-            counts = torch.zeros(2, len(reqs), dtype=torch.int64, device=self.device)
-            counts[0].index_add_(0, seg, conv.long())
-            counts[1].index_add_(0, seg, fitted.long())
+            counts = torch.stack([m[a:b].sum() for m in (conv, fitted)
+                                  for a, b in zip(offs[:-1], offs[1:])]).view(2, len(reqs))
             depth_h = torch.empty(int(offs[-1]), dtype=torch.float32, pin_memory=True)
             counts_h = torch.empty(2, len(reqs), dtype=torch.int64, pin_memory=True)
             depth_h.copy_(out["depth"], non_blocking=True)
