@@ -6,8 +6,8 @@
 //
 // One CTA (8 warps) owns a 128 x BN output tile (or, split-K, one slice of
 // K of it: the weight-gradient products have 128 x 128 outputs and K = the
-// batch, so their K is spread over CTAs and the partial sums are added in a
-// fixed order by a second kernel).  K is consumed in chunks of 64 through two
+// batch, so their K is spread over CTAs and photic_mlp.cu adds the partial
+// sums in a fixed order).  K is consumed in chunks of 64 through two
 // buffers: all threads stage the A and B chunks into shared memory in the
 // canonical no-swizzle core-matrix layout (16-byte vector loads; an operand
 // stored with K as its rows is transposed 8 x 8 in registers on the way), one
@@ -202,7 +202,7 @@ __global__ void __launch_bounds__(kThreads) tn_gemm_kernel(const __grid_constant
   bool ok = true;
   // split-K: CTA z takes chunks [c0, c1) of K and writes a partial sum
   const int nchunks = (g.K + kBK - 1) / kBK;
-  const int per = g.ksplit > 1 ? (nchunks + g.ksplit - 1) / g.ksplit : nchunks;
+  const int per = (nchunks + b.slices - 1) / b.slices;  // (no slice is empty)
   const int c0 = slice * per;
   const int c1 = min(nchunks, c0 + per);
   // Wait for the MMAs of chunk kc (the n-th use of its buffer).  A wait that
@@ -257,12 +257,7 @@ __global__ void __launch_bounds__(kThreads) tn_gemm_kernel(const __grid_constant
   tc::fence_after_sync();
 
   const int64_t row = m0 + (warp & 3) * 32 + lane;
-  if (ok && c1 <= c0) {
-    // an empty split contributes zeros
-    if (row < g.M && warp < 4)
-      for (int j = 0; j < ncols; j++)
-        g.partial[((size_t)slice * g.M + row) * g.N + n0 + j] = 0.0f;
-  } else if (ok) {
+  if (ok) {
     // warps 0-3 and 4-7 share the TMEM lanes and take every other 16 columns
     for (int cc = (warp >> 2) * 16; cc < mma_n; cc += 32) {
       float v[16];
@@ -287,19 +282,6 @@ __global__ void __launch_bounds__(kThreads) tn_gemm_kernel(const __grid_constant
   tc::fence_before_sync();
   __syncthreads();
   if (warp == 0) tc::tmem_free(tmem, kTmemCols);
-}
-
-// C = sum over splits of the partial products, in split order (the sum is
-// the same on every run).
-__global__ void splitk_reduce_kernel(const float *partial, int S, int M, int N, float *C,
-                                     int ldc) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= (int64_t)M * N) return;
-  const int r = (int)(i / N), c = (int)(i % N);
-  float s = 0.0f;
-#pragma unroll 16  // the loads of sixteen splits in flight; the additions in order
-  for (int z = 0; z < S; z++) s += partial[(size_t)z * M * N + i];
-  C[(size_t)r * ldc + c] = s;
 }
 
 }  // namespace
@@ -336,42 +318,26 @@ cudaError_t launch_batch(const GemmBatch &b, int n, int M, int N, cudaStream_t s
 
 cudaError_t launch_gemm(const GemmArgs &g, cudaStream_t s) {
   if (g.M <= 0 || g.N <= 0) return cudaSuccess;
-  const int nchunks = (g.K + kBK - 1) / kBK;
   GemmBatch b{};
-  GemmArgs &a = b.g[0];
-  a = g;
-  int S = 1;
-  if (g.ksplit > 1 && g.partial && g.epi == EPI_F32 && nchunks > 1) {
-    const int per = (nchunks + g.ksplit - 1) / g.ksplit;
-    S = (nchunks + per - 1) / per;
-    a.ksplit = S;
-  } else {
-    a.ksplit = 1;
-    a.partial = nullptr;
-  }
-  a.vec = epilogue_vec(a);
-  b.slices = S;
-  cudaError_t e = launch_batch(b, 1, g.M, g.N, s);
-  if (e == cudaSuccess && S > 1) {
-    const int64_t n = (int64_t)g.M * g.N;
-    splitk_reduce_kernel<<<(unsigned)((n + 127) / 128), 128, 0, s>>>(a.partial, S, g.M, g.N, g.C,
-                                                                     g.ldc);
-    e = cudaGetLastError();
-  }
-  return e;
+  b.g[0] = g;
+  b.g[0].partial = nullptr;
+  b.g[0].vec = epilogue_vec(b.g[0]);
+  b.slices = 1;
+  return launch_batch(b, 1, g.M, g.N, s);
 }
 
-// Split-K products of one M and K in one launch, the partial sums left in
-// their scratch: [slices][M][N] each.  Returns the slices.
-cudaError_t launch_gemm_partials(const GemmArgs *g, int n, int *slices, cudaStream_t s) {
+// Products of one M and K in one launch, each cut into up to `ksplit` slices
+// of K and the partial sums left in their scratch: [slices][M][N] each.
+// Returns the slices.
+cudaError_t launch_gemm_partials(const GemmArgs *g, int n, int ksplit, int *slices,
+                                 cudaStream_t s) {
   GemmBatch b{};
   const int nchunks = (g[0].K + kBK - 1) / kBK;
-  const int per = (nchunks + g[0].ksplit - 1) / g[0].ksplit;
+  const int per = (nchunks + ksplit - 1) / ksplit;
   b.slices = (nchunks + per - 1) / per;
   int N = 0;
   for (int i = 0; i < n; i++) {
     b.g[i] = g[i];
-    b.g[i].ksplit = b.slices;
     b.g[i].vec = epilogue_vec(b.g[i]);
     N = g[i].N > N ? g[i].N : N;
   }

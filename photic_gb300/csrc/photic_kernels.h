@@ -265,8 +265,7 @@ struct GemmArgs {
   int epi;
   int k_rows;      // A and B are stored [K][lda], [K][ldb] (lda, ldb multiples of 8)
   int vec;         // set by launch_gemm: the epilogue's rows allow 16-byte accesses
-  int ksplit;      // > 1: split K over this many CTAs (EPI_F32 only) ...
-  float *partial;  // ... with partial sums in [ksplit][M][N] scratch
+  float *partial;  // launch_gemm_partials: the sums over slices of K, [slices][M][N]
 };
 constexpr int kGemmBatch = 4;
 struct GemmBatch {
@@ -274,7 +273,7 @@ struct GemmBatch {
   int slices;  // K slices of each product
 };
 cudaError_t launch_gemm(const GemmArgs &g, cudaStream_t s);
-cudaError_t launch_gemm_partials(const GemmArgs *g, int n, int *slices, cudaStream_t s);
+cudaError_t launch_gemm_partials(const GemmArgs *g, int n, int ksplit, int *slices, cudaStream_t s);
 
 // Surrogate MLP (photic_mlp.cu): 6 (padded 16) -> 128 -> 128 -> 128 -> 5
 // (padded 16).  FP32 master parameters, flat, in this order.

@@ -460,7 +460,6 @@ static int gemm(const void *A, int lda, const void *B, int ldb, int M, int N, in
                 float *C, int ldc, void *O, int ldo, float *Z, int ldz, const float *bias,
                 unsigned int *err, cudaStream_t s) {
   GemmArgs g{};
-  g.ksplit = 1;
   g.A = A;
   g.B = B;
   g.lda = lda;
@@ -545,14 +544,13 @@ cudaError_t mlp_backward(const MlpState &st, const float *x, const float *t, int
     ga[l].sbo = 1024;
     ga[l].epi = EPI_F32;
     ga[l].k_rows = 1;
-    ga[l].ksplit = kMlpSplitK;
     ga[l].partial = w.part[l];
     f.part[l] = w.part[l];
     f.cols[l] = ca.parts[l] = w.cols[l];
     ca.m[l] = dz[l];
     ca.C[l] = l < 3 ? kMlpH : kMlpOut;
   }
-  if (launch_gemm_partials(ga, 4, &f.slices, s) != cudaSuccess) bad = 1;
+  if (launch_gemm_partials(ga, 4, kMlpSplitK, &f.slices, s) != cudaSuccess) bad = 1;
   colsum_parts_kernel<<<dim3(kColParts * (kMlpH / 2) / 128, 4), 128, 0, s>>>(ca);
   grads_finish_kernel<<<kWeightBlocks + kBiasBlocks, 128, 0, s>>>(f);
   if (bad) return cudaErrorLaunchFailure;
