@@ -37,8 +37,12 @@ namespace photic {
 // above the bound goes back at a synchronisation, all of it when an
 // allocation fails, when a surrogate is destroyed and when the caller asks
 // (photic_release_workspace).  A capturing stream
-// keeps to the default pool, whose allocations become the graph's.
+// keeps to the default pool, whose allocations become the graph's.  The device
+// makes those when the graph is launched, and the launch fails if it cannot:
+// what it has no memory for is refused while capturing, so that the call takes
+// less.
 constexpr uint64_t kPoolKeepBytes = 512ull << 20;
+constexpr size_t kGraphSpareBytes = 32ull << 20;  // the driver's granularity, twice over
 namespace {
 std::mutex g_pool_mu;
 std::vector<cudaMemPool_t> g_pools;
@@ -67,11 +71,31 @@ cudaMemPool_t device_pool() {
 }
 }  // namespace
 
+namespace {
+// Whether the device has `bytes` left, the pool's unused part included.
+bool device_has(size_t bytes) {
+  // (neither call enters the stream that another thread may be capturing)
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  if (cudaThreadExchangeStreamCaptureMode(&mode) != cudaSuccess) return true;
+  size_t left = 0, total = 0;
+  bool known = cudaMemGetInfo(&left, &total) == cudaSuccess;
+  if (known && left < bytes) {
+    (void)ws_trim();
+    known = cudaMemGetInfo(&left, &total) == cudaSuccess;
+  }
+  cudaThreadExchangeStreamCaptureMode(&mode);
+  return !known || left >= bytes;
+}
+}  // namespace
+
 cudaError_t ws_alloc(void **p, size_t bytes, cudaStream_t s) {
   cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
   const cudaError_t c = cudaStreamIsCapturing(s, &cs);
   if (c != cudaSuccess) return c;
-  cudaMemPool_t pool = cs == cudaStreamCaptureStatusNone ? device_pool() : nullptr;
+  const bool capturing = cs != cudaStreamCaptureStatusNone;
+  if (capturing && bytes > kGraphSpareBytes && !device_has(bytes + kGraphSpareBytes))
+    return cudaErrorMemoryAllocation;
+  cudaMemPool_t pool = capturing ? nullptr : device_pool();
   cudaError_t e = pool ? cudaMallocFromPoolAsync(p, bytes, pool, s) : cudaMallocAsync(p, bytes, s);
   if (pool && e == cudaErrorMemoryAllocation) {
     cudaMemPoolTrimTo(pool, 0);
