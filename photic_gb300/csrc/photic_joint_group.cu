@@ -426,11 +426,8 @@ __global__ void __launch_bounds__(kBlock) joint_group_kernel(const __grid_consta
             a.sw.evals[it] = capped ? -1 : m.icount;
             a.sw.fault[it] = m.ifault;
           }
-          __threadfence();
-          __syncwarp(gmask);
-          int mine = 0;
-          if (gl == 0) mine = start_done(a.sw, slot, item_k, fp.n_hstarts, ynewlo, early);
-          mine = __shfl_sync(gmask, mine, 0, G);
+          const bool mine =
+              start_done(a.sw, slot, item_k, fp.n_hstarts, ynewlo, early, gmask, G, gl);
           has = false;
           if (!rest && !mine && gl == 0)  // the pixel's other starts run in the next launch
             a.rest[first + atomicAdd(a.rest_count + bin, 1)] = (int32_t)slot;

@@ -938,13 +938,9 @@ __global__ void __launch_bounds__(BLOCK, C > 1 ? 12 : 1) region_kernel(const __g
             a.sw.evals[it] = capped ? -1 : m.icount;
             a.sw.fault[it] = m.ifault;
           }
-          __threadfence();
-          __syncwarp();
-          int mine = 0;
-          if (lane == 0)
-            mine = start_done(a.sw, slot, item_k, n_starts, capped ? kNaN : ynewlo, early);
-          mine = __shfl_sync(kFull, mine, 0);
-          if (!mine) break;
+          if (!start_done(a.sw, slot, item_k, n_starts, capped ? kNaN : ynewlo, early, kFull, 32,
+                          lane))
+            break;
           const StartChoice c = choose_start(a.sw, slot, n_starts, early);
           if (c.invalid) {
             if (lane == 0 && o.status) o.status[p] = PHOTIC_PX_INVALID;

@@ -19,10 +19,9 @@
 namespace photic {
 
 // Publish start k's completion (its record is written); true for the one
-// caller that is to compare the pixel's records.  Called by one lane, the
-// group's record writes fenced before.
-__device__ __forceinline__ bool start_done(const StartWork &w, int64_t slot, int k, int n_starts,
-                                           double y, double early) {
+// caller that is to compare the pixel's records.  One lane's part of the next.
+__device__ __forceinline__ bool start_done_lane(const StartWork &w, int64_t slot, int k,
+                                                int n_starts, double y, double early) {
   if (sf::lt(y, early) && sf::lt(y, 1.0e4)) atomicMin(w.exit_k + slot, k);
   __threadfence();
   const unsigned long long bit = 1ull << k;
@@ -35,6 +34,22 @@ __device__ __forceinline__ bool start_done(const StartWork &w, int64_t slot, int
   const bool mine = !(atomicOr(w.done + slot, 1ull << 63) >> 63);
   if (mine) __threadfence();
   return mine;
+}
+
+// The same for the `width` lanes of `mask`, of which gl is the caller's rank
+// and which have written the record between them: one answer.  The lanes that
+// then read the other starts' records are behind the first lane's look at who
+// has written them by the second barrier; exchanges order no memory.
+__device__ __forceinline__ bool start_done(const StartWork &w, int64_t slot, int k, int n_starts,
+                                           double y, double early, unsigned mask, int width,
+                                           int gl) {
+  __threadfence();
+  __syncwarp(mask);
+  int mine = 0;
+  if (gl == 0) mine = start_done_lane(w, slot, k, n_starts, y, early);
+  mine = __shfl_sync(mask, mine, 0, width);
+  __syncwarp(mask);
+  return mine != 0;
 }
 
 // Whether start k of the pixel whose word is *exit_k is still wanted: one

@@ -39,6 +39,7 @@ static inline int __shfl_sync(unsigned, int v, int from, int) {
   return r;
 }
 static inline void __threadfence() {}
+static inline void __syncwarp(unsigned) { pthread_barrier_wait(&g_meet); }
 static inline int atomicMin(int *p, int v) { return *p < v ? *p : (*p = v); }
 static inline unsigned long long atomicOr(unsigned long long *p, unsigned long long v) {
   const unsigned long long o = *p;
