@@ -493,8 +493,9 @@ def main():
     if rank == 0:
         # kernels of this library per step: the surrogate's feature kernel,
         # per 2^20-row chunk its standardisation + 4 GEMMs + de-normalisation,
-        # the seed polish and the inversion
-        launches = args.steps * (1 + 6 * ((tile + (1 << 20) - 1) >> 20) + 1 + 1)
+        # the seed polish and the inversion (starts by lanes, the last ones by
+        # groups of lanes, the comparison of each pixel's starts)
+        launches = args.steps * (1 + 6 * ((tile + (1 << 20) - 1) >> 20) + 1 + 3)
         line = {"metric": METRIC, "value": value, "unit": UNIT, "n_gpus": ws,
                 "steps": args.steps, "warmup": args.warmup, "ms_per_step": ms_step,
                 "higher_is_better": True, "scaling": "weak", "vs_baseline": None,
