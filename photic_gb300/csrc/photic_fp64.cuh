@@ -167,8 +167,8 @@ static __device__ PHOTIC_NOINLINE void band_term_general(const SceneConsts &sc, 
 // The same bits with the divisions, square roots, comparisons and most of the
 // exponentials on the integer and FP32 pipes (photic_softfp.cuh).  The
 // products stay on the FP64 pipe: thirty integer instructions each beside it
-// cost more in instruction fetch than they saved (1024 x 320 scene 346 -> 325
-// ms without them, 41 x 29 general fit 335 -> 299, 8 009 stacks 217 -> 201).
+// cost more in instruction fetch than they saved (1024 x 320 scene 346 -> 316
+// ms without them, 41 x 29 general fit 335 -> 294, 8 009 stacks 217 -> 201).
 // A product by the unit secant of a nadir view is skipped (exact).
 // The soft operations need normal operands of moderate exponent: the tests
 // below cover each, and a term that fails one (an exact zero, an absurd

@@ -284,7 +284,8 @@ __device__ __forceinline__ void load_spectrum(const InvertArgs &args, int64_t p,
 // does, and groups of lanes finish them (invert_few_kernel).  Nothing waits:
 // a warp takes the next records in order that are ready, or none.  1024 x 320
 // pixels 307 -> 299 ms, 20 011 of eight bands 112 -> 83, a 701 x 997 tile of
-// seeds 278 -> 264, the lookup-table loop over 509 x 400 91 -> 86.
+// seeds 278 -> 264; four lookup-table loops over 509 x 400, whose rarest
+// starts take 5 000 evaluations, 115 to 153 ms -> 111 to 146.
 // counted: the warp's starts in LeftStarts::live, -1 before its first call.
 // true: the warp ends.
 template <int BS, class Px>

@@ -55,7 +55,7 @@ constexpr int kStage = 72 + 3 * kMaxScenes + 64;
 // With more than a coordinate a lane the simplex (35 KB at n = 66) lies in
 // global memory, a slab for every resident warp, 59 MB in all and so in L2:
 // in shared memory it held an SM to five warps, with the FP64 pipe half idle;
-// eleven are resident now.  A lane reads and writes only its own columns.
+// twelve are resident now.  A lane reads and writes only its own columns.
 template <int C, int CG>
 struct Shape {
   static constexpr int kMaxN = C == 1 ? 32 : CG;
@@ -295,8 +295,8 @@ __device__ __noinline__ void serve_copy(const RegionArgs &a, int64_t p, int64_t 
 }
 
 // (The launch bound's minimum: without one the compiler held the kernel to 128
-// registers and spilled; with twelve one-warp blocks the large shapes get 168,
-// 41 x 29 general fit 241 -> 230 ms.)
+// registers and spilled; with twelve one-warp blocks the large shapes may take
+// 168 and take 157, 41 x 29 general fit 241 -> 230 ms.)
 template <int C, int CG, int BLOCK>
 __global__ void __launch_bounds__(BLOCK, C > 1 ? 12 : 1) region_kernel(const __grid_constant__ RegionArgs a) {
   using Sh = Shape<C, CG>;
