@@ -638,8 +638,8 @@ __global__ void __launch_bounds__(BS) invert_kernel(const __grid_constant__ Inve
 // `bottom` set evaluates the bottom's path, the lane `apart` below it the
 // columns' and the term (valid there).
 __device__ __forceinline__ void band_term_pair(const SceneConsts &sc, int b, double sec_sun,
-                                               bool bottom, int apart, unsigned mask, double H,
-                                               double rho, double P, double lnP, double G, double X,
+                                               bool bottom, int apart, unsigned mask, double mean,
+                                               double H, double rho, double P, double lnP, double G, double X,
                                                double pw, double r, BandTerm &t) {
   double u, K;
   bool ok = band_medium(sc, b, P, lnP, G, X, pw, u, K), deep;
@@ -650,11 +650,7 @@ __device__ __forceinline__ void band_term_pair(const SceneConsts &sc, int b, dou
   const int fB = __shfl_down_sync(mask, (ok ? 1 : 0) | (deep ? 2 : 0), apart);
   if (bottom) return;
   ok = band_close(u, K, e, eB, (fB & 2) != 0, rho, r, t) && ok && (fB & 1) != 0;
-  if (!ok) {
-    BandTerm g;
-    band_term_general(sc, b, sec_sun, H, rho, P, lnP, G, X, pw, r, &g);
-    t = g;
-  }
+  if (!ok) band_term_again(sc, b, sec_sun, false, mean, H, rho, P, lnP, G, X, pw, r, t);
 }
 
 // The same queue of starts for few positions: a group of eight lanes a start,
@@ -831,11 +827,11 @@ __global__ void __launch_bounds__(kFewBlock) invert_few_kernel(const __grid_cons
       const double P = 0.01 * fabs(X[3]), Gg = 0.01 * fabs(X[4]), Xx = 0.01 * fabs(X[5]);
       BandTerm t;
       if constexpr (kPair)
-        band_term_pair(sc, band, sc.sec_sun, gl >= kPaths, kPaths, gmask, H, qB * sc.refl[band], P,
-                       log(P), Gg, Xx, my_pw, my_rrs, t);
+        band_term_pair(sc, band, sc.sec_sun, gl >= kPaths, kPaths, gmask, mean, H,
+                       qB * sc.refl[band], P, log(P), Gg, Xx, my_pw, my_rrs, t);
       else
-        band_term(sc, gl, sc.sec_sun, false, H, qB * sc.refl[gl], P, log(P), Gg, Xx, my_pw, my_rrs,
-                  t);
+        band_term(sc, gl, sc.sec_sun, false, mean, H, qB * sc.refl[gl], P, log(P), Gg, Xx, my_pw,
+                  my_rrs, t);
       if (gl < nb) {
         dd[gl] = t.dd;
         kk[gl] = t.K;

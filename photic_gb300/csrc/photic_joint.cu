@@ -129,7 +129,7 @@ __device__ __forceinline__ double jcost(const JointArgs &a, const JPixel<K, NB> 
     for (int b = 0; b < NB; b++) {
       if (b < nb) {
         BandTerm t;
-        band_term(sc, b, px.sec_sun[s], kDetails, H, qB * sc.refl[b], P, lnP, G, X, px.pw[s][b],
+        band_term(sc, b, px.sec_sun[s], kDetails, px.mean, H, qB * sc.refl[b], P, lnP, G, X, px.pw[s][b],
                   px.rrs[s][b], t);
         err = err + t.dd;
         const double Kb = t.K;

@@ -313,7 +313,8 @@ __global__ void __launch_bounds__(kBlock) joint_group_kernel(const __grid_consta
       const double Xx = 0.01 * fabs(x[cP + 2]);
       const double lnP = log(P);
       BandTerm t;
-      band_term(sc, bb, my_sec, final_eval, H, qB * sc.refl[bb], P, lnP, Gg, Xx, my_pw, my_rrs, t);
+      band_term(sc, bb, my_sec, final_eval, mean, H, qB * sc.refl[bb], P, lnP, Gg, Xx, my_pw,
+                my_rrs, t);
       g.dd[gl] = t.dd;
       g.kk[gl] = t.K;
       if (final_eval) g.io[gl] = t.rrs_B / t.rrs;

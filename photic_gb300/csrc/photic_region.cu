@@ -674,7 +674,8 @@ __global__ void __launch_bounds__(BLOCK, C > 1 ? 12 : 1) region_kernel(const __g
 #pragma unroll 1
         for (int k = 1; k < nbt; k++) rho += wB[r * nbt + k] * sc.refl_k[k][b];
         BandTerm t;
-        band_term(sc, b, a.sec_sun[s], final_eval, H, rho, P, lnP, Gg, Xx, pw, my_rrs[h], t);
+        // (no mean: its test took registers that the large shapes lack, 193 -> 196 ms)
+        band_term(sc, b, a.sec_sun[s], final_eval, 1.0, H, rho, P, lnP, Gg, Xx, pw, my_rrs[h], t);
         dd[tau] = t.dd;
         kk[tau] = t.K;
         if (final_eval) {
